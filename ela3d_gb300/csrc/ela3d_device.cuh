@@ -37,7 +37,7 @@ constexpr unsigned long long kTestWaitLimitNs = 20000000ull;
 // loads, so every consumer wait expires and the kernel returns
 // DEV_ERR_TIMEOUT: the failure path of a lost transfer, exercised without a
 // fault (the waits are bounded, nothing spins forever).
-// CTL_PF_X lets the producer warp prefetch into L1 the C-PML memory
+// CTL_PF_X lets the producer warp prefetch into L2 the C-PML memory
 // variables of the x slab, CTL_PF_YZ those of the y and z slabs into L2
 // (performance hints; results do not depend on them).
 enum : int { CTL_WITHHOLD_LOADS = 1, CTL_PF_X = 2, CTL_PF_YZ = 4 };
@@ -178,6 +178,17 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, i
 __device__ __forceinline__ void cp_async_16(void *dst, const void *src, uint32_t src_bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(src_bytes)
                : "memory");
+}
+
+// Asynchronous copy of B = 4, 8 or 16 bytes global -> shared (both addresses
+// aligned to B); 16 bytes go through L2 only.
+template <int B>
+__device__ __forceinline__ void cp_async_vec(void *dst, const void *src) {
+  static_assert(B == 4 || B == 8 || B == 16, "cp.async size");
+  if constexpr (B == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(dst)), "l"(src), "n"(B) : "memory");
 }
 
 // Arrive on bar once every cp.async this thread issued before has landed

@@ -14,7 +14,8 @@
 //  - consumer warps compute plane k from stages k and k+1 (the z+1
 //    neighbours) and keep the z-1 neighbours in registers; each thread owns
 //    16 bytes of consecutive x cells of one row (float4 / double2);
-//  - C-PML memory variables are read and written only in the PML slabs;
+//  - C-PML memory variables are read and written only in the PML slabs, each
+//    thread copying its own cells' one plane ahead (PsiSlots);
 //  - cells outside the update ranges of the reference's loops keep their
 //    value (the Dirichlet edges); receivers are sampled after the velocity
 //    update and the force source is added after that (simpelmodel.cpp:592-622).
@@ -73,10 +74,16 @@ struct Geo {
   static constexpr int V_V = V_RHO + sz(W1);      // vx vy vz (C)
   static constexpr int V_STAGE = V_V + 3 * sz(C);
   static constexpr int V_TX = (int)sizeof(T) * (2 * W0 + 2 * Y1 + 4 * C + 2 * W1);
+  // memory-variable slots (PsiSlots): one 16-byte (or smaller) vector per
+  // consumer thread for each of the three variables of each axis
+  static constexpr int PSI_BYTES = 9 * NT * VEC * (int)sizeof(T);
   // mbarriers (full[NS], empty[NS]) live after the stages, so the TMA
-  // destinations start at the (aligned) base of dynamic shared memory
-  static constexpr int S_SMEM = NS * S_STAGE + 16 * NS;
-  static constexpr int V_SMEM = NS * V_STAGE + 16 * NS;
+  // destinations start at the (aligned) base of dynamic shared memory; the
+  // memory-variable slots follow them
+  static constexpr int S_PSI = al(NS * S_STAGE + 16 * NS);
+  static constexpr int V_PSI = al(NS * V_STAGE + 16 * NS);
+  static constexpr int S_SMEM = S_PSI + PSI_BYTES;
+  static constexpr int V_SMEM = V_PSI + PSI_BYTES;
 };
 
 template <typename T>
@@ -89,27 +96,35 @@ __device__ __forceinline__ int tiles_x_of(const ShotDesc<T> &s, int TX) {
 __device__ __forceinline__ float div_fast(float a, float b) { return __fdividef(a, b); }
 __device__ __forceinline__ double div_fast(double a, double b) { return a / b; }
 
+// Arithmetic with the rounding written out: these are never fused with a
+// neighbouring operation.
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ float sub_rn(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(a, b); }
+
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-// L1 prefetch of every 128-byte line of [p, p + bytes).
-__device__ __forceinline__ void prefetch_l1(const void *p, int bytes) {
+// L2 prefetch of every 128-byte line of [p, p + bytes).
+__device__ __forceinline__ void prefetch_l2(const void *p, int bytes) {
   const uintptr_t a = reinterpret_cast<uintptr_t>(p);
   for (uintptr_t q = a & ~uintptr_t(127); q < a + (uintptr_t)bytes; q += 128)
-    asm volatile("prefetch.global.L1 [%0];" ::"l"(q));
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(q));
 }
 
-// L1 prefetch of the x-slab C-PML memory variables var0 .. var0+2 that the
-// consumers of a tile will load: every row of the tile crosses the x slab
-// at the tile's edge columns, so without it every consumer warp waits on
-// DRAM once per plane.  Issued by the producer warp's lanes (one (variable,
-// row) pair per lane) when a plane's stage is requested, NS-2 planes ahead
-// of the consumers.  A hint: no result depends on it.  (Prefetching the y
-// and z slabs into L1 the same way measured slower: whole warps load those
-// rows and planes, and the extra lines crowd L1.)
-// The y- and z-slab rows are brought into L2 instead (CTL_PF_YZ), with bulk
-// prefetches that need no L1 space.
+// L2 prefetch of the C-PML memory variables var0 .. var0+2 that the
+// consumers of a tile will copy into their slots (PsiSlots, which reach one
+// plane ahead and read through L2): issued by the producer warp's lanes (one
+// (variable, row) pair per lane) when a plane's stage is requested, NS-2
+// planes ahead of the consumers.  A hint: no result depends on it.  The x
+// slab's row ends are short and unaligned (CTL_PF_X, line by line); the rows
+// of the y and z slabs are whole (CTL_PF_YZ, bulk prefetches).
 __device__ __forceinline__ void prefetch_l2_bulk(const void *p, int bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
@@ -151,8 +166,8 @@ struct PsiPrefetch {
   }
   __device__ __forceinline__ void plane(int k) const {
     if (k < 0 || k >= nz) return;
-    if (lbytes) prefetch_l1(left + k * pstride, lbytes);
-    if (rbytes) prefetch_l1(right + k * pstride, rbytes);
+    if (lbytes) prefetch_l2(left + k * pstride, lbytes);
+    if (rbytes) prefetch_l2(right + k * pstride, rbytes);
     if (yrow) prefetch_l2_bulk(yrow + k * ystride, wbytes);
     if (zrow && (k < zl || k >= zr)) prefetch_l2_bulk(zrow + (k < zl ? k : zl + (k - zr)) * zstride, wbytes);
   }
@@ -353,6 +368,50 @@ __device__ __forceinline__ bool flow_ready(uint64_t *ready, uint32_t parity, uns
   return true;
 }
 
+// C-PML memory variables of one thread's cells, one plane ahead.  A thread
+// reads the variables of its own V cells only, so it copies them with
+// cp.async into slots of shared memory that no other thread touches: no
+// barrier is needed, only its own wait.  The copies of plane k+1 are issued
+// once plane k's variables are used (their stores precede the copies in
+// program order, so a slot is never refilled before it was read), and land
+// while plane k's update, stores and the next stage wait run.  Loaded into
+// registers at the top of the plane instead, their latency was exposed in
+// every plane of every warp that crosses a layer (grids near the L2 size ran
+// at 0.7-0.8 of their rate without layers), and 36 of them stayed live across
+// the plane's update.  Built-in choices, 10 layer cells, Gcell-updates/s:
+// 101^3 33.2 -> 36.5, 128^3 36.0 -> 40.7, 192^3 41.1 -> 42.2, 256^3 47.5 ->
+// 48.7; the two kernels at 128^3 29.8 -> 33.5.
+template <typename T, int NT, int V>
+struct PsiSlots {
+  unsigned char *base;   // this thread's slot of variable 0
+  static constexpr int B = V * (int)sizeof(T);
+  __device__ __forceinline__ PsiSlots(unsigned char *psi, int tid) : base(psi + tid * B) {}
+  // variables 0..2 of `axis` from p, p + stride, p + 2 stride
+  __device__ __forceinline__ void fetch(int axis, const T *p, long long stride) const {
+#pragma unroll
+    for (int v = 0; v < 3; ++v) cp_async_vec<B>(base + (axis * 3 + v) * NT * B, p + v * stride);
+  }
+  // d <- d / K + psi with psi <- b psi + a d, written back to p.  RAW: d
+  // holds plain differences, to be multiplied by 1/h first.  AFIRST: which
+  // of the two products is rounded before the fused add.
+  template <bool RAW, bool AFIRST, typename A>
+  __device__ __forceinline__ void apply(int axis, int v, T *p, const A &a, const A &b, const A &ik, T h,
+                                        T (&d)[V]) const {
+    T q[V];
+    ld_vec(reinterpret_cast<const T *>(base + (axis * 3 + v) * NT * B), q);
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      const T ae = at(a, e), be = at(b, e), x = RAW ? mul_rn(d[e], h) : d[e];
+      q[e] = AFIRST ? fma_rn(ae, x, mul_rn(be, q[e])) : fma_rn(be, q[e], mul_rn(ae, x));
+      d[e] = fma_rn(x, at(ik, e), q[e]);
+    }
+    st_vec(p, q);
+  }
+  // profile value of cell e: one per cell (x) or one for the row or plane
+  static __device__ __forceinline__ T at(const T (&a)[V], int e) { return a[e]; }
+  static __device__ __forceinline__ T at(const T &a, int) { return a; }
+};
+
 // ----------------------------------------------------------- stress ----
 // The stress half-step over one work item (the block's consumer warps).
 // STAGE is the byte stride of the ring's stages.  FLOW (the dataflow
@@ -362,9 +421,9 @@ __device__ __forceinline__ bool flow_ready(uint64_t *ready, uint32_t parity, uns
 // and the z-1 plane, written during this launch, bypasses L1.
 template <typename T, int TX, int TY, int NS, int CPT, int MB, int STAGE, bool FLOW>
 __device__ __forceinline__ bool stress_item(const ShotDesc<T> &sd, const Item &item, const unsigned char *smem,
-                                            uint64_t *full, uint64_t *empty, unsigned &n, unsigned *__restrict__ err,
-                                            unsigned long long wait_ns, int tid, uint64_t *ready = nullptr,
-                                            uint32_t ready_parity = 0) {
+                                            unsigned char *psi, uint64_t *full, uint64_t *empty, unsigned &n,
+                                            unsigned *__restrict__ err, unsigned long long wait_ns, int tid,
+                                            uint64_t *ready = nullptr, uint32_t ready_parity = 0) {
   using G = Geo<T, TX, TY, NS, CPT, MB>;
   constexpr int V = G::VEC, H = G::H, WW = G::WW;
   const int lane = tid & 31;
@@ -440,8 +499,19 @@ __device__ __forceinline__ bool stress_item(const ShotDesc<T> &sd, const Item &i
   T *gy = psi_y + ((long long)item.k0 * yw + ys) * px + xg;
   const long long dgx = (long long)ny * xw, dgy = (long long)yw * px;
   long long g = (long long)item.k0 * plane + rowoff;
+  // the memory variables of plane k (x and y slab pointers at that plane)
+  const PsiSlots<T, G::NT, V> slots(psi, tid);
+  auto fetch_psi = [&](int k, const T *ax_, const T *ay_) {
+    if (in_x) slots.fetch(0, ax_ + PSI_S0 * psx, psx);
+    if (in_y) slots.fetch(1, ay_ + PSI_S0 * psy, psy);
+    if (live && (k < zl || k >= zr)) {
+      const int zs = k < zl ? k : zl + (k - zr);
+      slots.fetch(2, psi_z + PSI_S0 * psz + ((long long)zs * ny + y) * px + xg, psz);
+    }
+  };
+  fetch_psi(item.k0, gx, gy);
   for (int k = item.k0; k < item.k1; ++k, gx += dgx, gy += dgy, g += plane) {
-    // memory variables and z profile first: their latency overlaps the wait
+    // z profile first: its latency overlaps the wait
     const bool plane_z = k < zl || k >= zr;       // the plane lies in the z slab
     const bool in_z = live && plane_z;
     const int zs = k < zl ? k : zl + (k - zr);
@@ -450,34 +520,12 @@ __device__ __forceinline__ bool stress_item(const ShotDesc<T> &sd, const Item &i
       az = prof_z[PR_A * nz + k]; bz = prof_z[PR_B * nz + k]; ikz = prof_z[PR_IK * nz + k];
       azh = prof_z[PR_AH * nz + k]; bzh = prof_z[PR_BH * nz + k]; ikzh = prof_z[PR_IKH * nz + k];
     }
-    T px0[V], px1[V], px2[V], py0[V], py1[V], py2[V], pz0[V], pz1[V], pz2[V];
     T *gz = psi_z + ((long long)zs * ny + y) * px + xg;
-    if (in_x) {
-      ld_vec_rw(gx + PSI_S0 * psx, px0);
-      ld_vec_rw(gx + PSI_S1 * psx, px1);
-      ld_vec_rw(gx + PSI_S2 * psx, px2);
-    } else {
-#pragma unroll
-      for (int e = 0; e < V; ++e) px0[e] = px1[e] = px2[e] = T(0);
-    }
-    if (in_y) {
-      ld_vec_rw(gy + PSI_S0 * psy, py0);
-      ld_vec_rw(gy + PSI_S1 * psy, py1);
-      ld_vec_rw(gy + PSI_S2 * psy, py2);
-    } else {
-#pragma unroll
-      for (int e = 0; e < V; ++e) py0[e] = py1[e] = py2[e] = T(0);
-    }
-    if (in_z) {
-      ld_vec_rw(gz + PSI_S0 * psz, pz0);
-      ld_vec_rw(gz + PSI_S1 * psz, pz1);
-      ld_vec_rw(gz + PSI_S2 * psz, pz2);
-    } else {
-#pragma unroll
-      for (int e = 0; e < V; ++e) pz0[e] = pz1[e] = pz2[e] = T(0);
-    }
 
-    if (!wait_planes<NS>(full, n, k == item.k0, wait_ns, err, lane)) return false;
+    if (!wait_planes<NS>(full, n, k == item.k0, wait_ns, err, lane)) {
+      cp_async_wait_all();   // (no copy outlives its thread)
+      return false;
+    }
     const int s0 = (int)(n % NS), s1 = (int)((n + 1) % NS);
     const unsigned char *cur = smem + s0 * STAGE;
     const unsigned char *nxt = smem + s1 * STAGE;
@@ -530,115 +578,111 @@ __device__ __forceinline__ bool stress_item(const ShotDesc<T> &sd, const Item &i
 
     // this plane's update masks: bit e of byte c = component c of cell e
     const unsigned mk = k >= 1 ? mbits : (mbits & 0xffffff00u);
-    // The y- and z-direction C-PML terms are evaluated only for rows /
-    // planes inside the slabs (elsewhere a = 0 and 1/K = 1 and the terms
-    // are exact no-ops).  Memory variables are updated whether or not the
-    // cell's stress is: a cell outside the update ranges never uses them.
-    auto compute = [&](auto PY, auto PZ) {
-      constexpr bool pyo = decltype(PY)::value, pzo = decltype(PZ)::value;
+    // The nine velocity derivatives.  Those along y and z that only enter a
+    // sum stay plain differences D with a factor S (1/h, or 1 once the C-PML
+    // term has been applied), so the sum is one fma either way.  Every
+    // rounding is written out (fma_rn, mul_rn, add_rn), operand order
+    // included: results are the same bits whatever the compiler contracts,
+    // in every tile variant and schedule.
+    T exx[V], eyx[V], ezx[V], eyy[V], exy[V], ezy[V], ezz[V], exz[V], eyz[V];
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      const T vx_xp = (e < V - 1) ? vx_c[e + 1] : vx_e;
+      const T vy_xm = (e > 0) ? vy_c[e - 1] : vy_w;
+      const T vz_xm = (e > 0) ? vz_c[e - 1] : vz_w;
+      exx[e] = mul_rn(sub_rn(vx_xp, vx_c[e]), idx);
+      eyx[e] = mul_rn(sub_rn(vy_c[e], vy_xm), idx);
+      ezx[e] = mul_rn(sub_rn(vz_c[e], vz_xm), idx);
+      eyy[e] = mul_rn(sub_rn(vy_c[e], vy_ym[e]), idy);
+      exy[e] = sub_rn(vx_yp[e], vx_c[e]);   // D
+      ezy[e] = sub_rn(vz_yp[e], vz_c[e]);   // D
+      ezz[e] = mul_rn(sub_rn(vz_c[e], vz_zm[e]), idz);
+      exz[e] = sub_rn(vx_zp[e], vx_c[e]);   // D
+      eyz[e] = sub_rn(vy_zp[e], vy_c[e]);   // D
+      vz_zm[e] = vz_c[e];
+    }
+    // C-PML terms, only for the cells inside a slab (elsewhere a = 0 and
+    // 1/K = 1 and the terms are exact no-ops).  Memory variables are updated
+    // whether or not the cell's stress is: a cell outside the update ranges
+    // never uses them.
+    constexpr bool F32 = sizeof(T) == 4;
+    T sy = idy, sz = idz;
+    cp_async_wait_all();
+    if (in_x) {
+      slots.template apply<false, false>(0, 0, gx + PSI_S0 * psx, axh, bxh, ikxh, idx, exx);
+      slots.template apply<false, false>(0, 1, gx + PSI_S1 * psx, ax, bx, ikx, idx, eyx);
+      slots.template apply<false, false>(0, 2, gx + PSI_S2 * psx, ax, bx, ikx, idx, ezx);
+    }
+    if (in_y) {
+      slots.template apply<false, F32>(1, 0, gy + PSI_S0 * psy, ay, by, iky, idy, eyy);
+      slots.template apply<true, F32>(1, 1, gy + PSI_S1 * psy, ayh, byh, ikyh, idy, exy);
+      slots.template apply<true, F32>(1, 2, gy + PSI_S2 * psy, ayh, byh, ikyh, idy, ezy);
+      sy = T(1);
+    }
+    if (in_z) {
+      slots.template apply<false, F32>(2, 0, gz + PSI_S0 * psz, az, bz, ikz, idz, ezz);
+      slots.template apply<true, F32>(2, 1, gz + PSI_S1 * psz, azh, bzh, ikzh, idz, exz);
+      if (F32 && row_y) slots.template apply<true, true>(2, 2, gz + PSI_S2 * psz, azh, bzh, ikzh, idz, eyz);
+      else slots.template apply<true, false>(2, 2, gz + PSI_S2 * psz, azh, bzh, ikzh, idz, eyz);
+      sz = T(1);
+    }
+    if (!last) fetch_psi(k + 1, gx + dgx, gy + dgy);
+
+    // normal stresses, simpelmodel.cpp:378-413: c + (p * u + q * w), which
+    // product is rounded first by template (X, Y, Z: the modulus times the
+    // component's own derivative is the fused one)
+    auto normal = [&](auto X, auto Y, auto Z) {
+      constexpr bool fx = decltype(X)::value, fy = decltype(Y)::value, fz = decltype(Z)::value;
 #pragma unroll
       for (int e = 0; e < V; ++e) {
-        const int x = xg + e;
-        const T vx_xp = (e < V - 1) ? vx_c[e + 1] : vx_e;
-        const T vy_xm = (e > 0) ? vy_c[e - 1] : vy_w;
-        const T vz_xm = (e > 0) ? vz_c[e - 1] : vz_w;
-        const T cs_xm = (e > 0) ? cs_c[e - 1] : cs_w;
-        const T rho_xm = (e > 0) ? rho_c[e - 1] : rho_w;
-
-        // normal stresses, simpelmodel.cpp:378-413
-        {
-          const bool m = (mk >> (0 + e)) & 1u;
-          const T vp = cp_c[e], vs = cs_c[e], rhos = rho_c[e];
-          const T lambda = rhos * (vp * vp - T(2) * vs * vs);
-          const T l2m = rhos * vp * vp;
-          const T DT_l2m = dt * l2m, DT_l = dt * lambda;
-          T dvx_dx = (vx_xp - vx_c[e]) * idx;
-          T dvy_dy = (vy_c[e] - vy_ym[e]) * idy;
-          T dvz_dz = (vz_c[e] - vz_zm[e]) * idz;
-          const T qx = bxh[e] * px0[e] + axh[e] * dvx_dx;
-          dvx_dx = dvx_dx * ikxh[e] + qx;
-          px0[e] = qx;
-          if constexpr (pyo) {
-            const T qy = by * py0[e] + ay * dvy_dy;
-            dvy_dy = dvy_dy * iky + qy;
-            py0[e] = qy;
-          }
-          if constexpr (pzo) {
-            const T qz = bz * pz0[e] + az * dvz_dz;
-            dvz_dz = dvz_dz * ikz + qz;
-            pz0[e] = qz;
-          }
-          if (m) {
-            sxx[e] = DT_l2m * dvx_dx + DT_l * (dvy_dy + dvz_dz) + sxx[e];
-            syy[e] = DT_l * (dvx_dx + dvz_dz) + DT_l2m * dvy_dy + syy[e];
-            szz[e] = DT_l * (dvx_dx + dvy_dy) + DT_l2m * dvz_dz + szz[e];
-          }
+        const T vp = cp_c[e], vs = cs_c[e], rhos = rho_c[e];
+        const T lambda = mul_rn(rhos, fma_rn(vp, vp, -mul_rn(mul_rn(T(2), vs), vs)));
+        const T DT_l2m = mul_rn(dt, mul_rn(mul_rn(rhos, vp), vp)), DT_l = mul_rn(dt, lambda);
+        const T tx = add_rn(eyy[e], ezz[e]), ty = add_rn(exx[e], ezz[e]), tz = add_rn(exx[e], eyy[e]);
+        auto two = [&](auto own, T d, T t) {
+          return decltype(own)::value ? fma_rn(DT_l2m, d, mul_rn(DT_l, t)) : fma_rn(DT_l, t, mul_rn(DT_l2m, d));
+        };
+        if ((mk >> (0 + e)) & 1u) {
+          sxx[e] = add_rn(two(std::bool_constant<fx>{}, exx[e], tx), sxx[e]);
+          syy[e] = add_rn(two(std::bool_constant<fy>{}, eyy[e], ty), syy[e]);
+          szz[e] = add_rn(two(std::bool_constant<fz>{}, ezz[e], tz), szz[e]);
         }
-        // sigma_xy, :416-442
-        {
-          const bool m = (mk >> (8 + e)) & 1u;
-          const T vs = (cs_xm + cs_yp[e]) / T(2);
-          const T rhos = (rho_xm + rho_yp[e]) / T(2);
-          const T DT_mu = dt * (rhos * vs * vs);
-          T dvy_dx = (vy_c[e] - vy_xm) * idx;
-          T dvx_dy = (vx_yp[e] - vx_c[e]) * idy;
-          const T qx = bx[e] * px1[e] + ax[e] * dvy_dx;
-          dvy_dx = dvy_dx * ikx[e] + qx;
-          px1[e] = qx;
-          if constexpr (pyo) {
-            const T qy = byh * py1[e] + ayh * dvx_dy;
-            dvx_dy = dvx_dy * ikyh + qy;
-            py1[e] = qy;
-          }
-          if (m) sxy[e] = DT_mu * (dvy_dx + dvx_dy) + sxy[e];
-        }
-        // sigma_xz, :445-471 (z+1 of plane nz-1 is the zero plane)
-        {
-          const bool m = (mk >> (16 + e)) & 1u;
-          const T vs = (cs_xm + cs_zp[e]) / T(2);
-          const T rhos = (rho_xm + rho_zp[e]) / T(2);
-          const T DT_mu = dt * (rhos * vs * vs);
-          T dvz_dx = (vz_c[e] - vz_xm) * idx;
-          T dvx_dz = (vx_zp[e] - vx_c[e]) * idz;
-          const T qx = bx[e] * px2[e] + ax[e] * dvz_dx;
-          dvz_dx = dvz_dx * ikx[e] + qx;
-          px2[e] = qx;
-          if constexpr (pzo) {
-            const T qz = bzh * pz1[e] + azh * dvx_dz;
-            dvx_dz = dvx_dz * ikzh + qz;
-            pz1[e] = qz;
-          }
-          if (m) sxz[e] = DT_mu * (dvz_dx + dvx_dz) + sxz[e];
-        }
-        // sigma_yz, :473-498
-        {
-          const bool m = (mk >> (24 + e)) & 1u;
-          const T vs = (cs_yp[e] + cs_zp[e]) / T(2);
-          const T rhos = (rho_yp[e] + rho_zp[e]) / T(2);
-          const T DT_mu = dt * (rhos * vs * vs);
-          T dvz_dy = (vz_yp[e] - vz_c[e]) * idy;
-          T dvy_dz = (vy_zp[e] - vy_c[e]) * idz;
-          if constexpr (pyo) {
-            const T qy = byh * py2[e] + ayh * dvz_dy;
-            dvz_dy = dvz_dy * ikyh + qy;
-            py2[e] = qy;
-          }
-          if constexpr (pzo) {
-            const T qz = bzh * pz2[e] + azh * dvy_dz;
-            dvy_dz = dvy_dz * ikzh + qz;
-            pz2[e] = qz;
-          }
-          if (m) syz[e] = DT_mu * (dvz_dy + dvy_dz) + syz[e];
-        }
-        vz_zm[e] = vz_c[e];
       }
     };
-    if (row_y) {
-      if (plane_z) compute(std::true_type{}, std::true_type{});
-      else compute(std::true_type{}, std::false_type{});
-    } else {
-      if (plane_z) compute(std::false_type{}, std::true_type{});
-      else compute(std::false_type{}, std::false_type{});
+    constexpr std::true_type own{};
+    constexpr std::false_type other{};
+    if (!F32) normal(own, own, own);
+    else if (plane_z) normal(own, own, other);
+    else if (row_y) normal(own, other, own);
+    else normal(other, own, own);
+
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      const T cs_xm = (e > 0) ? cs_c[e - 1] : cs_w;
+      const T rho_xm = (e > 0) ? rho_c[e - 1] : rho_w;
+      auto dt_mu = [&](T c0, T c1, T r0, T r1) {   // dt mu of the averaged density and velocity
+        const T vs = mul_rn(add_rn(c0, c1), T(0.5)), rhos = mul_rn(add_rn(r0, r1), T(0.5));
+        return mul_rn(dt, mul_rn(mul_rn(rhos, vs), vs));
+      };
+      // sigma_xy, :416-442
+      {
+        const T mu = dt_mu(cs_xm, cs_yp[e], rho_xm, rho_yp[e]);
+        if ((mk >> (8 + e)) & 1u) sxy[e] = fma_rn(mu, fma_rn(exy[e], sy, eyx[e]), sxy[e]);
+      }
+      // sigma_xz, :445-471 (z+1 of plane nz-1 is the zero plane)
+      {
+        const T mu = dt_mu(cs_xm, cs_zp[e], rho_xm, rho_zp[e]);
+        if ((mk >> (16 + e)) & 1u) sxz[e] = fma_rn(mu, fma_rn(exz[e], sz, ezx[e]), sxz[e]);
+      }
+      // sigma_yz, :473-498
+      {
+        const T mu = dt_mu(cs_yp[e], cs_zp[e], rho_yp[e], rho_zp[e]);
+        // (a derivative whose C-PML term was applied has S = 1, and its
+        // product with S is exact)
+        const bool z_fused = F32 ? row_y : !plane_z;
+        const T t = z_fused ? fma_rn(eyz[e], sz, mul_rn(ezy[e], sy)) : fma_rn(ezy[e], sy, mul_rn(eyz[e], sz));
+        if ((mk >> (24 + e)) & 1u) syz[e] = fma_rn(mu, t, syz[e]);
+      }
     }
 
     if (live) {
@@ -648,21 +692,6 @@ __device__ __forceinline__ bool stress_item(const ShotDesc<T> &sd, const Item &i
       st_vec(f6 + g, sxy);
       st_vec(f7 + g, sxz);
       st_vec(f8 + g, syz);
-      if (in_x) {
-        st_vec(gx + PSI_S0 * psx, px0);
-        st_vec(gx + PSI_S1 * psx, px1);
-        st_vec(gx + PSI_S2 * psx, px2);
-      }
-      if (in_y) {
-        st_vec(gy + PSI_S0 * psy, py0);
-        st_vec(gy + PSI_S1 * psy, py1);
-        st_vec(gy + PSI_S2 * psy, py2);
-      }
-      if (in_z) {
-        st_vec(gz + PSI_S0 * psz, pz0);
-        st_vec(gz + PSI_S1 * psz, pz1);
-        st_vec(gz + PSI_S2 * psz, pz2);
-      }
     }
     n += last ? 2 : 1;
   }
@@ -674,9 +703,10 @@ __device__ __forceinline__ bool stress_item(const ShotDesc<T> &sd, const Item &i
 // stress_item for STAGE and FLOW), with the receivers and the force source.
 template <typename T, int TX, int TY, int NS, int CPT, int MB, int STAGE, bool FLOW>
 __device__ __forceinline__ bool velocity_item(const ShotDesc<T> &sd, const Item &item, int tick,
-                                              const unsigned char *smem, uint64_t *full, uint64_t *empty,
-                                              unsigned &n, unsigned *__restrict__ err, unsigned long long wait_ns,
-                                              int tid, uint64_t *ready = nullptr, uint32_t ready_parity = 0) {
+                                              const unsigned char *smem, unsigned char *psi, uint64_t *full,
+                                              uint64_t *empty, unsigned &n, unsigned *__restrict__ err,
+                                              unsigned long long wait_ns, int tid, uint64_t *ready = nullptr,
+                                              uint32_t ready_parity = 0) {
   using G = Geo<T, TX, TY, NS, CPT, MB>;
   constexpr int V = G::VEC, H = G::H, WW = G::WW;
   constexpr int CS = G::SC / (int)sizeof(T);
@@ -763,6 +793,17 @@ __device__ __forceinline__ bool velocity_item(const ShotDesc<T> &sd, const Item 
   T *gy = psi_y + ((long long)item.k0 * yw + ys) * px + xg;
   const long long dgx = (long long)ny * xw, dgy = (long long)yw * px;
   long long g = (long long)item.k0 * plane + rowoff;
+  // the memory variables of plane k (x and y slab pointers at that plane)
+  const PsiSlots<T, G::NT, V> slots(psi, tid);
+  auto fetch_psi = [&](int k, const T *ax_, const T *ay_) {
+    if (in_x) slots.fetch(0, ax_ + PSI_V0 * psx, psx);
+    if (in_y) slots.fetch(1, ay_ + PSI_V0 * psy, psy);
+    if (live && (k < zl || k >= zr)) {
+      const int zs = k < zl ? k : zl + (k - zr);
+      slots.fetch(2, psi_z + PSI_V0 * psz + ((long long)zs * ny + y) * px + xg, psz);
+    }
+  };
+  fetch_psi(item.k0, gx, gy);
   for (int k = item.k0; k < item.k1; ++k, gx += dgx, gy += dgy, g += plane) {
     const bool plane_z = k < zl || k >= zr;       // the plane lies in the z slab
     const bool in_z = live && plane_z;
@@ -772,32 +813,7 @@ __device__ __forceinline__ bool velocity_item(const ShotDesc<T> &sd, const Item 
       az = prof_z[PR_A * nz + k]; bz = prof_z[PR_B * nz + k]; ikz = prof_z[PR_IK * nz + k];
       azh = prof_z[PR_AH * nz + k]; bzh = prof_z[PR_BH * nz + k]; ikzh = prof_z[PR_IKH * nz + k];
     }
-    T px0[V], px1[V], px2[V], py0[V], py1[V], py2[V], pz0[V], pz1[V], pz2[V];
     T *gz = psi_z + ((long long)zs * ny + y) * px + xg;
-    if (in_x) {
-      ld_vec_rw(gx + PSI_V0 * psx, px0);
-      ld_vec_rw(gx + PSI_V1 * psx, px1);
-      ld_vec_rw(gx + PSI_V2 * psx, px2);
-    } else {
-#pragma unroll
-      for (int e = 0; e < V; ++e) px0[e] = px1[e] = px2[e] = T(0);
-    }
-    if (in_y) {
-      ld_vec_rw(gy + PSI_V0 * psy, py0);
-      ld_vec_rw(gy + PSI_V1 * psy, py1);
-      ld_vec_rw(gy + PSI_V2 * psy, py2);
-    } else {
-#pragma unroll
-      for (int e = 0; e < V; ++e) py0[e] = py1[e] = py2[e] = T(0);
-    }
-    if (in_z) {
-      ld_vec_rw(gz + PSI_V0 * psz, pz0);
-      ld_vec_rw(gz + PSI_V1 * psz, pz1);
-      ld_vec_rw(gz + PSI_V2 * psz, pz2);
-    } else {
-#pragma unroll
-      for (int e = 0; e < V; ++e) pz0[e] = pz1[e] = pz2[e] = T(0);
-    }
 
     int rlo = 0, rhi = 0;   // receivers of this plane
     if (item_rec) {
@@ -805,7 +821,10 @@ __device__ __forceinline__ bool velocity_item(const ShotDesc<T> &sd, const Item 
       rhi = rec_plane[k + 1];
     }
 
-    if (!wait_planes<NS>(full, n, k == item.k0, wait_ns, err, lane)) return false;
+    if (!wait_planes<NS>(full, n, k == item.k0, wait_ns, err, lane)) {
+      cp_async_wait_all();   // (no copy outlives its thread)
+      return false;
+    }
     const int s0 = (int)(n % NS), s1 = (int)((n + 1) % NS);
     const unsigned char *cur = smem + s0 * STAGE;
     const unsigned char *nxt = smem + s1 * STAGE;
@@ -850,96 +869,61 @@ __device__ __forceinline__ bool velocity_item(const ShotDesc<T> &sd, const Item 
 
     // this plane's update masks: bit e of byte c = component c of cell e
     const unsigned mk = (k >= 1 ? (mbits & 0x00ffffu) : 0u) | (k <= nz - 2 ? (mbits & 0xff0000u) : 0u);
-    // y/z C-PML terms only inside the slabs; memory variables updated
-    // whether or not the cell's velocity is (as in the stress half-step)
-    auto compute = [&](auto PY, auto PZ) {
-      constexpr bool pyo = decltype(PY)::value, pzo = decltype(PZ)::value;
+    // the nine stress derivatives (x1: of vx's update along x, and so on);
+    // y and z as plain differences with a factor, roundings written out (as
+    // in the stress half-step)
+    T x1[V], x2[V], x3[V], y1[V], y2[V], y3[V], z1[V], z2[V], z3[V];
 #pragma unroll
-      for (int e = 0; e < V; ++e) {
-        const int x = xg + e;
-        const T sxx_xm = (e > 0) ? sxx_c[e - 1] : sxx_w;
-        const T rho_xm = (e > 0) ? rho_c[e - 1] : rho_w;
-        const T sxy_xp = (e < V - 1) ? sxy_c[e + 1] : sxy_e;
-        const T sxz_xp = (e < V - 1) ? sxz_c[e + 1] : sxz_e;
-        // vx, simpelmodel.cpp:502-530
-        {
-          const bool m = (mk >> (0 + e)) & 1u;
-          const T rhos = (rho_c[e] + rho_xm) / T(2);
-          const T DT_over_rho = div_fast(dt, rhos);
-          T d1 = (sxx_c[e] - sxx_xm) * idx;
-          T d2 = (sxy_c[e] - sxy_ym[e]) * idy;
-          T d3 = (sxz_c[e] - sxz_zm[e]) * idz;
-          const T qx = bx[e] * px0[e] + ax[e] * d1;
-          d1 = d1 * ikx[e] + qx;
-          px0[e] = qx;
-          if constexpr (pyo) {
-            const T qy = by * py0[e] + ay * d2;
-            d2 = d2 * iky + qy;
-            py0[e] = qy;
-          }
-          if constexpr (pzo) {
-            const T qz = bz * pz0[e] + az * d3;
-            d3 = d3 * ikz + qz;
-            pz0[e] = qz;
-          }
-          if (m) vx[e] = DT_over_rho * (d1 + d2 + d3) + vx[e];
-        }
-        // vy, :532-559
-        {
-          const bool m = (mk >> (8 + e)) & 1u;
-          const T rhos = (rho_c[e] + rho_yp[e]) / T(2);
-          const T DT_over_rho = div_fast(dt, rhos);
-          T d1 = (sxy_xp - sxy_c[e]) * idx;
-          T d2 = (syy_yp[e] - syy_c[e]) * idy;
-          T d3 = (syz_c[e] - syz_zm[e]) * idz;
-          const T qx = bxh[e] * px1[e] + axh[e] * d1;
-          d1 = d1 * ikxh[e] + qx;
-          px1[e] = qx;
-          if constexpr (pyo) {
-            const T qy = byh * py1[e] + ayh * d2;
-            d2 = d2 * ikyh + qy;
-            py1[e] = qy;
-          }
-          if constexpr (pzo) {
-            const T qz = bz * pz1[e] + az * d3;
-            d3 = d3 * ikz + qz;
-            pz1[e] = qz;
-          }
-          if (m) vy[e] = DT_over_rho * (d1 + d2 + d3) + vy[e];
-        }
-        // vz, :563-590
-        {
-          const bool m = (mk >> (16 + e)) & 1u;
-          const T rhos = (rho_c[e] + rho_zp[e]) / T(2);
-          const T DT_over_rho = div_fast(dt, rhos);
-          T d1 = (sxz_xp - sxz_c[e]) * idx;
-          T d2 = (syz_c[e] - syz_ym[e]) * idy;
-          T d3 = (szz_zp[e] - szz_c[e]) * idz;
-          const T qx = bxh[e] * px2[e] + axh[e] * d1;
-          d1 = d1 * ikxh[e] + qx;
-          px2[e] = qx;
-          if constexpr (pyo) {
-            const T qy = by * py2[e] + ay * d2;
-            d2 = d2 * iky + qy;
-            py2[e] = qy;
-          }
-          if constexpr (pzo) {
-            const T qz = bzh * pz2[e] + azh * d3;
-            d3 = d3 * ikzh + qz;
-            pz2[e] = qz;
-          }
-          if (m) vz[e] = DT_over_rho * (d1 + d2 + d3) + vz[e];
-        }
-        sxz_zm[e] = sxz_c[e];
-        syz_zm[e] = syz_c[e];
-      }
+    for (int e = 0; e < V; ++e) {
+      const T sxx_xm = (e > 0) ? sxx_c[e - 1] : sxx_w;
+      const T sxy_xp = (e < V - 1) ? sxy_c[e + 1] : sxy_e;
+      const T sxz_xp = (e < V - 1) ? sxz_c[e + 1] : sxz_e;
+      x1[e] = mul_rn(sub_rn(sxx_c[e], sxx_xm), idx);
+      x2[e] = sub_rn(sxy_c[e], sxy_ym[e]);
+      x3[e] = sub_rn(sxz_c[e], sxz_zm[e]);
+      y1[e] = mul_rn(sub_rn(sxy_xp, sxy_c[e]), idx);
+      y2[e] = sub_rn(syy_yp[e], syy_c[e]);
+      y3[e] = sub_rn(syz_c[e], syz_zm[e]);
+      z1[e] = mul_rn(sub_rn(sxz_xp, sxz_c[e]), idx);
+      z2[e] = sub_rn(syz_c[e], syz_ym[e]);
+      z3[e] = sub_rn(szz_zp[e], szz_c[e]);
+      sxz_zm[e] = sxz_c[e];
+      syz_zm[e] = syz_c[e];
+    }
+    // C-PML terms only inside the slabs; memory variables updated whether or
+    // not the cell's velocity is (as in the stress half-step)
+    constexpr bool F32 = sizeof(T) == 4;
+    T sy = idy, sz = idz;
+    cp_async_wait_all();
+    if (in_x) {
+      slots.template apply<false, false>(0, 0, gx + PSI_V0 * psx, ax, bx, ikx, idx, x1);
+      slots.template apply<false, false>(0, 1, gx + PSI_V1 * psx, axh, bxh, ikxh, idx, y1);
+      slots.template apply<false, false>(0, 2, gx + PSI_V2 * psx, axh, bxh, ikxh, idx, z1);
+    }
+    if (in_y) {
+      slots.template apply<true, F32>(1, 0, gy + PSI_V0 * psy, ay, by, iky, idy, x2);
+      slots.template apply<true, F32>(1, 1, gy + PSI_V1 * psy, ayh, byh, ikyh, idy, y2);
+      slots.template apply<true, F32>(1, 2, gy + PSI_V2 * psy, ay, by, iky, idy, z2);
+      sy = T(1);
+    }
+    if (in_z) {
+      slots.template apply<true, F32>(2, 0, gz + PSI_V0 * psz, az, bz, ikz, idz, x3);
+      slots.template apply<true, F32>(2, 1, gz + PSI_V1 * psz, az, bz, ikz, idz, y3);
+      slots.template apply<true, F32>(2, 2, gz + PSI_V2 * psz, azh, bzh, ikzh, idz, z3);
+      sz = T(1);
+    }
+    if (!last) fetch_psi(k + 1, gx + dgx, gy + dgy);
+
+    auto update = [&](bool m, T r0, T r1, T d1, T d2, T d3, T &v) {
+      const T DT_over_rho = div_fast(dt, mul_rn(add_rn(r0, r1), T(0.5)));
+      if (m) v = fma_rn(DT_over_rho, fma_rn(d3, sz, fma_rn(d2, sy, d1)), v);
     };
-    if (row_y) {
-      if (plane_z) compute(std::true_type{}, std::true_type{});
-      else compute(std::true_type{}, std::false_type{});
-    } else {
-      if (plane_z) compute(std::false_type{}, std::true_type{});
-      else compute(std::false_type{}, std::false_type{});
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      const T rho_xm = (e > 0) ? rho_c[e - 1] : rho_w;
+      update((mk >> (0 + e)) & 1u, rho_c[e], rho_xm, x1[e], x2[e], x3[e], vx[e]);          // simpelmodel.cpp:502-530
+      update((mk >> (8 + e)) & 1u, rho_c[e], rho_yp[e], y1[e], y2[e], y3[e], vy[e]);       // :532-559
+      update((mk >> (16 + e)) & 1u, rho_c[e], rho_zp[e], z1[e], z2[e], z3[e], vz[e]);      // :563-590
     }
 
     if (live) {
@@ -1004,21 +988,6 @@ __device__ __forceinline__ bool velocity_item(const ShotDesc<T> &sd, const Item 
       st_vec(f0 + g, vx);
       st_vec(f1 + g, vy);
       st_vec(f2 + g, vz);
-      if (in_x) {
-        st_vec(gx + PSI_V0 * psx, px0);
-        st_vec(gx + PSI_V1 * psx, px1);
-        st_vec(gx + PSI_V2 * psx, px2);
-      }
-      if (in_y) {
-        st_vec(gy + PSI_V0 * psy, py0);
-        st_vec(gy + PSI_V1 * psy, py1);
-        st_vec(gy + PSI_V2 * psy, py2);
-      }
-      if (in_z) {
-        st_vec(gz + PSI_V0 * psz, pz0);
-        st_vec(gz + PSI_V1 * psz, pz1);
-        st_vec(gz + PSI_V2 * psz, pz2);
-      }
     }
     n += last ? 2 : 1;
   }
@@ -1071,8 +1040,8 @@ __global__ void __launch_bounds__(Geo<T, TX, TY, NS, CPT, MB>::THREADS, Geo<T, T
   unsigned n = 0;  // index of the load holding the current plane
   for (int ii = range.x; ii < range.y; ++ii) {
     const Item item = items[ii];
-    if (!stress_item<T, TX, TY, NS, CPT, MB, G::S_STAGE, false>(shots[item.shot], item, smem, full, empty, n, err,
-                                                                 wait_ns, tid))
+    if (!stress_item<T, TX, TY, NS, CPT, MB, G::S_STAGE, false>(shots[item.shot], item, smem, smem + G::S_PSI, full,
+                                                                 empty, n, err, wait_ns, tid))
       return;
   }
 }
@@ -1108,8 +1077,8 @@ __global__ void __launch_bounds__(Geo<T, TX, TY, NS, CPT, MB>::THREADS, Geo<T, T
   unsigned n = 0;
   for (int ii = range.x; ii < range.y; ++ii) {
     const Item item = items[ii];
-    if (!velocity_item<T, TX, TY, NS, CPT, MB, G::V_STAGE, false>(shots[item.shot], item, tick, smem, full, empty,
-                                                                   n, err, wait_ns, tid))
+    if (!velocity_item<T, TX, TY, NS, CPT, MB, G::V_STAGE, false>(shots[item.shot], item, tick, smem, smem + G::V_PSI,
+                                                                   full, empty, n, err, wait_ns, tid))
       return;
   }
 }
@@ -1156,7 +1125,8 @@ struct Flow {
   static constexpr int STAGE = G::S_STAGE > G::V_STAGE ? G::S_STAGE : G::V_STAGE;
   static constexpr int RB = 8;
   static_assert(RB >= NS / 2 + 2, "ready barriers for the items in flight");
-  static constexpr int SMEM = NS * STAGE + 16 * NS + 8 * RB + 4 * RB;
+  static constexpr int PSI = G::al(NS * STAGE + 16 * NS + 8 * RB + 4 * RB);   // memory-variable slots
+  static constexpr int SMEM = PSI + G::PSI_BYTES;
 };
 
 __device__ __forceinline__ int ld_relaxed_gpu(const int *p) {
@@ -1310,11 +1280,11 @@ __global__ void __launch_bounds__(Geo<T, TX, TY, NS, CPT, MB>::THREADS, Geo<T, T
     ++idx;
     bool ok;
     if (fi.kind == 0)
-      ok = stress_item<T, TX, TY, NS, CPT, MB, F::STAGE, true>(sd, fi.it, smem, full, empty, n, err, wait_ns, tid,
-                                                                rb, rp);
+      ok = stress_item<T, TX, TY, NS, CPT, MB, F::STAGE, true>(sd, fi.it, smem, smem + F::PSI, full, empty, n, err,
+                                                                wait_ns, tid, rb, rp);
     else
-      ok = velocity_item<T, TX, TY, NS, CPT, MB, F::STAGE, true>(sd, fi.it, tick + fi.step, smem, full, empty, n,
-                                                                  err, wait_ns, tid, rb, rp);
+      ok = velocity_item<T, TX, TY, NS, CPT, MB, F::STAGE, true>(sd, fi.it, tick + fi.step, smem, smem + F::PSI, full,
+                                                                  empty, n, err, wait_ns, tid, rb, rp);
     if (!ok) return;
     // this warp's share of the item is written: it arrives (CTA scope) on
     // the item's counter, and the last warp to arrive releases the whole

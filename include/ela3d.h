@@ -267,8 +267,8 @@ typedef struct ela3d_tuning {
                                3 and 4), or 0 */
     int32_t blocks_per_sm;  /* cap on resident blocks per SM, 0 = occupancy limit, -1 */
     int32_t prefetch;       /* prefetch of the C-PML memory variables by the
-                               loading warp: bit 1 (2) x slab into L1, bit 2 (4)
-                               y and z slabs into L2; -1 = built-in choice
+                               loading warp: bit 1 (2) x slab, bit 2 (4)
+                               y and z slabs, into L2; -1 = built-in choice
                                (6; 2 or 0 for shots whose arrays fit in or
                                near the L2) */
     int32_t lag;            /* schedules 3 and 4: places in the work list
