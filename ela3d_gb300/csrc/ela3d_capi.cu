@@ -136,9 +136,12 @@ static TuneChoice resolve_tuning(const std::vector<ela3d_params> &ps, const floa
   const ela3d_params &p = ps[0];
   // (the size-aware default applies to single shots; many shots give
   // round-robin chunks enough to go around)
-  TuneChoice c = ps.size() == 1 ? default_choice(p.precision == ELA3D_FP64, p.nx, p.ny, p.nz,
-                                                 p.src_kind == ELA3D_SRC_EXPLOSIVE)
-                                : default_choice(p.precision == ELA3D_FP64, 0, 0, 0);
+  const bool open = !t || (t->variant < 0 && t->schedule < 0 && t->chunk <= 0 && t->blocks_per_sm < 0 &&
+                           t->prefetch < 0 && t->lag < 0);
+  TuneChoice c = ps.size() != 1 ? default_choice(p.precision == ELA3D_FP64, 0, 0, 0)
+                 : open         ? plan_choice(p)
+                                : default_choice(p.precision == ELA3D_FP64, p.nx, p.ny, p.nz,
+                                                 p.src_kind == ELA3D_SRC_EXPLOSIVE);
   const bool explicit_variant = t && t->variant >= 0;
   if (!explicit_variant) {
     TuneChoice cached{};

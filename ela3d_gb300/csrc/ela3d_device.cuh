@@ -58,7 +58,7 @@ enum { PSI_S0 = 0, PSI_S1, PSI_S2, PSI_V0, PSI_V1, PSI_V2 };
 enum { PR_A = 0, PR_B, PR_IK, PR_AH, PR_BH, PR_IKH };
 
 template <typename T>
-struct ShotDesc {
+struct alignas(16) ShotDesc {
   int nx, ny, nz, px;
   int tick0;          // step it of this shot = tick - tick0 (1-based)
   int nstep;

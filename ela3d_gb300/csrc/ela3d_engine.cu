@@ -419,6 +419,51 @@ TuneChoice default_choice(int fp64, int nx, int ny, int nz, bool explosive) {
   return c;
 }
 
+TuneChoice plan_choice(const ela3d_params &p) {
+  TuneChoice c = default_choice(p.precision == ELA3D_FP64, p.nx, p.ny, p.nz, p.src_kind == ELA3D_SRC_EXPLOSIVE);
+  if (c.kind != kScheduleFlowOverlap) return c;
+  int n = 0;
+  const Variant *v = variants(&n);
+  // The tile: the share of its threads that hold cells, times a weight for
+  // its shape.  Narrow tiles read more halo, which costs little while the
+  // arrays are near the L2 (126 MB) and more once they stream from HBM.
+  // Gcell-updates/s (128x7, 112x8, 64x14, 56x16, 32x28): 101^3 32.4 34.2 30.8
+  // 31.2 30.7; 128^3 42.2 28.7 40.3 35.7 40.2; 160^3 33.3 35.8 38.8 41.2 42.0;
+  // 192^3 37.7 40.2 43.1 38.8 43.1; 224^3 44.1 46.2 42.5 43.6 43.9; 256^3 48.5
+  // 40.8 46.8 43.3 43.5; 320^3 46.3 47.6 47.6 44.0 42.3; 150x211x93 29.7 31.4
+  // 34.8 35.5 37.5.
+  const double bytes = 12.0 * p.nx * p.ny * p.nz * 4.0;
+  const bool streams = bytes > 400e6;
+  const struct { int tx, ty; double w; } shapes[] = {
+      {128, 7, 1.0}, {112, 8, 0.985}, {64, 14, 0.96}, {56, 16, streams ? 0.88 : 0.93}, {32, 28, streams ? 0.85 : 0.98}};
+  double best = 0.0;
+  for (const auto &s : shapes)
+    for (int j = 0; j < n; ++j) {
+      if (v[j].fp64 || v[j].loads != LOAD_TMA || !v[j].flow || v[j].tx != s.tx || v[j].ty != s.ty) continue;
+      const long long cx = (p.nx + s.tx - 1) / s.tx * s.tx, cy = (p.ny + s.ty - 1) / s.ty * s.ty;
+      const double score = s.w * ((double)p.nx / cx) * ((double)p.ny / cy);
+      if (score > best) {
+        best = score;
+        c.variant = j;
+      }
+    }
+  // The chunk: about two items per block and half-step, for the claimed
+  // places to even out (256^3: 48.8 with 64 planes, 45.1 with 86), but no more
+  // than 80 planes (512^3: 51.0 at 64, 50.5 at 128, 48.8 in whole columns;
+  // 448^3 48.7 at 75, 44.8 whole; 384^3 49.7 at 96, 48.6 at 192) and no fewer
+  // than 2.
+  int dev = 0, sms = 152;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int tx = v[c.variant].tx, ty = v[c.variant].ty;
+  const long long tiles = (long long)((p.nx + tx - 1) / tx) * ((p.ny + ty - 1) / ty);
+  const long long per_col = std::max({1ll, (4ll * sms + tiles) / (2 * tiles), (long long)(p.nz + 79) / 80});
+  c.chunk = std::max(2, (int)((p.nz + per_col - 1) / per_col));
+  // the memory variables' copies reach one plane ahead; the prefetches add
+  // to that only where the variables come from DRAM
+  c.prefetch = streams ? kPrefetchDefault : 0;
+  return c;
+}
+
 // ------------------------------------------------------------ TMA maps --
 static PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
@@ -998,7 +1043,9 @@ class Engine final : public EngineBase {
       }
       if (flow_on() && flow_steps_ > 0) {
         while (seg > 0) {
-          const int k = std::min(seg, flow_steps_ * flow_passes_);
+          // (places in a launch's list are 32-bit)
+          const int passes = (int)std::min<long long>(flow_passes_, std::max(1ll, (1ll << 30) / std::max(1, flow_items_)));
+          const int k = std::min(seg, flow_steps_ * passes);
           ela3d_status st = launch_flow(tick_ + 1, k);
           if (st != ELA3D_OK) return st;
           tick_ += k;
@@ -1181,12 +1228,14 @@ class Engine final : public EngineBase {
       CK(cudaMalloc(&d_flow_, items.size() * sizeof(FlowItem)));
       flow_cap_ = items.size();
     }
-    if ((size_t)nflags > flags_cap_) {
+    // the claim counter sits behind the flags, on a line of its own
+    const size_t flags = ((size_t)nflags + 31) / 32 * 32 + 32;
+    if (flags > flags_cap_) {
       if (d_flags_) CK(cudaFree(d_flags_));
       d_flags_ = nullptr;
       flags_cap_ = 0;
-      CK(cudaMalloc(&d_flags_, (size_t)nflags * sizeof(int)));
-      flags_cap_ = (size_t)nflags;
+      CK(cudaMalloc(&d_flags_, flags * sizeof(int)));
+      flags_cap_ = flags;
     }
     CK(cudaMemcpy(d_flow_, items.data(), items.size() * sizeof(FlowItem), cudaMemcpyHostToDevice));
     for (size_t a = 0; a < active.size(); ++a) {
@@ -1198,7 +1247,7 @@ class Engine final : public EngineBase {
     if (st != ELA3D_OK) return st;
     flow_items_ = (int)items.size();
     flow_steps_ = K;
-    flags_used_ = (size_t)nflags;
+    flags_used_ = flags;
     return ELA3D_OK;
   }
 
@@ -1207,7 +1256,19 @@ class Engine final : public EngineBase {
     int ctl = (inject_ > 0 ? CTL_WITHHOLD_LOADS : 0) | prefetch_;
     inject_ = std::max(0, inject_ - nsteps);
     const int *dtick = nullptr;
-    void *args[] = {&d_desc_, &d_maps_, &d_flow_, &flow_items_, &flow_steps_, &nsteps, &tick, &dtick, &d_err_, &ctl};
+    // Blocks claim their places in the list (the counter behind the flags)
+    // once there are about 1.6 items per block and half-step: a block slowed
+    // by layer items then takes fewer.  With fewer items the fixed deal, every
+    // G-th place, is the better one (no atomic on the way to an item, and the
+    // same block keeps a tile).  Gcell-updates/s, claimed / dealt: 64^3 (1.05
+    // items per block) 17.1 / 17.8, 72^3 (1.4) 20.0 / 21.1, 256^3 (1.5) 45.1 /
+    // 47.0; 160^3 (1.6) 42.5 / 42.7; 192^3 (1.9) 43.4 / 43.0, 256^3 (1.9) 48.8
+    // / 46.9, 320^3 (3.0) 47.7 / 44.2, 512^3 (13.6) 50.5 / 46.7.
+    int *claim = d_flags_ + flags_used_ - 32;
+    const long long places = (long long)per_sm_flow_ * num_sms_ * 2 * flow_steps_;
+    if (100ll * flow_items_ < 155ll * places) claim = nullptr;
+    void *args[] = {&d_desc_, &d_maps_, &d_flow_, &flow_items_, &flow_steps_, &nsteps, &tick, &dtick, &d_err_, &ctl,
+                    &claim};
     CK(cudaMemsetAsync(d_flags_, 0, flags_used_ * sizeof(int), stream_));
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (timing_) {

@@ -90,6 +90,10 @@ struct TuneChoice {
 };
 // Built-in choice when the autotuner's cache has none for the workload.
 TuneChoice default_choice(int fp64, int nx, int ny, int nz, bool explosive = false);
+// The choice of a plan whose caller leaves every tuning field open: where
+// default_choice takes the dataflow kernel, with the tile that wastes least
+// of the grid and the chunk that suits claimed places.
+TuneChoice plan_choice(const ela3d_params &p);
 
 // Autotuner (ela3d_tune.cu): process-wide cache of measured best choices
 // keyed by the workload shape.

@@ -208,7 +208,6 @@ __device__ __forceinline__ void copy_box_async(unsigned char *dst, const T *base
 template <int NS, bool ASYNC, typename Issue, typename Prefetch>
 __device__ __forceinline__ bool produce_item(const Item &it, unsigned &n, uint64_t *full, uint64_t *empty,
                                              Issue issue, Prefetch &prefetch, int lane) {
-  prefetch.begin(it);
   for (int k = it.k0; k <= it.k1; ++k, ++n) {
     const int slot = (int)(n % NS);
     int good = 1;
@@ -239,8 +238,11 @@ __device__ __forceinline__ void produce(const Item *__restrict__ items, int2 ran
   if (ctl & CTL_WITHHOLD_LOADS) return;  // test mode: no stage is ever filled
   unsigned n = 0;
   bool ok = true;
-  for (int ii = range.x; ii < range.y && ok; ++ii) ok = produce_item<NS, ASYNC>(items[ii], n, full, empty, issue,
-                                                                                 prefetch, lane);
+  for (int ii = range.x; ii < range.y && ok; ++ii) {
+    const Item it = items[ii];
+    prefetch.begin(it);
+    ok = produce_item<NS, ASYNC>(it, n, full, empty, issue, prefetch, lane);
+  }
   produce_drain<NS, ASYNC>(n, ok, full, err, lane);
 }
 
@@ -251,8 +253,8 @@ struct ItemPrefetch {
   PsiPrefetch<T, TX, TY> pf;
   const ShotDesc<T> *shots;
   int lane, ctl, var0;
-  __device__ __forceinline__ void begin(const Item &it) {
-    const ShotDesc<T> &sd = shots[it.shot];
+  __device__ __forceinline__ void begin(const Item &it) { begin(it, shots[it.shot]); }
+  __device__ __forceinline__ void begin(const Item &it, const ShotDesc<T> &sd) {
     const int txs = tiles_x_of(sd, TX);
     pf.begin(sd, (it.tile % txs) * TX, (it.tile / txs) * TY, var0, lane, ctl);
   }
@@ -416,14 +418,13 @@ struct PsiSlots {
 // The stress half-step over one work item (the block's consumer warps).
 // STAGE is the byte stride of the ring's stages.  FLOW (the dataflow
 // kernel): the item's inputs were written by other blocks of the same
-// launch; nothing global is read before the producer has acquired the
-// item's dependencies and arrived on `ready` (phase parity ready_parity),
-// and the z-1 plane, written during this launch, bypasses L1.
+// launch; the caller has waited for the item's ready barrier, on which the
+// producer arrives once it has acquired the item's dependencies, and the z-1
+// plane, written during this launch, bypasses L1.
 template <typename T, int TX, int TY, int NS, int CPT, int MB, int STAGE, bool FLOW>
 __device__ __forceinline__ bool stress_item(const ShotDesc<T> &sd, const Item &item, const unsigned char *smem,
                                             unsigned char *psi, uint64_t *full, uint64_t *empty, unsigned &n,
-                                            unsigned *__restrict__ err, unsigned long long wait_ns, int tid,
-                                            uint64_t *ready = nullptr, uint32_t ready_parity = 0) {
+                                            unsigned *__restrict__ err, unsigned long long wait_ns, int tid) {
   using G = Geo<T, TX, TY, NS, CPT, MB>;
   constexpr int V = G::VEC, H = G::H, WW = G::WW;
   const int lane = tid & 31;
@@ -443,9 +444,6 @@ __device__ __forceinline__ bool stress_item(const ShotDesc<T> &sd, const Item &i
   T *const psi_x = sd.psi_x, *const psi_y = sd.psi_y, *const psi_z = sd.psi_z;
   const long long psx = sd.psx, psy = sd.psy, psz = sd.psz;
   const int xw = sd.xw, yw = sd.yw;
-
-  // FLOW: the producer has acquired the item's dependencies
-  if (FLOW && !flow_ready(ready, ready_parity, wait_ns, err, lane)) return false;
 
   // z-1 neighbour of vz for the first plane of the run
   T vz_zm[V];
@@ -758,8 +756,7 @@ template <typename T, int TX, int TY, int NS, int CPT, int MB, int STAGE, bool F
 __device__ __forceinline__ bool velocity_item(const ShotDesc<T> &sd, const Item &item, int tick,
                                               const unsigned char *smem, unsigned char *psi, uint64_t *full,
                                               uint64_t *empty, unsigned &n, unsigned *__restrict__ err,
-                                              unsigned long long wait_ns, int tid, uint64_t *ready = nullptr,
-                                              uint32_t ready_parity = 0) {
+                                              unsigned long long wait_ns, int tid) {
   using G = Geo<T, TX, TY, NS, CPT, MB>;
   constexpr int V = G::VEC, H = G::H, WW = G::WW;
   constexpr int CS = G::SC / (int)sizeof(T);
@@ -787,8 +784,6 @@ __device__ __forceinline__ bool velocity_item(const ShotDesc<T> &sd, const Item 
   const bool item_rec = sample && rec_plane[item.k1] > rec_plane[item.k0];
   const bool src_row = sd.src_kind == 0 && y == sd.src_j && sd.src_i >= xg && sd.src_i < xg + V &&
                        it_step >= 1 && it_step <= sd.nstep;
-
-  if (FLOW && !flow_ready(ready, ready_parity, wait_ns, err, lane)) return false;
 
   T sxz_zm[V], syz_zm[V];
 #pragma unroll
@@ -1117,9 +1112,14 @@ __global__ void __launch_bounds__(Geo<T, TX, TY, NS, CPT, MB>::THREADS, Geo<T, T
 // z-chunk) at one of list_steps steps; a launch of nsteps steps walks the
 // list again for every further list_steps steps (the item of list step s
 // in pass p runs step p * list_steps + s; items of steps >= nsteps are
-// skipped, so one list serves shorter launches); block b takes items
-// b, b + G, ... of every pass
-// (G blocks, all resident: the launch is cooperative).  Chunk j of a shot
+// skipped, so one list serves shorter launches).  A block takes the next
+// place whenever its loading warp is done with an item (an atomic counter,
+// read one item ahead), or, without a counter, places b, b + G, ... (G
+// blocks, all resident: the launch is cooperative); either way a block's
+// places ascend and every earlier place is taken.  The loading warp passes
+// the item and a copy of its shot's descriptor to the consumers in shared
+// memory: read from global memory, both miss L1 at every item, since each
+// acquire of the counters empties it.  Chunk j of a shot
 // covers planes [jC, (j+1)C) for stress and the same range shifted down by
 // one plane for velocity, so that
 //   stress (j, tile, step r)   reads v written by velocity (j and j+1) of
@@ -1153,8 +1153,18 @@ struct Flow {
   static constexpr int STAGE = G::S_STAGE > G::V_STAGE ? G::S_STAGE : G::V_STAGE;
   static constexpr int RB = 8;
   static_assert(RB >= NS / 2 + 2, "ready barriers for the items in flight");
-  static constexpr int PSI = G::al(NS * STAGE + 16 * NS + 8 * RB + 4 * RB);   // memory-variable slots
+  // per item in flight: the item (kind < 0: the list is done) and a copy of
+  // its shot's descriptor
+  struct alignas(16) Slot {
+    FlowItem fi;
+    ShotDesc<T> sd;
+  };
+  static_assert(sizeof(ShotDesc<T>) % 16 == 0 && sizeof(FlowItem) % 16 == 0, "descriptors are copied 16 bytes at a time");
+  static constexpr int READY = NS * STAGE + 16 * NS;
+  static constexpr int SLOTS = (READY + 8 * RB + 4 * RB + 15) & ~15;
+  static constexpr int PSI = (SLOTS + RB * (int)sizeof(Slot) + 15) & ~15;   // memory-variable slots
   static constexpr int SMEM = PSI + G::PSI_BYTES;
+  static_assert(SMEM <= 232448, "shared memory of one block");
 };
 
 __device__ __forceinline__ int ld_relaxed_gpu(const int *p) {
@@ -1229,7 +1239,7 @@ template <typename T, int TX, int TY, int NS, int CPT, int MB>
 __global__ void __launch_bounds__(Geo<T, TX, TY, NS, CPT, MB>::THREADS, Geo<T, TX, TY, NS, CPT, MB>::MINB)
     flow_kernel(const ShotDesc<T> *__restrict__ shots, const ShotMaps *__restrict__ maps,
                 const FlowItem *__restrict__ items, int nitems, int list_steps, int nsteps, int tick,
-                const int *__restrict__ dtick, unsigned *__restrict__ err, int ctl) {
+                const int *__restrict__ dtick, unsigned *__restrict__ err, int ctl, int *__restrict__ claim) {
   using G = Geo<T, TX, TY, NS, CPT, MB>;
   using F = Flow<T, TX, TY, NS, CPT, MB>;
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -1237,6 +1247,7 @@ __global__ void __launch_bounds__(Geo<T, TX, TY, NS, CPT, MB>::THREADS, Geo<T, T
   uint64_t *empty = full + NS;
   uint64_t *ready = empty + NS;   // F::RB barriers, one per item in flight
   int *arrived = reinterpret_cast<int *>(ready + F::RB);   // F::RB consumer-warp counters
+  typename F::Slot *slots = reinterpret_cast<typename F::Slot *>(smem + F::SLOTS);
   const int tid = threadIdx.x;
   if (tid == 0)
     for (int r = 0; r < F::RB; ++r) {
@@ -1245,74 +1256,85 @@ __global__ void __launch_bounds__(Geo<T, TX, TY, NS, CPT, MB>::THREADS, Geo<T, T
     }
   init_ring<NS, G::NCW, LOAD_TMA>(full, empty);
   const unsigned long long wait_ns = (ctl & CTL_WITHHOLD_LOADS) ? kTestWaitLimitNs : kWaitLimitNs;
-  const int pass_steps = list_steps > 0 ? list_steps : nsteps;   // (one pass if the list's length is unset)
 
   if (tid >= G::NT) {  // producer warp
     const int lane = tid - G::NT;
     if (ctl & CTL_WITHHOLD_LOADS) return;  // test mode: no stage is ever filled
     ItemPrefetch<T, TX, TY> pf_s{{}, shots, lane, ctl, PSI_S0};
     ItemPrefetch<T, TX, TY> pf_v{{}, shots, lane, ctl, PSI_V0};
+    const int pass_steps = list_steps > 0 ? list_steps : nsteps;   // (one pass if the list's length is unset)
+    const int total = nitems * ((nsteps + pass_steps - 1) / pass_steps);
     unsigned n = 0, idx = 0;
     bool ok = true;
-    for (int rep = 0; rep < nsteps && ok; rep += pass_steps)
-    for (int q = blockIdx.x; q < nitems && ok; q += gridDim.x) {
-      FlowItem fi = items[q];
-      // the block's next work item into L1: its consumers read it at their
-      // next item's start, and so does this warp (101^3: +0.4%)
-      if (lane == 0) {
-        const int qn = q + (int)gridDim.x < nitems ? q + (int)gridDim.x : (int)blockIdx.x;
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(items + qn));
+    int next = 0;   // lane 0: the place claimed next
+    if (lane == 0) next = claim ? atomicAdd(claim, 1) : (int)blockIdx.x;
+    while (true) {
+      const int q = __shfl_sync(0xffffffffu, next, 0);
+      const bool end = q >= total;
+      FlowItem fi{{0, 0, 0, 0}, -1, 0, 0, 0};
+      if (!end) {
+        // (the next claim is in flight while this item's loads are issued)
+        if (lane == 0) next = claim ? atomicAdd(claim, 1) : q + (int)gridDim.x;
+        fi = items[q % nitems];
+        fi.step += q / nitems * pass_steps;
+        if (fi.step >= nsteps) continue;   // a list of more steps than this launch runs
       }
-      fi.step += rep;
-      if (fi.step >= nsteps) continue;   // a list of more steps than this launch runs
-      const ShotDesc<T> &sd = shots[fi.it.shot];
+      // the item and its shot's descriptor for the consumers (their slot's
+      // last item, RB items ago, is done: see RB)
+      typename F::Slot &slot = slots[idx % F::RB];
+      if (!end) {
+        const uint4 *src = reinterpret_cast<const uint4 *>(shots + fi.it.shot);
+        uint4 *dst = reinterpret_cast<uint4 *>(&slot.sd);
+        for (int c = lane; c < (int)(sizeof(ShotDesc<T>) / 16); c += 32) dst[c] = __ldg(src + c);
+      }
+      if (lane == 0) slot.fi = fi;
+      __syncwarp();
       int good = 1;
       if (lane == 0) {
-        const int txs = (sd.nx + TX - 1) / TX, tys = (sd.ny + TY - 1) / TY;
-        good = flow_wait_deps(sd, fi, txs, tys, G::NCW, wait_ns);
-        if (good) mbar_arrive(&ready[idx % F::RB]);   // release the consumers' global reads
+        if (!end) {
+          const int txs = (slot.sd.nx + TX - 1) / TX, tys = (slot.sd.ny + TY - 1) / TY;
+          good = flow_wait_deps(slot.sd, fi, txs, tys, G::NCW, wait_ns);
+        }
+        if (good) mbar_arrive(&ready[idx % F::RB]);   // release the consumers' reads
       }
       ++idx;
-      if (!__shfl_sync(0xffffffffu, good, 0)) {
-        ok = false;
-        break;
-      }
+      ok = __shfl_sync(0xffffffffu, good, 0);
+      if (!ok || end) break;
       if (fi.kind == 0) {
-        auto issue = [&](const Item &it, int k, int slot, uint64_t *bar, int l) {
-          stress_issue<T, TX, TY, NS, CPT, MB, LOAD_TMA>(shots, maps, it, k, smem + slot * F::STAGE, bar, l);
+        auto issue = [&](const Item &it, int k, int st, uint64_t *bar, int l) {
+          stress_issue<T, TX, TY, NS, CPT, MB, LOAD_TMA>(shots, maps, it, k, smem + st * F::STAGE, bar, l);
         };
+        pf_s.begin(fi.it, slot.sd);
         ok = produce_item<NS, false>(fi.it, n, full, empty, issue, pf_s, lane);
       } else {
-        auto issue = [&](const Item &it, int k, int slot, uint64_t *bar, int l) {
-          velocity_issue<T, TX, TY, NS, CPT, MB, LOAD_TMA>(shots, maps, it, k, smem + slot * F::STAGE, bar, l);
+        auto issue = [&](const Item &it, int k, int st, uint64_t *bar, int l) {
+          velocity_issue<T, TX, TY, NS, CPT, MB, LOAD_TMA>(shots, maps, it, k, smem + st * F::STAGE, bar, l);
         };
+        pf_v.begin(fi.it, slot.sd);
         ok = produce_item<NS, false>(fi.it, n, full, empty, issue, pf_v, lane);
       }
+      if (!ok) break;
     }
     produce_drain<NS, false>(n, ok, full, err, lane);
     return;
   }
 
-  const int lane = tid & 31, warp = tid >> 5;
+  const int lane = tid & 31;
   if (dtick) tick += *dtick;
-  unsigned n = 0, idx = 0;
-  for (int rep = 0; rep < nsteps; rep += pass_steps)
-  for (int q = blockIdx.x; q < nitems; q += gridDim.x) {
-    FlowItem fi = items[q];
-    fi.step += rep;
-    if (fi.step >= nsteps) continue;
-    const ShotDesc<T> &sd = shots[fi.it.shot];
-    uint64_t *rb = &ready[idx % F::RB];
-    int *arr = &arrived[idx % F::RB];
-    const uint32_t rp = (idx / F::RB) & 1;
-    ++idx;
+  unsigned n = 0;
+  for (unsigned idx = 0;; ++idx) {
+    if (!flow_ready(&ready[idx % F::RB], (idx / F::RB) & 1, wait_ns, err, lane)) return;
+    const typename F::Slot &slot = slots[idx % F::RB];
+    const FlowItem fi = slot.fi;
+    if (fi.kind < 0) return;   // the list is done
+    const ShotDesc<T> &sd = slot.sd;
     bool ok;
     if (fi.kind == 0)
       ok = stress_item<T, TX, TY, NS, CPT, MB, F::STAGE, true>(sd, fi.it, smem, smem + F::PSI, full, empty, n, err,
-                                                                wait_ns, tid, rb, rp);
+                                                                wait_ns, tid);
     else
       ok = velocity_item<T, TX, TY, NS, CPT, MB, F::STAGE, true>(sd, fi.it, tick + fi.step, smem, smem + F::PSI, full,
-                                                                  empty, n, err, wait_ns, tid, rb, rp);
+                                                                  empty, n, err, wait_ns, tid);
     if (!ok) return;
     // this warp's share of the item is written: it arrives (CTA scope) on
     // the item's counter, and the last warp to arrive releases the whole
@@ -1320,13 +1342,12 @@ __global__ void __launch_bounds__(Geo<T, TX, TY, NS, CPT, MB>::THREADS, Geo<T, T
     // acquired -- so one gpu-scope fence per item instead of one per warp
     fence_proxy_async_global();
     __syncwarp();
-    if (lane == 0 && atom_acq_rel_cta_add(arr, 1) == G::NCW - 1) {
-      *arr = 0;   // re-armed for item idx + RB (no warp is that far ahead)
+    if (lane == 0 && atom_acq_rel_cta_add(&arrived[idx % F::RB], 1) == G::NCW - 1) {
+      arrived[idx % F::RB] = 0;   // re-armed for item idx + RB (no warp is that far ahead)
       const int txs = (sd.nx + TX - 1) / TX, tys = (sd.ny + TY - 1) / TY;
       int *flag = sd.flow_flags + ((size_t)fi.kind * sd.flow_chunks + fi.chunk) * (txs * tys) + fi.it.tile;
       red_release_gpu_add(flag, G::NCW);
     }
-    (void)warp;
   }
 }
 

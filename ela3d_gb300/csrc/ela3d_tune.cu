@@ -163,13 +163,16 @@ ela3d_status autotune(const std::vector<ela3d_params> &ps, const std::vector<con
     // retire, which batches and servers do: it is tried for single shots
     std::vector<TuneChoice> cands = schedules((int)ps.size(), vs[v].flow != nullptr && ps.size() == 1);
     if (ps.size() == 1) {
-      // the built-in choice for this shot is always among the candidates
-      // (its chunk is sized to the shot)
-      const TuneChoice d = default_choice(fp64, ps[0].nx, ps[0].ny, ps[0].nz, ps[0].src_kind == ELA3D_SRC_EXPLOSIVE);
-      bool have = d.variant != v;
-      for (const TuneChoice &c : cands)
-        have = have || (c.kind == d.kind && c.chunk == d.chunk && c.prefetch == d.prefetch && c.lag == d.lag);
-      if (!have) cands.push_back({0, d.kind, d.chunk, 0, d.prefetch, d.lag});
+      // the built-in choices for this shot are always among the candidates
+      // (their chunks are sized to the shot)
+      for (const TuneChoice &d : {default_choice(fp64, ps[0].nx, ps[0].ny, ps[0].nz,
+                                                 ps[0].src_kind == ELA3D_SRC_EXPLOSIVE),
+                                  plan_choice(ps[0])}) {
+        bool have = d.variant != v;
+        for (const TuneChoice &c : cands)
+          have = have || (c.kind == d.kind && c.chunk == d.chunk && c.prefetch == d.prefetch && c.lag == d.lag);
+        if (!have) cands.push_back({0, d.kind, d.chunk, 0, d.prefetch, d.lag});
+      }
     }
     for (TuneChoice c : cands) {
       c.variant = v;

@@ -290,7 +290,9 @@ typedef struct ela3d_tuning {
  * together; the autotuner tries them for single shots, and schedule 4 is
  * the built-in choice for a single FP32 shot without an explosive source,
  * its z-chunks sized for about 1.5 work items per block (ela3d_builtin_tuning
- * reports the choice). */
+ * reports the choice).  A plan whose caller leaves every field open refines
+ * that choice where it is schedule 4: the tile that wastes least of the grid,
+ * z-chunks for about two items per block and of at most 80 planes. */
 
 /* Times every compiled variant with the candidate schedules on these shots
  * (`steps` time steps each, after a warm-up) and returns the fastest choice;
