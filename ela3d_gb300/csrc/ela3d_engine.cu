@@ -397,8 +397,8 @@ TuneChoice default_choice(int fp64, int nx, int ny, int nz, bool explosive) {
     // vs 22.5, 160^3 30.8 vs 25.9, 192^3 38.9 vs 34.1, 224^3 42.6 vs 40.8,
     // 256^3 45.6 vs 44.5, 288^3 42.0 vs 41.2, 384^3 46.1 vs 44.9, 448^3
     // 42.2 vs 41.8, 512^3 47.0 vs 45.4, 1024^3 47.6 vs 44.7; only 320^3 is
-    // the other way, 42.8 vs 43.4.  An explosive source injects between the
-    // half-steps, so it keeps the two kernels.
+    // the other way, 42.8 vs 43.4.  (An explosive source keeps the two
+    // kernels here; plan_choice gives it the dataflow kernel.)
     if (!fp64 && !explosive && v[i].flow) {
       // (chunks of equal size: at 256^3 three 86-plane chunks per column ran
       // at 46.5 against 45.6 for four of 64 and 45.6 for 96 + 96 + 64)
@@ -420,7 +420,8 @@ TuneChoice default_choice(int fp64, int nx, int ny, int nz, bool explosive) {
 }
 
 TuneChoice plan_choice(const ela3d_params &p) {
-  TuneChoice c = default_choice(p.precision == ELA3D_FP64, p.nx, p.ny, p.nz, p.src_kind == ELA3D_SRC_EXPLOSIVE);
+  // (explosive sources too: 201^3 242 us a step on the two kernels, 204 here)
+  TuneChoice c = default_choice(p.precision == ELA3D_FP64, p.nx, p.ny, p.nz);
   if (c.kind != kScheduleFlowOverlap) return c;
   int n = 0;
   const Variant *v = variants(&n);
@@ -977,11 +978,10 @@ class Engine final : public EngineBase {
   }
 
   // The dataflow kernel runs when the schedule asks for it and it can: a
-  // compiled dataflow kernel, resident blocks, and no explosive source (its
-  // injection into the stresses runs as a kernel between the steps).
+  // compiled dataflow kernel and resident blocks.
   bool flow_on() const {
     return (choice_.kind == kScheduleFlow || choice_.kind == kScheduleFlowOverlap) && var_ && var_->flow &&
-           per_sm_flow_ > 0 && !any_explosive_;
+           per_sm_flow_ > 0;
   }
 
   // Retire shots once they reach their nstep (batches with uneven lengths):
@@ -1282,6 +1282,11 @@ class Engine final : public EngineBase {
       pending_.push_back({e0, e1, nullptr, nsteps});
     }
     launches_ += 1;
+    // the last step's explosive sources (the kernel adds those of the others)
+    if (any_explosive_) {
+      CK(Fp<T>::explosive(d_desc_, (int)shots_.size(), tick + nsteps - 1, nullptr, stream_));
+      launches_ += 1;
+    }
     return ELA3D_OK;
   }
 

@@ -24,6 +24,8 @@
 // threads return.
 #pragma once
 
+#include <limits.h>
+
 #include <type_traits>
 
 #include "ela3d_device.cuh"
@@ -420,11 +422,14 @@ struct PsiSlots {
 // kernel): the item's inputs were written by other blocks of the same
 // launch; the caller has waited for the item's ready barrier, on which the
 // producer arrives once it has acquired the item's dependencies, and the z-1
-// plane, written during this launch, bypasses L1.
+// plane, written during this launch, bypasses L1.  inject_tick (FLOW): the
+// tick of the step before, whose explosive source is still to be added to
+// the source cell's stresses (INT_MIN: none).
 template <typename T, int TX, int TY, int NS, int CPT, int MB, int STAGE, bool FLOW>
 __device__ __forceinline__ bool stress_item(const ShotDesc<T> &sd, const Item &item, const unsigned char *smem,
                                             unsigned char *psi, uint64_t *full, uint64_t *empty, unsigned &n,
-                                            unsigned *__restrict__ err, unsigned long long wait_ns, int tid) {
+                                            unsigned *__restrict__ err, unsigned long long wait_ns, int tid,
+                                            int inject_tick = INT_MIN) {
   using G = Geo<T, TX, TY, NS, CPT, MB>;
   constexpr int V = G::VEC, H = G::H, WW = G::WW;
   const int lane = tid & 31;
@@ -444,6 +449,11 @@ __device__ __forceinline__ bool stress_item(const ShotDesc<T> &sd, const Item &i
   T *const psi_x = sd.psi_x, *const psi_y = sd.psi_y, *const psi_z = sd.psi_z;
   const long long psx = sd.psx, psy = sd.psy, psz = sd.psz;
   const int xw = sd.xw, yw = sd.yw;
+  // the thread whose cells hold an explosive source, in a step that follows
+  // one with an injection
+  const int inject = inject_tick == INT_MIN ? 0 : inject_tick - sd.tick0;
+  const bool src_row = FLOW && inject >= 1 && inject <= sd.nstep && sd.src_kind == 1 && y == sd.src_j &&
+                       sd.src_i >= xg && sd.src_i < xg + V;
 
   // z-1 neighbour of vz for the first plane of the run
   T vz_zm[V];
@@ -565,6 +575,24 @@ __device__ __forceinline__ bool stress_item(const ShotDesc<T> &sd, const Item &i
     ld_vec(bsig + 3 * CS + sc, sxy);
     ld_vec(bsig + 4 * CS + sc, sxz);
     ld_vec(bsig + 5 * CS + sc, syz);
+
+    // explosive source of the step before, simpelmodel.cpp:607-622, as
+    // explosive_kernel adds it: this item is the first to read the cell since
+    if (FLOW && src_row && k == sd.src_k) {
+      const T s = sd.stf[inject - 1];
+      const int ns = sd.nstep + 1;
+#pragma unroll
+      for (int e = 0; e < V; ++e)
+        if (xg + e == sd.src_i) {
+          const T l2m = mul_rn(mul_rn(rho_c[e], cp_c[e]), cp_c[e]);
+          sxx[e] = fma_rn(mul_rn(mul_rn(sd.expl_w[0], s), dt), l2m, sxx[e]);
+          syy[e] = fma_rn(mul_rn(mul_rn(sd.expl_w[1], s), dt), l2m, syy[e]);
+          szz[e] = fma_rn(mul_rn(mul_rn(sd.expl_w[2], s), dt), l2m, szz[e]);
+          sd.src_trace[inject] = sxx[e];
+          sd.src_trace[ns + inject] = syy[e];
+          sd.src_trace[2 * ns + inject] = szz[e];
+        }
+    }
 
     // stage s0 is no longer read by this warp (s1 still is, as the next plane)
     const bool last = (k == item.k1 - 1);
@@ -1119,7 +1147,10 @@ __global__ void __launch_bounds__(Geo<T, TX, TY, NS, CPT, MB>::THREADS, Geo<T, T
 // places ascend and every earlier place is taken.  The loading warp passes
 // the item and a copy of its shot's descriptor to the consumers in shared
 // memory: read from global memory, both miss L1 at every item, since each
-// acquire of the counters empties it.  Chunk j of a shot
+// acquire of the counters empties it.  An explosive source acts on the
+// stresses after a step: the next step's stress item adds it as it reads the
+// cell, and explosive_kernel adds the last step's after the launch.  Chunk j
+// of a shot
 // covers planes [jC, (j+1)C) for stress and the same range shifted down by
 // one plane for velocity, so that
 //   stress (j, tile, step r)   reads v written by velocity (j and j+1) of
@@ -1331,7 +1362,7 @@ __global__ void __launch_bounds__(Geo<T, TX, TY, NS, CPT, MB>::THREADS, Geo<T, T
     bool ok;
     if (fi.kind == 0)
       ok = stress_item<T, TX, TY, NS, CPT, MB, F::STAGE, true>(sd, fi.it, smem, smem + F::PSI, full, empty, n, err,
-                                                                wait_ns, tid);
+                                                                wait_ns, tid, fi.step > 0 ? tick + fi.step - 1 : INT_MIN);
     else
       ok = velocity_item<T, TX, TY, NS, CPT, MB, F::STAGE, true>(sd, fi.it, tick + fi.step, smem, smem + F::PSI, full,
                                                                   empty, n, err, wait_ns, tid);

@@ -283,16 +283,16 @@ typedef struct ela3d_tuning {
  * item `lag` places after the last item it waits for, so it runs soon
  * after them, while their results are still in L2; schedule 3 keeps the
  * time steps in sequence, schedule 4 lets a step start where the previous
- * one is done.  Results are bit-identical to schedules 0-2.  Shots with an
- * explosive source run the two-kernel path with schedule 1.  The work list
+ * one is done.  Results are bit-identical to schedules 0-2.  The work list
  * is built on the host for the shots running, again whenever shots join or
  * retire, so these schedules suit a plan or a batch of shots that run
  * together; the autotuner tries them for single shots, and schedule 4 is
  * the built-in choice for a single FP32 shot without an explosive source,
  * its z-chunks sized for about 1.5 work items per block (ela3d_builtin_tuning
  * reports the choice).  A plan whose caller leaves every field open refines
- * that choice where it is schedule 4: the tile that wastes least of the grid,
- * z-chunks for about two items per block and of at most 80 planes. */
+ * that choice where it is schedule 4, and takes schedule 4 for an explosive
+ * source too: the tile that wastes least of the grid, z-chunks for about two
+ * items per block and of at most 80 planes. */
 
 /* Times every compiled variant with the candidate schedules on these shots
  * (`steps` time steps each, after a warm-up) and returns the fastest choice;
