@@ -236,6 +236,7 @@ ela3d_status ela3d_model_generate(const ela3d_model_spec *model, int32_t nx, int
   ela3d_status st = status_from_cuda(cudaMalloc(&d, 3 * n * sizeof(float)), "cudaMalloc");
   if (st != ELA3D_OK) return st;
   st = status_from_cuda(launch_model_f32(spec, nx, ny, nz, nx, d, d + n, d + 2 * n, 0), "model kernel");
+  for (float *a : {cp, cs, rho}) populate_host(a, n * sizeof(float));   // (while the kernel runs)
   if (st == ELA3D_OK) st = status_from_cuda(cudaDeviceSynchronize(), "model kernel");
   if (st == ELA3D_OK) st = status_from_cuda(cudaMemcpy(cp, d, n * sizeof(float), cudaMemcpyDeviceToHost), "copy");
   if (st == ELA3D_OK) st = status_from_cuda(cudaMemcpy(cs, d + n, n * sizeof(float), cudaMemcpyDeviceToHost), "copy");

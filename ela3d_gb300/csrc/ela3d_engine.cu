@@ -3,6 +3,8 @@
 #include "ela3d_engine.h"
 
 #include <cudaTypedefs.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <cmath>
@@ -11,6 +13,7 @@
 #include <cstring>
 #include <mutex>
 #include <numeric>
+#include <thread>
 
 namespace ela3d {
 
@@ -37,6 +40,40 @@ ela3d_status status_from_cuda(cudaError_t e, const char *what) {
     set_last_error(msg);          \
     return ELA3D_ERR_INVALID_ARG; \
   } while (0)
+
+// Backs a result buffer with memory before the GPU writes to it.  A device
+// to host copy into pages that no one has touched takes a GPU page fault for
+// each (a fresh 67 MB array: 57 ms, 0.6 ms once its pages exist); the kernel
+// populates them far faster, a few threads in parallel faster still.  Pages
+// that exist are left as they are, contents included; where the call is not
+// supported the copy simply faults as before.
+void populate_host(void *buf, size_t bytes) {
+#ifdef MADV_POPULATE_WRITE
+  constexpr size_t kPart = 4u << 20;   // a thread for every so many bytes
+  if (bytes < (64u << 10)) return;
+  const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+  const uintptr_t lo = (uintptr_t)buf / page * page, hi = ((uintptr_t)buf + bytes + page - 1) / page * page;
+  const int parts =
+      (int)std::max<size_t>(1, std::min<size_t>({8, bytes / kPart, std::max(1u, std::thread::hardware_concurrency())}));
+  const uintptr_t step = ((hi - lo) / parts + page - 1) / page * page;
+  auto part = [=](int q) {
+    const uintptr_t a = lo + q * step, b = std::min(hi, a + step);
+    if (a < b) madvise((void *)a, b - a, MADV_POPULATE_WRITE);
+  };
+  std::vector<std::thread> ts;
+  int q = 1;
+  try {
+    for (; q < parts; ++q) ts.emplace_back(part, q);
+  } catch (const std::exception &) {   // no more threads: the rest below
+  }
+  part(0);
+  for (; q < parts; ++q) part(q);
+  for (auto &t : ts) t.join();
+#else
+  (void)buf;
+  (void)bytes;
+#endif
+}
 
 ela3d_status validate_params(const ela3d_params &p) {
   if (p.nx < 3 || p.ny < 3 || p.nz < 3) BAD("grid must be at least 3 cells on each axis");
@@ -1459,6 +1496,7 @@ class Engine final : public EngineBase {
     const int nx = s.d.nx, ny = s.d.ny, nz = s.d.nz;
     const size_t n = (size_t)nx * ny * nz;
     if ((sizeof(T) == 8) == (out_fp64 != 0)) {
+      populate_host(out, n * sizeof(T));
       CK(cudaMemcpy2DAsync(out, nx * sizeof(T), s.d.f[comp], s.d.px * sizeof(T), nx * sizeof(T), (size_t)ny * nz,
                            cudaMemcpyDeviceToHost, stream_));
       CK(cudaStreamSynchronize(stream_));

@@ -19,6 +19,8 @@ namespace ela3d {
 void set_last_error(const std::string &msg);
 const char *last_error();
 ela3d_status status_from_cuda(cudaError_t e, const char *what);
+// Backs [buf, buf + bytes) with memory ahead of a device to host copy.
+void populate_host(void *buf, size_t bytes);
 
 // Validates a parameter block (grid, spacing, source, receivers).
 ela3d_status validate_params(const ela3d_params &p);
