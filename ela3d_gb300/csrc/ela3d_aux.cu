@@ -4,6 +4,8 @@
 // FP64 total-energy reduction used by the stability monitor.
 #include <math.h>
 
+#include <algorithm>
+
 #include "ela3d_internal.h"
 
 namespace ela3d {
@@ -124,8 +126,17 @@ __global__ void explosive_kernel(const ShotDesc<T> *shots, int nshots, int tick,
 // (1/(4mu)) sigma:sigma - lambda / (4mu(3lambda+2mu)) tr(sigma)^2, cell-local,
 // accumulated in FP64 (no counterpart in the reference; the stability monitor).
 // Two passes in a fixed order, so repeated calls on one state agree to the
-// bit: one block per z-plane writes the plane's sum to part[k], then one
-// block adds the planes in order (energy_sum_kernel).
+// bit: kEnergyParts blocks per z-plane write their sums to part[], then one
+// block adds them in order (energy_sum_kernel).
+//
+// The FP64 pipe bounds it (two lanes a cycle on each SM), so the FP32 kernel
+// spends as few FP64 operations as it can: the strain energy is one quotient
+// (ss D - lambda tr^2) / (4 mu D) with D = 3 lambda + 2 mu, the quotients of
+// four cells are brought to one denominator, and the twelve values of a cell
+// are widened with integer operations (widen_normal).  The denominators' product stays
+// in range for moduli between 1e-38 and 1e38.  FP64 plans, whose values may be
+// larger, keep one division per term.  FP32, ms a call before and now: 101^3
+// 0.23 and 0.12, 201^3 1.57 and 0.59, 256^3 2.54 and 1.10, 400^3 9.2 and 4.1.
 __device__ __forceinline__ double block_sum_f64(double v) {
   __shared__ double part[32];
   for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
@@ -139,15 +150,87 @@ __device__ __forceinline__ double block_sum_f64(double v) {
   return v;  // valid in thread 0
 }
 
-template <typename T>
-__global__ void energy_plane_kernel(const ShotDesc<T> *shot, int nx, int ny, double *part) {
-  const ShotDesc<T> &sd = *shot;
-  const int k = blockIdx.x;
-  const long long cells = (long long)nx * ny;
+// A zero or normal float as a double, by its bits: exact.
+__device__ __forceinline__ double widen_normal(float f) {
+  const unsigned b = __float_as_uint(f);
+  const unsigned hi = (b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u);
+  return __hiloint2double((b << 1) ? (int)hi : 0, (int)(b << 29));
+}
+__device__ __forceinline__ bool subnormal_or_special(float f) {   // also infinities and NaN
+  const unsigned b = __float_as_uint(f) << 1;
+  return b != 0 && (b < 0x01000000u || b >= 0xff000000u);
+}
+
+// Twice the kinetic energy density of one cell, and its strain energy density
+// as (n / 4) / d.
+__device__ __forceinline__ void energy_cell(const double (&v)[12], double &k, double &n, double &d) {
+  k = v[11] * (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+  const double mu = v[11] * (v[10] * v[10]), l2m = v[11] * (v[9] * v[9]), lam = l2m - 2.0 * mu;
+  const double tr = v[3] + v[4] + v[5], D = 3.0 * l2m - 4.0 * mu;
+  if (mu > 0.0) {
+    const double ss = v[3] * v[3] + v[4] * v[4] + v[5] * v[5] + 2.0 * (v[6] * v[6] + v[7] * v[7] + v[8] * v[8]);
+    n = ss * D - lam * (tr * tr);
+    d = mu * D;
+  } else {   // a fluid cell: tr^2 / (18 lambda)
+    n = lam > 0.0 ? tr * tr * (4.0 / 18.0) : 0.0;
+    d = lam > 0.0 ? lam : 1.0;
+  }
+}
+
+constexpr int kEnergyThreads = 256;
+
+__global__ void __launch_bounds__(kEnergyThreads)
+    energy_plane_kernel(const ShotDesc<float> *shot, int nx, int ny, int k0, double *part) {
+  const ShotDesc<float> &sd = *shot;
+  const int gx = (nx + 3) / 4;             // groups of four cells in a row
+  const unsigned groups = (unsigned)gx * ny;   // (fewer than 2^31: a grid holds at most 2^34 cells)
+  const long long plane = (long long)(k0 + blockIdx.y) * ny * sd.px;
+  double kin = 0.0, strain = 0.0;
+  for (unsigned q = blockIdx.x * kEnergyThreads + threadIdx.x; q < groups; q += gridDim.x * kEnergyThreads) {
+    const unsigned y = q / gx, x = 4 * (q - y * gx);
+    const long long o = plane + (long long)y * sd.px + x;
+    float f[12][4];
+#pragma unroll
+    for (int c = 0; c < 9; ++c) ld_vec_rw(sd.f[c] + o, f[c]);
+    ld_vec_rw(sd.cp + o, f[9]);
+    ld_vec_rw(sd.cs + o, f[10]);
+    ld_vec_rw(sd.rho + o, f[11]);
+    double n[4], d[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      n[e] = 0.0;
+      d[e] = 1.0;
+      if (x + e >= (unsigned)nx) continue;   // a padding column
+      bool slow = false;
+#pragma unroll
+      for (int c = 0; c < 12; ++c) slow |= subnormal_or_special(f[c][e]);
+      double v[12], k;
+      if (slow) {
+#pragma unroll
+        for (int c = 0; c < 12; ++c) v[c] = f[c][e];
+      } else {
+#pragma unroll
+        for (int c = 0; c < 12; ++c) v[c] = widen_normal(f[c][e]);
+      }
+      energy_cell(v, k, n[e], d[e]);
+      kin += k;
+    }
+    const double n01 = n[0] * d[1] + n[1] * d[0], d01 = d[0] * d[1];
+    const double n23 = n[2] * d[3] + n[3] * d[2], d23 = d[2] * d[3];
+    strain += (n01 * d23 + n23 * d01) / (d01 * d23);
+  }
+  const double acc = block_sum_f64(0.5 * kin + 0.25 * strain);
+  if (threadIdx.x == 0) part[(long long)blockIdx.y * gridDim.x + blockIdx.x] = acc;
+}
+
+__global__ void __launch_bounds__(kEnergyThreads)
+    energy_plane_kernel(const ShotDesc<double> *shot, int nx, int ny, int k0, double *part) {
+  const ShotDesc<double> &sd = *shot;
+  const long long cells = (long long)nx * ny, plane = (long long)(k0 + blockIdx.y) * ny * sd.px;
   double acc = 0.0;
-  for (long long q = threadIdx.x; q < cells; q += blockDim.x) {
+  for (long long q = blockIdx.x * kEnergyThreads + threadIdx.x; q < cells; q += (long long)gridDim.x * kEnergyThreads) {
     const long long y = q / nx, x = q - y * nx;
-    const long long o = ((long long)k * ny + y) * sd.px + x;
+    const long long o = plane + y * sd.px + x;
     const double rho = sd.rho[o], cp = sd.cp[o], cs = sd.cs[o];
     const double mu = rho * cs * cs, lam = rho * (cp * cp - 2.0 * cs * cs);
     const double vx = sd.f[0][o], vy = sd.f[1][o], vz = sd.f[2][o];
@@ -164,14 +247,14 @@ __global__ void energy_plane_kernel(const ShotDesc<T> *shot, int nx, int ny, dou
     acc += e;
   }
   acc = block_sum_f64(acc);
-  if (threadIdx.x == 0) part[k] = acc;
+  if (threadIdx.x == 0) part[(long long)blockIdx.y * gridDim.x + blockIdx.x] = acc;
 }
 
 template <typename T>
-__global__ void energy_sum_kernel(const ShotDesc<T> *shot, const double *part, int nz, double *out) {
+__global__ void energy_sum_kernel(const ShotDesc<T> *shot, const double *part, long long parts, double *out) {
   const ShotDesc<T> &sd = *shot;
   double acc = 0.0;
-  for (int k = threadIdx.x; k < nz; k += blockDim.x) acc += part[k];
+  for (long long k = threadIdx.x; k < parts; k += blockDim.x) acc += part[k];
   acc = block_sum_f64(acc);
   if (threadIdx.x == 0) *out = acc * (double)(1.0 / sd.idx) * (double)(1.0 / sd.idy) * (double)(1.0 / sd.idz);
 }
@@ -229,13 +312,21 @@ cudaError_t launch_explosive_f64(const ShotDesc<double> *shots, int nshots, int 
   explosive_kernel<double><<<(nshots + 63) / 64, 64, 0, s>>>(shots, nshots, tick, dtick);
   return cudaGetLastError();
 }
-// out[0] = the energy; out[1 .. nz] = the per-plane sums (scratch)
+// out[0] = the energy; the blocks' sums follow (scratch, kEnergyParts per
+// plane).  Blocks per plane: enough that a plane's cells give each thread
+// about two groups of four, at most kEnergyParts.
 template <typename T>
 static cudaError_t launch_energy(const ShotDesc<T> *shot, int nx, int ny, int nz, double *out, cudaStream_t s) {
-  energy_plane_kernel<T><<<nz, 256, 0, s>>>(shot, nx, ny, out + 1);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  energy_sum_kernel<T><<<1, 256, 0, s>>>(shot, out + 1, nz, out);
+  const long long per = 8ll * kEnergyThreads;   // cells a block takes at least
+  const int parts = (int)std::max(1ll, std::min<long long>(kEnergyParts, ((long long)nx * ny + per - 1) / per));
+  // (planes are the grid's y dimension: at most 65535 of them in a launch)
+  for (int k = 0; k < nz; k += 65535) {
+    const int planes = std::min(65535, nz - k);
+    energy_plane_kernel<<<dim3(parts, planes), kEnergyThreads, 0, s>>>(shot, nx, ny, k, out + 1 + (long long)k * parts);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  energy_sum_kernel<T><<<1, 1024, 0, s>>>(shot, out + 1, (long long)nz * parts, out);
   return cudaGetLastError();
 }
 cudaError_t launch_energy_f32(const ShotDesc<float> *shot, int nx, int ny, int nz, double *out, cudaStream_t s) {

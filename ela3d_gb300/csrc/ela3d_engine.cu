@@ -1515,13 +1515,13 @@ class Engine final : public EngineBase {
     const Shot<T> &s = *shots_[shot];
     const ShotDesc<T> *dd = d_desc_ ? d_desc_ + shot : nullptr;
     if (!dd) BAD("engine not finalized");
-    // the result and one partial sum per plane (grown to the largest nz seen)
+    // the result and the planes' partial sums (grown to the largest nz seen)
     if (energy_cap_ < s.d.nz + 1) {
       CK(cudaStreamSynchronize(stream_));
       if (d_energy_) cudaFree(d_energy_);
       d_energy_ = nullptr;
       energy_cap_ = 0;
-      CK(cudaMalloc(&d_energy_, sizeof(double) * (size_t)(s.d.nz + 1)));
+      CK(cudaMalloc(&d_energy_, sizeof(double) * ((size_t)s.d.nz * kEnergyParts + 1)));
       energy_cap_ = s.d.nz + 1;
     }
     CK(Fp<T>::energy(dd, s.d.nx, s.d.ny, s.d.nz, d_energy_, stream_));

@@ -60,7 +60,9 @@ cudaError_t launch_explosive_f64(const ShotDesc<double> *shots, int nshots, int 
 // Device step counter of replayable graphs: *dtick = value / *dtick += delta.
 cudaError_t launch_tick_set(int *dtick, int value, cudaStream_t s);
 cudaError_t launch_tick_add(int *dtick, int delta, cudaStream_t s);
-// Total energy of one shot, accumulated into *out (double, device).
+// Total energy of one shot into *out (double, device), followed by room for
+// kEnergyParts sums per plane.
+constexpr int kEnergyParts = 16;
 cudaError_t launch_energy_f32(const ShotDesc<float> *shot, int nx, int ny, int nz, double *out, cudaStream_t s);
 cudaError_t launch_energy_f64(const ShotDesc<double> *shot, int nx, int ny, int nz, double *out, cudaStream_t s);
 
