@@ -138,7 +138,8 @@ static TuneChoice resolve_tuning(const std::vector<ela3d_params> &ps, const floa
   // round-robin chunks enough to go around)
   const bool open = !t || (t->variant < 0 && t->schedule < 0 && t->chunk <= 0 && t->blocks_per_sm < 0 &&
                            t->prefetch < 0 && t->lag < 0);
-  TuneChoice c = ps.size() != 1 ? default_choice(p.precision == ELA3D_FP64, 0, 0, 0)
+  TuneChoice c = ps.size() != 1 ? (open ? batch_choice(ps, p.precision == ELA3D_FP64)
+                                        : default_choice(p.precision == ELA3D_FP64, 0, 0, 0))
                  : open         ? plan_choice(p)
                                 : default_choice(p.precision == ELA3D_FP64, p.nx, p.ny, p.nz,
                                                  p.src_kind == ELA3D_SRC_EXPLOSIVE);

@@ -40,7 +40,9 @@ constexpr unsigned long long kTestWaitLimitNs = 20000000ull;
 // CTL_PF_X lets the producer warp prefetch into L2 the C-PML memory
 // variables of the x slab, CTL_PF_YZ those of the y and z slabs into L2
 // (performance hints; results do not depend on them).
-enum : int { CTL_WITHHOLD_LOADS = 1, CTL_PF_X = 2, CTL_PF_YZ = 4 };
+// CTL_RETIRE: the dataflow kernel passes over the items of a shot that has
+// done its nstep steps.
+enum : int { CTL_WITHHOLD_LOADS = 1, CTL_PF_X = 2, CTL_PF_YZ = 4, CTL_RETIRE = 8 };
 
 // How a kernel's loading warp fills a stage: one lane issues TMA tiled loads
 // (LOAD_TMA, every production variant), or all 32 lanes copy 16-byte chunks

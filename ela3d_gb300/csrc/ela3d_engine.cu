@@ -226,7 +226,9 @@ bool build_flow_schedule(const std::vector<FlowShape> &shots, int tx, int ty, in
   flag_off->clear();
   nchunks->clear();
   *nflags = 0;
-  if (chunk < 2 || gap < 1 || nsteps < 1 || nsteps > 255 || tx < 1 || ty < 1 || shots.size() >= (1u << 16)) {
+  bool sized = true;
+  for (const FlowShape &f : shots) sized = sized && (f.chunk == 0 ? chunk >= 2 : f.chunk >= 2);
+  if (!sized || (shots.empty() && chunk < 2) || gap < 1 || nsteps < 1 || nsteps > 255 || tx < 1 || ty < 1 || shots.size() >= (1u << 16)) {
     *why = "dataflow schedule: chunk >= 2, gap >= 1, 1 <= nsteps <= 255, fewer than 65536 shots";
     return false;
   }
@@ -238,7 +240,7 @@ bool build_flow_schedule(const std::vector<FlowShape> &shots, int tx, int ty, in
   // unless steps may overlap).  The list is ordered by key, ties by (step,
   // kind, shot, chunk, tile): the items are generated in that tie order and
   // sorted stably by key (a counting sort when the keys are dense).
-  struct Shape { int txs, tys, nt, J; long long step_base; std::vector<long long> ks, kv, kv_prev; };
+  struct Shape { int txs, tys, nt, J, C; long long step_base; std::vector<long long> ks, kv, kv_prev; };
   std::vector<Shape> sh(shots.size());
   size_t total = 0;
   for (size_t s = 0; s < shots.size(); ++s) {
@@ -246,7 +248,8 @@ bool build_flow_schedule(const std::vector<FlowShape> &shots, int tx, int ty, in
     h.txs = (shots[s].nx + tx - 1) / tx;
     h.tys = (shots[s].ny + ty - 1) / ty;
     h.nt = h.txs * h.tys;
-    h.J = (shots[s].nz + chunk - 1) / chunk;
+    h.C = shots[s].chunk ? shots[s].chunk : chunk;
+    h.J = (shots[s].nz + h.C - 1) / h.C;
     if (h.J >= (1 << 14) || h.nt >= (1 << 25)) {
       *why = "dataflow schedule: too many z-chunks or tiles for one shot";
       return false;
@@ -373,8 +376,8 @@ bool build_flow_schedule(const std::vector<FlowShape> &shots, int tx, int ty, in
     g2 -= first[sidx];
     const Shape &h = sh[sidx];
     const int j = (int)(g2 / h.nt), t = (int)(g2 % h.nt), nz = shots[sidx].nz;
-    const int k0 = kind == 0 ? j * chunk : std::max(j * chunk - 1, 0);
-    const int k1 = kind == 0 ? std::min((j + 1) * chunk, nz) : (j == h.J - 1 ? nz : (j + 1) * chunk - 1);
+    const int k0 = kind == 0 ? j * h.C : std::max(j * h.C - 1, 0);
+    const int k1 = kind == 0 ? std::min((j + 1) * h.C, nz) : (j == h.J - 1 ? nz : (j + 1) * h.C - 1);
     (*items)[q] = FlowItem{{shots[sidx].id, t, k0, k1}, kind, r, j, 0};
   }
   return true;
@@ -456,49 +459,98 @@ TuneChoice default_choice(int fp64, int nx, int ny, int nz, bool explosive) {
   return c;
 }
 
+// The tile: the share of its threads that hold cells, times a weight for its
+// shape.  Narrow tiles read more halo, which costs little while the arrays are
+// near the L2 (126 MB) and more once they stream from HBM.  Single shots,
+// Gcell-updates/s (128x7, 112x8, 64x14, 56x16, 32x28): 101^3 32.4 34.2 30.8
+// 31.2 30.7; 128^3 42.2 28.7 40.3 35.7 40.2; 160^3 33.3 35.8 38.8 41.2 42.0;
+// 192^3 37.7 40.2 43.1 38.8 43.1; 224^3 44.1 46.2 42.5 43.6 43.9; 256^3 48.5
+// 40.8 46.8 43.3 43.5; 320^3 46.3 47.6 47.6 44.0 42.3; 150x211x93 29.7 31.4
+// 34.8 35.5 37.5.  For several shots the cells' summed time decides.
+static int pick_tile(const std::vector<ela3d_params> &ps, bool streams, int fallback) {
+  int n = 0;
+  const Variant *v = variants(&n);
+  const struct { int tx, ty; double w; } shapes[] = {
+      {128, 7, 1.0}, {112, 8, 0.985}, {64, 14, 0.96}, {56, 16, streams ? 0.88 : 0.93}, {32, 28, streams ? 0.85 : 0.98}};
+  int pick = fallback;
+  double best = 0.0;
+  for (const auto &s : shapes)
+    for (int j = 0; j < n; ++j) {
+      if (v[j].fp64 || v[j].loads != LOAD_TMA || !v[j].flow || v[j].tx != s.tx || v[j].ty != s.ty) continue;
+      double cells = 0.0, taken = 0.0;
+      for (const ela3d_params &p : ps) {
+        cells += (double)p.nx * p.ny * p.nz;
+        taken += (double)((p.nx + s.tx - 1) / s.tx * s.tx) * ((p.ny + s.ty - 1) / s.ty * s.ty) * p.nz;
+      }
+      const double score = s.w * cells / taken;
+      if (score > best) {
+        best = score;
+        pick = j;
+      }
+    }
+  return pick;
+}
+
+static int device_sms() {
+  int dev = 0, sms = 152;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
+// The chunk: about two items per block and half-step, for the claimed places
+// to even out (256^3: 48.8 Gcell-updates/s with 64 planes, 45.1 with 86), but
+// no more than 80 planes (512^3: 51.0 at 64, 50.5 at 128, 48.8 in whole
+// columns; 448^3 48.7 at 75, 44.8 whole; 384^3 49.7 at 96, 48.6 at 192) and no
+// fewer than 2.
+int flow_chunk(int nz, long long tiles, int blocks, int most) {
+  long long per_col = std::max({1ll, (4ll * blocks + tiles) / (2 * tiles), (long long)(nz + most - 1) / most});
+  per_col = std::min(per_col, 16000ll);   // (a schedule holds fewer than 2^14 chunks per column)
+  return std::max(2, (int)((nz + per_col - 1) / per_col));
+}
+
 TuneChoice plan_choice(const ela3d_params &p) {
   // (explosive sources too: 201^3 242 us a step on the two kernels, 204 here)
   TuneChoice c = default_choice(p.precision == ELA3D_FP64, p.nx, p.ny, p.nz);
   if (c.kind != kScheduleFlowOverlap) return c;
   int n = 0;
   const Variant *v = variants(&n);
-  // The tile: the share of its threads that hold cells, times a weight for
-  // its shape.  Narrow tiles read more halo, which costs little while the
-  // arrays are near the L2 (126 MB) and more once they stream from HBM.
-  // Gcell-updates/s (128x7, 112x8, 64x14, 56x16, 32x28): 101^3 32.4 34.2 30.8
-  // 31.2 30.7; 128^3 42.2 28.7 40.3 35.7 40.2; 160^3 33.3 35.8 38.8 41.2 42.0;
-  // 192^3 37.7 40.2 43.1 38.8 43.1; 224^3 44.1 46.2 42.5 43.6 43.9; 256^3 48.5
-  // 40.8 46.8 43.3 43.5; 320^3 46.3 47.6 47.6 44.0 42.3; 150x211x93 29.7 31.4
-  // 34.8 35.5 37.5.
-  const double bytes = 12.0 * p.nx * p.ny * p.nz * 4.0;
-  const bool streams = bytes > 400e6;
-  const struct { int tx, ty; double w; } shapes[] = {
-      {128, 7, 1.0}, {112, 8, 0.985}, {64, 14, 0.96}, {56, 16, streams ? 0.88 : 0.93}, {32, 28, streams ? 0.85 : 0.98}};
-  double best = 0.0;
-  for (const auto &s : shapes)
-    for (int j = 0; j < n; ++j) {
-      if (v[j].fp64 || v[j].loads != LOAD_TMA || !v[j].flow || v[j].tx != s.tx || v[j].ty != s.ty) continue;
-      const long long cx = (p.nx + s.tx - 1) / s.tx * s.tx, cy = (p.ny + s.ty - 1) / s.ty * s.ty;
-      const double score = s.w * ((double)p.nx / cx) * ((double)p.ny / cy);
-      if (score > best) {
-        best = score;
-        c.variant = j;
-      }
-    }
-  // The chunk: about two items per block and half-step, for the claimed
-  // places to even out (256^3: 48.8 with 64 planes, 45.1 with 86), but no more
-  // than 80 planes (512^3: 51.0 at 64, 50.5 at 128, 48.8 in whole columns;
-  // 448^3 48.7 at 75, 44.8 whole; 384^3 49.7 at 96, 48.6 at 192) and no fewer
-  // than 2.
-  int dev = 0, sms = 152;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const bool streams = 12.0 * p.nx * p.ny * p.nz * 4.0 > 400e6;
+  c.variant = pick_tile({p}, streams, c.variant);
   const int tx = v[c.variant].tx, ty = v[c.variant].ty;
-  const long long tiles = (long long)((p.nx + tx - 1) / tx) * ((p.ny + ty - 1) / ty);
-  const long long per_col = std::max({1ll, (4ll * sms + tiles) / (2 * tiles), (long long)(p.nz + 79) / 80});
-  c.chunk = std::max(2, (int)((p.nz + per_col - 1) / per_col));
+  c.chunk = flow_chunk(p.nz, (long long)((p.nx + tx - 1) / tx) * ((p.ny + ty - 1) / ty), device_sms(), 80);
   // the memory variables' copies reach one plane ahead; the prefetches add
   // to that only where the variables come from DRAM
   c.prefetch = streams ? kPrefetchDefault : 0;
+  return c;
+}
+
+// Shots that run together.  Known ones (a batch) take the dataflow kernel with
+// the tile that suits all of them best and chunks of up to 48 planes, no
+// prefetch; Gcell-updates/s against the two kernels with 128x7 tiles and
+// 10-plane chunks: eight 192^3 shots of one model 45.2 against 36.6, ten uneven
+// grids (edges 64-320) 39.0 against 35.6.  (80 planes 43.8 and 38.3; with all
+// prefetches 43.7 and 38.0.)
+// A server's shots are prepared while others run: the dataflow kernel would
+// hold every SM for many steps and keep the preparation's kernels waiting, so
+// a server keeps the two kernels, on the tile that was best for uneven grids
+// (ten of them, 32-plane chunks: 38.5, 128x7 with 10 planes 35.6); chunk 0:
+// sized for the shots running.
+TuneChoice batch_choice(const std::vector<ela3d_params> &ps, int fp64) {
+  TuneChoice c = default_choice(fp64, 0, 0, 0);
+  int n = 0;
+  const Variant *v = variants(&n);
+  if (fp64 || !v[c.variant].flow) return c;
+  c.prefetch = 0;
+  c.lag = 0;
+  c.chunk = 0;
+  if (ps.empty()) {
+    for (int j = 0; j < n; ++j)
+      if (!v[j].fp64 && v[j].loads == LOAD_TMA && v[j].tx == 64 && v[j].ty == 14) c.variant = j;
+    c.kind = 1;
+  } else {
+    c.variant = pick_tile(ps, true, c.variant);
+    c.kind = kScheduleFlowOverlap;
+  }
   return c;
 }
 
@@ -1058,6 +1110,13 @@ class Engine final : public EngineBase {
     return best;
   }
 
+  // Steps until every shot has reached its nstep.
+  int steps_to_last() const {
+    int most = 1;
+    for (auto &sp : shots_) most = std::max(most, sp->d.tick0 + sp->p.nstep - tick_);
+    return most;
+  }
+
   ela3d_status enqueue(int nsteps) override {
     if (!finalized_) BAD("engine not finalized");
     if (nsteps < 0) BAD("nsteps must be >= 0");
@@ -1066,7 +1125,13 @@ class Engine final : public EngineBase {
       if (retire_) {
         ela3d_status st = rebuild_schedule();
         if (st != ELA3D_OK) return st;
-        seg = std::min(seg, steps_to_boundary());
+        // (the dataflow kernel passes over finished shots itself: a launch
+        // ends at a shot's last step only for an explosive source's sake,
+        // whose last injection comes after the launch)
+        if (flow_on() && flow_steps_ > 0 && !any_explosive_)
+          seg = std::min({seg, steps_to_last(), std::max(1, flow_steps_ * flow_walks_)});
+        else
+          seg = std::min(seg, steps_to_boundary());
         if (nblocks_ == 0) {  // nothing active: time passes, no work
           tick_ += seg;
           nsteps -= seg;
@@ -1081,7 +1146,7 @@ class Engine final : public EngineBase {
       if (flow_on() && flow_steps_ > 0) {
         while (seg > 0) {
           // (places in a launch's list are 32-bit)
-          const int passes = (int)std::min<long long>(flow_passes_, std::max(1ll, (1ll << 30) / std::max(1, flow_items_)));
+          const int passes = (int)std::min<long long>(flow_walks_, std::max(1ll, (1ll << 30) / std::max(1, flow_items_)));
           const int k = std::min(seg, flow_steps_ * passes);
           ela3d_status st = launch_flow(tick_ + 1, k);
           if (st != ELA3D_OK) return st;
@@ -1197,11 +1262,25 @@ class Engine final : public EngineBase {
       nblocks_ = 0;
       return ELA3D_OK;
     }
+    flow_items_ = 0;
+    flow_steps_ = 0;
+    if (flow_on()) {
+      nblocks_ = 1;   // (something is active)
+      return rebuild_flow(key);
+    }
     std::vector<Item> items;
     std::vector<int2> ranges;
     const int kind = choice_.kind >= kScheduleFlow ? 1 : choice_.kind;
-    build_schedule(shapes, var_->tx, var_->ty, kind, std::max(choice_.chunk, 1), per_sm_ * num_sms_, &items,
-                   &ranges);
+    int chunk = choice_.chunk;
+    if (chunk <= 0) {
+      // sized for the shots running: 32 planes once they fill the GPU,
+      // shorter while that leaves fewer than about six items per block
+      long long planes = 0;
+      for (const ShotShape &sh : shapes)
+        planes += (long long)((sh.nx + var_->tx - 1) / var_->tx) * ((sh.ny + var_->ty - 1) / var_->ty) * sh.nz;
+      chunk = (int)std::max<long long>(8, std::min<long long>(32, planes / (6ll * per_sm_ * num_sms_)));
+    }
+    build_schedule(shapes, var_->tx, var_->ty, kind, chunk, per_sm_ * num_sms_, &items, &ranges);
     if (items.empty()) BAD("empty schedule");
     for (const Item &it : items)
       if (it.k1 <= it.k0) BAD("internal: empty work item");
@@ -1222,9 +1301,6 @@ class Engine final : public EngineBase {
     CK(cudaMemcpy(d_ranges_, ranges.data(), ranges.size() * sizeof(int2), cudaMemcpyHostToDevice));
     nblocks_ = (int)ranges.size();
     nitems_ = (int)items.size();
-    flow_items_ = 0;
-    flow_steps_ = 0;
-    if (flow_on()) return rebuild_flow(key);
     return ELA3D_OK;
   }
 
@@ -1234,15 +1310,23 @@ class Engine final : public EngineBase {
   // point at them.
   ela3d_status rebuild_flow(const std::vector<int> &active) {
     std::vector<FlowShape> shapes;
-    long long per_step = 0;
+    long long per_step = 0, tiles = 0;
     const int C = std::max(choice_.chunk, 2);
+    auto tiles_of = [&](const ShotDesc<T> &d) {
+      return (long long)((d.nx + var_->tx - 1) / var_->tx) * ((d.ny + var_->ty - 1) / var_->ty);
+    };
+    for (int q : active) tiles += tiles_of(shots_[q]->d);
     for (int q : active) {
       const ShotDesc<T> &d = shots_[q]->d;
-      shapes.push_back({d.nx, d.ny, d.nz, q});
-      const long long nt = (long long)((d.nx + var_->tx - 1) / var_->tx) * ((d.ny + var_->ty - 1) / var_->ty);
-      per_step += 2 * nt * ((d.nz + C - 1) / C);
+      const int c = choice_.chunk > 0 ? C : flow_chunk(d.nz, tiles, per_sm_flow_ * num_sms_, 48);
+      shapes.push_back({d.nx, d.ny, d.nz, q, c});
+      per_step += 2 * tiles_of(d) * ((d.nz + c - 1) / c);
     }
-    const int K = (int)std::max<long long>(1, std::min<long long>(flow_max_steps_, kFlowMaxItems / std::max(1ll, per_step)));
+    // (shots that run together change more often than a plan's, and their
+    // longer steps hide the seam between two walks of a short list)
+    const long long most = active.size() > 1 ? kFlowBatchItems : kFlowMaxItems;
+    const int K = (int)std::max<long long>(1, std::min<long long>(flow_max_steps_, most / std::max(1ll, per_step)));
+    flow_walks_ = active.size() > 1 ? std::max(flow_passes_, (kFlowSteps * kFlowPasses + K - 1) / K) : flow_passes_;
     std::vector<FlowItem> items;
     std::vector<int> off, nch;
     int nflags = 0;
@@ -1290,7 +1374,7 @@ class Engine final : public EngineBase {
 
   // One launch of the dataflow kernel: steps tick .. tick + nsteps - 1.
   ela3d_status launch_flow(int tick, int nsteps) {
-    int ctl = (inject_ > 0 ? CTL_WITHHOLD_LOADS : 0) | prefetch_;
+    int ctl = (inject_ > 0 ? CTL_WITHHOLD_LOADS : 0) | prefetch_ | (retire_ ? CTL_RETIRE : 0);
     inject_ = std::max(0, inject_ - nsteps);
     const int *dtick = nullptr;
     // Blocks claim their places in the list (the counter behind the flags)
@@ -1782,7 +1866,8 @@ class Engine final : public EngineBase {
   // ELA3D_FLOW_PASSES=<n> the passes per launch (experiments)
   int flow_max_steps_ = kFlowSteps;
   int flow_passes_ = kFlowPasses;
-  static constexpr long long kFlowMaxItems = 1 << 20;
+  static constexpr long long kFlowMaxItems = 1 << 20, kFlowBatchItems = 1 << 14;
+  int flow_walks_ = kFlowPasses;   // walks of the list in one launch
   FlowItem *d_flow_ = nullptr;
   int *d_flags_ = nullptr;
   size_t flow_cap_ = 0, flags_cap_ = 0, flags_used_ = 0;

@@ -70,6 +70,7 @@ void build_schedule(const std::vector<ShotShape> &shots, int tx, int ty, int kin
 struct FlowShape {
   int nx, ny, nz;
   int id;   // shot index written into the items
+  int chunk = 0;   // planes per z-chunk of this shot (0: the schedule's)
 };
 bool build_flow_schedule(const std::vector<FlowShape> &shots, int tx, int ty, int chunk, int gap, bool overlap,
                          int nsteps, std::vector<FlowItem> *items, std::vector<int> *flag_off,
@@ -85,7 +86,7 @@ constexpr int kScheduleFlow = 3;
 constexpr int kScheduleFlowOverlap = 4;
 struct TuneChoice {
   int variant;     // index into variants()
-  int kind, chunk; // schedule
+  int kind, chunk; // schedule (chunk 0 = sized for the shots running)
   int blocks_per_sm;  // 0 = occupancy limit
   int prefetch = kPrefetchDefault;  // CTL_PF_* bits
   int lag = 0;     // kinds 3, 4: gap in items (0 = three rounds of the grid)
@@ -96,6 +97,13 @@ TuneChoice default_choice(int fp64, int nx, int ny, int nz, bool explosive = fal
 // default_choice takes the dataflow kernel, with the tile that wastes least
 // of the grid and the chunk that suits claimed places.
 TuneChoice plan_choice(const ela3d_params &p);
+// The same for shots that run together (none given: a server, whose shots are
+// not known yet): one tile for all, chunk 0 = sized for each shot.
+TuneChoice batch_choice(const std::vector<ela3d_params> &ps, int fp64);
+// Planes per z-chunk (at most `most`) of a dataflow schedule for a column of
+// nz planes, when the shots running have `tiles` tiles in all and there are
+// `blocks` blocks.
+int flow_chunk(int nz, long long tiles, int blocks, int most);
 
 // Autotuner (ela3d_tune.cu): process-wide cache of measured best choices
 // keyed by the workload shape.

@@ -355,7 +355,10 @@ ela3d_status ela3d_server_create(const ela3d_server_config *cfg, ela3d_server **
     ela3d_params probe{};
     ela3d_params_default(&probe);
     probe.precision = cfg->precision;
-    TuneChoice c = default_choice(cfg->precision == ELA3D_FP64, 0, 0, 0);
+    const ela3d_tuning &t = cfg->tune;
+    const bool open = t.variant < 0 && t.schedule < 0 && t.chunk <= 0 && t.blocks_per_sm < 0 && t.prefetch < 0 && t.lag < 0;
+    TuneChoice c = open ? batch_choice({}, cfg->precision == ELA3D_FP64)
+                        : default_choice(cfg->precision == ELA3D_FP64, 0, 0, 0);
     if (cfg->tune.variant >= 0) c.variant = cfg->tune.variant;
     if (cfg->tune.schedule >= 0) c.kind = cfg->tune.schedule;
     if (cfg->tune.chunk > 0) c.chunk = cfg->tune.chunk;

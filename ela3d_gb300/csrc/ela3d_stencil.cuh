@@ -1297,6 +1297,7 @@ __global__ void __launch_bounds__(Geo<T, TX, TY, NS, CPT, MB>::THREADS, Geo<T, T
     const int total = nitems * ((nsteps + pass_steps - 1) / pass_steps);
     unsigned n = 0, idx = 0;
     bool ok = true;
+    if (dtick) tick += *dtick;
     int next = 0;   // lane 0: the place claimed next
     if (lane == 0) next = claim ? atomicAdd(claim, 1) : (int)blockIdx.x;
     while (true) {
@@ -1320,6 +1321,10 @@ __global__ void __launch_bounds__(Geo<T, TX, TY, NS, CPT, MB>::THREADS, Geo<T, T
       }
       if (lane == 0) slot.fi = fi;
       __syncwarp();
+      if (!end && (ctl & CTL_RETIRE) && tick + fi.step - slot.sd.tick0 > slot.sd.nstep) {
+        __syncwarp();   // (the slot is filled again next)
+        continue;
+      }
       int good = 1;
       if (lane == 0) {
         if (!end) {
