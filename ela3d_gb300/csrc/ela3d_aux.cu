@@ -82,15 +82,15 @@ __global__ void stf_kernel(StfArgs p, T *out) {
   out[i] = (T)s;
 }
 
+// One warp per row (a row index is k*ny + j), rows of a warp `stride` apart.
 template <typename T>
-__global__ void pad_kernel(const float *__restrict__ src, T *__restrict__ dst, int nx, int ny, int nz,
-                           int px) {
-  const long long n = (long long)px * ny * nz;
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n;
-       q += (long long)gridDim.x * blockDim.x) {
-    const int x = (int)(q % px);
-    const long long r = q / px;  // row index = k*ny + j
-    dst[q] = x < nx ? (T)src[r * nx + x] : T(0);
+__global__ void pad_kernel(const float *__restrict__ src, T *__restrict__ dst, int nx, long long rows, int px) {
+  const int lane = threadIdx.x & 31;
+  const long long stride = (long long)gridDim.x * (blockDim.x >> 5);
+  for (long long r = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5); r < rows; r += stride) {
+    const float *a = src + r * nx;
+    T *b = dst + r * px;
+    for (int x = lane; x < px; x += 32) b[x] = x < nx ? (T)__ldg(a + x) : T(0);
   }
 }
 
@@ -295,11 +295,13 @@ cudaError_t launch_stf_f64(const StfArgs &a, double *out, cudaStream_t s) {
   return cudaGetLastError();
 }
 cudaError_t launch_pad_f32(const float *src, float *dst, int nx, int ny, int nz, int px, cudaStream_t s) {
-  pad_kernel<float><<<blocks_for((long long)px * ny * nz, 256, 4096), 256, 0, s>>>(src, dst, nx, ny, nz, px);
+  const long long rows = (long long)ny * nz;
+  pad_kernel<float><<<blocks_for(rows, 8, 4096), 256, 0, s>>>(src, dst, nx, rows, px);
   return cudaGetLastError();
 }
 cudaError_t launch_pad_f64(const float *src, double *dst, int nx, int ny, int nz, int px, cudaStream_t s) {
-  pad_kernel<double><<<blocks_for((long long)px * ny * nz, 256, 4096), 256, 0, s>>>(src, dst, nx, ny, nz, px);
+  const long long rows = (long long)ny * nz;
+  pad_kernel<double><<<blocks_for(rows, 8, 4096), 256, 0, s>>>(src, dst, nx, rows, px);
   return cudaGetLastError();
 }
 cudaError_t launch_explosive_f32(const ShotDesc<float> *shots, int nshots, int tick, const int *dtick,
