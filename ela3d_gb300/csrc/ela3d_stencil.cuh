@@ -93,11 +93,6 @@ __device__ __forceinline__ int tiles_x_of(const ShotDesc<T> &s, int TX) {
   return (s.nx + TX - 1) / TX;
 }
 
-// dt / rho_avg: FP32 uses the hardware reciprocal-based divide (<= 2 ulp
-// from the IEEE quotient); FP64 keeps the IEEE division.
-__device__ __forceinline__ float div_fast(float a, float b) { return __fdividef(a, b); }
-__device__ __forceinline__ double div_fast(double a, double b) { return a / b; }
-
 // Arithmetic with the rounding written out: these are never fused with a
 // neighbouring operation.
 __device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
@@ -108,6 +103,62 @@ __device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, 
 __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ float sub_rn(float a, float b) { return __fsub_rn(a, b); }
 __device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(a, b); }
+
+// dt / rho_avg of two densities: FP32 uses the hardware reciprocal-based
+// divide (<= 2 ulp from the IEEE quotient).
+__device__ __forceinline__ float dt_over_rho(float dt, float r0, float r1) {
+  return __fdividef(dt, mul_rn(add_rn(r0, r1), 0.5f));
+}
+// FP64: the IEEE quotient dt / ((r0 + r1) / 2) = 2 dt / R, with fewer FP64
+// operations than a general division: the FP64 pipe (two lanes a cycle on
+// each SM) bounds the FP64 kernels.  R = r0 + r1 is a sum of two float32 model
+// values.  Its reciprocal starts from the FP32 unit (relative error 2^-22,
+// widened and narrowed by integer operations), takes one cubic Newton step
+// (e = 1 - R y; y (1 + e + e^2)), and the quotient one Markstein correction
+// (P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990): q + (2 dt - q R) y rounds to the IEEE
+// quotient, because a quotient by a 26-bit R stays 2^-27 of an ulp away from
+// the midpoints between doubles, far more than the correction's error.
+// Anything outside the normal float32 range divides as usual.
+__device__ __forceinline__ double dt_over_rho(double dt, double r0, double r1) {
+  const double R = add_rn(r0, r1), a = 2.0 * dt;
+  const int hi = __double2hiint(R);
+  // 2^-100 <= R < 2^100
+  if ((unsigned)(hi - 0x39b00000) >= 0x0c800000u) return a / R;
+  const float rf = __uint_as_float(((unsigned)(hi - 0x38000000) << 3) | ((unsigned)__double2loint(R) >> 29));
+  float yf;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(rf));
+  const unsigned yb = __float_as_uint(yf);
+  const double y0 = __hiloint2double((int)((yb >> 3) + 0x38000000u), (int)(yb << 29));
+  const double e = fma_rn(-R, y0, 1.0);
+  const double y = fma_rn(y0, fma_rn(e, e, e), y0);
+  const double q = mul_rn(a, y);
+  return fma_rn(fma_rn(-q, R, a), y, q);
+}
+
+// dt mu of the averaged shear velocity S / 2 and density R / 2:
+// dt ((R/2 S/2) S/2).  FP64 takes the halves out as one factor 1/8 (exact).
+__device__ __forceinline__ float dt_mu(float dt, float c0, float c1, float r0, float r1) {
+  const float vs = mul_rn(add_rn(c0, c1), 0.5f), rhos = mul_rn(add_rn(r0, r1), 0.5f);
+  return mul_rn(dt, mul_rn(mul_rn(rhos, vs), vs));
+}
+__device__ __forceinline__ double dt_mu(double dt, double c0, double c1, double r0, double r1) {
+  const double S = add_rn(c0, c1), R = add_rn(r0, r1);
+  return mul_rn(0.125 * dt, mul_rn(mul_rn(R, S), S));
+}
+
+// dt (lambda + 2 mu) and dt lambda of one cell: lambda = rho (vp^2 - 2 vs^2).
+__device__ __forceinline__ void dt_moduli(float dt, float vp, float vs, float rho, float &l2m, float &lam) {
+  l2m = mul_rn(dt, mul_rn(mul_rn(rho, vp), vp));
+  lam = mul_rn(dt, mul_rn(rho, fma_rn(vp, vp, -mul_rn(mul_rn(2.0f, vs), vs))));
+}
+// FP64: the model's values are float32 numbers, so the squares are exact and
+// rho (vp vp) rounds to what (rho vp) vp does.
+__device__ __forceinline__ void dt_moduli(double dt, double vp, double vs, double rho, double &l2m, double &lam) {
+  const double vp2 = mul_rn(vp, vp);
+  l2m = mul_rn(dt, mul_rn(rho, vp2));
+  lam = mul_rn(dt, mul_rn(rho, fma_rn(-2.0, mul_rn(vs, vs), vp2)));
+}
 
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -661,9 +712,8 @@ __device__ __forceinline__ bool stress_item(const ShotDesc<T> &sd, const Item &i
       constexpr bool fx = decltype(X)::value, fy = decltype(Y)::value, fz = decltype(Z)::value;
 #pragma unroll
       for (int e = 0; e < V; ++e) {
-        const T vp = cp_c[e], vs = cs_c[e], rhos = rho_c[e];
-        const T lambda = mul_rn(rhos, fma_rn(vp, vp, -mul_rn(mul_rn(T(2), vs), vs)));
-        const T DT_l2m = mul_rn(dt, mul_rn(mul_rn(rhos, vp), vp)), DT_l = mul_rn(dt, lambda);
+        T DT_l2m, DT_l;
+        dt_moduli(dt, cp_c[e], cs_c[e], rho_c[e], DT_l2m, DT_l);
         const T tx = add_rn(eyy[e], ezz[e]), ty = add_rn(exx[e], ezz[e]), tz = add_rn(exx[e], eyy[e]);
         auto two = [&](auto own, T d, T t) {
           return decltype(own)::value ? fma_rn(DT_l2m, d, mul_rn(DT_l, t)) : fma_rn(DT_l, t, mul_rn(DT_l2m, d));
@@ -686,23 +736,19 @@ __device__ __forceinline__ bool stress_item(const ShotDesc<T> &sd, const Item &i
     for (int e = 0; e < V; ++e) {
       const T cs_xm = (e > 0) ? cs_c[e - 1] : cs_w;
       const T rho_xm = (e > 0) ? rho_c[e - 1] : rho_w;
-      auto dt_mu = [&](T c0, T c1, T r0, T r1) {   // dt mu of the averaged density and velocity
-        const T vs = mul_rn(add_rn(c0, c1), T(0.5)), rhos = mul_rn(add_rn(r0, r1), T(0.5));
-        return mul_rn(dt, mul_rn(mul_rn(rhos, vs), vs));
-      };
       // sigma_xy, :416-442
       {
-        const T mu = dt_mu(cs_xm, cs_yp[e], rho_xm, rho_yp[e]);
+        const T mu = dt_mu(dt, cs_xm, cs_yp[e], rho_xm, rho_yp[e]);
         if ((mk >> (8 + e)) & 1u) sxy[e] = fma_rn(mu, fma_rn(exy[e], sy, eyx[e]), sxy[e]);
       }
       // sigma_xz, :445-471 (z+1 of plane nz-1 is the zero plane)
       {
-        const T mu = dt_mu(cs_xm, cs_zp[e], rho_xm, rho_zp[e]);
+        const T mu = dt_mu(dt, cs_xm, cs_zp[e], rho_xm, rho_zp[e]);
         if ((mk >> (16 + e)) & 1u) sxz[e] = fma_rn(mu, fma_rn(exz[e], sz, ezx[e]), sxz[e]);
       }
       // sigma_yz, :473-498
       {
-        const T mu = dt_mu(cs_yp[e], cs_zp[e], rho_yp[e], rho_zp[e]);
+        const T mu = dt_mu(dt, cs_yp[e], cs_zp[e], rho_yp[e], rho_zp[e]);
         // (a derivative whose C-PML term was applied has S = 1, and its
         // product with S is exact)
         const bool z_fused = F32 ? row_y : !plane_z;
@@ -991,8 +1037,11 @@ __device__ __forceinline__ bool velocity_item(const ShotDesc<T> &sd, const Item 
     if (!last) fetch_psi(k + 1, gx + dgx, gy + dgy);
 
     auto update = [&](bool m, T r0, T r1, T d1, T d2, T d3, T &v) {
-      const T DT_over_rho = div_fast(dt, mul_rn(add_rn(r0, r1), T(0.5)));
-      if (m) v = fma_rn(DT_over_rho, fma_rn(d3, sz, fma_rn(d2, sy, d1)), v);
+      // (FP32 divides for every cell: a branch around it costs more.  FP64
+      // leaves out the cells outside the range, whose density may be 0.)
+      T b = T(0);
+      if (F32 || m) b = dt_over_rho(dt, r0, r1);
+      if (m) v = fma_rn(b, fma_rn(d3, sz, fma_rn(d2, sy, d1)), v);
     };
 #pragma unroll
     for (int e = 0; e < V; ++e) {
