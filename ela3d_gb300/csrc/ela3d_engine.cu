@@ -466,17 +466,22 @@ TuneChoice default_choice(int fp64, int nx, int ny, int nz, bool explosive) {
 // 31.2 30.7; 128^3 42.2 28.7 40.3 35.7 40.2; 160^3 33.3 35.8 38.8 41.2 42.0;
 // 192^3 37.7 40.2 43.1 38.8 43.1; 224^3 44.1 46.2 42.5 43.6 43.9; 256^3 48.5
 // 40.8 46.8 43.3 43.5; 320^3 46.3 47.6 47.6 44.0 42.3; 150x211x93 29.7 31.4
-// 34.8 35.5 37.5.  For several shots the cells' summed time decides.
-static int pick_tile(const std::vector<ela3d_params> &ps, bool streams, int fallback) {
+// 34.8 35.5 37.5.  FP64 is bound by its arithmetic, and a thread without a
+// cell costs as much as one with: 101^3 with 32x7, 16x14 and 8x28 tiles (76%,
+// 81% and 88% used) 3.34, 3.65 and 3.83; 180^3 (93%, 93%, 90%) 4.57, 4.62 and
+// 4.48.  For several shots the cells' summed time decides.
+static int pick_tile(const std::vector<ela3d_params> &ps, bool fp64, bool streams, int fallback) {
   int n = 0;
   const Variant *v = variants(&n);
-  const struct { int tx, ty; double w; } shapes[] = {
-      {128, 7, 1.0}, {112, 8, 0.985}, {64, 14, 0.96}, {56, 16, streams ? 0.88 : 0.93}, {32, 28, streams ? 0.85 : 0.98}};
+  const struct { bool fp64; int tx, ty; double w; } shapes[] = {
+      {false, 128, 7, 1.0}, {false, 112, 8, 0.985}, {false, 64, 14, 0.96}, {false, 56, 16, streams ? 0.88 : 0.93},
+      {false, 32, 28, streams ? 0.85 : 0.98}, {true, 32, 7, 1.0}, {true, 16, 14, 1.0}, {true, 8, 28, 1.0}};
   int pick = fallback;
   double best = 0.0;
   for (const auto &s : shapes)
-    for (int j = 0; j < n; ++j) {
-      if (v[j].fp64 || v[j].loads != LOAD_TMA || !v[j].flow || v[j].tx != s.tx || v[j].ty != s.ty) continue;
+    for (int j = 0; j < n && s.fp64 == fp64; ++j) {
+      if ((v[j].fp64 != 0) != fp64 || v[j].loads != LOAD_TMA || !v[j].flow || v[j].tx != s.tx || v[j].ty != s.ty)
+        continue;
       double cells = 0.0, taken = 0.0;
       for (const ela3d_params &p : ps) {
         cells += (double)p.nx * p.ny * p.nz;
@@ -510,14 +515,19 @@ int flow_chunk(int nz, long long tiles, int blocks, int most) {
 
 TuneChoice plan_choice(const ela3d_params &p) {
   // (explosive sources too: 201^3 242 us a step on the two kernels, 204 here)
-  TuneChoice c = default_choice(p.precision == ELA3D_FP64, p.nx, p.ny, p.nz);
-  if (c.kind != kScheduleFlowOverlap) return c;
+  // and FP64 (101^3 335 us a step on the two kernels, 270 here; 160x128x144
+  // 722, 645)
+  const bool fp64 = p.precision == ELA3D_FP64;
+  TuneChoice c = default_choice(fp64, p.nx, p.ny, p.nz);
   int n = 0;
   const Variant *v = variants(&n);
-  const bool streams = 12.0 * p.nx * p.ny * p.nz * 4.0 > 400e6;
-  c.variant = pick_tile({p}, streams, c.variant);
+  if (!v[c.variant].flow) return c;
+  c.kind = kScheduleFlowOverlap;
+  c.lag = 0;
+  const bool streams = !fp64 && 12.0 * p.nx * p.ny * p.nz * 4.0 > 400e6;
+  c.variant = pick_tile({p}, fp64, streams, c.variant);
   const int tx = v[c.variant].tx, ty = v[c.variant].ty;
-  c.chunk = flow_chunk(p.nz, (long long)((p.nx + tx - 1) / tx) * ((p.ny + ty - 1) / ty), device_sms(), 80);
+  c.chunk = flow_chunk(p.nz, (long long)((p.nx + tx - 1) / tx) * ((p.ny + ty - 1) / ty), device_sms(), fp64 ? 32 : 80);
   // the memory variables' copies reach one plane ahead; the prefetches add
   // to that only where the variables come from DRAM
   c.prefetch = streams ? kPrefetchDefault : 0;
@@ -539,7 +549,7 @@ TuneChoice batch_choice(const std::vector<ela3d_params> &ps, int fp64) {
   TuneChoice c = default_choice(fp64, 0, 0, 0);
   int n = 0;
   const Variant *v = variants(&n);
-  if (fp64 || !v[c.variant].flow) return c;
+  if (!v[c.variant].flow || (fp64 && ps.empty())) return c;
   c.prefetch = 0;
   c.lag = 0;
   c.chunk = 0;
@@ -548,7 +558,7 @@ TuneChoice batch_choice(const std::vector<ela3d_params> &ps, int fp64) {
       if (!v[j].fp64 && v[j].loads == LOAD_TMA && v[j].tx == 64 && v[j].ty == 14) c.variant = j;
     c.kind = 1;
   } else {
-    c.variant = pick_tile(ps, true, c.variant);
+    c.variant = pick_tile(ps, fp64 != 0, true, c.variant);
     c.kind = kScheduleFlowOverlap;
   }
   return c;

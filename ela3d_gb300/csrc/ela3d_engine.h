@@ -93,9 +93,9 @@ struct TuneChoice {
 };
 // Built-in choice when the autotuner's cache has none for the workload.
 TuneChoice default_choice(int fp64, int nx, int ny, int nz, bool explosive = false);
-// The choice of a plan whose caller leaves every tuning field open: where
-// default_choice takes the dataflow kernel, with the tile that wastes least
-// of the grid and the chunk that suits claimed places.
+// The choice of a plan whose caller leaves every tuning field open: the
+// dataflow kernel with the tile that wastes least of the grid and the chunk
+// that suits claimed places.
 TuneChoice plan_choice(const ela3d_params &p);
 // The same for shots that run together (none given: a server, whose shots are
 // not known yet): one tile for all, chunk 0 = sized for each shot.

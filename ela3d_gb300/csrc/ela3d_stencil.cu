@@ -61,6 +61,9 @@ static const Variant kVariants[] = {
     // five 32-wide tiles, 67% of two 112-wide ones)
     make_variant<float, 56, 16, 4>(),
     make_variant<float, 32, 28, 4>(),
+    // and narrow FP64 tiles: its arithmetic bounds FP64, idle lanes included
+    make_variant<double, 16, 14, 4, 1>(),
+    make_variant<double, 8, 28, 4, 1>(),
 };
 
 const Variant *variants(int *count) {

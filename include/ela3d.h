@@ -290,9 +290,10 @@ typedef struct ela3d_tuning {
  * the built-in choice for a single FP32 shot without an explosive source,
  * its z-chunks sized for about 1.5 work items per block (ela3d_builtin_tuning
  * reports the choice).  A plan whose caller leaves every field open refines
- * that choice where it is schedule 4, and takes schedule 4 for an explosive
- * source too: the tile that wastes least of the grid, z-chunks for about two
- * items per block and of at most 80 planes. */
+ * that choice, and takes schedule 4 for an explosive source and in FP64 too:
+ * the tile that wastes least of the grid, z-chunks for about two items per
+ * block and of at most 80 planes (FP64 32).  A batch with open fields takes
+ * schedule 4 as well, one tile for all its shots and chunks for each. */
 
 /* Times every compiled variant with the candidate schedules on these shots
  * (`steps` time steps each, after a warm-up) and returns the fastest choice;

@@ -53,3 +53,74 @@ def test_open_plan_equals_two_kernels(n, explosive):
     assert np.abs(want[0]).max() > 0
     for a, b in zip(got, want):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("n", [(32, 14, 20), (33, 15, 64), (16, 28, 70), (101, 101, 33), (9, 57, 40), (3, 3, 3)])
+@pytest.mark.parametrize("explosive", [False, True], ids=["force", "explosive"])
+def test_open_fp64_plan_equals_two_kernels(n, explosive):
+    """The same in FP64: each of its tiles and one cell past their edges."""
+    import ela3d_gb300 as E
+    from ela3d_gb300 import media
+
+    nx, ny, nz = n
+    p = E.ShotParams(nx=nx, ny=ny, nz=nz, nstep=23, dt=1e-3, npml=max(0, min(8, (min(n) - 2) // 3)), f0=25.0, t0=0.01,
+                     k_max=1.5, src=(nx // 2, ny // 3, nz // 2), precision=E.FP64, angle_force=25.0,
+                     src_kind=E.SRC_EXPLOSIVE if explosive else E.SRC_FORCE,
+                     rec=np.array([[nx // 2, ny // 3, nz // 2], [0, ny - 1, 0], [nx - 1, 0, nz - 1]], np.int32))
+    cp, cs, rho = media.anticline_layers(nx, ny, nz, depths=(nz * 0.3, nz * 0.6, nz * 0.8, 2 * nz), amp=nz * 0.1,
+                                         sigma=max(nx, ny) * 0.2, seed=3)
+    first = next(i for i, v in enumerate(E.variants()) if v.fp64)
+    want = _run(p, cp, cs, rho, variant=first, schedule=1, chunk=8)
+    got = _run(p, cp, cs, rho)
+    assert np.abs(want[0]).max() > 0
+    for a, b in zip(got, want):
+        assert np.array_equal(a, b)
+
+
+def test_open_batch_equals_shots_alone(built):
+    """A batch with open tuning: uneven grids, lengths and source kinds (the
+    shots that end first are passed over), and two shots of one model."""
+    import ela3d_gb300 as E
+    from ela3d_gb300 import media
+
+    shots = []
+    for i, (n, steps, kind) in enumerate([((70, 33, 90), 31, 0), ((33, 64, 40), 9, 1), ((129, 15, 60), 57, 0),
+                                          ((70, 33, 90), 44, 0)]):
+        m = shots[0][1:] if i == 3 else media.anticline_layers(
+            *n, depths=(n[2] * 0.3, n[2] * 0.7, n[2], 2 * n[2]), amp=4, sigma=n[0] * 0.2, seed=i)
+        rec = np.array([[n[0] // 2, n[1] // 2, 12 + q] for q in range(5)], np.int32)
+        shots.append((E.ShotParams(nx=n[0], ny=n[1], nz=n[2], nstep=steps, dt=1e-3, npml=5, f0=25.0, t0=0.005,
+                                   src=(n[0] // 2, n[1] // 2, 12), src_kind=kind, rec=rec), *m))
+    for group in (shots, [s for s in shots if s[0].src_kind == E.SRC_FORCE]):
+        with E.Batch(group) as b:
+            b.run(20)
+            b.run(40)
+            for q, s in enumerate(group):
+                with E.Plan(*s, variant=0, schedule=1, chunk=8) as plan:
+                    plan.run(s[0].nstep)
+                    assert np.array_equal(b.seismograms(q), plan.seismograms())
+                    assert np.array_equal(b.source_trace(q), plan.source_trace())
+                    for c in range(9):
+                        assert np.array_equal(b.field(q, c), plan.field(c)), (q, c)
+
+
+@pytest.mark.parametrize("scale", [1e-36, 1e-20, 1.0, 1e30])
+def test_fp64_densities_of_any_size(built, scale):
+    """The FP64 kernels' own dt / rho quotient and, for sums of densities
+    outside its range (1e-36 and 1e30 kg/m^3 times the usual), the general
+    division, against the FP64 oracle: the tolerance of the FP64 parity tests."""
+    import oracle
+    from conftest import rel_l2
+    from ela3d_gb300 import FP64, Plan, ShotParams, media
+
+    nx, ny, nz = 37, 30, 33
+    p = ShotParams(nx=nx, ny=ny, nz=nz, nstep=40, dt=1e-3, npml=6, f0=25.0, t0=0.02, src=(18, 15, 16),
+                   rec=np.array([[10, 15, 16], [25, 20, 10]], np.int32), precision=FP64)
+    cp, cs, rho = media.anticline_layers(nx, ny, nz, depths=(8, 15, 24, 60), amp=3, sigma=8, seed=4)
+    rho = (rho.astype(np.float64) * scale).astype(np.float32)
+    want, fields = oracle.run(p, cp, cs, rho, p.nstep, fp64=True)
+    with Plan(p, cp, cs, rho) as plan:
+        plan.run(p.nstep)
+        assert np.abs(want).max() > 0 and rel_l2(plan.seismograms(fp64=True), want) < 1e-11
+        for c in range(9):
+            assert rel_l2(plan.field(c, fp64=True), fields[c]) < 1e-11, c
