@@ -104,15 +104,102 @@ __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(
 __device__ __forceinline__ float sub_rn(float a, float b) { return __fsub_rn(a, b); }
 __device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(a, b); }
 
-// dt / rho_avg of two densities: FP32 uses the hardware reciprocal-based
-// divide (<= 2 ulp from the IEEE quotient).
-__device__ __forceinline__ float dt_over_rho(float dt, float r0, float r1) {
-  return __fdividef(dt, mul_rn(add_rn(r0, r1), 0.5f));
+// The same over the V cells of a thread; operands are arrays (a value per
+// cell) or one value for all.  FP32 cells go two at a time through the packed
+// f32x2 instructions, with the same roundings: half the instructions.
+template <typename T, int V> constexpr bool kPacked = sizeof(T) == 4 && V % 2 == 0;
+struct Pair { unsigned long long v; };
+__device__ __forceinline__ Pair pair_of(float a, float b) {
+  Pair p;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(p.v) : "f"(a), "f"(b));
+  return p;
 }
-// FP64: the IEEE quotient dt / ((r0 + r1) / 2) = 2 dt / R, with fewer FP64
+template <int V> __device__ __forceinline__ Pair pair_at(const float (&a)[V], int e) { return pair_of(a[e], a[e + 1]); }
+__device__ __forceinline__ Pair pair_at(const float &a, int) { return pair_of(a, a); }
+template <typename T, int V> __device__ __forceinline__ T cell_at(const T (&a)[V], int e) { return a[e]; }
+template <typename T> __device__ __forceinline__ T cell_at(const T &a, int) { return a; }
+template <int V> __device__ __forceinline__ void put_pair(float (&d)[V], int e, Pair p) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(d[e]), "=f"(d[e + 1]) : "l"(p.v));
+}
+// d = a b + c
+template <typename T, int V, typename A, typename B, typename C>
+__device__ __forceinline__ void fma_v(T (&d)[V], const A &a, const B &b, const C &c) {
+#pragma unroll
+  for (int e = 0; e < V; e += kPacked<T, V> ? 2 : 1) {
+    if constexpr (kPacked<T, V>) {
+      Pair p;
+      asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(p.v) : "l"(pair_at(a, e).v), "l"(pair_at(b, e).v), "l"(pair_at(c, e).v));
+      put_pair(d, e, p);
+    } else {
+      d[e] = fma_rn(cell_at(a, e), cell_at(b, e), cell_at(c, e));
+    }
+  }
+}
+template <typename T, int V, typename A, typename B>
+__device__ __forceinline__ void mul_v(T (&d)[V], const A &a, const B &b) {
+#pragma unroll
+  for (int e = 0; e < V; e += kPacked<T, V> ? 2 : 1) {
+    if constexpr (kPacked<T, V>) {
+      Pair p;
+      asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(p.v) : "l"(pair_at(a, e).v), "l"(pair_at(b, e).v));
+      put_pair(d, e, p);
+    } else {
+      d[e] = mul_rn(cell_at(a, e), cell_at(b, e));
+    }
+  }
+}
+template <typename T, int V, typename A, typename B>
+__device__ __forceinline__ void add_v(T (&d)[V], const A &a, const B &b) {
+#pragma unroll
+  for (int e = 0; e < V; e += kPacked<T, V> ? 2 : 1) {
+    if constexpr (kPacked<T, V>) {
+      Pair p;
+      asm("add.rn.f32x2 %0, %1, %2;" : "=l"(p.v) : "l"(pair_at(a, e).v), "l"(pair_at(b, e).v));
+      put_pair(d, e, p);
+    } else {
+      d[e] = add_rn(cell_at(a, e), cell_at(b, e));
+    }
+  }
+}
+// d = a - b (FP32: a + (-1) b in one rounding, the same value)
+template <typename T, int V, typename A, typename B>
+__device__ __forceinline__ void sub_v(T (&d)[V], const A &a, const B &b) {
+  if constexpr (kPacked<T, V>) {
+    fma_v(d, b, T(-1), a);
+  } else {
+#pragma unroll
+    for (int e = 0; e < V; ++e) d[e] = sub_rn(cell_at(a, e), cell_at(b, e));
+  }
+}
+// the cells' west neighbours (first: the value west of cell 0) and east ones
+template <typename T, int V>
+__device__ __forceinline__ void west_of(T (&d)[V], const T (&a)[V], T first) {
+#pragma unroll
+  for (int e = 0; e < V; ++e) d[e] = e > 0 ? a[e > 0 ? e - 1 : 0] : first;
+}
+template <typename T, int V>
+__device__ __forceinline__ void east_of(T (&d)[V], const T (&a)[V], T last) {
+#pragma unroll
+  for (int e = 0; e < V; ++e) d[e] = e < V - 1 ? a[e < V - 1 ? e + 1 : e] : last;
+}
+// s <- n for the cells whose bit is set in m (all of them when `all`)
+template <typename T, int V>
+__device__ __forceinline__ void keep_masked(T (&s)[V], const T (&n)[V], unsigned m, bool all) {
+  if (V > 1 && all) {
+#pragma unroll
+    for (int e = 0; e < V; ++e) s[e] = n[e];
+  } else {
+#pragma unroll
+    for (int e = 0; e < V; ++e) s[e] = ((m >> e) & 1u) ? n[e] : s[e];
+  }
+}
+
+// dt / (R / 2), R the sum of two densities: FP32 uses the hardware
+// reciprocal-based divide (<= 2 ulp from the IEEE quotient).
+__device__ __forceinline__ float dt_over_rho(float dt, float R) { return __fdividef(dt, mul_rn(R, 0.5f)); }
+// FP64: the IEEE quotient dt / (R / 2) = 2 dt / R, with fewer FP64
 // operations than a general division: the FP64 pipe (two lanes a cycle on
-// each SM) bounds the FP64 kernels.  R = r0 + r1 is a sum of two float32 model
-// values.  Its reciprocal starts from the FP32 unit (relative error 2^-22,
+// each SM) bounds the FP64 kernels.  R is a sum of two float32 model values.  Its reciprocal starts from the FP32 unit (relative error 2^-22,
 // widened and narrowed by integer operations), takes one cubic Newton step
 // (e = 1 - R y; y (1 + e + e^2)), and the quotient one Markstein correction
 // (P. Markstein, "Computation of elementary functions on the IBM RISC
@@ -120,8 +207,8 @@ __device__ __forceinline__ float dt_over_rho(float dt, float r0, float r1) {
 // quotient, because a quotient by a 26-bit R stays 2^-27 of an ulp away from
 // the midpoints between doubles, far more than the correction's error.
 // Anything outside the normal float32 range divides as usual.
-__device__ __forceinline__ double dt_over_rho(double dt, double r0, double r1) {
-  const double R = add_rn(r0, r1), a = 2.0 * dt;
+__device__ __forceinline__ double dt_over_rho(double dt, double R) {
+  const double a = 2.0 * dt;
   const int hi = __double2hiint(R);
   // 2^-100 <= R < 2^100
   if ((unsigned)(hi - 0x39b00000) >= 0x0c800000u) return a / R;
@@ -137,27 +224,77 @@ __device__ __forceinline__ double dt_over_rho(double dt, double r0, double r1) {
 }
 
 // dt mu of the averaged shear velocity S / 2 and density R / 2:
-// dt ((R/2 S/2) S/2).  FP64 takes the halves out as one factor 1/8 (exact).
-__device__ __forceinline__ float dt_mu(float dt, float c0, float c1, float r0, float r1) {
-  const float vs = mul_rn(add_rn(c0, c1), 0.5f), rhos = mul_rn(add_rn(r0, r1), 0.5f);
-  return mul_rn(dt, mul_rn(mul_rn(rhos, vs), vs));
-}
-__device__ __forceinline__ double dt_mu(double dt, double c0, double c1, double r0, double r1) {
-  const double S = add_rn(c0, c1), R = add_rn(r0, r1);
-  return mul_rn(0.125 * dt, mul_rn(mul_rn(R, S), S));
+// dt ((R/2 S/2) S/2), the halves taken out as one factor 1/8 (exact: the
+// products only change their exponents).
+template <typename T, int V>
+__device__ __forceinline__ void dt_mu(T (&mu)[V], T dt8, const T (&c0)[V], const T (&c1)[V], const T (&r0)[V],
+                                      const T (&r1)[V]) {
+  T S[V];
+  add_v(S, c0, c1);
+  add_v(mu, r0, r1);
+  mul_v(mu, mu, S);
+  mul_v(mu, mu, S);
+  mul_v(mu, mu, dt8);
 }
 
-// dt (lambda + 2 mu) and dt lambda of one cell: lambda = rho (vp^2 - 2 vs^2).
-__device__ __forceinline__ void dt_moduli(float dt, float vp, float vs, float rho, float &l2m, float &lam) {
-  l2m = mul_rn(dt, mul_rn(mul_rn(rho, vp), vp));
-  lam = mul_rn(dt, mul_rn(rho, fma_rn(vp, vp, -mul_rn(mul_rn(2.0f, vs), vs))));
-}
-// FP64: the model's values are float32 numbers, so the squares are exact and
+// dt (lambda + 2 mu) and dt lambda: lambda = rho (vp^2 - 2 vs^2).  FP64: the
+// model's values are float32 numbers, so the squares are exact and
 // rho (vp vp) rounds to what (rho vp) vp does.
-__device__ __forceinline__ void dt_moduli(double dt, double vp, double vs, double rho, double &l2m, double &lam) {
-  const double vp2 = mul_rn(vp, vp);
-  l2m = mul_rn(dt, mul_rn(rho, vp2));
-  lam = mul_rn(dt, mul_rn(rho, fma_rn(-2.0, mul_rn(vs, vs), vp2)));
+template <typename T, int V>
+__device__ __forceinline__ void dt_moduli(T dt, const T (&vp)[V], const T (&vs)[V], const T (&rho)[V], T (&l2m)[V],
+                                          T (&lam)[V]) {
+  if constexpr (sizeof(T) == 4) {
+    mul_v(l2m, rho, vp);
+    mul_v(l2m, l2m, vp);
+    mul_v(lam, vs, T(-2));
+    mul_v(lam, lam, vs);
+    fma_v(lam, vp, vp, lam);
+  } else {
+    T vp2[V];
+    mul_v(vp2, vp, vp);
+    mul_v(l2m, rho, vp2);
+    mul_v(lam, vs, vs);
+    fma_v(lam, lam, T(-2), vp2);
+  }
+  mul_v(l2m, l2m, dt);
+  mul_v(lam, lam, rho);
+  mul_v(lam, lam, dt);
+}
+
+// v + dt / rho_avg (d1 + d2 sy + d3 sz) for the cells of the mask.  (FP32
+// divides for every cell: a branch around it costs more.  FP64 leaves out the
+// cells outside the range, whose density may be 0.)
+template <typename T, int V>
+__device__ __forceinline__ void velocity_update(T dt, T sy, T sz, const T (&r0)[V], const T (&r1)[V], const T (&d1)[V],
+                                                const T (&d2)[V], const T (&d3)[V], T (&v)[V], unsigned m, bool all) {
+  T b[V], t[V];
+  add_v(b, r0, r1);
+#pragma unroll
+  for (int e = 0; e < V; ++e)
+    if (sizeof(T) == 4 || ((m >> e) & 1u)) b[e] = dt_over_rho(dt, b[e]);
+  fma_v(t, d2, sy, d1);
+  fma_v(t, d3, sz, t);
+  fma_v(t, b, t, v);
+  keep_masked(v, t, m, all);
+}
+
+// sig + (l2m d + lam (t0 + t1)) for the cells of the mask; OWN: the product
+// with the component's own derivative d is the fused one, the other is
+// rounded first.
+template <bool OWN, typename T, int V>
+__device__ __forceinline__ void normal_stress(const T (&l2m)[V], const T (&lam)[V], const T (&d)[V], const T (&t0)[V],
+                                              const T (&t1)[V], T (&sig)[V], unsigned m, bool all) {
+  T t[V], u[V];
+  add_v(t, t0, t1);
+  if constexpr (OWN) {
+    mul_v(u, lam, t);
+    fma_v(t, l2m, d, u);
+  } else {
+    mul_v(u, l2m, d);
+    fma_v(t, lam, t, u);
+  }
+  add_v(t, t, sig);
+  keep_masked(sig, t, m, all);
 }
 
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
@@ -452,19 +589,24 @@ struct PsiSlots {
   template <bool RAW, bool AFIRST, typename A>
   __device__ __forceinline__ void apply(int axis, int v, T *p, const A &a, const A &b, const A &ik, T h,
                                         T (&d)[V]) const {
-    T q[V];
+    T q[V], x[V], t[V];
     ld_vec(reinterpret_cast<const T *>(base + (axis * 3 + v) * NT * B), q);
+    if constexpr (RAW) {
+      mul_v(x, d, h);
+    } else {
 #pragma unroll
-    for (int e = 0; e < V; ++e) {
-      const T ae = at(a, e), be = at(b, e), x = RAW ? mul_rn(d[e], h) : d[e];
-      q[e] = AFIRST ? fma_rn(ae, x, mul_rn(be, q[e])) : fma_rn(be, q[e], mul_rn(ae, x));
-      d[e] = fma_rn(x, at(ik, e), q[e]);
+      for (int e = 0; e < V; ++e) x[e] = d[e];
     }
+    if constexpr (AFIRST) {
+      mul_v(t, b, q);
+      fma_v(q, a, x, t);
+    } else {
+      mul_v(t, a, x);
+      fma_v(q, b, q, t);
+    }
+    fma_v(d, x, ik, q);
     st_vec(p, q);
   }
-  // profile value of cell e: one per cell (x) or one for the row or plane
-  static __device__ __forceinline__ T at(const T (&a)[V], int e) { return a[e]; }
-  static __device__ __forceinline__ T at(const T &a, int) { return a; }
 };
 
 // ----------------------------------------------------------- stress ----
@@ -554,6 +696,9 @@ __device__ __forceinline__ bool stress_item(const ShotDesc<T> &sd, const Item &i
     mbits |= ((x >= 1) && (x <= nx - 1) ? 1u : 0u) << (16 + e);            // sigma_xz
     mbits |= ((y <= ny - 2) && (x <= nx - 1) ? 1u : 0u) << (24 + e);       // sigma_yz
   }
+  constexpr unsigned kCells = (1u << V) - 1;
+  const bool item_all = __all_sync(0xffffffffu, mbits == (kCells | kCells << 8 | kCells << 16 | kCells << 24));
+  const T dt8 = T(0.125) * dt;
   T *gx = psi_x + ((long long)item.k0 * ny + y) * xw + xs;
   T *gy = psi_y + ((long long)item.k0 * yw + ys) * px + xg;
   const long long dgx = (long long)ny * xw, dgy = (long long)yw * px;
@@ -662,21 +807,27 @@ __device__ __forceinline__ bool stress_item(const ShotDesc<T> &sd, const Item &i
     // included: results are the same bits whatever the compiler contracts,
     // in every tile variant and schedule.
     T exx[V], eyx[V], ezx[V], eyy[V], exy[V], ezy[V], ezz[V], exz[V], eyz[V];
+    {
+      T n[V];
+      east_of(n, vx_c, vx_e);
+      sub_v(exx, n, vx_c);
+      mul_v(exx, exx, idx);
+      west_of(n, vy_c, vy_w);
+      sub_v(eyx, vy_c, n);
+      mul_v(eyx, eyx, idx);
+      west_of(n, vz_c, vz_w);
+      sub_v(ezx, vz_c, n);
+      mul_v(ezx, ezx, idx);
+      sub_v(eyy, vy_c, vy_ym);
+      mul_v(eyy, eyy, idy);
+      sub_v(exy, vx_yp, vx_c);   // D
+      sub_v(ezy, vz_yp, vz_c);   // D
+      sub_v(ezz, vz_c, vz_zm);
+      mul_v(ezz, ezz, idz);
+      sub_v(exz, vx_zp, vx_c);   // D
+      sub_v(eyz, vy_zp, vy_c);   // D
 #pragma unroll
-    for (int e = 0; e < V; ++e) {
-      const T vx_xp = (e < V - 1) ? vx_c[e + 1] : vx_e;
-      const T vy_xm = (e > 0) ? vy_c[e - 1] : vy_w;
-      const T vz_xm = (e > 0) ? vz_c[e - 1] : vz_w;
-      exx[e] = mul_rn(sub_rn(vx_xp, vx_c[e]), idx);
-      eyx[e] = mul_rn(sub_rn(vy_c[e], vy_xm), idx);
-      ezx[e] = mul_rn(sub_rn(vz_c[e], vz_xm), idx);
-      eyy[e] = mul_rn(sub_rn(vy_c[e], vy_ym[e]), idy);
-      exy[e] = sub_rn(vx_yp[e], vx_c[e]);   // D
-      ezy[e] = sub_rn(vz_yp[e], vz_c[e]);   // D
-      ezz[e] = mul_rn(sub_rn(vz_c[e], vz_zm[e]), idz);
-      exz[e] = sub_rn(vx_zp[e], vx_c[e]);   // D
-      eyz[e] = sub_rn(vy_zp[e], vy_c[e]);   // D
-      vz_zm[e] = vz_c[e];
+      for (int e = 0; e < V; ++e) vz_zm[e] = vz_c[e];
     }
     // C-PML terms, only for the cells inside a slab (elsewhere a = 0 and
     // 1/K = 1 and the terms are exact no-ops).  Memory variables are updated
@@ -705,56 +856,54 @@ __device__ __forceinline__ bool stress_item(const ShotDesc<T> &sd, const Item &i
     }
     if (!last) fetch_psi(k + 1, gx + dgx, gy + dgy);
 
-    // normal stresses, simpelmodel.cpp:378-413: c + (p * u + q * w), which
-    // product is rounded first by template (X, Y, Z: the modulus times the
-    // component's own derivative is the fused one)
-    auto normal = [&](auto X, auto Y, auto Z) {
-      constexpr bool fx = decltype(X)::value, fy = decltype(Y)::value, fz = decltype(Z)::value;
-#pragma unroll
-      for (int e = 0; e < V; ++e) {
-        T DT_l2m, DT_l;
-        dt_moduli(dt, cp_c[e], cs_c[e], rho_c[e], DT_l2m, DT_l);
-        const T tx = add_rn(eyy[e], ezz[e]), ty = add_rn(exx[e], ezz[e]), tz = add_rn(exx[e], eyy[e]);
-        auto two = [&](auto own, T d, T t) {
-          return decltype(own)::value ? fma_rn(DT_l2m, d, mul_rn(DT_l, t)) : fma_rn(DT_l, t, mul_rn(DT_l2m, d));
-        };
-        if ((mk >> (0 + e)) & 1u) {
-          sxx[e] = add_rn(two(std::bool_constant<fx>{}, exx[e], tx), sxx[e]);
-          syy[e] = add_rn(two(std::bool_constant<fy>{}, eyy[e], ty), syy[e]);
-          szz[e] = add_rn(two(std::bool_constant<fz>{}, ezz[e], tz), szz[e]);
-        }
-      }
-    };
-    constexpr std::true_type own{};
-    constexpr std::false_type other{};
-    if (!F32) normal(own, own, own);
-    else if (plane_z) normal(own, own, other);
-    else if (row_y) normal(own, other, own);
-    else normal(other, own, own);
+    // normal stresses, simpelmodel.cpp:378-413
+    const bool all = item_all && k >= 1;   // no cell of the warp is outside the ranges
+    T DT_l2m[V], DT_l[V];
+    dt_moduli(dt, cp_c, cs_c, rho_c, DT_l2m, DT_l);
+    if (!F32) {
+      normal_stress<true>(DT_l2m, DT_l, exx, eyy, ezz, sxx, mk, all);
+      normal_stress<true>(DT_l2m, DT_l, eyy, exx, ezz, syy, mk, all);
+      normal_stress<true>(DT_l2m, DT_l, ezz, exx, eyy, szz, mk, all);
+    } else if (plane_z) {
+      normal_stress<true>(DT_l2m, DT_l, exx, eyy, ezz, sxx, mk, all);
+      normal_stress<true>(DT_l2m, DT_l, eyy, exx, ezz, syy, mk, all);
+      normal_stress<false>(DT_l2m, DT_l, ezz, exx, eyy, szz, mk, all);
+    } else if (row_y) {
+      normal_stress<true>(DT_l2m, DT_l, exx, eyy, ezz, sxx, mk, all);
+      normal_stress<false>(DT_l2m, DT_l, eyy, exx, ezz, syy, mk, all);
+      normal_stress<true>(DT_l2m, DT_l, ezz, exx, eyy, szz, mk, all);
+    } else {
+      normal_stress<false>(DT_l2m, DT_l, exx, eyy, ezz, sxx, mk, all);
+      normal_stress<true>(DT_l2m, DT_l, eyy, exx, ezz, syy, mk, all);
+      normal_stress<true>(DT_l2m, DT_l, ezz, exx, eyy, szz, mk, all);
+    }
 
-#pragma unroll
-    for (int e = 0; e < V; ++e) {
-      const T cs_xm = (e > 0) ? cs_c[e - 1] : cs_w;
-      const T rho_xm = (e > 0) ? rho_c[e - 1] : rho_w;
-      // sigma_xy, :416-442
-      {
-        const T mu = dt_mu(dt, cs_xm, cs_yp[e], rho_xm, rho_yp[e]);
-        if ((mk >> (8 + e)) & 1u) sxy[e] = fma_rn(mu, fma_rn(exy[e], sy, eyx[e]), sxy[e]);
+    // the shear stresses: sigma_xy :416-442, sigma_xz :445-471 (z+1 of plane
+    // nz-1 is the zero plane), sigma_yz :473-498
+    {
+      T cw[V], rw[V], mu[V], t[V];
+      west_of(cw, cs_c, cs_w);
+      west_of(rw, rho_c, rho_w);
+      dt_mu(mu, dt8, cw, cs_yp, rw, rho_yp);
+      fma_v(t, exy, sy, eyx);
+      fma_v(t, mu, t, sxy);
+      keep_masked(sxy, t, mk >> 8, all);
+      dt_mu(mu, dt8, cw, cs_zp, rw, rho_zp);
+      fma_v(t, exz, sz, ezx);
+      fma_v(t, mu, t, sxz);
+      keep_masked(sxz, t, mk >> 16, all);
+      dt_mu(mu, dt8, cs_yp, cs_zp, rho_yp, rho_zp);
+      // (a derivative whose C-PML term was applied has S = 1, and its
+      // product with S is exact)
+      if (F32 ? row_y : !plane_z) {
+        mul_v(t, ezy, sy);
+        fma_v(t, eyz, sz, t);
+      } else {
+        mul_v(t, eyz, sz);
+        fma_v(t, ezy, sy, t);
       }
-      // sigma_xz, :445-471 (z+1 of plane nz-1 is the zero plane)
-      {
-        const T mu = dt_mu(dt, cs_xm, cs_zp[e], rho_xm, rho_zp[e]);
-        if ((mk >> (16 + e)) & 1u) sxz[e] = fma_rn(mu, fma_rn(exz[e], sz, ezx[e]), sxz[e]);
-      }
-      // sigma_yz, :473-498
-      {
-        const T mu = dt_mu(dt, cs_yp[e], cs_zp[e], rho_yp[e], rho_zp[e]);
-        // (a derivative whose C-PML term was applied has S = 1, and its
-        // product with S is exact)
-        const bool z_fused = F32 ? row_y : !plane_z;
-        const T t = z_fused ? fma_rn(eyz[e], sz, mul_rn(ezy[e], sy)) : fma_rn(ezy[e], sy, mul_rn(eyz[e], sz));
-        if ((mk >> (24 + e)) & 1u) syz[e] = fma_rn(mu, t, syz[e]);
-      }
+      fma_v(t, mu, t, syz);
+      keep_masked(syz, t, mk >> 24, all);
     }
 
     if (live) {
@@ -911,6 +1060,8 @@ __device__ __forceinline__ bool velocity_item(const ShotDesc<T> &sd, const Item 
     mbits |= ((y <= ny - 2) && (x <= nx - 2) ? 1u : 0u) << (8 + e);         // vy (with k >= 1)
     mbits |= ((y >= 1) && (x <= nx - 2) ? 1u : 0u) << (16 + e);             // vz (with k <= nz-2)
   }
+  constexpr unsigned kCells = (1u << V) - 1;
+  const bool item_all = __all_sync(0xffffffffu, mbits == (kCells | kCells << 8 | kCells << 16));
   T *gx = psi_x + ((long long)item.k0 * ny + y) * xw + xs;
   T *gy = psi_y + ((long long)item.k0 * yw + ys) * px + xg;
   const long long dgx = (long long)ny * xw, dgy = (long long)yw * px;
@@ -995,22 +1146,28 @@ __device__ __forceinline__ bool velocity_item(const ShotDesc<T> &sd, const Item 
     // y and z as plain differences with a factor, roundings written out (as
     // in the stress half-step)
     T x1[V], x2[V], x3[V], y1[V], y2[V], y3[V], z1[V], z2[V], z3[V];
+    {
+      T n[V];
+      west_of(n, sxx_c, sxx_w);
+      sub_v(x1, sxx_c, n);
+      mul_v(x1, x1, idx);
+      sub_v(x2, sxy_c, sxy_ym);
+      sub_v(x3, sxz_c, sxz_zm);
+      east_of(n, sxy_c, sxy_e);
+      sub_v(y1, n, sxy_c);
+      mul_v(y1, y1, idx);
+      sub_v(y2, syy_yp, syy_c);
+      sub_v(y3, syz_c, syz_zm);
+      east_of(n, sxz_c, sxz_e);
+      sub_v(z1, n, sxz_c);
+      mul_v(z1, z1, idx);
+      sub_v(z2, syz_c, syz_ym);
+      sub_v(z3, szz_zp, szz_c);
 #pragma unroll
-    for (int e = 0; e < V; ++e) {
-      const T sxx_xm = (e > 0) ? sxx_c[e - 1] : sxx_w;
-      const T sxy_xp = (e < V - 1) ? sxy_c[e + 1] : sxy_e;
-      const T sxz_xp = (e < V - 1) ? sxz_c[e + 1] : sxz_e;
-      x1[e] = mul_rn(sub_rn(sxx_c[e], sxx_xm), idx);
-      x2[e] = sub_rn(sxy_c[e], sxy_ym[e]);
-      x3[e] = sub_rn(sxz_c[e], sxz_zm[e]);
-      y1[e] = mul_rn(sub_rn(sxy_xp, sxy_c[e]), idx);
-      y2[e] = sub_rn(syy_yp[e], syy_c[e]);
-      y3[e] = sub_rn(syz_c[e], syz_zm[e]);
-      z1[e] = mul_rn(sub_rn(sxz_xp, sxz_c[e]), idx);
-      z2[e] = sub_rn(syz_c[e], syz_ym[e]);
-      z3[e] = sub_rn(szz_zp[e], szz_c[e]);
-      sxz_zm[e] = sxz_c[e];
-      syz_zm[e] = syz_c[e];
+      for (int e = 0; e < V; ++e) {
+        sxz_zm[e] = sxz_c[e];
+        syz_zm[e] = syz_c[e];
+      }
     }
     // C-PML terms only inside the slabs; memory variables updated whether or
     // not the cell's velocity is (as in the stress half-step)
@@ -1036,20 +1193,12 @@ __device__ __forceinline__ bool velocity_item(const ShotDesc<T> &sd, const Item 
     }
     if (!last) fetch_psi(k + 1, gx + dgx, gy + dgy);
 
-    auto update = [&](bool m, T r0, T r1, T d1, T d2, T d3, T &v) {
-      // (FP32 divides for every cell: a branch around it costs more.  FP64
-      // leaves out the cells outside the range, whose density may be 0.)
-      T b = T(0);
-      if (F32 || m) b = dt_over_rho(dt, r0, r1);
-      if (m) v = fma_rn(b, fma_rn(d3, sz, fma_rn(d2, sy, d1)), v);
-    };
-#pragma unroll
-    for (int e = 0; e < V; ++e) {
-      const T rho_xm = (e > 0) ? rho_c[e - 1] : rho_w;
-      update((mk >> (0 + e)) & 1u, rho_c[e], rho_xm, x1[e], x2[e], x3[e], vx[e]);          // simpelmodel.cpp:502-530
-      update((mk >> (8 + e)) & 1u, rho_c[e], rho_yp[e], y1[e], y2[e], y3[e], vy[e]);       // :532-559
-      update((mk >> (16 + e)) & 1u, rho_c[e], rho_zp[e], z1[e], z2[e], z3[e], vz[e]);      // :563-590
-    }
+    const bool all = item_all && k >= 1 && k <= nz - 2;   // no cell of the warp is outside the ranges
+    T rw[V];
+    west_of(rw, rho_c, rho_w);
+    velocity_update(dt, sy, sz, rho_c, rw, x1, x2, x3, vx, mk, all);              // simpelmodel.cpp:502-530
+    velocity_update(dt, sy, sz, rho_c, rho_yp, y1, y2, y3, vy, mk >> 8, all);     // :532-559
+    velocity_update(dt, sy, sz, rho_c, rho_zp, z1, z2, z3, vz, mk >> 16, all);    // :563-590
 
     // receivers in this warp's cells (velocity after the update, :593-602)
     if (rlo < rhi)
