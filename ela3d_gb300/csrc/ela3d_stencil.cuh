@@ -64,7 +64,10 @@ struct Geo {
   static constexpr int S_CP = S_RHO + sz(W1);
   static constexpr int S_SIG = S_CP + sz(C);  // six centre boxes follow
   static constexpr int S_STAGE = S_SIG + 6 * sz(C);
-  static constexpr int S_TX = (int)sizeof(T) * (5 * W1 + 7 * C);
+  // bytes of the two parts a stage is loaded in: what the plane below also
+  // needs (vx vy cs rho, as its z+1 neighbours), and the rest
+  static constexpr int S_TXA = (int)sizeof(T) * 4 * W1;
+  static constexpr int S_TXB = (int)sizeof(T) * (W1 + 7 * C);
   // velocity stage
   static constexpr int V_SXX = 0;                 // W0
   static constexpr int V_SYY = V_SXX + sz(W0);    // Y1
@@ -75,15 +78,17 @@ struct Geo {
   static constexpr int V_RHO = V_SYZ + sz(Y1);    // W1
   static constexpr int V_V = V_RHO + sz(W1);      // vx vy vz (C)
   static constexpr int V_STAGE = V_V + 3 * sz(C);
-  static constexpr int V_TX = (int)sizeof(T) * (2 * W0 + 2 * Y1 + 4 * C + 2 * W1);
+  static constexpr int V_TXA = (int)sizeof(T) * (C + W1);   // szz, rho
+  static constexpr int V_TXB = (int)sizeof(T) * (2 * W0 + 2 * Y1 + 3 * C + W1);
   // memory-variable slots (PsiSlots): one 16-byte (or smaller) vector per
   // consumer thread for each of the three variables of each axis
   static constexpr int PSI_BYTES = 9 * NT * VEC * (int)sizeof(T);
-  // mbarriers (full[NS], empty[NS]) live after the stages, so the TMA
+  // mbarriers (full[2][NS], empty[NS]) live after the stages, so the TMA
   // destinations start at the (aligned) base of dynamic shared memory; the
   // memory-variable slots follow them
-  static constexpr int S_PSI = al(NS * S_STAGE + 16 * NS);
-  static constexpr int V_PSI = al(NS * V_STAGE + 16 * NS);
+  static constexpr int BARS = 24 * NS;
+  static constexpr int S_PSI = al(NS * S_STAGE + BARS);
+  static constexpr int V_PSI = al(NS * V_STAGE + BARS);
   static constexpr int S_SMEM = S_PSI + PSI_BYTES;
   static constexpr int V_SMEM = V_PSI + PSI_BYTES;
 };
@@ -392,7 +397,11 @@ __device__ __forceinline__ void copy_box_async(unsigned char *dst, const T *base
 // goes to stage n % NS; before reusing a stage lane 0 waits for the
 // consumers' release of load n - NS on that stage's empty barrier.  Item i
 // contributes planes k0 .. k1 (k1 is the look-ahead plane, possibly nz,
-// which the TMA fills with zeros).
+// which the TMA fills with zeros).  A stage has two full barriers: full[s] for
+// the part that the plane below reads too, full[NS + s] for the rest.  The
+// consumers of plane k wait for the rest of k and the first part of k + 1, so
+// the rest of k + 1 has a plane's time more to arrive, and the look-ahead
+// plane's rest is not loaded at all.
 // With ASYNC every lane copies a share of each plane's boxes (cp.async)
 // instead of lane 0 issuing TMA loads.
 template <int NS, bool ASYNC, typename Issue, typename Prefetch>
@@ -403,7 +412,7 @@ __device__ __forceinline__ bool produce_item(const Item &it, unsigned &n, uint64
     int good = 1;
     if (lane == 0 && n >= NS) good = mbar_wait_bounded(&empty[slot], (uint32_t)(((n / NS) - 1) & 1));
     if (!__shfl_sync(0xffffffffu, good, 0)) return false;
-    if (ASYNC || lane == 0) issue(it, k, slot, &full[slot], lane);
+    if (ASYNC || lane == 0) issue(it, k, slot, &full[slot], &full[NS + slot], k == it.k1, lane);
     prefetch.plane(k);
   }
   return true;
@@ -418,7 +427,8 @@ __device__ __forceinline__ void produce_drain(unsigned n, bool ok, uint64_t *ful
   if (lane != 0) return;
   if (!ok) atomicOr(err, DEV_ERR_TIMEOUT);
   for (unsigned q = (n > NS ? n - NS : 0); q < n; ++q)
-    mbar_wait_bounded(&full[q % NS], (uint32_t)((q / NS) & 1), 200000000ull);
+    for (int part = 0; part < 2; ++part)
+      mbar_wait_bounded(&full[part * NS + q % NS], (uint32_t)((q / NS) & 1), 200000000ull);
 }
 
 template <int NS, bool ASYNC, typename Issue, typename Prefetch>
@@ -452,12 +462,13 @@ struct ItemPrefetch {
 };
 
 // ------------------------------------------------------- stage loads ----
-// One stress plane: vx vy vz cs rho with their halos, cp and the six
-// stresses of the tile (box shapes in ela3d_device.cuh, ShotMaps).
+// One stress plane.  First part: vx vy cs rho with their halos; the rest: vz
+// with its halo, cp and the six stresses of the tile (box shapes in
+// ela3d_device.cuh, ShotMaps).  `ahead`: the look-ahead plane, first part only.
 template <typename T, int TX, int TY, int NS, int CPT, int MB, int LOAD>
 __device__ __forceinline__ void stress_issue(const ShotDesc<T> *__restrict__ shots,
                                              const ShotMaps *__restrict__ maps, const Item &it, int k,
-                                             unsigned char *st, uint64_t *bar, int lane) {
+                                             unsigned char *st, uint64_t *bar, uint64_t *rest, bool ahead, int lane) {
   using G = Geo<T, TX, TY, NS, CPT, MB>;
   constexpr int H = G::H;
   const int txs = tiles_x_of(shots[it.shot], TX);
@@ -466,74 +477,94 @@ __device__ __forceinline__ void stress_issue(const ShotDesc<T> *__restrict__ sho
     const ShotDesc<T> &sd = shots[it.shot];
     copy_box_async<T, TX + H, TY + 1>(st + G::S_VX, sd.f[0], sd, x0, y0, k, lane);
     copy_box_async<T, TX + H, TY + 1>(st + G::S_VY, sd.f[1], sd, x0 - H, y0 - 1, k, lane);
-    copy_box_async<T, TX + H, TY + 1>(st + G::S_VZ, sd.f[2], sd, x0 - H, y0, k, lane);
     copy_box_async<T, TX + H, TY + 1>(st + G::S_CS, sd.cs, sd, x0 - H, y0, k, lane);
     copy_box_async<T, TX + H, TY + 1>(st + G::S_RHO, sd.rho, sd, x0 - H, y0, k, lane);
-    copy_box_async<T, TX, TY>(st + G::S_CP, sd.cp, sd, x0, y0, k, lane);
-#pragma unroll
-    for (int c = 0; c < 6; ++c) copy_box_async<T, TX, TY>(st + G::S_SIG + c * G::SC, sd.f[3 + c], sd, x0, y0, k, lane);
     cp_async_arrive_noinc(bar);
+    if (!ahead) {
+      copy_box_async<T, TX + H, TY + 1>(st + G::S_VZ, sd.f[2], sd, x0 - H, y0, k, lane);
+      copy_box_async<T, TX, TY>(st + G::S_CP, sd.cp, sd, x0, y0, k, lane);
+#pragma unroll
+      for (int c = 0; c < 6; ++c)
+        copy_box_async<T, TX, TY>(st + G::S_SIG + c * G::SC, sd.f[3 + c], sd, x0, y0, k, lane);
+    }
+    cp_async_arrive_noinc(rest);
     return;
   }
   const CUtensorMap *m = maps[it.shot].stress;
-  mbar_arrive_expect_tx(bar, G::S_TX);
+  mbar_arrive_expect_tx(bar, G::S_TXA);
   tma_load_3d(st + G::S_VX, &m[0], x0, y0, k, bar);
   tma_load_3d(st + G::S_VY, &m[1], x0 - H, y0 - 1, k, bar);
-  tma_load_3d(st + G::S_VZ, &m[2], x0 - H, y0, k, bar);
   tma_load_3d(st + G::S_CS, &m[3], x0 - H, y0, k, bar);
   tma_load_3d(st + G::S_RHO, &m[4], x0 - H, y0, k, bar);
-  tma_load_3d(st + G::S_CP, &m[5], x0, y0, k, bar);
+  if (ahead) {
+    mbar_arrive(rest);
+    return;
+  }
+  mbar_arrive_expect_tx(rest, G::S_TXB);
+  tma_load_3d(st + G::S_VZ, &m[2], x0 - H, y0, k, rest);
+  tma_load_3d(st + G::S_CP, &m[5], x0, y0, k, rest);
 #pragma unroll
-  for (int c = 0; c < 6; ++c) tma_load_3d(st + G::S_SIG + c * G::SC, &m[6 + c], x0, y0, k, bar);
+  for (int c = 0; c < 6; ++c) tma_load_3d(st + G::S_SIG + c * G::SC, &m[6 + c], x0, y0, k, rest);
 }
 
-// One velocity plane: the six stresses with the halos the divergence needs,
-// rho with its halo, and vx vy vz of the tile.
+// One velocity plane.  First part: szz and rho (with its halo); the rest: the
+// other stresses with the halos the divergence needs, and vx vy vz of the tile.
 template <typename T, int TX, int TY, int NS, int CPT, int MB, int LOAD>
 __device__ __forceinline__ void velocity_issue(const ShotDesc<T> *__restrict__ shots,
                                                const ShotMaps *__restrict__ maps, const Item &it, int k,
-                                               unsigned char *st, uint64_t *bar, int lane) {
+                                               unsigned char *st, uint64_t *bar, uint64_t *rest, bool ahead,
+                                               int lane) {
   using G = Geo<T, TX, TY, NS, CPT, MB>;
   constexpr int H = G::H;
   const int txs = tiles_x_of(shots[it.shot], TX);
   const int x0 = (it.tile % txs) * TX, y0 = (it.tile / txs) * TY;
   if constexpr (LOAD == LOAD_CP_ASYNC) {
     const ShotDesc<T> &sd = shots[it.shot];
-    copy_box_async<T, TX + H, TY>(st + G::V_SXX, sd.f[3], sd, x0 - H, y0, k, lane);
-    copy_box_async<T, TX, TY + 1>(st + G::V_SYY, sd.f[4], sd, x0, y0, k, lane);
     copy_box_async<T, TX, TY>(st + G::V_SZZ, sd.f[5], sd, x0, y0, k, lane);
-    copy_box_async<T, TX + H, TY + 1>(st + G::V_SXY, sd.f[6], sd, x0, y0 - 1, k, lane);
-    copy_box_async<T, TX + H, TY>(st + G::V_SXZ, sd.f[7], sd, x0, y0, k, lane);
-    copy_box_async<T, TX, TY + 1>(st + G::V_SYZ, sd.f[8], sd, x0, y0 - 1, k, lane);
     copy_box_async<T, TX + H, TY + 1>(st + G::V_RHO, sd.rho, sd, x0 - H, y0, k, lane);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) copy_box_async<T, TX, TY>(st + G::V_V + c * G::SC, sd.f[c], sd, x0, y0, k, lane);
     cp_async_arrive_noinc(bar);
+    if (!ahead) {
+      copy_box_async<T, TX + H, TY>(st + G::V_SXX, sd.f[3], sd, x0 - H, y0, k, lane);
+      copy_box_async<T, TX, TY + 1>(st + G::V_SYY, sd.f[4], sd, x0, y0, k, lane);
+      copy_box_async<T, TX + H, TY + 1>(st + G::V_SXY, sd.f[6], sd, x0, y0 - 1, k, lane);
+      copy_box_async<T, TX + H, TY>(st + G::V_SXZ, sd.f[7], sd, x0, y0, k, lane);
+      copy_box_async<T, TX, TY + 1>(st + G::V_SYZ, sd.f[8], sd, x0, y0 - 1, k, lane);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) copy_box_async<T, TX, TY>(st + G::V_V + c * G::SC, sd.f[c], sd, x0, y0, k, lane);
+    }
+    cp_async_arrive_noinc(rest);
     return;
   }
   const CUtensorMap *m = maps[it.shot].vel;
-  mbar_arrive_expect_tx(bar, G::V_TX);
-  tma_load_3d(st + G::V_SXX, &m[0], x0 - H, y0, k, bar);
-  tma_load_3d(st + G::V_SYY, &m[1], x0, y0, k, bar);
+  mbar_arrive_expect_tx(bar, G::V_TXA);
   tma_load_3d(st + G::V_SZZ, &m[2], x0, y0, k, bar);
-  tma_load_3d(st + G::V_SXY, &m[3], x0, y0 - 1, k, bar);
-  tma_load_3d(st + G::V_SXZ, &m[4], x0, y0, k, bar);
-  tma_load_3d(st + G::V_SYZ, &m[5], x0, y0 - 1, k, bar);
   tma_load_3d(st + G::V_RHO, &m[6], x0 - H, y0, k, bar);
+  if (ahead) {
+    mbar_arrive(rest);
+    return;
+  }
+  mbar_arrive_expect_tx(rest, G::V_TXB);
+  tma_load_3d(st + G::V_SXX, &m[0], x0 - H, y0, k, rest);
+  tma_load_3d(st + G::V_SYY, &m[1], x0, y0, k, rest);
+  tma_load_3d(st + G::V_SXY, &m[3], x0, y0 - 1, k, rest);
+  tma_load_3d(st + G::V_SXZ, &m[4], x0, y0, k, rest);
+  tma_load_3d(st + G::V_SYZ, &m[5], x0, y0 - 1, k, rest);
 #pragma unroll
-  for (int c = 0; c < 3; ++c) tma_load_3d(st + G::V_V + c * G::SC, &m[7 + c], x0, y0, k, bar);
+  for (int c = 0; c < 3; ++c) tma_load_3d(st + G::V_V + c * G::SC, &m[7 + c], x0, y0, k, rest);
 }
 
-// Waits for the stages of loads n and n+1 (planes k and k+1); load n was
-// already waited for as the previous plane's k+1 unless k is the first plane
-// of its work item.  False when a wait passed its limit; the caller records
-// the timeout and returns.
+// Waits for the whole stage of load n (plane k) and the first part of load
+// n+1 (plane k+1); load n's first part was already waited for as the previous
+// plane's k+1 unless k is the first plane of its work item.  False when a wait
+// passed its limit; the caller records the timeout and returns.
 template <int NS>
 __device__ __forceinline__ bool wait_planes(uint64_t *full, unsigned n, bool first, unsigned long long wait_ns,
                                             unsigned *err, int lane) {
   const int s0 = (int)(n % NS), s1 = (int)((n + 1) % NS);
-  bool ok = !first || mbar_wait_bounded(&full[s0], (uint32_t)((n / NS) & 1), wait_ns);
-  ok = ok && mbar_wait_bounded(&full[s1], (uint32_t)(((n + 1) / NS) & 1), wait_ns);
+  const uint32_t p0 = (uint32_t)((n / NS) & 1), p1 = (uint32_t)(((n + 1) / NS) & 1);
+  bool ok = !first || mbar_wait_bounded(&full[s0], p0, wait_ns);
+  ok = ok && mbar_wait_bounded(&full[NS + s0], p0, wait_ns);
+  ok = ok && mbar_wait_bounded(&full[s1], p1, wait_ns);
   if (__any_sync(0xffffffffu, !ok)) {
     if (lane == 0) atomicOr(err, DEV_ERR_TIMEOUT);
     return false;
@@ -1244,14 +1275,15 @@ __device__ __forceinline__ bool velocity_item(const ShotDesc<T> &sd, const Item 
 }
 
 // ------------------------------------------------- half-step kernels ----
-// Barrier set-up shared by the kernels: full[s] expects the producer's one
-// arrival plus the stage's bytes (TMA) or one arrival per lane (cp.async);
-// empty[s] one arrival per consumer warp.
+// Barrier set-up shared by the kernels: full[s] and full[NS + s] (the parts of
+// a stage) expect the producer's one arrival plus the part's bytes (TMA) or
+// one arrival per lane (cp.async); empty[s] one arrival per consumer warp.
 template <int NS, int NCW, int LOAD>
 __device__ __forceinline__ void init_ring(uint64_t *full, uint64_t *empty) {
   if (threadIdx.x == 0) {
     for (int s = 0; s < NS; ++s) {
       mbar_init(&full[s], LOAD == LOAD_TMA ? 1 : 32);
+      mbar_init(&full[NS + s], LOAD == LOAD_TMA ? 1 : 32);
       mbar_init(&empty[s], NCW);
     }
     fence_mbar_init();
@@ -1269,7 +1301,7 @@ __global__ void __launch_bounds__(Geo<T, TX, TY, NS, CPT, MB>::THREADS, Geo<T, T
   using G = Geo<T, TX, TY, NS, CPT, MB>;
   extern __shared__ __align__(1024) unsigned char smem[];
   uint64_t *full = reinterpret_cast<uint64_t *>(smem + NS * G::S_STAGE);
-  uint64_t *empty = full + NS;
+  uint64_t *empty = full + 2 * NS;
 
   const int tid = threadIdx.x;
   const int2 range = ranges[blockIdx.x];
@@ -1277,8 +1309,8 @@ __global__ void __launch_bounds__(Geo<T, TX, TY, NS, CPT, MB>::THREADS, Geo<T, T
   init_ring<NS, G::NCW, LOAD>(full, empty);
 
   if (tid >= G::NT) {  // producer warp
-    auto issue = [&](const Item &it, int k, int slot, uint64_t *bar, int lane) {
-      stress_issue<T, TX, TY, NS, CPT, MB, LOAD>(shots, maps, it, k, smem + slot * G::S_STAGE, bar, lane);
+    auto issue = [&](const Item &it, int k, int slot, uint64_t *bar, uint64_t *rest, bool ahead, int lane) {
+      stress_issue<T, TX, TY, NS, CPT, MB, LOAD>(shots, maps, it, k, smem + slot * G::S_STAGE, bar, rest, ahead, lane);
     };
     ItemPrefetch<T, TX, TY> prefetch{{}, shots, tid - G::NT, ctl, PSI_S0};
     produce<NS, LOAD == LOAD_CP_ASYNC>(items, range, full, empty, issue, prefetch, err, ctl, tid - G::NT);
@@ -1303,7 +1335,7 @@ __global__ void __launch_bounds__(Geo<T, TX, TY, NS, CPT, MB>::THREADS, Geo<T, T
   using G = Geo<T, TX, TY, NS, CPT, MB>;
   extern __shared__ __align__(1024) unsigned char smem[];
   uint64_t *full = reinterpret_cast<uint64_t *>(smem + NS * G::V_STAGE);
-  uint64_t *empty = full + NS;
+  uint64_t *empty = full + 2 * NS;
 
   const int tid = threadIdx.x;
   const int2 range = ranges[blockIdx.x];
@@ -1311,8 +1343,8 @@ __global__ void __launch_bounds__(Geo<T, TX, TY, NS, CPT, MB>::THREADS, Geo<T, T
   init_ring<NS, G::NCW, LOAD>(full, empty);
 
   if (tid >= G::NT) {  // producer warp
-    auto issue = [&](const Item &it, int k, int slot, uint64_t *bar, int lane) {
-      velocity_issue<T, TX, TY, NS, CPT, MB, LOAD>(shots, maps, it, k, smem + slot * G::V_STAGE, bar, lane);
+    auto issue = [&](const Item &it, int k, int slot, uint64_t *bar, uint64_t *rest, bool ahead, int lane) {
+      velocity_issue<T, TX, TY, NS, CPT, MB, LOAD>(shots, maps, it, k, smem + slot * G::V_STAGE, bar, rest, ahead, lane);
     };
     ItemPrefetch<T, TX, TY> prefetch{{}, shots, tid - G::NT, ctl, PSI_V0};
     produce<NS, LOAD == LOAD_CP_ASYNC>(items, range, full, empty, issue, prefetch, err, ctl, tid - G::NT);
@@ -1389,7 +1421,7 @@ struct Flow {
     ShotDesc<T> sd;
   };
   static_assert(sizeof(ShotDesc<T>) % 16 == 0 && sizeof(FlowItem) % 16 == 0, "descriptors are copied 16 bytes at a time");
-  static constexpr int READY = NS * STAGE + 16 * NS;
+  static constexpr int READY = NS * STAGE + G::BARS;
   static constexpr int SLOTS = (READY + 8 * RB + 4 * RB + 15) & ~15;
   static constexpr int PSI = (SLOTS + RB * (int)sizeof(Slot) + 15) & ~15;   // memory-variable slots
   static constexpr int SMEM = PSI + G::PSI_BYTES;
@@ -1473,7 +1505,7 @@ __global__ void __launch_bounds__(Geo<T, TX, TY, NS, CPT, MB>::THREADS, Geo<T, T
   using F = Flow<T, TX, TY, NS, CPT, MB>;
   extern __shared__ __align__(1024) unsigned char smem[];
   uint64_t *full = reinterpret_cast<uint64_t *>(smem + NS * F::STAGE);
-  uint64_t *empty = full + NS;
+  uint64_t *empty = full + 2 * NS;
   uint64_t *ready = empty + NS;   // F::RB barriers, one per item in flight
   int *arrived = reinterpret_cast<int *>(ready + F::RB);   // F::RB consumer-warp counters
   typename F::Slot *slots = reinterpret_cast<typename F::Slot *>(smem + F::SLOTS);
@@ -1535,14 +1567,14 @@ __global__ void __launch_bounds__(Geo<T, TX, TY, NS, CPT, MB>::THREADS, Geo<T, T
       ok = __shfl_sync(0xffffffffu, good, 0);
       if (!ok || end) break;
       if (fi.kind == 0) {
-        auto issue = [&](const Item &it, int k, int st, uint64_t *bar, int l) {
-          stress_issue<T, TX, TY, NS, CPT, MB, LOAD_TMA>(shots, maps, it, k, smem + st * F::STAGE, bar, l);
+        auto issue = [&](const Item &it, int k, int st, uint64_t *bar, uint64_t *rest, bool ahead, int l) {
+          stress_issue<T, TX, TY, NS, CPT, MB, LOAD_TMA>(shots, maps, it, k, smem + st * F::STAGE, bar, rest, ahead, l);
         };
         pf_s.begin(fi.it, slot.sd);
         ok = produce_item<NS, false>(fi.it, n, full, empty, issue, pf_s, lane);
       } else {
-        auto issue = [&](const Item &it, int k, int st, uint64_t *bar, int l) {
-          velocity_issue<T, TX, TY, NS, CPT, MB, LOAD_TMA>(shots, maps, it, k, smem + st * F::STAGE, bar, l);
+        auto issue = [&](const Item &it, int k, int st, uint64_t *bar, uint64_t *rest, bool ahead, int l) {
+          velocity_issue<T, TX, TY, NS, CPT, MB, LOAD_TMA>(shots, maps, it, k, smem + st * F::STAGE, bar, rest, ahead, l);
         };
         pf_v.begin(fi.it, slot.sd);
         ok = produce_item<NS, false>(fi.it, n, full, empty, issue, pf_v, lane);
