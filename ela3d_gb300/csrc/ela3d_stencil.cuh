@@ -187,16 +187,13 @@ __device__ __forceinline__ void east_of(T (&d)[V], const T (&a)[V], T last) {
 #pragma unroll
   for (int e = 0; e < V; ++e) d[e] = e < V - 1 ? a[e < V - 1 ? e + 1 : e] : last;
 }
-// s <- n for the cells whose bit is set in m (all of them when `all`)
+// s <- n for the cells whose bit is set in m (selects: a branch for warps
+// without a masked cell costs more than it saves, 101^3 36.3 against 37.1
+// Gcell-updates/s)
 template <typename T, int V>
-__device__ __forceinline__ void keep_masked(T (&s)[V], const T (&n)[V], unsigned m, bool all) {
-  if (V > 1 && all) {
+__device__ __forceinline__ void keep_masked(T (&s)[V], const T (&n)[V], unsigned m) {
 #pragma unroll
-    for (int e = 0; e < V; ++e) s[e] = n[e];
-  } else {
-#pragma unroll
-    for (int e = 0; e < V; ++e) s[e] = ((m >> e) & 1u) ? n[e] : s[e];
-  }
+  for (int e = 0; e < V; ++e) s[e] = ((m >> e) & 1u) ? n[e] : s[e];
 }
 
 // dt / (R / 2), R the sum of two densities: FP32 uses the hardware
@@ -271,7 +268,7 @@ __device__ __forceinline__ void dt_moduli(T dt, const T (&vp)[V], const T (&vs)[
 // cells outside the range, whose density may be 0.)
 template <typename T, int V>
 __device__ __forceinline__ void velocity_update(T dt, T sy, T sz, const T (&r0)[V], const T (&r1)[V], const T (&d1)[V],
-                                                const T (&d2)[V], const T (&d3)[V], T (&v)[V], unsigned m, bool all) {
+                                                const T (&d2)[V], const T (&d3)[V], T (&v)[V], unsigned m) {
   T b[V], t[V];
   add_v(b, r0, r1);
 #pragma unroll
@@ -280,7 +277,7 @@ __device__ __forceinline__ void velocity_update(T dt, T sy, T sz, const T (&r0)[
   fma_v(t, d2, sy, d1);
   fma_v(t, d3, sz, t);
   fma_v(t, b, t, v);
-  keep_masked(v, t, m, all);
+  keep_masked(v, t, m);
 }
 
 // sig + (l2m d + lam (t0 + t1)) for the cells of the mask; OWN: the product
@@ -288,7 +285,7 @@ __device__ __forceinline__ void velocity_update(T dt, T sy, T sz, const T (&r0)[
 // rounded first.
 template <bool OWN, typename T, int V>
 __device__ __forceinline__ void normal_stress(const T (&l2m)[V], const T (&lam)[V], const T (&d)[V], const T (&t0)[V],
-                                              const T (&t1)[V], T (&sig)[V], unsigned m, bool all) {
+                                              const T (&t1)[V], T (&sig)[V], unsigned m) {
   T t[V], u[V];
   add_v(t, t0, t1);
   if constexpr (OWN) {
@@ -299,7 +296,7 @@ __device__ __forceinline__ void normal_stress(const T (&l2m)[V], const T (&lam)[
     fma_v(t, lam, t, u);
   }
   add_v(t, t, sig);
-  keep_masked(sig, t, m, all);
+  keep_masked(sig, t, m);
 }
 
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
@@ -562,7 +559,12 @@ __device__ __forceinline__ bool wait_planes(uint64_t *full, unsigned n, bool fir
                                             unsigned *err, int lane) {
   const int s0 = (int)(n % NS), s1 = (int)((n + 1) % NS);
   const uint32_t p0 = (uint32_t)((n / NS) & 1), p1 = (uint32_t)(((n + 1) / NS) & 1);
-  bool ok = !first || mbar_wait_bounded(&full[s0], p0, wait_ns);
+  // all three have usually completed: one vote
+  bool ok = !first || mbar_try_wait(&full[s0], p0);
+  ok &= mbar_try_wait(&full[NS + s0], p0);
+  ok &= mbar_try_wait(&full[s1], p1);
+  if (__all_sync(0xffffffffu, ok)) return true;
+  ok = !first || mbar_wait_bounded(&full[s0], p0, wait_ns);
   ok = ok && mbar_wait_bounded(&full[NS + s0], p0, wait_ns);
   ok = ok && mbar_wait_bounded(&full[s1], p1, wait_ns);
   if (__any_sync(0xffffffffu, !ok)) {
@@ -727,35 +729,32 @@ __device__ __forceinline__ bool stress_item(const ShotDesc<T> &sd, const Item &i
     mbits |= ((x >= 1) && (x <= nx - 1) ? 1u : 0u) << (16 + e);            // sigma_xz
     mbits |= ((y <= ny - 2) && (x <= nx - 1) ? 1u : 0u) << (24 + e);       // sigma_yz
   }
-  constexpr unsigned kCells = (1u << V) - 1;
-  const bool item_all = __all_sync(0xffffffffu, mbits == (kCells | kCells << 8 | kCells << 16 | kCells << 24));
   const T dt8 = T(0.125) * dt;
   T *gx = psi_x + ((long long)item.k0 * ny + y) * xw + xs;
   T *gy = psi_y + ((long long)item.k0 * yw + ys) * px + xg;
   const long long dgx = (long long)ny * xw, dgy = (long long)yw * px;
   long long g = (long long)item.k0 * plane + rowoff;
-  // the memory variables of plane k (x and y slab pointers at that plane)
+  // the memory variables of the first plane; each plane then copies the next
+  // one's as it has used its own
   const PsiSlots<T, G::NT, V> slots(psi, tid);
-  auto fetch_psi = [&](int k, const T *ax_, const T *ay_) {
-    if (in_x) slots.fetch(0, ax_ + PSI_S0 * psx, psx);
-    if (in_y) slots.fetch(1, ay_ + PSI_S0 * psy, psy);
+  auto fetch_z = [&](int k) {
     if (live && (k < zl || k >= zr)) {
       const int zs = k < zl ? k : zl + (k - zr);
       slots.fetch(2, psi_z + PSI_S0 * psz + ((long long)zs * ny + y) * px + xg, psz);
     }
   };
-  fetch_psi(item.k0, gx, gy);
+  if (in_x) slots.fetch(0, gx + PSI_S0 * psx, psx);
+  if (in_y) slots.fetch(1, gy + PSI_S0 * psy, psy);
+  fetch_z(item.k0);
   for (int k = item.k0; k < item.k1; ++k, gx += dgx, gy += dgy, g += plane) {
     // z profile first: its latency overlaps the wait
     const bool plane_z = k < zl || k >= zr;       // the plane lies in the z slab
     const bool in_z = live && plane_z;
-    const int zs = k < zl ? k : zl + (k - zr);
     T az = 0, bz = 1, ikz = 1, azh = 0, bzh = 1, ikzh = 1;
     if (in_z) {
       az = prof_z[PR_A * nz + k]; bz = prof_z[PR_B * nz + k]; ikz = prof_z[PR_IK * nz + k];
       azh = prof_z[PR_AH * nz + k]; bzh = prof_z[PR_BH * nz + k]; ikzh = prof_z[PR_IKH * nz + k];
     }
-    T *gz = psi_z + ((long long)zs * ny + y) * px + xg;
 
     if (!wait_planes<NS>(full, n, k == item.k0, wait_ns, err, lane)) {
       cp_async_wait_all();   // (no copy outlives its thread)
@@ -871,42 +870,45 @@ __device__ __forceinline__ bool stress_item(const ShotDesc<T> &sd, const Item &i
       slots.template apply<false, false>(0, 0, gx + PSI_S0 * psx, axh, bxh, ikxh, idx, exx);
       slots.template apply<false, false>(0, 1, gx + PSI_S1 * psx, ax, bx, ikx, idx, eyx);
       slots.template apply<false, false>(0, 2, gx + PSI_S2 * psx, ax, bx, ikx, idx, ezx);
+      if (!last) slots.fetch(0, gx + PSI_S0 * psx + dgx, psx);
     }
     if (in_y) {
       slots.template apply<false, F32>(1, 0, gy + PSI_S0 * psy, ay, by, iky, idy, eyy);
       slots.template apply<true, F32>(1, 1, gy + PSI_S1 * psy, ayh, byh, ikyh, idy, exy);
       slots.template apply<true, F32>(1, 2, gy + PSI_S2 * psy, ayh, byh, ikyh, idy, ezy);
+      if (!last) slots.fetch(1, gy + PSI_S0 * psy + dgy, psy);
       sy = T(1);
     }
     if (in_z) {
+      const int zs = k < zl ? k : zl + (k - zr);
+      T *gz = psi_z + ((long long)zs * ny + y) * px + xg;
       slots.template apply<false, F32>(2, 0, gz + PSI_S0 * psz, az, bz, ikz, idz, ezz);
       slots.template apply<true, F32>(2, 1, gz + PSI_S1 * psz, azh, bzh, ikzh, idz, exz);
       if (F32 && row_y) slots.template apply<true, true>(2, 2, gz + PSI_S2 * psz, azh, bzh, ikzh, idz, eyz);
       else slots.template apply<true, false>(2, 2, gz + PSI_S2 * psz, azh, bzh, ikzh, idz, eyz);
       sz = T(1);
     }
-    if (!last) fetch_psi(k + 1, gx + dgx, gy + dgy);
+    if (!last) fetch_z(k + 1);
 
     // normal stresses, simpelmodel.cpp:378-413
-    const bool all = item_all && k >= 1;   // no cell of the warp is outside the ranges
     T DT_l2m[V], DT_l[V];
     dt_moduli(dt, cp_c, cs_c, rho_c, DT_l2m, DT_l);
     if (!F32) {
-      normal_stress<true>(DT_l2m, DT_l, exx, eyy, ezz, sxx, mk, all);
-      normal_stress<true>(DT_l2m, DT_l, eyy, exx, ezz, syy, mk, all);
-      normal_stress<true>(DT_l2m, DT_l, ezz, exx, eyy, szz, mk, all);
+      normal_stress<true>(DT_l2m, DT_l, exx, eyy, ezz, sxx, mk);
+      normal_stress<true>(DT_l2m, DT_l, eyy, exx, ezz, syy, mk);
+      normal_stress<true>(DT_l2m, DT_l, ezz, exx, eyy, szz, mk);
     } else if (plane_z) {
-      normal_stress<true>(DT_l2m, DT_l, exx, eyy, ezz, sxx, mk, all);
-      normal_stress<true>(DT_l2m, DT_l, eyy, exx, ezz, syy, mk, all);
-      normal_stress<false>(DT_l2m, DT_l, ezz, exx, eyy, szz, mk, all);
+      normal_stress<true>(DT_l2m, DT_l, exx, eyy, ezz, sxx, mk);
+      normal_stress<true>(DT_l2m, DT_l, eyy, exx, ezz, syy, mk);
+      normal_stress<false>(DT_l2m, DT_l, ezz, exx, eyy, szz, mk);
     } else if (row_y) {
-      normal_stress<true>(DT_l2m, DT_l, exx, eyy, ezz, sxx, mk, all);
-      normal_stress<false>(DT_l2m, DT_l, eyy, exx, ezz, syy, mk, all);
-      normal_stress<true>(DT_l2m, DT_l, ezz, exx, eyy, szz, mk, all);
+      normal_stress<true>(DT_l2m, DT_l, exx, eyy, ezz, sxx, mk);
+      normal_stress<false>(DT_l2m, DT_l, eyy, exx, ezz, syy, mk);
+      normal_stress<true>(DT_l2m, DT_l, ezz, exx, eyy, szz, mk);
     } else {
-      normal_stress<false>(DT_l2m, DT_l, exx, eyy, ezz, sxx, mk, all);
-      normal_stress<true>(DT_l2m, DT_l, eyy, exx, ezz, syy, mk, all);
-      normal_stress<true>(DT_l2m, DT_l, ezz, exx, eyy, szz, mk, all);
+      normal_stress<false>(DT_l2m, DT_l, exx, eyy, ezz, sxx, mk);
+      normal_stress<true>(DT_l2m, DT_l, eyy, exx, ezz, syy, mk);
+      normal_stress<true>(DT_l2m, DT_l, ezz, exx, eyy, szz, mk);
     }
 
     // the shear stresses: sigma_xy :416-442, sigma_xz :445-471 (z+1 of plane
@@ -918,11 +920,11 @@ __device__ __forceinline__ bool stress_item(const ShotDesc<T> &sd, const Item &i
       dt_mu(mu, dt8, cw, cs_yp, rw, rho_yp);
       fma_v(t, exy, sy, eyx);
       fma_v(t, mu, t, sxy);
-      keep_masked(sxy, t, mk >> 8, all);
+      keep_masked(sxy, t, mk >> 8);
       dt_mu(mu, dt8, cw, cs_zp, rw, rho_zp);
       fma_v(t, exz, sz, ezx);
       fma_v(t, mu, t, sxz);
-      keep_masked(sxz, t, mk >> 16, all);
+      keep_masked(sxz, t, mk >> 16);
       dt_mu(mu, dt8, cs_yp, cs_zp, rho_yp, rho_zp);
       // (a derivative whose C-PML term was applied has S = 1, and its
       // product with S is exact)
@@ -934,7 +936,7 @@ __device__ __forceinline__ bool stress_item(const ShotDesc<T> &sd, const Item &i
         fma_v(t, ezy, sy, t);
       }
       fma_v(t, mu, t, syz);
-      keep_masked(syz, t, mk >> 24, all);
+      keep_masked(syz, t, mk >> 24);
     }
 
     if (live) {
@@ -1091,33 +1093,30 @@ __device__ __forceinline__ bool velocity_item(const ShotDesc<T> &sd, const Item 
     mbits |= ((y <= ny - 2) && (x <= nx - 2) ? 1u : 0u) << (8 + e);         // vy (with k >= 1)
     mbits |= ((y >= 1) && (x <= nx - 2) ? 1u : 0u) << (16 + e);             // vz (with k <= nz-2)
   }
-  constexpr unsigned kCells = (1u << V) - 1;
-  const bool item_all = __all_sync(0xffffffffu, mbits == (kCells | kCells << 8 | kCells << 16));
   T *gx = psi_x + ((long long)item.k0 * ny + y) * xw + xs;
   T *gy = psi_y + ((long long)item.k0 * yw + ys) * px + xg;
   const long long dgx = (long long)ny * xw, dgy = (long long)yw * px;
   long long g = (long long)item.k0 * plane + rowoff;
-  // the memory variables of plane k (x and y slab pointers at that plane)
+  // the memory variables of the first plane; each plane then copies the next
+  // one's as it has used its own
   const PsiSlots<T, G::NT, V> slots(psi, tid);
-  auto fetch_psi = [&](int k, const T *ax_, const T *ay_) {
-    if (in_x) slots.fetch(0, ax_ + PSI_V0 * psx, psx);
-    if (in_y) slots.fetch(1, ay_ + PSI_V0 * psy, psy);
+  auto fetch_z = [&](int k) {
     if (live && (k < zl || k >= zr)) {
       const int zs = k < zl ? k : zl + (k - zr);
       slots.fetch(2, psi_z + PSI_V0 * psz + ((long long)zs * ny + y) * px + xg, psz);
     }
   };
-  fetch_psi(item.k0, gx, gy);
+  if (in_x) slots.fetch(0, gx + PSI_V0 * psx, psx);
+  if (in_y) slots.fetch(1, gy + PSI_V0 * psy, psy);
+  fetch_z(item.k0);
   for (int k = item.k0; k < item.k1; ++k, gx += dgx, gy += dgy, g += plane) {
     const bool plane_z = k < zl || k >= zr;       // the plane lies in the z slab
     const bool in_z = live && plane_z;
-    const int zs = k < zl ? k : zl + (k - zr);
     T az = 0, bz = 1, ikz = 1, azh = 0, bzh = 1, ikzh = 1;
     if (in_z) {
       az = prof_z[PR_A * nz + k]; bz = prof_z[PR_B * nz + k]; ikz = prof_z[PR_IK * nz + k];
       azh = prof_z[PR_AH * nz + k]; bzh = prof_z[PR_BH * nz + k]; ikzh = prof_z[PR_IKH * nz + k];
     }
-    T *gz = psi_z + ((long long)zs * ny + y) * px + xg;
 
     int rlo = 0, rhi = 0;   // receivers of this plane
     if (item_rec) {
@@ -1209,27 +1208,30 @@ __device__ __forceinline__ bool velocity_item(const ShotDesc<T> &sd, const Item 
       slots.template apply<false, false>(0, 0, gx + PSI_V0 * psx, ax, bx, ikx, idx, x1);
       slots.template apply<false, false>(0, 1, gx + PSI_V1 * psx, axh, bxh, ikxh, idx, y1);
       slots.template apply<false, false>(0, 2, gx + PSI_V2 * psx, axh, bxh, ikxh, idx, z1);
+      if (!last) slots.fetch(0, gx + PSI_V0 * psx + dgx, psx);
     }
     if (in_y) {
       slots.template apply<true, F32>(1, 0, gy + PSI_V0 * psy, ay, by, iky, idy, x2);
       slots.template apply<true, F32>(1, 1, gy + PSI_V1 * psy, ayh, byh, ikyh, idy, y2);
       slots.template apply<true, F32>(1, 2, gy + PSI_V2 * psy, ay, by, iky, idy, z2);
+      if (!last) slots.fetch(1, gy + PSI_V0 * psy + dgy, psy);
       sy = T(1);
     }
     if (in_z) {
+      const int zs = k < zl ? k : zl + (k - zr);
+      T *gz = psi_z + ((long long)zs * ny + y) * px + xg;
       slots.template apply<true, F32>(2, 0, gz + PSI_V0 * psz, az, bz, ikz, idz, x3);
       slots.template apply<true, F32>(2, 1, gz + PSI_V1 * psz, az, bz, ikz, idz, y3);
       slots.template apply<true, F32>(2, 2, gz + PSI_V2 * psz, azh, bzh, ikzh, idz, z3);
       sz = T(1);
     }
-    if (!last) fetch_psi(k + 1, gx + dgx, gy + dgy);
+    if (!last) fetch_z(k + 1);
 
-    const bool all = item_all && k >= 1 && k <= nz - 2;   // no cell of the warp is outside the ranges
     T rw[V];
     west_of(rw, rho_c, rho_w);
-    velocity_update(dt, sy, sz, rho_c, rw, x1, x2, x3, vx, mk, all);              // simpelmodel.cpp:502-530
-    velocity_update(dt, sy, sz, rho_c, rho_yp, y1, y2, y3, vy, mk >> 8, all);     // :532-559
-    velocity_update(dt, sy, sz, rho_c, rho_zp, z1, z2, z3, vz, mk >> 16, all);    // :563-590
+    velocity_update(dt, sy, sz, rho_c, rw, x1, x2, x3, vx, mk);              // simpelmodel.cpp:502-530
+    velocity_update(dt, sy, sz, rho_c, rho_yp, y1, y2, y3, vy, mk >> 8);     // :532-559
+    velocity_update(dt, sy, sz, rho_c, rho_zp, z1, z2, z3, vz, mk >> 16);    // :563-590
 
     // receivers in this warp's cells (velocity after the update, :593-602)
     if (rlo < rhi)
