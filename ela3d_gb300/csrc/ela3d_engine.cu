@@ -459,14 +459,24 @@ TuneChoice default_choice(int fp64, int nx, int ny, int nz, bool explosive) {
   return c;
 }
 
+static int device_sms() {
+  int dev = 0, sms = 152;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
 // The tile: the share of its threads that hold cells, times a weight for its
 // shape.  Narrow tiles read more halo, which costs little while the arrays are
 // near the L2 (126 MB) and more once they stream from HBM.  Single shots,
-// Gcell-updates/s (128x7, 112x8, 64x14, 56x16, 32x28): 101^3 32.4 34.2 30.8
-// 31.2 30.7; 128^3 42.2 28.7 40.3 35.7 40.2; 160^3 33.3 35.8 38.8 41.2 42.0;
-// 192^3 37.7 40.2 43.1 38.8 43.1; 224^3 44.1 46.2 42.5 43.6 43.9; 256^3 48.5
-// 40.8 46.8 43.3 43.5; 320^3 46.3 47.6 47.6 44.0 42.3; 150x211x93 29.7 31.4
-// 34.8 35.5 37.5.  FP64 is bound by its arithmetic, and a thread without a
+// Gcell-updates/s with seven consumer warps (128x7, 112x8, 64x14, 56x16, 32x28):
+// 101^3 35.7 38.1 34.1 34.7 33.3; 128^3 43.6 29.9 43.1 37.8 42.5; 160^3 34.8
+// 37.7 40.5 42.6 43.5; 192^3 41.0 43.2 46.6 42.8 45.2; 256^3 49.0 41.2 47.4
+// 44.1 43.9; 384^3 50.2 46.8 48.8 44.2 43.3; 150x211x93 31.6 33.0 36.4 37.0
+// 39.0; with eight (128x8, 112x9, 64x16, 56x18, 32x32): 36.1 35.3 33.7 33.8
+// 30.3; 46.2 29.3 46.2 34.0 45.7; 36.0 37.2 43.0 41.9 45.2; 42.8 42.7 47.7 42.0
+// 46.1; 49.2 39.3 48.2 43.2 44.1; 50.3 46.4 49.0 43.3 43.0; 31.5 33.4 37.2
+// 37.5 40.2.  A tile that leaves fewer two-plane items than there are blocks
+// counts for less (64^3: 64x14 19.5, 64x16 17.2).  FP64 is bound by its arithmetic, and a thread without a
 // cell costs as much as one with: 101^3 with 32x7, 16x14 and 8x28 tiles (76%,
 // 81% and 88% used) 3.34, 3.65 and 3.83; 180^3 (93%, 93%, 90%) 4.57, 4.62 and
 // 4.48.  For several shots the cells' summed time decides.
@@ -475,31 +485,29 @@ static int pick_tile(const std::vector<ela3d_params> &ps, bool fp64, bool stream
   const Variant *v = variants(&n);
   const struct { bool fp64; int tx, ty; double w; } shapes[] = {
       {false, 128, 7, 1.0}, {false, 112, 8, 0.985}, {false, 64, 14, 0.96}, {false, 56, 16, streams ? 0.88 : 0.93},
-      {false, 32, 28, streams ? 0.85 : 0.98}, {true, 32, 7, 1.0}, {true, 16, 14, 1.0}, {true, 8, 28, 1.0}};
+      {false, 32, 28, streams ? 0.85 : 0.98}, {false, 128, 8, 1.01}, {false, 112, 9, 0.99}, {false, 64, 16, 0.975},
+      {false, 56, 18, streams ? 0.88 : 0.94}, {false, 32, 32, streams ? 0.86 : 1.0}, {true, 32, 7, 1.0}, {true, 16, 14, 1.0}, {true, 8, 28, 1.0}};
+  const double sms = device_sms();
   int pick = fallback;
   double best = 0.0;
   for (const auto &s : shapes)
     for (int j = 0; j < n && s.fp64 == fp64; ++j) {
       if ((v[j].fp64 != 0) != fp64 || v[j].loads != LOAD_TMA || !v[j].flow || v[j].tx != s.tx || v[j].ty != s.ty)
         continue;
-      double cells = 0.0, taken = 0.0;
+      double cells = 0.0, taken = 0.0, items = 0.0;
       for (const ela3d_params &p : ps) {
         cells += (double)p.nx * p.ny * p.nz;
-        taken += (double)((p.nx + s.tx - 1) / s.tx * s.tx) * ((p.ny + s.ty - 1) / s.ty * s.ty) * p.nz;
+        const double tiles = (double)((p.nx + s.tx - 1) / s.tx) * ((p.ny + s.ty - 1) / s.ty);
+        taken += tiles * s.tx * s.ty * p.nz;
+        items += tiles * ((p.nz + 1) / 2);
       }
-      const double score = s.w * cells / taken;
+      const double score = s.w * cells / taken * std::min(1.0, items / sms);
       if (score > best) {
         best = score;
         pick = j;
       }
     }
   return pick;
-}
-
-static int device_sms() {
-  int dev = 0, sms = 152;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms;
 }
 
 // The chunk: about two items per block and half-step, for the claimed places

@@ -21,8 +21,8 @@ static Variant make_variant() {
   v.ns = NS;
   v.ns_vel = NSV;
   v.threads = G::THREADS;
-  v.stress_smem = G::S_SMEM;
-  v.vel_smem = GV::V_SMEM;
+  v.stress_smem = kKernelSmem<G, StressRing<G>>;
+  v.vel_smem = kKernelSmem<GV, VelocityRing<GV>>;
   v.halo = G::H;
   v.loads = LOAD;
   v.stress = reinterpret_cast<const void *>(&stress_kernel<T, TX, TY, NS, CPT, MB, LOAD>);
@@ -61,6 +61,15 @@ static const Variant kVariants[] = {
     // five 32-wide tiles, 67% of two 112-wide ones)
     make_variant<float, 56, 16, 4>(),
     make_variant<float, 32, 28, 4>(),
+    // FP32 tiles of eight consumer warps (their launch splits its registers
+    // unevenly): grids are often multiples of 8 or 16 rows, and near the L2
+    // size the warps are what limits the kernel (128^3 43.6 -> 46.2
+    // Gcell-updates/s, 192^3 46.6 -> 47.7)
+    make_variant<float, 128, 8, 4>(),
+    make_variant<float, 64, 16, 4>(),
+    make_variant<float, 32, 32, 4>(),
+    make_variant<float, 112, 9, 4>(),
+    make_variant<float, 56, 18, 4>(),
     // and narrow FP64 tiles: its arithmetic bounds FP64, idle lanes included
     make_variant<double, 16, 14, 4, 1>(),
     make_variant<double, 8, 28, 4, 1>(),

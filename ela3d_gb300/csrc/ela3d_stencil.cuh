@@ -38,16 +38,23 @@ struct Geo {
   static constexpr int H = Vec<T>::N;    // halo width in x (16 bytes, the TMA x alignment)
   static constexpr int TX = TX_, TY = TY_, NS = NS_;
   static constexpr int NTX = TX / VEC;
-  static constexpr int NT = NTX * TY;      // consumer threads
-  static constexpr int NCW = NT / 32;      // consumer warps
-  static constexpr int THREADS = NT + 32;  // + one producer warp
+  static constexpr int NCW = (NTX * TY + 31) / 32;   // consumer warps
+  static constexpr int NT = 32 * NCW;      // consumer threads (a last few may have no cells)
+  // Seven consumer warps and the loading warp fill the register file at up to
+  // 255 registers a thread.  Eight consumer warps cannot: the loading warp would
+  // be a ninth, a sub-partition's third.  They are launched as three warpgroups
+  // of 168 registers a thread, and the loading warp's group hands registers over
+  // to the consumers (setmaxnreg; 8 x 216 + 4 x 72 = 12 x 168).
+  static constexpr bool SPLIT = NCW == 8 && sizeof(T) == 4;
+  static constexpr int CONSUMER_REGS = 216, LOADER_REGS = 72;
+  static_assert(8 * CONSUMER_REGS + 4 * LOADER_REGS <= 12 * 168, "registers of the launch");
+  static constexpr int THREADS = SPLIT ? 384 : NT + 32;  // + the loading warp (or its group)
   // blocks per SM the register budget is sized for (64K registers per SM):
   // two blocks of four warps keep 255 registers per thread; fewer cells per
   // thread trade registers for resident warps
   static constexpr int MINB = MINB_ ? MINB_ : (THREADS <= 128 ? 2 : 1);
   static constexpr int WW = TX + H;
   static_assert(H % VEC == 0 && TX % H == 0 && TX + H <= 256 && TY + 1 <= 256, "tile shape");
-  static_assert(NT % 32 == 0, "consumer threads must fill whole warps");
   __host__ __device__ static constexpr int al(int b) { return (b + 127) & ~127; }
   static constexpr int C = TX * TY;          // center box
   static constexpr int W1 = WW * (TY + 1);   // wide box with one extra row
@@ -55,43 +62,83 @@ struct Geo {
   static constexpr int Y1 = TX * (TY + 1);   // narrow box with one extra row
   __host__ __device__ static constexpr int sz(int e) { return al(e * (int)sizeof(T)); }
   static constexpr int SC = (C * (int)sizeof(T) + 127) & ~127;  // bytes of a centre box
-  // stress stage: vx vy vz cs rho (W1), cp s0..s5 (C)
+  // A plane is held in two parts, each in a ring of its own: the first part is
+  // what the plane below reads too (as its z+1 neighbours), the second the
+  // rest.  The first ring has NS places; the second does with one place less
+  // where shared memory is short.
+  // stress: vx vy cs rho (W1) | vz (W1), cp and the six stresses (C)
   static constexpr int S_VX = 0;
   static constexpr int S_VY = S_VX + sz(W1);
-  static constexpr int S_VZ = S_VY + sz(W1);
-  static constexpr int S_CS = S_VZ + sz(W1);
+  static constexpr int S_CS = S_VY + sz(W1);
   static constexpr int S_RHO = S_CS + sz(W1);
-  static constexpr int S_CP = S_RHO + sz(W1);
+  static constexpr int S_A = S_RHO + sz(W1);
+  static constexpr int S_VZ = 0;
+  static constexpr int S_CP = S_VZ + sz(W1);
   static constexpr int S_SIG = S_CP + sz(C);  // six centre boxes follow
-  static constexpr int S_STAGE = S_SIG + 6 * sz(C);
-  // bytes of the two parts a stage is loaded in: what the plane below also
-  // needs (vx vy cs rho, as its z+1 neighbours), and the rest
-  static constexpr int S_TXA = (int)sizeof(T) * 4 * W1;
+  static constexpr int S_B = S_SIG + 6 * sz(C);
+  static constexpr int S_TXA = (int)sizeof(T) * 4 * W1;   // bytes loaded
   static constexpr int S_TXB = (int)sizeof(T) * (W1 + 7 * C);
-  // velocity stage
+  // velocity: szz (C), rho (W1) | sxx syy sxy sxz syz with their halos, vx vy vz (C)
+  static constexpr int V_SZZ = 0;
+  static constexpr int V_RHO = V_SZZ + sz(C);
+  static constexpr int V_A = V_RHO + sz(W1);
   static constexpr int V_SXX = 0;                 // W0
   static constexpr int V_SYY = V_SXX + sz(W0);    // Y1
-  static constexpr int V_SZZ = V_SYY + sz(Y1);    // C
-  static constexpr int V_SXY = V_SZZ + sz(C);     // W1
+  static constexpr int V_SXY = V_SYY + sz(Y1);    // W1
   static constexpr int V_SXZ = V_SXY + sz(W1);    // W0
   static constexpr int V_SYZ = V_SXZ + sz(W0);    // Y1
-  static constexpr int V_RHO = V_SYZ + sz(Y1);    // W1
-  static constexpr int V_V = V_RHO + sz(W1);      // vx vy vz (C)
-  static constexpr int V_STAGE = V_V + 3 * sz(C);
-  static constexpr int V_TXA = (int)sizeof(T) * (C + W1);   // szz, rho
+  static constexpr int V_V = V_SYZ + sz(Y1);      // vx vy vz (C)
+  static constexpr int V_B = V_V + 3 * sz(C);
+  static constexpr int V_TXA = (int)sizeof(T) * (C + W1);
   static constexpr int V_TXB = (int)sizeof(T) * (2 * W0 + 2 * Y1 + 3 * C + W1);
   // memory-variable slots (PsiSlots): one 16-byte (or smaller) vector per
   // consumer thread for each of the three variables of each axis
   static constexpr int PSI_BYTES = 9 * NT * VEC * (int)sizeof(T);
-  // mbarriers (full[2][NS], empty[NS]) live after the stages, so the TMA
-  // destinations start at the (aligned) base of dynamic shared memory; the
-  // memory-variable slots follow them
-  static constexpr int BARS = 24 * NS;
-  static constexpr int S_PSI = al(NS * S_STAGE + BARS);
-  static constexpr int V_PSI = al(NS * V_STAGE + BARS);
-  static constexpr int S_SMEM = S_PSI + PSI_BYTES;
-  static constexpr int V_SMEM = V_PSI + PSI_BYTES;
+  static constexpr int MAX_SMEM = 232448;   // of one block
+  // places of the second ring for parts of a and b bytes, with `other` bytes
+  // of shared memory beside the rings
+  __host__ __device__ static constexpr int places_b(int a, int b, int other) {
+    return NS * (a + b) + 32 * NS + PSI_BYTES + other <= MAX_SMEM / MINB ? NS : NS - 1;
+  }
 };
+
+// The two rings of a kernel's planes, at the (aligned) base of dynamic shared
+// memory, and their mbarriers behind them: full (TMA bytes landed) and empty
+// (all consumer warps done) for every place.
+template <int NA_, int NB_, int A_, int B_>
+struct Ring {
+  static constexpr int NA = NA_, NB = NB_, A = A_, B = B_;
+  static constexpr int BARRIERS = NA * A + NB * B;
+  static constexpr int BYTES = BARRIERS + 16 * (NA + NB);
+  unsigned char *base;
+  __device__ __forceinline__ unsigned char *a(int s) const { return base + s * A; }
+  __device__ __forceinline__ unsigned char *b(int s) const { return base + NA * A + s * B; }
+  __device__ __forceinline__ uint64_t *bars() const { return reinterpret_cast<uint64_t *>(base + BARRIERS); }
+  __device__ __forceinline__ uint64_t *full_a(int s) const { return bars() + s; }
+  __device__ __forceinline__ uint64_t *full_b(int s) const { return bars() + NA + s; }
+  __device__ __forceinline__ uint64_t *empty_a(int s) const { return bars() + NA + NB + s; }
+  __device__ __forceinline__ uint64_t *empty_b(int s) const { return bars() + 2 * NA + NB + s; }
+};
+
+// A place in a ring of N, and the parity of the pass over it.
+template <int N>
+struct Place {
+  int s = 0;
+  uint32_t parity = 0;
+  __device__ __forceinline__ void next() {
+    if (++s == N) {
+      s = 0;
+      parity ^= 1;
+    }
+  }
+};
+
+template <int REGS> __device__ __forceinline__ void more_registers() {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS));
+}
+template <int REGS> __device__ __forceinline__ void fewer_registers() {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS));
+}
 
 template <typename T>
 __device__ __forceinline__ int tiles_x_of(const ShotDesc<T> &s, int TX) {
@@ -390,57 +437,60 @@ __device__ __forceinline__ void copy_box_async(unsigned char *dst, const T *base
 
 
 // Producer warp: walks the block's items and issues every plane's loads
-// (lane 0) and the plane's memory-variable prefetches (all lanes).  Load n
-// goes to stage n % NS; before reusing a stage lane 0 waits for the
-// consumers' release of load n - NS on that stage's empty barrier.  Item i
-// contributes planes k0 .. k1 (k1 is the look-ahead plane, possibly nz,
-// which the TMA fills with zeros).  A stage has two full barriers: full[s] for
-// the part that the plane below reads too, full[NS + s] for the rest.  The
-// consumers of plane k wait for the rest of k and the first part of k + 1, so
-// the rest of k + 1 has a plane's time more to arrive, and the look-ahead
-// plane's rest is not loaded at all.
+// (lane 0) and the plane's memory-variable prefetches (all lanes).  An item's
+// planes k0 .. k1 - 1 take a place in both rings, its look-ahead plane k1
+// (possibly nz, which the TMA fills with zeros) one in the first ring only.
+// The consumers of plane k need both parts of k and the first part of k + 1,
+// so the first parts run one plane ahead of the second.  Before a place is
+// filled again lane 0 waits for the consumers' release of what it held.  (A
+// fresh barrier counts as having completed a phase of parity 1.)
 // With ASYNC every lane copies a share of each plane's boxes (cp.async)
 // instead of lane 0 issuing TMA loads.
-template <int NS, bool ASYNC, typename Issue, typename Prefetch>
-__device__ __forceinline__ bool produce_item(const Item &it, unsigned &n, uint64_t *full, uint64_t *empty,
-                                             Issue issue, Prefetch &prefetch, int lane) {
-  for (int k = it.k0; k <= it.k1; ++k, ++n) {
-    const int slot = (int)(n % NS);
+template <typename R>
+struct Loads {
+  Place<R::NA> a;
+  Place<R::NB> b;
+  unsigned na = 0, nb = 0;   // parts loaded so far
+};
+
+template <bool ASYNC, typename R, typename IssueA, typename IssueB, typename Prefetch>
+__device__ __forceinline__ bool produce_item(const Item &it, const R &ring, Loads<R> &ld, IssueA issue_a,
+                                             IssueB issue_b, Prefetch &prefetch, int lane) {
+  for (int k = it.k0 - 1; k < it.k1; ++k) {
+    const bool both = k >= it.k0;
     int good = 1;
-    if (lane == 0 && n >= NS) good = mbar_wait_bounded(&empty[slot], (uint32_t)(((n / NS) - 1) & 1));
+    if (lane == 0) {
+      good = mbar_wait_bounded(ring.empty_a(ld.a.s), ld.a.parity ^ 1);
+      if (both) good = good && mbar_wait_bounded(ring.empty_b(ld.b.s), ld.b.parity ^ 1);
+    }
     if (!__shfl_sync(0xffffffffu, good, 0)) return false;
-    if (ASYNC || lane == 0) issue(it, k, slot, &full[slot], &full[NS + slot], k == it.k1, lane);
-    prefetch.plane(k);
+    if (ASYNC || lane == 0) {
+      issue_a(k + 1, ring.a(ld.a.s), ring.full_a(ld.a.s));
+      if (both) issue_b(k, ring.b(ld.b.s), ring.full_b(ld.b.s));
+    }
+    ld.a.next();
+    ++ld.na;
+    if (both) {
+      ld.b.next();
+      ++ld.nb;
+    }
+    prefetch.plane(k + 1);
   }
   return true;
 }
 
 // The block must not exit with copies in flight: waits (bounded) for the
-// last NS loads, and reports a timeout seen earlier.
-template <int NS, bool ASYNC>
-__device__ __forceinline__ void produce_drain(unsigned n, bool ok, uint64_t *full, unsigned *__restrict__ err,
+// last loads of each ring, and reports a timeout seen earlier.
+template <bool ASYNC, typename R>
+__device__ __forceinline__ void produce_drain(const R &ring, const Loads<R> &ld, bool ok, unsigned *__restrict__ err,
                                               int lane) {
   if (ASYNC) cp_async_wait_all();
   if (lane != 0) return;
   if (!ok) atomicOr(err, DEV_ERR_TIMEOUT);
-  for (unsigned q = (n > NS ? n - NS : 0); q < n; ++q)
-    for (int part = 0; part < 2; ++part)
-      mbar_wait_bounded(&full[part * NS + q % NS], (uint32_t)((q / NS) & 1), 200000000ull);
-}
-
-template <int NS, bool ASYNC, typename Issue, typename Prefetch>
-__device__ __forceinline__ void produce(const Item *__restrict__ items, int2 range, uint64_t *full, uint64_t *empty,
-                                        Issue issue, Prefetch &prefetch, unsigned *__restrict__ err, int ctl,
-                                        int lane) {
-  if (ctl & CTL_WITHHOLD_LOADS) return;  // test mode: no stage is ever filled
-  unsigned n = 0;
-  bool ok = true;
-  for (int ii = range.x; ii < range.y && ok; ++ii) {
-    const Item it = items[ii];
-    prefetch.begin(it);
-    ok = produce_item<NS, ASYNC>(it, n, full, empty, issue, prefetch, lane);
-  }
-  produce_drain<NS, ASYNC>(n, ok, full, err, lane);
+  for (unsigned q = ld.na > R::NA ? ld.na - R::NA : 0; q < ld.na; ++q)
+    mbar_wait_bounded(ring.full_a(q % R::NA), (uint32_t)((q / R::NA) & 1), 200000000ull);
+  for (unsigned q = ld.nb > R::NB ? ld.nb - R::NB : 0; q < ld.nb; ++q)
+    mbar_wait_bounded(ring.full_b(q % R::NB), (uint32_t)((q / R::NB) & 1), 200000000ull);
 }
 
 // The producer lanes' memory-variable prefetcher for one half-step (var0 =
@@ -459,114 +509,116 @@ struct ItemPrefetch {
 };
 
 // ------------------------------------------------------- stage loads ----
-// One stress plane.  First part: vx vy cs rho with their halos; the rest: vz
-// with its halo, cp and the six stresses of the tile (box shapes in
-// ela3d_device.cuh, ShotMaps).  `ahead`: the look-ahead plane, first part only.
-template <typename T, int TX, int TY, int NS, int CPT, int MB, int LOAD>
-__device__ __forceinline__ void stress_issue(const ShotDesc<T> *__restrict__ shots,
-                                             const ShotMaps *__restrict__ maps, const Item &it, int k,
-                                             unsigned char *st, uint64_t *bar, uint64_t *rest, bool ahead, int lane) {
-  using G = Geo<T, TX, TY, NS, CPT, MB>;
-  constexpr int H = G::H;
-  const int txs = tiles_x_of(shots[it.shot], TX);
+// The two parts of one stress plane (box shapes in ela3d_device.cuh, ShotMaps):
+// vx vy cs rho with their halos | vz with its halo, cp and the six stresses.
+template <typename G, int LOAD, typename T>
+__device__ __forceinline__ void stress_issue_a(const ShotDesc<T> &sd, const ShotMaps &maps, const Item &it, int k,
+                                         unsigned char *st, uint64_t *bar, int lane) {
+  constexpr int H = G::H, TX = G::TX, TY = G::TY;
+  const int txs = tiles_x_of(sd, TX);
   const int x0 = (it.tile % txs) * TX, y0 = (it.tile / txs) * TY;
   if constexpr (LOAD == LOAD_CP_ASYNC) {
-    const ShotDesc<T> &sd = shots[it.shot];
     copy_box_async<T, TX + H, TY + 1>(st + G::S_VX, sd.f[0], sd, x0, y0, k, lane);
     copy_box_async<T, TX + H, TY + 1>(st + G::S_VY, sd.f[1], sd, x0 - H, y0 - 1, k, lane);
     copy_box_async<T, TX + H, TY + 1>(st + G::S_CS, sd.cs, sd, x0 - H, y0, k, lane);
     copy_box_async<T, TX + H, TY + 1>(st + G::S_RHO, sd.rho, sd, x0 - H, y0, k, lane);
     cp_async_arrive_noinc(bar);
-    if (!ahead) {
-      copy_box_async<T, TX + H, TY + 1>(st + G::S_VZ, sd.f[2], sd, x0 - H, y0, k, lane);
-      copy_box_async<T, TX, TY>(st + G::S_CP, sd.cp, sd, x0, y0, k, lane);
-#pragma unroll
-      for (int c = 0; c < 6; ++c)
-        copy_box_async<T, TX, TY>(st + G::S_SIG + c * G::SC, sd.f[3 + c], sd, x0, y0, k, lane);
-    }
-    cp_async_arrive_noinc(rest);
-    return;
+  } else {
+    const CUtensorMap *m = maps.stress;
+    mbar_arrive_expect_tx(bar, G::S_TXA);
+    tma_load_3d(st + G::S_VX, &m[0], x0, y0, k, bar);
+    tma_load_3d(st + G::S_VY, &m[1], x0 - H, y0 - 1, k, bar);
+    tma_load_3d(st + G::S_CS, &m[3], x0 - H, y0, k, bar);
+    tma_load_3d(st + G::S_RHO, &m[4], x0 - H, y0, k, bar);
   }
-  const CUtensorMap *m = maps[it.shot].stress;
-  mbar_arrive_expect_tx(bar, G::S_TXA);
-  tma_load_3d(st + G::S_VX, &m[0], x0, y0, k, bar);
-  tma_load_3d(st + G::S_VY, &m[1], x0 - H, y0 - 1, k, bar);
-  tma_load_3d(st + G::S_CS, &m[3], x0 - H, y0, k, bar);
-  tma_load_3d(st + G::S_RHO, &m[4], x0 - H, y0, k, bar);
-  if (ahead) {
-    mbar_arrive(rest);
-    return;
-  }
-  mbar_arrive_expect_tx(rest, G::S_TXB);
-  tma_load_3d(st + G::S_VZ, &m[2], x0 - H, y0, k, rest);
-  tma_load_3d(st + G::S_CP, &m[5], x0, y0, k, rest);
-#pragma unroll
-  for (int c = 0; c < 6; ++c) tma_load_3d(st + G::S_SIG + c * G::SC, &m[6 + c], x0, y0, k, rest);
 }
 
-// One velocity plane.  First part: szz and rho (with its halo); the rest: the
-// other stresses with the halos the divergence needs, and vx vy vz of the tile.
-template <typename T, int TX, int TY, int NS, int CPT, int MB, int LOAD>
-__device__ __forceinline__ void velocity_issue(const ShotDesc<T> *__restrict__ shots,
-                                               const ShotMaps *__restrict__ maps, const Item &it, int k,
-                                               unsigned char *st, uint64_t *bar, uint64_t *rest, bool ahead,
-                                               int lane) {
-  using G = Geo<T, TX, TY, NS, CPT, MB>;
-  constexpr int H = G::H;
-  const int txs = tiles_x_of(shots[it.shot], TX);
+template <typename G, int LOAD, typename T>
+__device__ __forceinline__ void stress_issue_b(const ShotDesc<T> &sd, const ShotMaps &maps, const Item &it, int k,
+                                         unsigned char *st, uint64_t *bar, int lane) {
+  constexpr int H = G::H, TX = G::TX, TY = G::TY;
+  const int txs = tiles_x_of(sd, TX);
   const int x0 = (it.tile % txs) * TX, y0 = (it.tile / txs) * TY;
   if constexpr (LOAD == LOAD_CP_ASYNC) {
-    const ShotDesc<T> &sd = shots[it.shot];
+    copy_box_async<T, TX + H, TY + 1>(st + G::S_VZ, sd.f[2], sd, x0 - H, y0, k, lane);
+    copy_box_async<T, TX, TY>(st + G::S_CP, sd.cp, sd, x0, y0, k, lane);
+#pragma unroll
+    for (int c = 0; c < 6; ++c) copy_box_async<T, TX, TY>(st + G::S_SIG + c * G::SC, sd.f[3 + c], sd, x0, y0, k, lane);
+    cp_async_arrive_noinc(bar);
+  } else {
+    const CUtensorMap *m = maps.stress;
+    mbar_arrive_expect_tx(bar, G::S_TXB);
+    tma_load_3d(st + G::S_VZ, &m[2], x0 - H, y0, k, bar);
+    tma_load_3d(st + G::S_CP, &m[5], x0, y0, k, bar);
+#pragma unroll
+    for (int c = 0; c < 6; ++c) tma_load_3d(st + G::S_SIG + c * G::SC, &m[6 + c], x0, y0, k, bar);
+  }
+}
+
+// The two parts of one velocity plane: szz, rho with its halo | the other
+// stresses with the halos the divergence needs, and vx vy vz of the tile.
+template <typename G, int LOAD, typename T>
+__device__ __forceinline__ void velocity_issue_a(const ShotDesc<T> &sd, const ShotMaps &maps, const Item &it, int k,
+                                         unsigned char *st, uint64_t *bar, int lane) {
+  constexpr int H = G::H, TX = G::TX, TY = G::TY;
+  const int txs = tiles_x_of(sd, TX);
+  const int x0 = (it.tile % txs) * TX, y0 = (it.tile / txs) * TY;
+  if constexpr (LOAD == LOAD_CP_ASYNC) {
     copy_box_async<T, TX, TY>(st + G::V_SZZ, sd.f[5], sd, x0, y0, k, lane);
     copy_box_async<T, TX + H, TY + 1>(st + G::V_RHO, sd.rho, sd, x0 - H, y0, k, lane);
     cp_async_arrive_noinc(bar);
-    if (!ahead) {
-      copy_box_async<T, TX + H, TY>(st + G::V_SXX, sd.f[3], sd, x0 - H, y0, k, lane);
-      copy_box_async<T, TX, TY + 1>(st + G::V_SYY, sd.f[4], sd, x0, y0, k, lane);
-      copy_box_async<T, TX + H, TY + 1>(st + G::V_SXY, sd.f[6], sd, x0, y0 - 1, k, lane);
-      copy_box_async<T, TX + H, TY>(st + G::V_SXZ, sd.f[7], sd, x0, y0, k, lane);
-      copy_box_async<T, TX, TY + 1>(st + G::V_SYZ, sd.f[8], sd, x0, y0 - 1, k, lane);
-#pragma unroll
-      for (int c = 0; c < 3; ++c) copy_box_async<T, TX, TY>(st + G::V_V + c * G::SC, sd.f[c], sd, x0, y0, k, lane);
-    }
-    cp_async_arrive_noinc(rest);
-    return;
+  } else {
+    const CUtensorMap *m = maps.vel;
+    mbar_arrive_expect_tx(bar, G::V_TXA);
+    tma_load_3d(st + G::V_SZZ, &m[2], x0, y0, k, bar);
+    tma_load_3d(st + G::V_RHO, &m[6], x0 - H, y0, k, bar);
   }
-  const CUtensorMap *m = maps[it.shot].vel;
-  mbar_arrive_expect_tx(bar, G::V_TXA);
-  tma_load_3d(st + G::V_SZZ, &m[2], x0, y0, k, bar);
-  tma_load_3d(st + G::V_RHO, &m[6], x0 - H, y0, k, bar);
-  if (ahead) {
-    mbar_arrive(rest);
-    return;
-  }
-  mbar_arrive_expect_tx(rest, G::V_TXB);
-  tma_load_3d(st + G::V_SXX, &m[0], x0 - H, y0, k, rest);
-  tma_load_3d(st + G::V_SYY, &m[1], x0, y0, k, rest);
-  tma_load_3d(st + G::V_SXY, &m[3], x0, y0 - 1, k, rest);
-  tma_load_3d(st + G::V_SXZ, &m[4], x0, y0, k, rest);
-  tma_load_3d(st + G::V_SYZ, &m[5], x0, y0 - 1, k, rest);
-#pragma unroll
-  for (int c = 0; c < 3; ++c) tma_load_3d(st + G::V_V + c * G::SC, &m[7 + c], x0, y0, k, rest);
 }
 
-// Waits for the whole stage of load n (plane k) and the first part of load
-// n+1 (plane k+1); load n's first part was already waited for as the previous
-// plane's k+1 unless k is the first plane of its work item.  False when a wait
-// passed its limit; the caller records the timeout and returns.
-template <int NS>
-__device__ __forceinline__ bool wait_planes(uint64_t *full, unsigned n, bool first, unsigned long long wait_ns,
+template <typename G, int LOAD, typename T>
+__device__ __forceinline__ void velocity_issue_b(const ShotDesc<T> &sd, const ShotMaps &maps, const Item &it, int k,
+                                         unsigned char *st, uint64_t *bar, int lane) {
+  constexpr int H = G::H, TX = G::TX, TY = G::TY;
+  const int txs = tiles_x_of(sd, TX);
+  const int x0 = (it.tile % txs) * TX, y0 = (it.tile / txs) * TY;
+  if constexpr (LOAD == LOAD_CP_ASYNC) {
+    copy_box_async<T, TX + H, TY>(st + G::V_SXX, sd.f[3], sd, x0 - H, y0, k, lane);
+    copy_box_async<T, TX, TY + 1>(st + G::V_SYY, sd.f[4], sd, x0, y0, k, lane);
+    copy_box_async<T, TX + H, TY + 1>(st + G::V_SXY, sd.f[6], sd, x0, y0 - 1, k, lane);
+    copy_box_async<T, TX + H, TY>(st + G::V_SXZ, sd.f[7], sd, x0, y0, k, lane);
+    copy_box_async<T, TX, TY + 1>(st + G::V_SYZ, sd.f[8], sd, x0, y0 - 1, k, lane);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) copy_box_async<T, TX, TY>(st + G::V_V + c * G::SC, sd.f[0 + c], sd, x0, y0, k, lane);
+    cp_async_arrive_noinc(bar);
+  } else {
+    const CUtensorMap *m = maps.vel;
+    mbar_arrive_expect_tx(bar, G::V_TXB);
+    tma_load_3d(st + G::V_SXX, &m[0], x0 - H, y0, k, bar);
+    tma_load_3d(st + G::V_SYY, &m[1], x0, y0, k, bar);
+    tma_load_3d(st + G::V_SXY, &m[3], x0, y0 - 1, k, bar);
+    tma_load_3d(st + G::V_SXZ, &m[4], x0, y0, k, bar);
+    tma_load_3d(st + G::V_SYZ, &m[5], x0, y0 - 1, k, bar);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) tma_load_3d(st + G::V_V + c * G::SC, &m[7 + c], x0, y0, k, bar);
+  }
+}
+
+// Waits for both parts of plane k (places a, b) and the first part of plane
+// k + 1 (place ahead); a was already waited for as the previous plane's ahead
+// unless k is the first plane of its work item.  False when a wait passed its
+// limit; the caller returns.
+template <typename R>
+__device__ __forceinline__ bool wait_planes(const R &ring, const Place<R::NA> &a, const Place<R::NB> &b,
+                                            const Place<R::NA> &ahead, bool first, unsigned long long wait_ns,
                                             unsigned *err, int lane) {
-  const int s0 = (int)(n % NS), s1 = (int)((n + 1) % NS);
-  const uint32_t p0 = (uint32_t)((n / NS) & 1), p1 = (uint32_t)(((n + 1) / NS) & 1);
   // all three have usually completed: one vote
-  bool ok = !first || mbar_try_wait(&full[s0], p0);
-  ok &= mbar_try_wait(&full[NS + s0], p0);
-  ok &= mbar_try_wait(&full[s1], p1);
+  bool ok = !first || mbar_try_wait(ring.full_a(a.s), a.parity);
+  ok &= mbar_try_wait(ring.full_b(b.s), b.parity);
+  ok &= mbar_try_wait(ring.full_a(ahead.s), ahead.parity);
   if (__all_sync(0xffffffffu, ok)) return true;
-  ok = !first || mbar_wait_bounded(&full[s0], p0, wait_ns);
-  ok = ok && mbar_wait_bounded(&full[NS + s0], p0, wait_ns);
-  ok = ok && mbar_wait_bounded(&full[s1], p1, wait_ns);
+  ok = !first || mbar_wait_bounded(ring.full_a(a.s), a.parity, wait_ns);
+  ok = ok && mbar_wait_bounded(ring.full_b(b.s), b.parity, wait_ns);
+  ok = ok && mbar_wait_bounded(ring.full_a(ahead.s), ahead.parity, wait_ns);
   if (__any_sync(0xffffffffu, !ok)) {
     if (lane == 0) atomicOr(err, DEV_ERR_TIMEOUT);
     return false;
@@ -644,26 +696,28 @@ struct PsiSlots {
 
 // ----------------------------------------------------------- stress ----
 // The stress half-step over one work item (the block's consumer warps).
-// STAGE is the byte stride of the ring's stages.  FLOW (the dataflow
+// a, b: the places of the item's first plane in the rings.  FLOW (the dataflow
 // kernel): the item's inputs were written by other blocks of the same
 // launch; the caller has waited for the item's ready barrier, on which the
 // producer arrives once it has acquired the item's dependencies, and the z-1
 // plane, written during this launch, bypasses L1.  inject_tick (FLOW): the
 // tick of the step before, whose explosive source is still to be added to
 // the source cell's stresses (INT_MIN: none).
-template <typename T, int TX, int TY, int NS, int CPT, int MB, int STAGE, bool FLOW>
-__device__ __forceinline__ bool stress_item(const ShotDesc<T> &sd, const Item &item, const unsigned char *smem,
-                                            unsigned char *psi, uint64_t *full, uint64_t *empty, unsigned &n,
-                                            unsigned *__restrict__ err, unsigned long long wait_ns, int tid,
-                                            int inject_tick = INT_MIN) {
-  using G = Geo<T, TX, TY, NS, CPT, MB>;
+template <typename G, bool FLOW, typename T, typename R>
+__device__ __forceinline__ bool stress_item(const ShotDesc<T> &sd, const Item &item, const R &ring, Place<R::NA> &a,
+                                            Place<R::NB> &b, unsigned char *psi, unsigned *__restrict__ err,
+                                            unsigned long long wait_ns, int tid, int inject_tick = INT_MIN) {
+  constexpr int TX = G::TX, TY = G::TY;
   constexpr int V = G::VEC, H = G::H, WW = G::WW;
   const int lane = tid & 31;
-  const int tx = tid % G::NTX, ty = tid / G::NTX;
+  const int tx = tid % G::NTX;
+  // (a thread without cells reads the last row's and has its row outside any grid)
+  const bool spare = G::NT != G::NTX * TY && tid >= G::NTX * TY;
+  const int ty = spare ? TY - 1 : tid / G::NTX;
   const int nx = sd.nx, ny = sd.ny, nz = sd.nz, px = sd.px;
   const int txs = (nx + TX - 1) / TX;
   const int x0 = (item.tile % txs) * TX, y0 = (item.tile / txs) * TY;
-  const int xg = x0 + tx * V, y = y0 + ty;
+  const int xg = x0 + tx * V, y = spare ? INT_MAX / 2 : y0 + ty;
   const bool live = (xg < nx) && (y < ny);
   const T dt = sd.dt, idx = sd.idx, idy = sd.idy, idz = sd.idz;
   const long long plane = (long long)ny * px;
@@ -756,20 +810,20 @@ __device__ __forceinline__ bool stress_item(const ShotDesc<T> &sd, const Item &i
       azh = prof_z[PR_AH * nz + k]; bzh = prof_z[PR_BH * nz + k]; ikzh = prof_z[PR_IKH * nz + k];
     }
 
-    if (!wait_planes<NS>(full, n, k == item.k0, wait_ns, err, lane)) {
+    Place<R::NA> ahead = a;
+    ahead.next();
+    if (!wait_planes(ring, a, b, ahead, k == item.k0, wait_ns, err, lane)) {
       cp_async_wait_all();   // (no copy outlives its thread)
       return false;
     }
-    const int s0 = (int)(n % NS), s1 = (int)((n + 1) % NS);
-    const unsigned char *cur = smem + s0 * STAGE;
-    const unsigned char *nxt = smem + s1 * STAGE;
+    const unsigned char *cur = ring.a(a.s), *rest = ring.b(b.s), *nxt = ring.a(ahead.s);
     const T *bvx = reinterpret_cast<const T *>(cur + G::S_VX);
     const T *bvy = reinterpret_cast<const T *>(cur + G::S_VY);
-    const T *bvz = reinterpret_cast<const T *>(cur + G::S_VZ);
+    const T *bvz = reinterpret_cast<const T *>(rest + G::S_VZ);
     const T *bcs = reinterpret_cast<const T *>(cur + G::S_CS);
     const T *brho = reinterpret_cast<const T *>(cur + G::S_RHO);
-    const T *bcp = reinterpret_cast<const T *>(cur + G::S_CP);
-    const T *bsig = reinterpret_cast<const T *>(cur + G::S_SIG);
+    const T *bcp = reinterpret_cast<const T *>(rest + G::S_CP);
+    const T *bsig = reinterpret_cast<const T *>(rest + G::S_SIG);
     constexpr int CS = G::SC / (int)sizeof(T);
 
     T vx_c[V], vx_yp[V], vx_zp[V], vy_c[V], vy_ym[V], vy_zp[V], vz_c[V], vz_yp[V];
@@ -820,12 +874,13 @@ __device__ __forceinline__ bool stress_item(const ShotDesc<T> &sd, const Item &i
         }
     }
 
-    // stage s0 is no longer read by this warp (s1 still is, as the next plane)
+    // this warp no longer reads the plane's places (ahead still is, as the next plane)
     const bool last = (k == item.k1 - 1);
     __syncwarp();
     if (lane == 0) {
-      mbar_arrive(&empty[s0]);
-      if (last) mbar_arrive(&empty[s1]);
+      mbar_arrive(ring.empty_a(a.s));
+      mbar_arrive(ring.empty_b(b.s));
+      if (last) mbar_arrive(ring.empty_a(ahead.s));
     }
 
     // this plane's update masks: bit e of byte c = component c of cell e
@@ -947,7 +1002,9 @@ __device__ __forceinline__ bool stress_item(const ShotDesc<T> &sd, const Item &i
       st_vec(f7 + g, sxz);
       st_vec(f8 + g, syz);
     }
-    n += last ? 2 : 1;
+    a = ahead;
+    if (last) a.next();
+    b.next();
   }
   return true;
 }
@@ -962,12 +1019,12 @@ __device__ __forceinline__ bool stress_item(const ShotDesc<T> &sd, const Item &i
 // every warp of the plane's tiles: 64^3 with 64 receivers 22.1 us a step
 // that way, 20.6 this way and without receivers; 101^3 with 11, 29.6 and
 // 28.7.)
-template <typename T, int NTX, int V>
+template <int NTX, int TY, typename T, int V>
 __device__ __forceinline__ void sample_receivers(const int4 *__restrict__ rec, int lo, int end, int x0, int y0,
                                                  int tid, const T (&vx)[V], const T (&vy)[V], const T (&vz)[V],
                                                  T *out, int nsamp) {
   const int lane = tid & 31, t0 = tid - lane;                // the warp's first thread
-  const int ya = y0 + t0 / NTX, yb = y0 + (t0 + 31) / NTX;   // its first and last row
+  const int ya = y0 + t0 / NTX, yb = y0 + min((t0 + 31) / NTX, TY - 1);   // its first and last row
   // the first receiver at or after (ya, x0) lies in [lo, hi]
   for (int hi = end; hi - lo > 32;) {
     const int step = (hi - lo + 31) / 32, q = lo + lane * step;
@@ -1007,21 +1064,23 @@ __device__ __forceinline__ void sample_receivers(const int4 *__restrict__ rec, i
 }
 
 // The velocity half-step over one work item at step `tick` (see
-// stress_item for STAGE and FLOW), with the receivers and the force source.
-template <typename T, int TX, int TY, int NS, int CPT, int MB, int STAGE, bool FLOW>
-__device__ __forceinline__ bool velocity_item(const ShotDesc<T> &sd, const Item &item, int tick,
-                                              const unsigned char *smem, unsigned char *psi, uint64_t *full,
-                                              uint64_t *empty, unsigned &n, unsigned *__restrict__ err,
-                                              unsigned long long wait_ns, int tid) {
-  using G = Geo<T, TX, TY, NS, CPT, MB>;
+// stress_item for a, b and FLOW), with the receivers and the force source.
+template <typename G, bool FLOW, typename T, typename R>
+__device__ __forceinline__ bool velocity_item(const ShotDesc<T> &sd, const Item &item, int tick, const R &ring,
+                                              Place<R::NA> &a, Place<R::NB> &b, unsigned char *psi,
+                                              unsigned *__restrict__ err, unsigned long long wait_ns, int tid) {
+  constexpr int TX = G::TX, TY = G::TY;
   constexpr int V = G::VEC, H = G::H, WW = G::WW;
   constexpr int CS = G::SC / (int)sizeof(T);
   const int lane = tid & 31;
-  const int tx = tid % G::NTX, ty = tid / G::NTX;
+  const int tx = tid % G::NTX;
+  // (a thread without cells reads the last row's and has its row outside any grid)
+  const bool spare = G::NT != G::NTX * TY && tid >= G::NTX * TY;
+  const int ty = spare ? TY - 1 : tid / G::NTX;
   const int nx = sd.nx, ny = sd.ny, nz = sd.nz, px = sd.px;
   const int txs = (nx + TX - 1) / TX;
   const int x0 = (item.tile % txs) * TX, y0 = (item.tile / txs) * TY;
-  const int xg = x0 + tx * V, y = y0 + ty;
+  const int xg = x0 + tx * V, y = spare ? INT_MAX / 2 : y0 + ty;
   const bool live = (xg < nx) && (y < ny);
   const T dt = sd.dt, idx = sd.idx, idy = sd.idy, idz = sd.idz;
   const long long plane = (long long)ny * px;
@@ -1124,21 +1183,21 @@ __device__ __forceinline__ bool velocity_item(const ShotDesc<T> &sd, const Item 
       rhi = rec_plane[k + 1];
     }
 
-    if (!wait_planes<NS>(full, n, k == item.k0, wait_ns, err, lane)) {
+    Place<R::NA> ahead = a;
+    ahead.next();
+    if (!wait_planes(ring, a, b, ahead, k == item.k0, wait_ns, err, lane)) {
       cp_async_wait_all();   // (no copy outlives its thread)
       return false;
     }
-    const int s0 = (int)(n % NS), s1 = (int)((n + 1) % NS);
-    const unsigned char *cur = smem + s0 * STAGE;
-    const unsigned char *nxt = smem + s1 * STAGE;
-    const T *bsxx = reinterpret_cast<const T *>(cur + G::V_SXX);
-    const T *bsyy = reinterpret_cast<const T *>(cur + G::V_SYY);
+    const unsigned char *cur = ring.a(a.s), *rest = ring.b(b.s), *nxt = ring.a(ahead.s);
+    const T *bsxx = reinterpret_cast<const T *>(rest + G::V_SXX);
+    const T *bsyy = reinterpret_cast<const T *>(rest + G::V_SYY);
     const T *bszz = reinterpret_cast<const T *>(cur + G::V_SZZ);
-    const T *bsxy = reinterpret_cast<const T *>(cur + G::V_SXY);
-    const T *bsxz = reinterpret_cast<const T *>(cur + G::V_SXZ);
-    const T *bsyz = reinterpret_cast<const T *>(cur + G::V_SYZ);
+    const T *bsxy = reinterpret_cast<const T *>(rest + G::V_SXY);
+    const T *bsxz = reinterpret_cast<const T *>(rest + G::V_SXZ);
+    const T *bsyz = reinterpret_cast<const T *>(rest + G::V_SYZ);
     const T *brho = reinterpret_cast<const T *>(cur + G::V_RHO);
-    const T *bv = reinterpret_cast<const T *>(cur + G::V_V);
+    const T *bv = reinterpret_cast<const T *>(rest + G::V_V);
 
     T sxx_c[V], syy_c[V], syy_yp[V], szz_c[V], szz_zp[V], sxy_c[V], sxy_ym[V], sxz_c[V];
     T syz_c[V], syz_ym[V], rho_c[V], rho_yp[V], rho_zp[V], vx[V], vy[V], vz[V];
@@ -1166,8 +1225,9 @@ __device__ __forceinline__ bool velocity_item(const ShotDesc<T> &sd, const Item 
     const bool last = (k == item.k1 - 1);
     __syncwarp();
     if (lane == 0) {
-      mbar_arrive(&empty[s0]);
-      if (last) mbar_arrive(&empty[s1]);
+      mbar_arrive(ring.empty_a(a.s));
+      mbar_arrive(ring.empty_b(b.s));
+      if (last) mbar_arrive(ring.empty_a(ahead.s));
     }
 
     // this plane's update masks: bit e of byte c = component c of cell e
@@ -1235,7 +1295,7 @@ __device__ __forceinline__ bool velocity_item(const ShotDesc<T> &sd, const Item 
 
     // receivers in this warp's cells (velocity after the update, :593-602)
     if (rlo < rhi)
-      sample_receivers<T, G::NTX, V>(sd.rec_sorted, rlo, rhi, x0, y0, tid, vx, vy, vz, sd.seis + samp, sd.nsamp);
+      sample_receivers<G::NTX, TY>(sd.rec_sorted, rlo, rhi, x0, y0, tid, vx, vy, vz, sd.seis + samp, sd.nsamp);
     if (live) {
       // force source after the update (cudazerocopy.cu:451-453)
       if (src_row && k == sd.src_k) {
@@ -1271,27 +1331,53 @@ __device__ __forceinline__ bool velocity_item(const ShotDesc<T> &sd, const Item 
       st_vec(f1 + g, vy);
       st_vec(f2 + g, vz);
     }
-    n += last ? 2 : 1;
+    a = ahead;
+    if (last) a.next();
+    b.next();
   }
   return true;
 }
 
 // ------------------------------------------------- half-step kernels ----
-// Barrier set-up shared by the kernels: full[s] and full[NS + s] (the parts of
-// a stage) expect the producer's one arrival plus the part's bytes (TMA) or
-// one arrival per lane (cp.async); empty[s] one arrival per consumer warp.
-template <int NS, int NCW, int LOAD>
-__device__ __forceinline__ void init_ring(uint64_t *full, uint64_t *empty) {
+// Barrier set-up shared by the kernels: full expects the producer's one
+// arrival plus the part's bytes (TMA) or one arrival per lane (cp.async);
+// empty one arrival per consumer warp.
+template <int NCW, int LOAD, typename R>
+__device__ __forceinline__ void init_ring(const R &ring) {
   if (threadIdx.x == 0) {
-    for (int s = 0; s < NS; ++s) {
-      mbar_init(&full[s], LOAD == LOAD_TMA ? 1 : 32);
-      mbar_init(&full[NS + s], LOAD == LOAD_TMA ? 1 : 32);
-      mbar_init(&empty[s], NCW);
+    for (int s = 0; s < R::NA + R::NB; ++s) {
+      mbar_init(ring.bars() + s, LOAD == LOAD_TMA ? 1 : 32);
+      mbar_init(ring.bars() + R::NA + R::NB + s, NCW);
     }
     fence_mbar_init();
   }
   __syncthreads();
 }
+
+// The loading warp of the half-step kernels: the block's items in turn.
+template <bool ASYNC, typename R, typename IssueA, typename IssueB, typename Prefetch>
+__device__ __forceinline__ void produce(const Item *__restrict__ items, int2 range, const R &ring, IssueA issue_a,
+                                        IssueB issue_b, Prefetch &prefetch, unsigned *__restrict__ err, int ctl,
+                                        int lane) {
+  if (ctl & CTL_WITHHOLD_LOADS) return;  // test mode: no place is ever filled
+  Loads<R> ld;
+  bool ok = true;
+  for (int ii = range.x; ii < range.y && ok; ++ii) {
+    const Item it = items[ii];
+    prefetch.begin(it);
+    ok = produce_item<ASYNC>(
+        it, ring, ld, [&](int k, unsigned char *st, uint64_t *bar) { issue_a(it, k, st, bar, lane); },
+        [&](int k, unsigned char *st, uint64_t *bar) { issue_b(it, k, st, bar, lane); }, prefetch, lane);
+  }
+  produce_drain<ASYNC>(ring, ld, ok, err, lane);
+}
+
+// Rings of the half-step kernels, and their shared memory: the rings, the
+// memory-variable slots behind them.
+template <typename G> using StressRing = Ring<G::NS, G::places_b(G::S_A, G::S_B, 128), G::S_A, G::S_B>;
+template <typename G> using VelocityRing = Ring<G::NS, G::places_b(G::V_A, G::V_B, 128), G::V_A, G::V_B>;
+template <typename G, typename R> constexpr int kPsiOffset = (R::BYTES + 127) & ~127;
+template <typename G, typename R> constexpr int kKernelSmem = kPsiOffset<G, R> + G::PSI_BYTES;
 
 // (tick and dtick are unused by the stress half-step; the parameter list is
 // shared with the velocity kernel so both launch from one argument array)
@@ -1301,30 +1387,37 @@ __global__ void __launch_bounds__(Geo<T, TX, TY, NS, CPT, MB>::THREADS, Geo<T, T
                   const Item *__restrict__ items, const int2 *__restrict__ ranges, int tick,
                   const int *__restrict__ dtick, unsigned *__restrict__ err, int ctl) {
   using G = Geo<T, TX, TY, NS, CPT, MB>;
+  using R = StressRing<G>;
   extern __shared__ __align__(1024) unsigned char smem[];
-  uint64_t *full = reinterpret_cast<uint64_t *>(smem + NS * G::S_STAGE);
-  uint64_t *empty = full + 2 * NS;
+  const R ring{smem};
 
   const int tid = threadIdx.x;
   const int2 range = ranges[blockIdx.x];
   if (range.x >= range.y) return;
-  init_ring<NS, G::NCW, LOAD>(full, empty);
+  init_ring<G::NCW, LOAD>(ring);
 
   if (tid >= G::NT) {  // producer warp
-    auto issue = [&](const Item &it, int k, int slot, uint64_t *bar, uint64_t *rest, bool ahead, int lane) {
-      stress_issue<T, TX, TY, NS, CPT, MB, LOAD>(shots, maps, it, k, smem + slot * G::S_STAGE, bar, rest, ahead, lane);
+    if constexpr (G::SPLIT) fewer_registers<G::LOADER_REGS>();
+    const int lane = tid - G::NT;
+    if (lane >= 32) return;   // (the rest of its group)
+    auto issue_a = [&](const Item &it, int k, unsigned char *st, uint64_t *bar, int l) {
+      stress_issue_a<G, LOAD>(shots[it.shot], maps[it.shot], it, k, st, bar, l);
     };
-    ItemPrefetch<T, TX, TY> prefetch{{}, shots, tid - G::NT, ctl, PSI_S0};
-    produce<NS, LOAD == LOAD_CP_ASYNC>(items, range, full, empty, issue, prefetch, err, ctl, tid - G::NT);
+    auto issue_b = [&](const Item &it, int k, unsigned char *st, uint64_t *bar, int l) {
+      stress_issue_b<G, LOAD>(shots[it.shot], maps[it.shot], it, k, st, bar, l);
+    };
+    ItemPrefetch<T, TX, TY> prefetch{{}, shots, lane, ctl, PSI_S0};
+    produce<LOAD == LOAD_CP_ASYNC>(items, range, ring, issue_a, issue_b, prefetch, err, ctl, lane);
     return;
   }
+  if constexpr (G::SPLIT) more_registers<G::CONSUMER_REGS>();
 
   const unsigned long long wait_ns = (ctl & CTL_WITHHOLD_LOADS) ? kTestWaitLimitNs : kWaitLimitNs;
-  unsigned n = 0;  // index of the load holding the current plane
+  Place<R::NA> a;
+  Place<R::NB> b;
   for (int ii = range.x; ii < range.y; ++ii) {
     const Item item = items[ii];
-    if (!stress_item<T, TX, TY, NS, CPT, MB, G::S_STAGE, false>(shots[item.shot], item, smem, smem + G::S_PSI, full,
-                                                                 empty, n, err, wait_ns, tid))
+    if (!stress_item<G, false>(shots[item.shot], item, ring, a, b, smem + kPsiOffset<G, R>, err, wait_ns, tid))
       return;
   }
 }
@@ -1335,33 +1428,41 @@ __global__ void __launch_bounds__(Geo<T, TX, TY, NS, CPT, MB>::THREADS, Geo<T, T
                     const Item *__restrict__ items, const int2 *__restrict__ ranges, int tick,
                     const int *__restrict__ dtick, unsigned *__restrict__ err, int ctl) {
   using G = Geo<T, TX, TY, NS, CPT, MB>;
+  using R = VelocityRing<G>;
   extern __shared__ __align__(1024) unsigned char smem[];
-  uint64_t *full = reinterpret_cast<uint64_t *>(smem + NS * G::V_STAGE);
-  uint64_t *empty = full + 2 * NS;
+  const R ring{smem};
 
   const int tid = threadIdx.x;
   const int2 range = ranges[blockIdx.x];
   if (range.x >= range.y) return;
-  init_ring<NS, G::NCW, LOAD>(full, empty);
+  init_ring<G::NCW, LOAD>(ring);
 
   if (tid >= G::NT) {  // producer warp
-    auto issue = [&](const Item &it, int k, int slot, uint64_t *bar, uint64_t *rest, bool ahead, int lane) {
-      velocity_issue<T, TX, TY, NS, CPT, MB, LOAD>(shots, maps, it, k, smem + slot * G::V_STAGE, bar, rest, ahead, lane);
+    if constexpr (G::SPLIT) fewer_registers<G::LOADER_REGS>();
+    const int lane = tid - G::NT;
+    if (lane >= 32) return;   // (the rest of its group)
+    auto issue_a = [&](const Item &it, int k, unsigned char *st, uint64_t *bar, int l) {
+      velocity_issue_a<G, LOAD>(shots[it.shot], maps[it.shot], it, k, st, bar, l);
     };
-    ItemPrefetch<T, TX, TY> prefetch{{}, shots, tid - G::NT, ctl, PSI_V0};
-    produce<NS, LOAD == LOAD_CP_ASYNC>(items, range, full, empty, issue, prefetch, err, ctl, tid - G::NT);
+    auto issue_b = [&](const Item &it, int k, unsigned char *st, uint64_t *bar, int l) {
+      velocity_issue_b<G, LOAD>(shots[it.shot], maps[it.shot], it, k, st, bar, l);
+    };
+    ItemPrefetch<T, TX, TY> prefetch{{}, shots, lane, ctl, PSI_V0};
+    produce<LOAD == LOAD_CP_ASYNC>(items, range, ring, issue_a, issue_b, prefetch, err, ctl, lane);
     return;
   }
+  if constexpr (G::SPLIT) more_registers<G::CONSUMER_REGS>();
 
   const unsigned long long wait_ns = (ctl & CTL_WITHHOLD_LOADS) ? kTestWaitLimitNs : kWaitLimitNs;
   // step counter: an argument for direct launches, device memory plus an
   // offset inside a replayable CUDA graph
   if (dtick) tick += *dtick;
-  unsigned n = 0;
+  Place<R::NA> a;
+  Place<R::NB> b;
   for (int ii = range.x; ii < range.y; ++ii) {
     const Item item = items[ii];
-    if (!velocity_item<T, TX, TY, NS, CPT, MB, G::V_STAGE, false>(shots[item.shot], item, tick, smem, smem + G::V_PSI,
-                                                                   full, empty, n, err, wait_ns, tid))
+    if (!velocity_item<G, false>(shots[item.shot], item, tick, ring, a, b, smem + kPsiOffset<G, R>, err, wait_ns,
+                                 tid))
       return;
   }
 }
@@ -1407,13 +1508,13 @@ __global__ void __launch_bounds__(Geo<T, TX, TY, NS, CPT, MB>::THREADS, Geo<T, T
 // item's ready barrier and then issues its loads; consumers read global
 // memory for the item only after that barrier.  Every wait is bounded: a wait that passes its limit
 // sets DEV_ERR_TIMEOUT and the block stops.
-// RB ready barriers: the producer is at most NS loads ahead of the slowest
-// consumer warp and every item takes at least two loads, so it never gets
+// RB ready barriers: the producer is at most NA loads ahead of the slowest
+// consumer warp and every item takes at least two of them, so it never gets
 // RB items ahead (a barrier is re-armed only after every warp passed it).
 template <typename T, int TX, int TY, int NS, int CPT, int MB>
 struct Flow {
   using G = Geo<T, TX, TY, NS, CPT, MB>;
-  static constexpr int STAGE = G::S_STAGE > G::V_STAGE ? G::S_STAGE : G::V_STAGE;
+  static constexpr int A = G::S_A > G::V_A ? G::S_A : G::V_A, B = G::S_B > G::V_B ? G::S_B : G::V_B;
   static constexpr int RB = 8;
   static_assert(RB >= NS / 2 + 2, "ready barriers for the items in flight");
   // per item in flight: the item (kind < 0: the list is done) and a copy of
@@ -1423,11 +1524,12 @@ struct Flow {
     ShotDesc<T> sd;
   };
   static_assert(sizeof(ShotDesc<T>) % 16 == 0 && sizeof(FlowItem) % 16 == 0, "descriptors are copied 16 bytes at a time");
-  static constexpr int READY = NS * STAGE + G::BARS;
+  using R = Ring<NS, G::places_b(A, B, RB * ((int)sizeof(Slot) + 12) + 128), A, B>;
+  static constexpr int READY = R::BYTES;
   static constexpr int SLOTS = (READY + 8 * RB + 4 * RB + 15) & ~15;
   static constexpr int PSI = (SLOTS + RB * (int)sizeof(Slot) + 15) & ~15;   // memory-variable slots
   static constexpr int SMEM = PSI + G::PSI_BYTES;
-  static_assert(SMEM <= 232448, "shared memory of one block");
+  static_assert(SMEM <= G::MAX_SMEM, "shared memory of one block");
 };
 
 __device__ __forceinline__ int ld_relaxed_gpu(const int *p) {
@@ -1447,54 +1549,34 @@ __device__ __forceinline__ int atom_acq_rel_cta_add(int *p, int v) {
   return old;
 }
 
-// Lane 0 of the producer: waits until every counter this item depends on
-// has reached its target.  The (up to ten) counters are read together, so
-// a satisfied item costs one L2 round trip.
+// The producer warp: waits until every counter this item depends on has
+// reached its target.  Each of the (up to ten) counters is read by a lane of
+// its own, so a satisfied item costs one L2 round trip.
 template <typename T>
 __device__ __forceinline__ bool flow_wait_deps(const ShotDesc<T> &sd, const FlowItem &fi, int txs, int tys, int ncw,
-                                               unsigned long long wait_ns) {
+                                               unsigned long long wait_ns, int lane) {
   const int ntiles = txs * tys;
   const int tile = fi.it.tile, tx = tile % txs, ty = tile / txs;
-  const int *base;
-  int c0, c1, target;
-  if (fi.kind == 0) {   // stress: velocity of the previous step, chunks j and j+1
-    base = sd.flow_flags + (size_t)sd.flow_chunks * ntiles;
-    c0 = fi.chunk;
-    c1 = fi.chunk + 1 < sd.flow_chunks ? fi.chunk + 1 : -1;
-    target = ncw * fi.step;
-  } else {              // velocity: stress of this step, chunks j-1 and j
-    base = sd.flow_flags;
-    c0 = fi.chunk;
-    c1 = fi.chunk > 0 ? fi.chunk - 1 : -1;
-    target = ncw * (fi.step + 1);
-  }
+  // stress: velocity of the previous step, chunks j and j+1; velocity: stress
+  // of this step, chunks j and j-1
+  const int target = ncw * (fi.kind == 0 ? fi.step : fi.step + 1);
   if (target <= 0) return true;
-  const int *p[10];
-  int np = 0;
-  const int nb[5][2] = {{tx, ty}, {tx - 1, ty}, {tx + 1, ty}, {tx, ty - 1}, {tx, ty + 1}};
-#pragma unroll
-  for (int q = 0; q < 5; ++q) {
-    const int x = nb[q][0], y = nb[q][1];
-    if (x < 0 || x >= txs || y < 0 || y >= tys) continue;
-    p[np++] = base + (size_t)c0 * ntiles + y * txs + x;
-    if (c1 >= 0) p[np++] = base + (size_t)c1 * ntiles + y * txs + x;
-  }
+  const int q = lane >> 1;   // 0: the tile itself, 1..4: its neighbours
+  const int x = tx + (q == 2) - (q == 1), y = ty + (q == 4) - (q == 3);
+  const int c = fi.chunk + ((lane & 1) ? (fi.kind == 0 ? 1 : -1) : 0);
+  const bool mine = lane < 10 && x >= 0 && x < txs && y >= 0 && y < tys && c >= 0 && c < sd.flow_chunks;
+  const int *p = sd.flow_flags + ((fi.kind == 0 ? (size_t)sd.flow_chunks : 0) + (mine ? c : 0)) * ntiles +
+                 (mine ? y * txs + x : 0);
   unsigned long long t0 = 0;
-  for (;;) {
-    int v[10];
-#pragma unroll
-    for (int q = 0; q < 10; ++q) v[q] = q < np ? ld_relaxed_gpu(p[q]) : target;
-    bool ok = true;
-#pragma unroll
-    for (int q = 0; q < 10; ++q) ok = ok && v[q] >= target;
-    if (ok) break;
+  while (!__all_sync(0xffffffffu, !mine || ld_relaxed_gpu(p) >= target)) {
     const unsigned long long t = globaltimer_ns();
     if (t0 == 0) t0 = t;
-    else if (t - t0 > wait_ns) return false;
+    else if (__any_sync(0xffffffffu, t - t0 > wait_ns)) return false;
     __nanosleep(64);
   }
   fence_acq_rel_gpu();
   fence_proxy_async_global();
+  __syncwarp();
   return true;
 }
 
@@ -1506,9 +1588,9 @@ __global__ void __launch_bounds__(Geo<T, TX, TY, NS, CPT, MB>::THREADS, Geo<T, T
   using G = Geo<T, TX, TY, NS, CPT, MB>;
   using F = Flow<T, TX, TY, NS, CPT, MB>;
   extern __shared__ __align__(1024) unsigned char smem[];
-  uint64_t *full = reinterpret_cast<uint64_t *>(smem + NS * F::STAGE);
-  uint64_t *empty = full + 2 * NS;
-  uint64_t *ready = empty + NS;   // F::RB barriers, one per item in flight
+  using R = typename F::R;
+  const R ring{smem};
+  uint64_t *ready = reinterpret_cast<uint64_t *>(smem + F::READY);   // F::RB barriers, one per item in flight
   int *arrived = reinterpret_cast<int *>(ready + F::RB);   // F::RB consumer-warp counters
   typename F::Slot *slots = reinterpret_cast<typename F::Slot *>(smem + F::SLOTS);
   const int tid = threadIdx.x;
@@ -1517,17 +1599,20 @@ __global__ void __launch_bounds__(Geo<T, TX, TY, NS, CPT, MB>::THREADS, Geo<T, T
       mbar_init(&ready[r], 1);
       arrived[r] = 0;
     }
-  init_ring<NS, G::NCW, LOAD_TMA>(full, empty);
+  init_ring<G::NCW, LOAD_TMA>(ring);
   const unsigned long long wait_ns = (ctl & CTL_WITHHOLD_LOADS) ? kTestWaitLimitNs : kWaitLimitNs;
 
   if (tid >= G::NT) {  // producer warp
+    if constexpr (G::SPLIT) fewer_registers<G::LOADER_REGS>();
     const int lane = tid - G::NT;
-    if (ctl & CTL_WITHHOLD_LOADS) return;  // test mode: no stage is ever filled
+    if (lane >= 32) return;   // (the rest of its group)
+    if (ctl & CTL_WITHHOLD_LOADS) return;  // test mode: no place is ever filled
     ItemPrefetch<T, TX, TY> pf_s{{}, shots, lane, ctl, PSI_S0};
     ItemPrefetch<T, TX, TY> pf_v{{}, shots, lane, ctl, PSI_V0};
     const int pass_steps = list_steps > 0 ? list_steps : nsteps;   // (one pass if the list's length is unset)
     const int total = nitems * ((nsteps + pass_steps - 1) / pass_steps);
-    unsigned n = 0, idx = 0;
+    Loads<R> ld;
+    unsigned idx = 0;
     bool ok = true;
     if (dtick) tick += *dtick;
     int next = 0;   // lane 0: the place claimed next
@@ -1557,39 +1642,40 @@ __global__ void __launch_bounds__(Geo<T, TX, TY, NS, CPT, MB>::THREADS, Geo<T, T
         __syncwarp();   // (the slot is filled again next)
         continue;
       }
-      int good = 1;
-      if (lane == 0) {
-        if (!end) {
-          const int txs = (slot.sd.nx + TX - 1) / TX, tys = (slot.sd.ny + TY - 1) / TY;
-          good = flow_wait_deps(slot.sd, fi, txs, tys, G::NCW, wait_ns);
-        }
-        if (good) mbar_arrive(&ready[idx % F::RB]);   // release the consumers' reads
+      if (!end) {
+        const int txs = (slot.sd.nx + TX - 1) / TX, tys = (slot.sd.ny + TY - 1) / TY;
+        ok = flow_wait_deps(slot.sd, fi, txs, tys, G::NCW, wait_ns, lane);
       }
+      if (ok && lane == 0) mbar_arrive(&ready[idx % F::RB]);   // release the consumers' reads
       ++idx;
-      ok = __shfl_sync(0xffffffffu, good, 0);
       if (!ok || end) break;
+      const ShotMaps &sm = maps[fi.it.shot];
       if (fi.kind == 0) {
-        auto issue = [&](const Item &it, int k, int st, uint64_t *bar, uint64_t *rest, bool ahead, int l) {
-          stress_issue<T, TX, TY, NS, CPT, MB, LOAD_TMA>(shots, maps, it, k, smem + st * F::STAGE, bar, rest, ahead, l);
-        };
         pf_s.begin(fi.it, slot.sd);
-        ok = produce_item<NS, false>(fi.it, n, full, empty, issue, pf_s, lane);
+        ok = produce_item<false>(
+            fi.it, ring, ld,
+            [&](int k, unsigned char *st, uint64_t *bar) { stress_issue_a<G, LOAD_TMA>(slot.sd, sm, fi.it, k, st, bar, lane); },
+            [&](int k, unsigned char *st, uint64_t *bar) { stress_issue_b<G, LOAD_TMA>(slot.sd, sm, fi.it, k, st, bar, lane); },
+            pf_s, lane);
       } else {
-        auto issue = [&](const Item &it, int k, int st, uint64_t *bar, uint64_t *rest, bool ahead, int l) {
-          velocity_issue<T, TX, TY, NS, CPT, MB, LOAD_TMA>(shots, maps, it, k, smem + st * F::STAGE, bar, rest, ahead, l);
-        };
         pf_v.begin(fi.it, slot.sd);
-        ok = produce_item<NS, false>(fi.it, n, full, empty, issue, pf_v, lane);
+        ok = produce_item<false>(
+            fi.it, ring, ld,
+            [&](int k, unsigned char *st, uint64_t *bar) { velocity_issue_a<G, LOAD_TMA>(slot.sd, sm, fi.it, k, st, bar, lane); },
+            [&](int k, unsigned char *st, uint64_t *bar) { velocity_issue_b<G, LOAD_TMA>(slot.sd, sm, fi.it, k, st, bar, lane); },
+            pf_v, lane);
       }
       if (!ok) break;
     }
-    produce_drain<NS, false>(n, ok, full, err, lane);
+    produce_drain<false>(ring, ld, ok, err, lane);
     return;
   }
+  if constexpr (G::SPLIT) more_registers<G::CONSUMER_REGS>();
 
   const int lane = tid & 31;
   if (dtick) tick += *dtick;
-  unsigned n = 0;
+  Place<R::NA> a;
+  Place<R::NB> b;
   for (unsigned idx = 0;; ++idx) {
     if (!flow_ready(&ready[idx % F::RB], (idx / F::RB) & 1, wait_ns, err, lane)) return;
     const typename F::Slot &slot = slots[idx % F::RB];
@@ -1598,11 +1684,10 @@ __global__ void __launch_bounds__(Geo<T, TX, TY, NS, CPT, MB>::THREADS, Geo<T, T
     const ShotDesc<T> &sd = slot.sd;
     bool ok;
     if (fi.kind == 0)
-      ok = stress_item<T, TX, TY, NS, CPT, MB, F::STAGE, true>(sd, fi.it, smem, smem + F::PSI, full, empty, n, err,
-                                                                wait_ns, tid, fi.step > 0 ? tick + fi.step - 1 : INT_MIN);
+      ok = stress_item<G, true>(sd, fi.it, ring, a, b, smem + F::PSI, err, wait_ns, tid,
+                                fi.step > 0 ? tick + fi.step - 1 : INT_MIN);
     else
-      ok = velocity_item<T, TX, TY, NS, CPT, MB, F::STAGE, true>(sd, fi.it, tick + fi.step, smem, smem + F::PSI, full,
-                                                                  empty, n, err, wait_ns, tid);
+      ok = velocity_item<G, true>(sd, fi.it, tick + fi.step, ring, a, b, smem + F::PSI, err, wait_ns, tid);
     if (!ok) return;
     // this warp's share of the item is written: it arrives (CTA scope) on
     // the item's counter, and the last warp to arrive releases the whole

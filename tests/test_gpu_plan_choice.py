@@ -28,7 +28,12 @@ def _run(p, cp, cs, rho, **kw):
     (113, 17, 50),      # one column past a 112-wide tile
     (127, 64, 90),      # 128x7
     (150, 211, 60),     # 32x28, claimed places
-    (130, 150, 160),    # claimed, 64x14
+    (130, 150, 160),    # claimed, 64-wide
+    (128, 32, 60),      # 128x8, eight consumer warps
+    (192, 48, 40),      # 64x16
+    (160, 64, 40),      # 32x32
+    (201, 63, 33),      # 112x9, whose last threads have no cells
+    (112, 36, 40),      # 56x18 or 112x9, one row past a tile's edge less
     (3, 3, 3),
     (400, 5, 3),
 ])
