@@ -550,9 +550,10 @@ TuneChoice plan_choice(const ela3d_params &p) {
 // prefetches 43.7 and 38.0.)
 // A server's shots are prepared while others run: the dataflow kernel would
 // hold every SM for many steps and keep the preparation's kernels waiting, so
-// a server keeps the two kernels, on the tile that was best for uneven grids
-// (ten of them, 32-plane chunks: 38.5, 128x7 with 10 planes 35.6); chunk 0:
-// sized for the shots running.
+// a server keeps the two kernels, on the tile that was best for bursts of
+// requests with lognormal edges (16, 15 and 20 of them, ms with 10-plane
+// chunks: 64x16 141 133 130, 64x14 145 136 134, 32x32 141 136 133, 128x8 150
+// 138 135; 64x16 with 32 planes 148 139 142).
 TuneChoice batch_choice(const std::vector<ela3d_params> &ps, int fp64) {
   TuneChoice c = default_choice(fp64, 0, 0, 0);
   int n = 0;
@@ -563,8 +564,9 @@ TuneChoice batch_choice(const std::vector<ela3d_params> &ps, int fp64) {
   c.chunk = 0;
   if (ps.empty()) {
     for (int j = 0; j < n; ++j)
-      if (!v[j].fp64 && v[j].loads == LOAD_TMA && v[j].tx == 64 && v[j].ty == 14) c.variant = j;
+      if (!v[j].fp64 && v[j].loads == LOAD_TMA && v[j].tx == 64 && v[j].ty == 16) c.variant = j;
     c.kind = 1;
+    c.chunk = 10;
   } else {
     c.variant = pick_tile(ps, fp64 != 0, true, c.variant);
     c.kind = kScheduleFlowOverlap;
@@ -1289,16 +1291,8 @@ class Engine final : public EngineBase {
     std::vector<Item> items;
     std::vector<int2> ranges;
     const int kind = choice_.kind >= kScheduleFlow ? 1 : choice_.kind;
-    int chunk = choice_.chunk;
-    if (chunk <= 0) {
-      // sized for the shots running: 32 planes once they fill the GPU,
-      // shorter while that leaves fewer than about six items per block
-      long long planes = 0;
-      for (const ShotShape &sh : shapes)
-        planes += (long long)((sh.nx + var_->tx - 1) / var_->tx) * ((sh.ny + var_->ty - 1) / var_->ty) * sh.nz;
-      chunk = (int)std::max<long long>(8, std::min<long long>(32, planes / (6ll * per_sm_ * num_sms_)));
-    }
-    build_schedule(shapes, var_->tx, var_->ty, kind, chunk, per_sm_ * num_sms_, &items, &ranges);
+    build_schedule(shapes, var_->tx, var_->ty, kind, std::max(choice_.chunk, 1), per_sm_ * num_sms_, &items,
+                   &ranges);
     if (items.empty()) BAD("empty schedule");
     for (const Item &it : items)
       if (it.k1 <= it.k0) BAD("internal: empty work item");
@@ -1340,11 +1334,19 @@ class Engine final : public EngineBase {
       shapes.push_back({d.nx, d.ny, d.nz, q, c});
       per_step += 2 * tiles_of(d) * ((d.nz + c - 1) / c);
     }
-    // (shots that run together change more often than a plan's, and their
-    // longer steps hide the seam between two walks of a short list)
-    const long long most = active.size() > 1 ? kFlowBatchItems : kFlowMaxItems;
-    const int K = (int)std::max<long long>(1, std::min<long long>(flow_max_steps_, most / std::max(1ll, per_step)));
-    flow_walks_ = active.size() > 1 ? std::max(flow_passes_, (kFlowSteps * kFlowPasses + K - 1) / K) : flow_passes_;
+    // The list's steps: building it costs the host about 16 us per 1000 items.
+    // A plan that streams from HBM gets all of flow_max_steps_ (512^3: 50 steps
+    // 51.0 Gcell-updates/s, 16 50.0); near the L2 size, and in FP64, ten do as
+    // well (101^3 35.4 and 35.3, 128^3 43.1 and 43.1).  Shots that run together change more
+    // often than a plan's, and their longer steps hide the seam between two
+    // walks of a short list.
+    double bytes = 0.0;
+    for (int q : active) bytes += 12.0 * sizeof(T) * shots_[q]->d.px * shots_[q]->d.ny * shots_[q]->d.nz;
+    const bool together = active.size() > 1, streams = sizeof(T) == 4 && bytes > 400e6;
+    const long long most = together ? kFlowBatchItems : kFlowMaxItems;
+    const int steps = together || streams ? flow_max_steps_ : std::min(flow_max_steps_, 10);
+    const int K = (int)std::max<long long>(1, std::min<long long>(steps, most / std::max(1ll, per_step)));
+    flow_walks_ = std::max(flow_passes_, (together || !streams) ? (kFlowSteps * kFlowPasses + K - 1) / K : 0);
     std::vector<FlowItem> items;
     std::vector<int> off, nch;
     int nflags = 0;
