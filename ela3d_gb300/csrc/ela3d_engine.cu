@@ -878,19 +878,29 @@ class Engine final : public EngineBase {
       const float *src[3] = {cp, cs, rho};
       T *dst[3] = {const_cast<T *>(d.cp), const_cast<T *>(d.cs), const_cast<T *>(d.rho)};
       const size_t compact = (size_t)nx * ny * nz * sizeof(float);
-      if (sizeof(T) == 4 && px == nx) {
-        for (int c = 0; c < 3; ++c) CK(cudaMemcpyAsync(dst[c], src[c], compact, cudaMemcpyHostToDevice, setup_));
-      } else {
-        // rows are padded (or widened): the arrays go up in one piece each,
-        // staged in the fields vx vy vz, which are zeroed again.  (A copy of
-        // rows that are no multiple of 128 bytes runs at a tenth of the
-        // link's rate: a plan of 201^3 cells took 5.5 ms to create, now 1.6.)
-        for (int c = 0; c < 3; ++c) {
-          float *stage = reinterpret_cast<float *>(d.f[c]);
-          CK(cudaMemcpyAsync(stage, src[c], compact, cudaMemcpyHostToDevice, setup_));
-          CK(Fp<T>::pad(stage, dst[c], nx, ny, nz, px, setup_));
-          CK(cudaMemsetAsync(stage, 0, compact, setup_));
+      for (int c = 0; c < 3; ++c) {
+        // page-locked arrays: the kernel that pads (and widens) the rows reads
+        // them over the link
+        cudaPointerAttributes at{};
+        const bool mapped = cudaPointerGetAttributes(&at, src[c]) == cudaSuccess && at.type == cudaMemoryTypeHost &&
+                            at.devicePointer && (uintptr_t)at.devicePointer % 16 == 0;
+        if (mapped) {
+          CK(Fp<T>::pad(static_cast<const float *>(at.devicePointer), dst[c], nx, ny, nz, px, setup_));
+          continue;
         }
+        cudaGetLastError();   // (a pointer CUDA does not know is no error)
+        if (sizeof(T) == 4 && px == nx) {
+          CK(cudaMemcpyAsync(dst[c], src[c], compact, cudaMemcpyHostToDevice, setup_));
+          continue;
+        }
+        // others go up in one piece each, staged in the fields vx vy vz, which
+        // are zeroed again.  (A copy of rows that are no multiple of 128 bytes
+        // runs at a tenth of the link's rate: a plan of 201^3 cells took 5.5
+        // ms to create, now 1.6.)
+        float *stage = reinterpret_cast<float *>(d.f[c]);
+        CK(cudaMemcpyAsync(stage, src[c], compact, cudaMemcpyHostToDevice, setup_));
+        CK(Fp<T>::pad(stage, dst[c], nx, ny, nz, px, setup_));
+        CK(cudaMemsetAsync(stage, 0, compact, setup_));
       }
     }
     // 4. source time function (FP64 on the device)
