@@ -478,15 +478,16 @@ static int device_sms() {
 // 37.5 40.2.  A tile that leaves fewer two-plane items than there are blocks
 // counts for less (64^3: 64x14 19.5, 64x16 17.2).  FP64 is bound by its arithmetic, and a thread without a
 // cell costs as much as one with: 101^3 with 32x7, 16x14 and 8x28 tiles (76%,
-// 81% and 88% used) 3.34, 3.65 and 3.83; 180^3 (93%, 93%, 90%) 4.57, 4.62 and
-// 4.48.  For several shots the cells' summed time decides.
+// 81% and 88% used) 3.46, 3.75 and 3.98; 180^3 (93%, 93%, 90%) 4.71, 4.75 and
+// 4.62; 128^3 with 32x7, 32x8 and 16x16 (96%, 100%, 100%) 4.63, 4.70 and 4.85.  For several shots the cells' summed time decides.
 static int pick_tile(const std::vector<ela3d_params> &ps, bool fp64, bool streams, int fallback) {
   int n = 0;
   const Variant *v = variants(&n);
   const struct { bool fp64; int tx, ty; double w; } shapes[] = {
       {false, 128, 7, 1.0}, {false, 112, 8, 0.985}, {false, 64, 14, 0.96}, {false, 56, 16, streams ? 0.88 : 0.93},
       {false, 32, 28, streams ? 0.85 : 0.98}, {false, 128, 8, 1.01}, {false, 112, 9, 0.99}, {false, 64, 16, 0.975},
-      {false, 56, 18, streams ? 0.88 : 0.94}, {false, 32, 32, streams ? 0.86 : 1.0}, {true, 32, 7, 1.0}, {true, 16, 14, 1.0}, {true, 8, 28, 1.0}};
+      {false, 56, 18, streams ? 0.88 : 0.94}, {false, 32, 32, streams ? 0.86 : 1.0}, {true, 32, 7, 1.0}, {true, 16, 14, 1.015}, {true, 8, 28, 1.0},
+      {true, 32, 8, 1.005}, {true, 16, 16, 1.03}};
   const double sms = device_sms();
   int pick = fallback;
   double best = 0.0;

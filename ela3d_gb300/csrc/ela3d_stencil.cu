@@ -73,6 +73,8 @@ static const Variant kVariants[] = {
     // and narrow FP64 tiles: its arithmetic bounds FP64, idle lanes included
     make_variant<double, 16, 14, 4, 1>(),
     make_variant<double, 8, 28, 4, 1>(),
+    make_variant<double, 32, 8, 4, 1>(),
+    make_variant<double, 16, 16, 4, 1>(),
 };
 
 const Variant *variants(int *count) {

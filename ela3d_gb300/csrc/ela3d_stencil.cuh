@@ -45,7 +45,7 @@ struct Geo {
   // be a ninth, a sub-partition's third.  They are launched as three warpgroups
   // of 168 registers a thread, and the loading warp's group hands registers over
   // to the consumers (setmaxnreg; 8 x 216 + 4 x 72 = 12 x 168).
-  static constexpr bool SPLIT = NCW == 8 && sizeof(T) == 4;
+  static constexpr bool SPLIT = NCW == 8;
   static constexpr int CONSUMER_REGS = 216, LOADER_REGS = 72;
   static_assert(8 * CONSUMER_REGS + 4 * LOADER_REGS <= 12 * 168, "registers of the launch");
   static constexpr int THREADS = SPLIT ? 384 : NT + 32;  // + the loading warp (or its group)
@@ -248,26 +248,33 @@ __device__ __forceinline__ void keep_masked(T (&s)[V], const T (&n)[V], unsigned
 __device__ __forceinline__ float dt_over_rho(float dt, float R) { return __fdividef(dt, mul_rn(R, 0.5f)); }
 // FP64: the IEEE quotient dt / (R / 2) = 2 dt / R, with fewer FP64
 // operations than a general division: the FP64 pipe (two lanes a cycle on
-// each SM) bounds the FP64 kernels.  R is a sum of two float32 model values.  Its reciprocal starts from the FP32 unit (relative error 2^-22,
-// widened and narrowed by integer operations), takes one cubic Newton step
-// (e = 1 - R y; y (1 + e + e^2)), and the quotient one Markstein correction
-// (P. Markstein, "Computation of elementary functions on the IBM RISC
-// System/6000 processor", 1990): q + (2 dt - q R) y rounds to the IEEE
-// quotient, because a quotient by a 26-bit R stays 2^-27 of an ulp away from
-// the midpoints between doubles, far more than the correction's error.
-// Anything outside the normal float32 range divides as usual.
+// each SM) bounds the FP64 kernels.  R is a sum of two float32 model values.
+// Its reciprocal is found in pairs of float32 numbers on the FP32 unit (R = rh
+// + rl; y = yf + yl from the hardware reciprocal yf of rh and one cubic Newton
+// step, e = 1 - R yf, yl = yf (e + e^2); relative error about 2^-44), and the
+// quotient takes one Markstein correction (P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", 1990): q + (2
+// dt - q R) y is off by 2^-88 before its rounding, while a quotient by a
+// 26-bit R stays 2^-80 away from the midpoints between doubles, so it rounds
+// to the IEEE quotient (2e8 random quotients agree).  Floats are widened by
+// integer operations.  Sums outside [2^-60, 2^60) divide as usual.
+__device__ __forceinline__ double widen_signed(float f) {   // (0 becomes 2^-127)
+  const unsigned b = __float_as_uint(f);
+  return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(b << 29));
+}
 __device__ __forceinline__ double dt_over_rho(double dt, double R) {
   const double a = 2.0 * dt;
   const int hi = __double2hiint(R);
-  // 2^-100 <= R < 2^100
-  if ((unsigned)(hi - 0x39b00000) >= 0x0c800000u) return a / R;
-  const float rf = __uint_as_float(((unsigned)(hi - 0x38000000) << 3) | ((unsigned)__double2loint(R) >> 29));
+  if ((unsigned)(hi - 0x3c300000) >= 0x07800000u) return a / R;
+  const unsigned lo = (unsigned)__double2loint(R);
+  const unsigned hb = ((unsigned)(hi - 0x38000000) << 3) | (lo >> 29);   // rh: the first 24 bits
+  const float rh = __uint_as_float(hb);
+  const float rl = (float)(lo & 0x1fffffffu) * __uint_as_float((hb & 0x7f800000u) - (52u << 23));
   float yf;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(rf));
-  const unsigned yb = __float_as_uint(yf);
-  const double y0 = __hiloint2double((int)((yb >> 3) + 0x38000000u), (int)(yb << 29));
-  const double e = fma_rn(-R, y0, 1.0);
-  const double y = fma_rn(y0, fma_rn(e, e, e), y0);
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(rh));
+  const float e = __fmaf_rn(-rl, yf, __fmaf_rn(-rh, yf, 1.0f));
+  const float yl = __fmul_rn(__fmaf_rn(e, e, e), yf);
+  const double y = add_rn(widen_signed(yf), widen_signed(yl));
   const double q = mul_rn(a, y);
   return fma_rn(fma_rn(-q, R, a), y, q);
 }

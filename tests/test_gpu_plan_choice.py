@@ -60,7 +60,8 @@ def test_open_plan_equals_two_kernels(n, explosive):
         assert np.array_equal(a, b)
 
 
-@pytest.mark.parametrize("n", [(32, 14, 20), (33, 15, 64), (16, 28, 70), (101, 101, 33), (9, 57, 40), (3, 3, 3)])
+@pytest.mark.parametrize("n", [(32, 14, 20), (33, 15, 64), (16, 28, 70), (101, 101, 33), (9, 57, 40), (3, 3, 3), (32, 16, 40),
+                               (64, 8, 33)])
 @pytest.mark.parametrize("explosive", [False, True], ids=["force", "explosive"])
 def test_open_fp64_plan_equals_two_kernels(n, explosive):
     """The same in FP64: each of its tiles and one cell past their edges."""
