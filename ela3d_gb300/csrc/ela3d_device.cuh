@@ -99,6 +99,7 @@ struct alignas(16) ShotDesc {
 struct ShotMaps {
   CUtensorMap stress[12];
   CUtensorMap vel[10];
+  CUtensorMap coef[8];   // the update coefficients TX x TY at (x0,y0), when the shot has them
 };
 
 // One work item: a z-run [k0, k1) of one x-y tile of one shot.

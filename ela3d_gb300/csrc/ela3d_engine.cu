@@ -7,6 +7,7 @@
 #include <unistd.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -621,7 +622,9 @@ struct Shot {
   int lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
   char *pool = nullptr;
   T *prof = nullptr;
-  size_t pool_bytes = 0, prof_bytes = 0;
+  T *coef = nullptr;   // update coefficients (FP64 dataflow kernel), or null
+  bool coef_own = false;
+  size_t pool_bytes = 0, prof_bytes = 0, coef_bytes = 0;
   int model_of = -1;   // shot that owns the model arrays (-1: self)
   ShotDesc<T> d{};
   ShotMaps maps{};
@@ -1031,8 +1034,13 @@ class Engine final : public EngineBase {
   void release_shot(Shot<T> &s) {
     if (s.pool) cudaFree(s.pool);
     if (s.prof) cudaFree(s.prof);
+    if (s.coef && s.coef_own) {
+      cudaFree(s.coef);
+      coef_bytes_held() -= (long long)s.coef_bytes;
+    }
     s.pool = nullptr;
     s.prof = nullptr;
+    s.coef = nullptr;
   }
 
   ela3d_status finalize(const TuneChoice *choice) override {
@@ -1047,6 +1055,11 @@ class Engine final : public EngineBase {
     var_ = &vs[c.variant];
     choice_ = c;
     prefetch_ = prefetch_env_ >= 0 ? prefetch_env_ : (c.prefetch & (CTL_PF_X | CTL_PF_YZ));
+    if (flow_wanted(c))
+      for (auto &sp : shots_) {
+        ela3d_status st = make_coef(*sp);
+        if (st != ELA3D_OK) return st;
+      }
     for (auto &sp : shots_) {
       ela3d_status st = encode_shot_maps(*sp);
       if (st != ELA3D_OK) return st;
@@ -1055,6 +1068,8 @@ class Engine final : public EngineBase {
     CK(cudaFuncSetAttribute(var_->velocity, cudaFuncAttributeMaxDynamicSharedMemorySize, var_->vel_smem));
     if (var_->flow)
       CK(cudaFuncSetAttribute(var_->flow, cudaFuncAttributeMaxDynamicSharedMemorySize, var_->flow_smem));
+    if (var_->flow_coef)
+      CK(cudaFuncSetAttribute(var_->flow_coef, cudaFuncAttributeMaxDynamicSharedMemorySize, var_->flow_coef_smem));
     ela3d_status ost = occupancy(c);
     if (ost != ELA3D_OK) return ost;
     if (!shots_.empty()) {
@@ -1074,9 +1089,61 @@ class Engine final : public EngineBase {
     prefetch_ = prefetch_env_ >= 0 ? prefetch_env_ : (c.prefetch & (CTL_PF_X | CTL_PF_YZ));
     ela3d_status ost = occupancy(c);
     if (ost != ELA3D_OK) return ost;
+    if (flow_wanted(c))
+      for (auto &sp : shots_) {
+        if (sp->coef) continue;
+        ela3d_status st = make_coef(*sp);
+        if (st == ELA3D_OK && sp->coef) st = encode_shot_maps(*sp);
+        if (st != ELA3D_OK) return st;
+        tables_dirty_ = true;
+      }
     sched_valid_ = false;
     sched_key_.clear();
     return rebuild_schedule();
+  }
+
+  static bool flow_wanted(const TuneChoice &c) { return c.kind == kScheduleFlow || c.kind == kScheduleFlowOverlap; }
+
+  // Device bytes that coefficient arrays hold in this process.
+  static std::atomic<long long> &coef_bytes_held() {
+    static std::atomic<long long> held{0};
+    return held;
+  }
+
+  // Update coefficients of an FP64 shot, for the dataflow kernel that reads
+  // them instead of deriving them from the model in every step: 43 of about 97
+  // FP64 operations per cell, and FP64 arithmetic is what bounds it (101^3 258
+  // us a step without them, 170 with; 160x128x144 618 and 395).  They take 64 bytes a cell beside the
+  // shot's other 130 or so, so they are an extra: at most kCoefBytes in a
+  // process and a quarter of the memory that is free; a shot that gets none
+  // runs the kernel without.  Shots of one model and time step share them.
+  ela3d_status make_coef(Shot<T> &s) {
+    if constexpr (sizeof(T) == 8) {
+      if (!var_->flow_coef || s.coef) return ELA3D_OK;
+      if (s.model_of >= 0 && shots_[s.model_of]->coef && shots_[s.model_of]->d.dt == s.d.dt) {
+        s.coef = shots_[s.model_of]->coef;
+        return ELA3D_OK;
+      }
+      const size_t bytes = 8 * sizeof(T) * (size_t)s.d.px * s.d.ny * s.d.nz;
+      size_t fr = 0, tot = 0;
+      CK(cudaMemGetInfo(&fr, &tot));
+      if (bytes > fr / 4) return ELA3D_OK;
+      if ((coef_bytes_held() += (long long)bytes) > kCoefBytes) {
+        coef_bytes_held() -= (long long)bytes;
+        return ELA3D_OK;
+      }
+      if (cudaMalloc(&s.coef, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        s.coef = nullptr;
+        coef_bytes_held() -= (long long)bytes;
+        return ELA3D_OK;
+      }
+      s.coef_own = true;
+      s.coef_bytes = bytes;
+      CK(launch_coef_f64(s.d, s.coef, setup_));
+      CK(cudaStreamSynchronize(setup_));
+    }
+    return ELA3D_OK;
   }
 
   // Resident blocks per SM of the half-step kernels and of the dataflow
@@ -1091,6 +1158,11 @@ class Engine final : public EngineBase {
     if (var_->flow) {
       int occ_f = 0;
       CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_f, var_->flow, var_->threads, var_->flow_smem));
+      if (var_->flow_coef) {
+        int occ_c = 0;
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_c, var_->flow_coef, var_->threads, var_->flow_coef_smem));
+        occ_f = std::min(occ_f, occ_c);
+      }
       per_sm_flow_ = occ_f;
       if (c.blocks_per_sm > 0) per_sm_flow_ = std::min(per_sm_flow_, c.blocks_per_sm);
     }
@@ -1245,6 +1317,8 @@ class Engine final : public EngineBase {
     ENC(&v[5], d.f[8], TX, TY + 1);      // syz
     ENC(&v[6], d.rho, TX + H, TY + 1);   // rho
     for (int q = 0; q < 3; ++q) ENC(&v[7 + q], d.f[q], TX, TY);
+    if (s.coef)
+      for (int q = 0; q < 8; ++q) ENC(&s.maps.coef[q], s.coef + (size_t)q * px * ny * nz, TX, TY);
 #undef ENC
     return ELA3D_OK;
   }
@@ -1399,6 +1473,8 @@ class Engine final : public EngineBase {
     if (st != ELA3D_OK) return st;
     flow_items_ = (int)items.size();
     flow_steps_ = K;
+    flow_coef_ = var_->flow_coef != nullptr;
+    for (int q : active) flow_coef_ = flow_coef_ && shots_[q]->coef;
     flags_used_ = flags;
     return ELA3D_OK;
   }
@@ -1428,7 +1504,9 @@ class Engine final : public EngineBase {
       CK(cudaEventRecord(e0, stream_));
     }
     const int grid = std::min(per_sm_flow_ * num_sms_, std::max(1, flow_items_));
-    CK(cudaLaunchCooperativeKernel(var_->flow, dim3(grid), dim3(var_->threads), args, var_->flow_smem, stream_));
+    const bool coef = flow_coef_;
+    CK(cudaLaunchCooperativeKernel(coef ? var_->flow_coef : var_->flow, dim3(grid), dim3(var_->threads), args,
+                                   coef ? var_->flow_coef_smem : var_->flow_smem, stream_));
     if (timing_) {
       CK(cudaEventRecord(e1, stream_));
       pending_.push_back({e0, e1, nullptr, nsteps});
@@ -1599,6 +1677,12 @@ class Engine final : public EngineBase {
     Shot<T> &s = *shots_[0];
     CK(cudaStreamSynchronize(stream_));
     CK(cudaMemcpy(s.pool, static_cast<const char *>(buf) + sizeof h, s.pool_bytes, cudaMemcpyHostToDevice));
+    if constexpr (sizeof(T) == 8) {   // (the model came with the checkpoint)
+      if (s.coef) {
+        CK(launch_coef_f64(s.d, s.coef, stream_));
+        CK(cudaStreamSynchronize(stream_));
+      }
+    }
     tick_ = s.d.tick0 + h.step;
     s.e_ref = h.e_ref;
     return ELA3D_OK;
@@ -1667,7 +1751,7 @@ class Engine final : public EngineBase {
     out->nsamp = s.nsamp;
     out->nrec = s.p.nrec;
     out->precision = sizeof(T) == 8 ? ELA3D_FP64 : ELA3D_FP32;
-    out->device_bytes = (int64_t)(s.pool_bytes + s.prof_bytes);
+    out->device_bytes = (int64_t)(s.pool_bytes + s.prof_bytes + s.coef_bytes);
     for (int a = 0; a < 3; ++a) { out->slab_lo[a] = s.lo[a]; out->slab_hi[a] = s.hi[a]; }
     return ELA3D_OK;
   }
@@ -1727,7 +1811,7 @@ class Engine final : public EngineBase {
 
   int64_t device_bytes() const override {
     int64_t b = 0;
-    for (auto &sp : shots_) b += (int64_t)(sp->pool_bytes + sp->prof_bytes);
+    for (auto &sp : shots_) b += (int64_t)(sp->pool_bytes + sp->prof_bytes + sp->coef_bytes);
     return b;
   }
 
@@ -1899,6 +1983,8 @@ class Engine final : public EngineBase {
   int flow_passes_ = kFlowPasses;
   static constexpr long long kFlowMaxItems = 1 << 20, kFlowBatchItems = 1 << 14;
   int flow_walks_ = kFlowPasses;   // walks of the list in one launch
+  bool flow_coef_ = false;         // every shot of the list has its coefficients
+  static constexpr long long kCoefBytes = 8ll << 30;
   FlowItem *d_flow_ = nullptr;
   int *d_flags_ = nullptr;
   size_t flow_cap_ = 0, flags_cap_ = 0, flags_used_ = 0;

@@ -22,10 +22,15 @@ struct Variant {
   const void *velocity;
   const void *flow;     // dataflow kernel (many steps per launch); null if not compiled
   int flow_smem;
+  const void *flow_coef;  // the same with coefficients from arrays; null if not compiled
+  int flow_coef_smem;
 };
 
 // All compiled variants (ela3d_stencil.cu).
 const Variant *variants(int *count);
+
+// The eight arrays of update coefficients of a shot (ela3d_stencil.cu).
+cudaError_t launch_coef_f64(const ShotDesc<double> &shot, double *out, cudaStream_t s);
 
 // Inputs of the FP64 profile kernel for one axis (ela3d_aux.cu).
 struct AxisProfileArgs {

@@ -29,9 +29,16 @@ static Variant make_variant() {
   v.velocity = reinterpret_cast<const void *>(&velocity_kernel<T, TX, TY, NSV, CPT, MB, LOAD>);
   v.flow = nullptr;
   v.flow_smem = 0;
+  v.flow_coef = nullptr;
+  v.flow_coef_smem = 0;
   if constexpr (LOAD == LOAD_TMA) {
-    v.flow = reinterpret_cast<const void *>(&flow_kernel<T, TX, TY, NS, CPT, MB>);
-    v.flow_smem = Flow<T, TX, TY, NS, CPT, MB>::SMEM;
+    v.flow = reinterpret_cast<const void *>(&flow_kernel<T, TX, TY, NS, CPT, MB, false>);
+    v.flow_smem = Flow<G, T, NS>::SMEM;
+    // FP64 with one cell per thread: also with coefficients from arrays
+    if constexpr (sizeof(T) == 8 && CPT == 1 && MB == 0) {
+      v.flow_coef = reinterpret_cast<const void *>(&flow_kernel<T, TX, TY, NS, CPT, MB, true>);
+      v.flow_coef_smem = Flow<Geo<T, TX, TY, NS, CPT, MB, true>, T, NS>::SMEM;
+    }
   }
   return v;
 }
@@ -76,6 +83,13 @@ static const Variant kVariants[] = {
     make_variant<double, 32, 8, 4, 1>(),
     make_variant<double, 16, 16, 4, 1>(),
 };
+
+cudaError_t launch_coef_f64(const ShotDesc<double> &shot, double *out, cudaStream_t s) {
+  const long long cells = (long long)shot.nz * shot.ny * shot.px;
+  const long long blocks = (cells + 255) / 256;
+  coef_kernel<double><<<(unsigned)(blocks < 4864 ? blocks : 4864), 256, 0, s>>>(shot, out, cells);
+  return cudaGetLastError();
+}
 
 const Variant *variants(int *count) {
   *count = (int)(sizeof(kVariants) / sizeof(kVariants[0]));

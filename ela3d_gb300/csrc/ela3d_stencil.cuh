@@ -32,8 +32,11 @@
 
 namespace ela3d {
 
-template <typename T, int TX_, int TY_, int NS_, int CPT_ = Vec<T>::N, int MINB_ = 0>
+// COEF: the update coefficients (dt lambda and so on) come from arrays
+// computed once per plan instead of from the model (FP64 dataflow kernels).
+template <typename T, int TX_, int TY_, int NS_, int CPT_ = Vec<T>::N, int MINB_ = 0, bool COEF_ = false>
 struct Geo {
+  static constexpr bool COEF = COEF_;
   static constexpr int VEC = CPT_;       // cells per thread (consecutive in x)
   static constexpr int H = Vec<T>::N;    // halo width in x (16 bytes, the TMA x alignment)
   static constexpr int TX = TX_, TY = TY_, NS = NS_;
@@ -66,31 +69,35 @@ struct Geo {
   // what the plane below reads too (as its z+1 neighbours), the second the
   // rest.  The first ring has NS places; the second does with one place less
   // where shared memory is short.
-  // stress: vx vy cs rho (W1) | vz (W1), cp and the six stresses (C)
+  // stress: vx vy cs rho (W1) | vz (W1), cp and the six stresses (C); with
+  // COEF: vx vy | vz, the five coefficients in cp's place, the stresses
   static constexpr int S_VX = 0;
   static constexpr int S_VY = S_VX + sz(W1);
   static constexpr int S_CS = S_VY + sz(W1);
   static constexpr int S_RHO = S_CS + sz(W1);
-  static constexpr int S_A = S_RHO + sz(W1);
+  static constexpr int S_A = COEF ? S_CS : S_RHO + sz(W1);
+  static constexpr int S_CENTRE = COEF ? 5 : 1;   // centre boxes before the stresses
   static constexpr int S_VZ = 0;
   static constexpr int S_CP = S_VZ + sz(W1);
-  static constexpr int S_SIG = S_CP + sz(C);  // six centre boxes follow
+  static constexpr int S_SIG = S_CP + S_CENTRE * sz(C);  // six centre boxes follow
   static constexpr int S_B = S_SIG + 6 * sz(C);
-  static constexpr int S_TXA = (int)sizeof(T) * 4 * W1;   // bytes loaded
-  static constexpr int S_TXB = (int)sizeof(T) * (W1 + 7 * C);
-  // velocity: szz (C), rho (W1) | sxx syy sxy sxz syz with their halos, vx vy vz (C)
+  static constexpr int S_TXA = (int)sizeof(T) * (COEF ? 2 : 4) * W1;   // bytes loaded
+  static constexpr int S_TXB = (int)sizeof(T) * (W1 + (S_CENTRE + 6) * C);
+  // velocity: szz (C), rho (W1) | sxx syy sxy sxz syz with their halos, vx vy
+  // vz (C); with COEF: szz | the same and three coefficients (C)
   static constexpr int V_SZZ = 0;
   static constexpr int V_RHO = V_SZZ + sz(C);
-  static constexpr int V_A = V_RHO + sz(W1);
+  static constexpr int V_A = COEF ? V_RHO : V_RHO + sz(W1);
   static constexpr int V_SXX = 0;                 // W0
   static constexpr int V_SYY = V_SXX + sz(W0);    // Y1
   static constexpr int V_SXY = V_SYY + sz(Y1);    // W1
   static constexpr int V_SXZ = V_SXY + sz(W1);    // W0
   static constexpr int V_SYZ = V_SXZ + sz(W0);    // Y1
   static constexpr int V_V = V_SYZ + sz(Y1);      // vx vy vz (C)
-  static constexpr int V_B = V_V + 3 * sz(C);
-  static constexpr int V_TXA = (int)sizeof(T) * (C + W1);
-  static constexpr int V_TXB = (int)sizeof(T) * (2 * W0 + 2 * Y1 + 3 * C + W1);
+  static constexpr int V_COEF = V_V + 3 * sz(C);
+  static constexpr int V_B = COEF ? V_COEF + 3 * sz(C) : V_COEF;
+  static constexpr int V_TXA = (int)sizeof(T) * (COEF ? C : C + W1);
+  static constexpr int V_TXB = (int)sizeof(T) * (2 * W0 + 2 * Y1 + (COEF ? 6 : 3) * C + W1);
   // memory-variable slots (PsiSlots): one 16-byte (or smaller) vector per
   // consumer thread for each of the three variables of each axis
   static constexpr int PSI_BYTES = 9 * NT * VEC * (int)sizeof(T);
@@ -317,17 +324,22 @@ __device__ __forceinline__ void dt_moduli(T dt, const T (&vp)[V], const T (&vs)[
   mul_v(lam, lam, dt);
 }
 
-// v + dt / rho_avg (d1 + d2 sy + d3 sz) for the cells of the mask.  (FP32
-// divides for every cell: a branch around it costs more.  FP64 leaves out the
-// cells outside the range, whose density may be 0.)
+// b = dt / rho_avg of the densities r0 and r1.  (FP32 divides for every cell: a
+// branch around it costs more.  FP64 leaves out the cells outside the mask,
+// whose density may be 0.)
 template <typename T, int V>
-__device__ __forceinline__ void velocity_update(T dt, T sy, T sz, const T (&r0)[V], const T (&r1)[V], const T (&d1)[V],
-                                                const T (&d2)[V], const T (&d3)[V], T (&v)[V], unsigned m) {
-  T b[V], t[V];
+__device__ __forceinline__ void dt_over_rho(T (&b)[V], T dt, const T (&r0)[V], const T (&r1)[V], unsigned m) {
   add_v(b, r0, r1);
 #pragma unroll
   for (int e = 0; e < V; ++e)
     if (sizeof(T) == 4 || ((m >> e) & 1u)) b[e] = dt_over_rho(dt, b[e]);
+}
+
+// v + b (d1 + d2 sy + d3 sz) for the cells of the mask.
+template <typename T, int V>
+__device__ __forceinline__ void velocity_update(T sy, T sz, const T (&b)[V], const T (&d1)[V], const T (&d2)[V],
+                                                const T (&d3)[V], T (&v)[V], unsigned m) {
+  T t[V];
   fma_v(t, d2, sy, d1);
   fma_v(t, d3, sz, t);
   fma_v(t, b, t, v);
@@ -535,8 +547,10 @@ __device__ __forceinline__ void stress_issue_a(const ShotDesc<T> &sd, const Shot
     mbar_arrive_expect_tx(bar, G::S_TXA);
     tma_load_3d(st + G::S_VX, &m[0], x0, y0, k, bar);
     tma_load_3d(st + G::S_VY, &m[1], x0 - H, y0 - 1, k, bar);
-    tma_load_3d(st + G::S_CS, &m[3], x0 - H, y0, k, bar);
-    tma_load_3d(st + G::S_RHO, &m[4], x0 - H, y0, k, bar);
+    if constexpr (!G::COEF) {
+      tma_load_3d(st + G::S_CS, &m[3], x0 - H, y0, k, bar);
+      tma_load_3d(st + G::S_RHO, &m[4], x0 - H, y0, k, bar);
+    }
   }
 }
 
@@ -556,7 +570,12 @@ __device__ __forceinline__ void stress_issue_b(const ShotDesc<T> &sd, const Shot
     const CUtensorMap *m = maps.stress;
     mbar_arrive_expect_tx(bar, G::S_TXB);
     tma_load_3d(st + G::S_VZ, &m[2], x0 - H, y0, k, bar);
-    tma_load_3d(st + G::S_CP, &m[5], x0, y0, k, bar);
+    if constexpr (G::COEF) {
+#pragma unroll
+      for (int c = 0; c < 5; ++c) tma_load_3d(st + G::S_CP + c * G::SC, &maps.coef[c], x0, y0, k, bar);
+    } else {
+      tma_load_3d(st + G::S_CP, &m[5], x0, y0, k, bar);
+    }
 #pragma unroll
     for (int c = 0; c < 6; ++c) tma_load_3d(st + G::S_SIG + c * G::SC, &m[6 + c], x0, y0, k, bar);
   }
@@ -578,7 +597,7 @@ __device__ __forceinline__ void velocity_issue_a(const ShotDesc<T> &sd, const Sh
     const CUtensorMap *m = maps.vel;
     mbar_arrive_expect_tx(bar, G::V_TXA);
     tma_load_3d(st + G::V_SZZ, &m[2], x0, y0, k, bar);
-    tma_load_3d(st + G::V_RHO, &m[6], x0 - H, y0, k, bar);
+    if constexpr (!G::COEF) tma_load_3d(st + G::V_RHO, &m[6], x0 - H, y0, k, bar);
   }
 }
 
@@ -607,6 +626,10 @@ __device__ __forceinline__ void velocity_issue_b(const ShotDesc<T> &sd, const Sh
     tma_load_3d(st + G::V_SYZ, &m[5], x0, y0 - 1, k, bar);
 #pragma unroll
     for (int c = 0; c < 3; ++c) tma_load_3d(st + G::V_V + c * G::SC, &m[7 + c], x0, y0, k, bar);
+    if constexpr (G::COEF) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) tma_load_3d(st + G::V_COEF + c * G::SC, &maps.coef[5 + c], x0, y0, k, bar);
+    }
   }
 }
 
@@ -846,15 +869,25 @@ __device__ __forceinline__ bool stress_item(const ShotDesc<T> &sd, const Item &i
     ld_vec(bvz + sl, vz_c);
     ld_vec(bvz + sl + WW, vz_yp);
     const T vz_w = bvz[sl - 1];
-    ld_vec(bcs + sl, cs_c);
-    ld_vec(bcs + sl + WW, cs_yp);
-    const T cs_w = bcs[sl - 1];
-    ld_vec(reinterpret_cast<const T *>(nxt + G::S_CS) + sl, cs_zp);
-    ld_vec(brho + sl, rho_c);
-    ld_vec(brho + sl + WW, rho_yp);
-    const T rho_w = brho[sl - 1];
-    ld_vec(reinterpret_cast<const T *>(nxt + G::S_RHO) + sl, rho_zp);
-    ld_vec(bcp + sc, cp_c);
+    T cs_w = T(0), rho_w = T(0);
+    T DT_l2m[V], DT_l[V], mu_xy[V], mu_xz[V], mu_yz[V];
+    if constexpr (G::COEF) {
+      ld_vec(bcp + 0 * CS + sc, DT_l2m);
+      ld_vec(bcp + 1 * CS + sc, DT_l);
+      ld_vec(bcp + 2 * CS + sc, mu_xy);
+      ld_vec(bcp + 3 * CS + sc, mu_xz);
+      ld_vec(bcp + 4 * CS + sc, mu_yz);
+    } else {
+      ld_vec(bcs + sl, cs_c);
+      ld_vec(bcs + sl + WW, cs_yp);
+      cs_w = bcs[sl - 1];
+      ld_vec(reinterpret_cast<const T *>(nxt + G::S_CS) + sl, cs_zp);
+      ld_vec(brho + sl, rho_c);
+      ld_vec(brho + sl + WW, rho_yp);
+      rho_w = brho[sl - 1];
+      ld_vec(reinterpret_cast<const T *>(nxt + G::S_RHO) + sl, rho_zp);
+      ld_vec(bcp + sc, cp_c);
+    }
     T sxx[V], syy[V], szz[V], sxy[V], sxz[V], syz[V];
     ld_vec(bsig + 0 * CS + sc, sxx);
     ld_vec(bsig + 1 * CS + sc, syy);
@@ -871,7 +904,8 @@ __device__ __forceinline__ bool stress_item(const ShotDesc<T> &sd, const Item &i
 #pragma unroll
       for (int e = 0; e < V; ++e)
         if (xg + e == sd.src_i) {
-          const T l2m = mul_rn(mul_rn(rho_c[e], cp_c[e]), cp_c[e]);
+          const long long gs = (long long)k * plane + rowoff + e;
+          const T l2m = mul_rn(mul_rn(sd.rho[gs], sd.cp[gs]), sd.cp[gs]);
           sxx[e] = fma_rn(mul_rn(mul_rn(sd.expl_w[0], s), dt), l2m, sxx[e]);
           syy[e] = fma_rn(mul_rn(mul_rn(sd.expl_w[1], s), dt), l2m, syy[e]);
           szz[e] = fma_rn(mul_rn(mul_rn(sd.expl_w[2], s), dt), l2m, szz[e]);
@@ -953,8 +987,7 @@ __device__ __forceinline__ bool stress_item(const ShotDesc<T> &sd, const Item &i
     if (!last) fetch_z(k + 1);
 
     // normal stresses, simpelmodel.cpp:378-413
-    T DT_l2m[V], DT_l[V];
-    dt_moduli(dt, cp_c, cs_c, rho_c, DT_l2m, DT_l);
+    if constexpr (!G::COEF) dt_moduli(dt, cp_c, cs_c, rho_c, DT_l2m, DT_l);
     if (!F32) {
       normal_stress<true>(DT_l2m, DT_l, exx, eyy, ezz, sxx, mk);
       normal_stress<true>(DT_l2m, DT_l, eyy, exx, ezz, syy, mk);
@@ -976,18 +1009,20 @@ __device__ __forceinline__ bool stress_item(const ShotDesc<T> &sd, const Item &i
     // the shear stresses: sigma_xy :416-442, sigma_xz :445-471 (z+1 of plane
     // nz-1 is the zero plane), sigma_yz :473-498
     {
-      T cw[V], rw[V], mu[V], t[V];
-      west_of(cw, cs_c, cs_w);
-      west_of(rw, rho_c, rho_w);
-      dt_mu(mu, dt8, cw, cs_yp, rw, rho_yp);
+      T cw[V], rw[V], t[V];
+      if constexpr (!G::COEF) {
+        west_of(cw, cs_c, cs_w);
+        west_of(rw, rho_c, rho_w);
+        dt_mu(mu_xy, dt8, cw, cs_yp, rw, rho_yp);
+      }
       fma_v(t, exy, sy, eyx);
-      fma_v(t, mu, t, sxy);
+      fma_v(t, mu_xy, t, sxy);
       keep_masked(sxy, t, mk >> 8);
-      dt_mu(mu, dt8, cw, cs_zp, rw, rho_zp);
+      if constexpr (!G::COEF) dt_mu(mu_xz, dt8, cw, cs_zp, rw, rho_zp);
       fma_v(t, exz, sz, ezx);
-      fma_v(t, mu, t, sxz);
+      fma_v(t, mu_xz, t, sxz);
       keep_masked(sxz, t, mk >> 16);
-      dt_mu(mu, dt8, cs_yp, cs_zp, rho_yp, rho_zp);
+      if constexpr (!G::COEF) dt_mu(mu_yz, dt8, cs_yp, cs_zp, rho_yp, rho_zp);
       // (a derivative whose C-PML term was applied has S = 1, and its
       // product with S is exact)
       if (F32 ? row_y : !plane_z) {
@@ -997,7 +1032,7 @@ __device__ __forceinline__ bool stress_item(const ShotDesc<T> &sd, const Item &i
         mul_v(t, eyz, sz);
         fma_v(t, ezy, sy, t);
       }
-      fma_v(t, mu, t, syz);
+      fma_v(t, mu_yz, t, syz);
       keep_masked(syz, t, mk >> 24);
     }
 
@@ -1221,10 +1256,19 @@ __device__ __forceinline__ bool velocity_item(const ShotDesc<T> &sd, const Item 
     const T sxz_e = bsxz[sr0 + V];
     ld_vec(bsyz + sc1, syz_c);
     ld_vec(bsyz + sc1 - TX, syz_ym);
-    ld_vec(brho + sl0, rho_c);
-    ld_vec(brho + sl0 + WW, rho_yp);
-    const T rho_w = brho[sl0 - 1];
-    ld_vec(reinterpret_cast<const T *>(nxt + G::V_RHO) + sl0, rho_zp);
+    T rho_w = T(0);
+    T bx_[V], by_[V], bz_[V];   // dt / rho of the three components
+    if constexpr (G::COEF) {
+      const T *bco = reinterpret_cast<const T *>(rest + G::V_COEF);
+      ld_vec(bco + 0 * CS + sc, bx_);
+      ld_vec(bco + 1 * CS + sc, by_);
+      ld_vec(bco + 2 * CS + sc, bz_);
+    } else {
+      ld_vec(brho + sl0, rho_c);
+      ld_vec(brho + sl0 + WW, rho_yp);
+      rho_w = brho[sl0 - 1];
+      ld_vec(reinterpret_cast<const T *>(nxt + G::V_RHO) + sl0, rho_zp);
+    }
     ld_vec(bv + 0 * CS + sc, vx);
     ld_vec(bv + 1 * CS + sc, vy);
     ld_vec(bv + 2 * CS + sc, vz);
@@ -1294,11 +1338,17 @@ __device__ __forceinline__ bool velocity_item(const ShotDesc<T> &sd, const Item 
     }
     if (!last) fetch_z(k + 1);
 
+    // simpelmodel.cpp:502-530, :532-559, :563-590
     T rw[V];
-    west_of(rw, rho_c, rho_w);
-    velocity_update(dt, sy, sz, rho_c, rw, x1, x2, x3, vx, mk);              // simpelmodel.cpp:502-530
-    velocity_update(dt, sy, sz, rho_c, rho_yp, y1, y2, y3, vy, mk >> 8);     // :532-559
-    velocity_update(dt, sy, sz, rho_c, rho_zp, z1, z2, z3, vz, mk >> 16);    // :563-590
+    if constexpr (!G::COEF) {
+      west_of(rw, rho_c, rho_w);
+      dt_over_rho(bx_, dt, rho_c, rw, mk);
+    }
+    velocity_update(sy, sz, bx_, x1, x2, x3, vx, mk);
+    if constexpr (!G::COEF) dt_over_rho(by_, dt, rho_c, rho_yp, mk >> 8);
+    velocity_update(sy, sz, by_, y1, y2, y3, vy, mk >> 8);
+    if constexpr (!G::COEF) dt_over_rho(bz_, dt, rho_c, rho_zp, mk >> 16);
+    velocity_update(sy, sz, bz_, z1, z2, z3, vz, mk >> 16);
 
     // receivers in this warp's cells (velocity after the update, :593-602)
     if (rlo < rhi)
@@ -1518,9 +1568,9 @@ __global__ void __launch_bounds__(Geo<T, TX, TY, NS, CPT, MB>::THREADS, Geo<T, T
 // RB ready barriers: the producer is at most NA loads ahead of the slowest
 // consumer warp and every item takes at least two of them, so it never gets
 // RB items ahead (a barrier is re-armed only after every warp passed it).
-template <typename T, int TX, int TY, int NS, int CPT, int MB>
+template <typename G_, typename T, int NS>
 struct Flow {
-  using G = Geo<T, TX, TY, NS, CPT, MB>;
+  using G = G_;
   static constexpr int A = G::S_A > G::V_A ? G::S_A : G::V_A, B = G::S_B > G::V_B ? G::S_B : G::V_B;
   static constexpr int RB = 8;
   static_assert(RB >= NS / 2 + 2, "ready barriers for the items in flight");
@@ -1587,13 +1637,13 @@ __device__ __forceinline__ bool flow_wait_deps(const ShotDesc<T> &sd, const Flow
   return true;
 }
 
-template <typename T, int TX, int TY, int NS, int CPT, int MB>
+template <typename T, int TX, int TY, int NS, int CPT, int MB, bool COEF>
 __global__ void __launch_bounds__(Geo<T, TX, TY, NS, CPT, MB>::THREADS, Geo<T, TX, TY, NS, CPT, MB>::MINB)
     flow_kernel(const ShotDesc<T> *__restrict__ shots, const ShotMaps *__restrict__ maps,
                 const FlowItem *__restrict__ items, int nitems, int list_steps, int nsteps, int tick,
                 const int *__restrict__ dtick, unsigned *__restrict__ err, int ctl, int *__restrict__ claim) {
-  using G = Geo<T, TX, TY, NS, CPT, MB>;
-  using F = Flow<T, TX, TY, NS, CPT, MB>;
+  using G = Geo<T, TX, TY, NS, CPT, MB, COEF>;
+  using F = Flow<G, T, NS>;
   extern __shared__ __align__(1024) unsigned char smem[];
   using R = typename F::R;
   const R ring{smem};
@@ -1708,6 +1758,48 @@ __global__ void __launch_bounds__(Geo<T, TX, TY, NS, CPT, MB>::THREADS, Geo<T, T
       int *flag = sd.flow_flags + ((size_t)fi.kind * sd.flow_chunks + fi.chunk) * (txs * tys) + fi.it.tile;
       red_release_gpu_add(flag, G::NCW);
     }
+  }
+}
+
+// The update coefficients of every cell, eight arrays of `cells` values each:
+// dt (lambda + 2 mu), dt lambda, dt mu of sigma_xy, sigma_xz and sigma_yz, and
+// dt / rho of vx, vy and vz -- by the functions that the kernels without them
+// use, so results are the same bits.  Neighbours outside the grid are zero, as
+// in the kernels' boxes.
+template <typename T>
+__global__ void __launch_bounds__(256) coef_kernel(const ShotDesc<T> sd, T *out, long long cells) {
+  const T dt = sd.dt;
+  const long long plane = (long long)sd.ny * sd.px;
+  for (long long i = blockIdx.x * 256ll + threadIdx.x; i < cells; i += gridDim.x * 256ll) {
+    const int k = (int)(i / plane);
+    const long long r = i - k * plane;
+    const int y = (int)(r / sd.px), x = (int)(r - (long long)y * sd.px);
+    T v[8] = {};
+    if (x < sd.nx) {
+      const bool w = x > 0, s = y + 1 < sd.ny, u = k + 1 < sd.nz;
+      const T cp[1] = {sd.cp[i]}, cs[1] = {sd.cs[i]}, rho[1] = {sd.rho[i]};
+      const T cw[1] = {w ? sd.cs[i - 1] : T(0)}, rw[1] = {w ? sd.rho[i - 1] : T(0)};
+      const T cy[1] = {s ? sd.cs[i + sd.px] : T(0)}, ry[1] = {s ? sd.rho[i + sd.px] : T(0)};
+      const T cz[1] = {u ? sd.cs[i + plane] : T(0)}, rz[1] = {u ? sd.rho[i + plane] : T(0)};
+      T a[1], b[1];
+      dt_moduli(dt, cp, cs, rho, a, b);
+      v[0] = a[0];
+      v[1] = b[0];
+      dt_mu(a, T(0.125) * dt, cw, cy, rw, ry);
+      v[2] = a[0];
+      dt_mu(a, T(0.125) * dt, cw, cz, rw, rz);
+      v[3] = a[0];
+      dt_mu(a, T(0.125) * dt, cy, cz, ry, rz);
+      v[4] = a[0];
+      dt_over_rho(a, dt, rho, rw, 1u);
+      v[5] = a[0];
+      dt_over_rho(a, dt, rho, ry, 1u);
+      v[6] = a[0];
+      dt_over_rho(a, dt, rho, rz, 1u);
+      v[7] = a[0];
+    }
+#pragma unroll
+    for (int c = 0; c < 8; ++c) out[c * cells + i] = v[c];
   }
 }
 

@@ -130,3 +130,36 @@ def test_fp64_densities_of_any_size(built, scale):
         assert np.abs(want).max() > 0 and rel_l2(plan.seismograms(fp64=True), want) < 1e-11
         for c in range(9):
             assert rel_l2(plan.field(c, fp64=True), fields[c]) < 1e-11, c
+
+
+def test_fp64_coefficients_follow_a_restored_model(built):
+    """An FP64 plan on the dataflow kernel runs from coefficients derived from
+    its model; a checkpoint brings its own model, and the plan then continues
+    as the saved one.  A batch's shots of one model share them, also when their
+    time steps differ."""
+    import ela3d_gb300 as E
+    from ela3d_gb300 import media
+
+    nx, ny, nz = 48, 40, 36
+    p = E.ShotParams(nx=nx, ny=ny, nz=nz, nstep=30, dt=1e-3, npml=6, f0=25.0, t0=0.01, src=(24, 20, 18),
+                     rec=np.array([[20, 20, 18], [30, 22, 12]], np.int32), precision=E.FP64)
+    m = media.anticline_layers(nx, ny, nz, depths=(10, 20, 30, 60), amp=3, sigma=9, seed=1)
+    other = media.anticline_layers(nx, ny, nz, depths=(8, 15, 22, 60), amp=4, sigma=7, seed=2)
+    first = next(i for i, v in enumerate(E.variants()) if v.fp64)
+    want = _run(p, *m, variant=first, schedule=1, chunk=8)
+    with E.Plan(p, *m) as a:
+        a.run(12)
+        saved = a.checkpoint()
+    with E.Plan(p, *other) as b:
+        b.restore(saved)
+        b.run(p.nstep - 12)
+        got = [b.seismograms(), b.source_trace()] + [b.field(c) for c in range(9)]
+    for x, y in zip(got, want):
+        assert np.array_equal(x, y)
+    shots = [(p, *m), (p.with_(dt=0.8e-3, src=(20, 18, 16)), *m), (p.with_(src=(30, 20, 16)), *m)]
+    with E.Batch(shots) as b:
+        b.run(p.nstep)
+        for q, s in enumerate(shots):
+            alone = _run(*s, variant=first, schedule=1, chunk=8)
+            assert np.array_equal(b.seismograms(q), alone[0])
+            assert np.array_equal(b.field(q, 2), alone[4])
