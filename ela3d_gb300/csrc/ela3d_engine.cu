@@ -513,12 +513,15 @@ static int pick_tile(const std::vector<ela3d_params> &ps, bool fp64, bool stream
 }
 
 // The chunk: about two items per block and half-step, for the claimed places
-// to even out (256^3: 48.8 Gcell-updates/s with 64 planes, 45.1 with 86), but
+// to even out (256^3: 48.8 Gcell-updates/s with 64 planes, 45.1 with 86;
+// 192x160x176 45.5, with 1.65 44.9); arrays near the L2 size 1.65, where an item's fixed costs weigh more (items per block:
+// 128^3 1.4 46.2, 1.7 47.1, 2.0 45.9, 2.7 42.3; 101^3 1.3 35.8, 1.45 38.2, 1.8
+// 37.2, 2.2 34.5; 180x120x100 1.3 37.2, 1.6 39.5, 2.05 38.9, 2.7 37.1).  But
 // no more than 80 planes (512^3: 51.0 at 64, 50.5 at 128, 48.8 in whole
 // columns; 448^3 48.7 at 75, 44.8 whole; 384^3 49.7 at 96, 48.6 at 192) and no
 // fewer than 2.
-int flow_chunk(int nz, long long tiles, int blocks, int most) {
-  long long per_col = std::max({1ll, (4ll * blocks + tiles) / (2 * tiles), (long long)(nz + most - 1) / most});
+int flow_chunk(int nz, long long tiles, double items, int most) {
+  long long per_col = std::max({1ll, (long long)(items / (double)tiles + 0.5), (long long)(nz + most - 1) / most});
   per_col = std::min(per_col, 16000ll);   // (a schedule holds fewer than 2^14 chunks per column)
   return std::max(2, (int)((nz + per_col - 1) / per_col));
 }
@@ -534,10 +537,11 @@ TuneChoice plan_choice(const ela3d_params &p) {
   if (!v[c.variant].flow) return c;
   c.kind = kScheduleFlowOverlap;
   c.lag = 0;
-  const bool streams = !fp64 && 12.0 * p.nx * p.ny * p.nz * 4.0 > 400e6;
+  const double bytes = 12.0 * p.nx * p.ny * p.nz * 4.0;
+  const bool streams = !fp64 && bytes > 400e6;
   c.variant = pick_tile({p}, fp64, streams, c.variant);
   const int tx = v[c.variant].tx, ty = v[c.variant].ty;
-  c.chunk = flow_chunk(p.nz, (long long)((p.nx + tx - 1) / tx) * ((p.ny + ty - 1) / ty), device_sms(), fp64 ? 32 : 80);
+  c.chunk = flow_chunk(p.nz, (long long)((p.nx + tx - 1) / tx) * ((p.ny + ty - 1) / ty), (fp64 || bytes > 170e6 ? 2.0 : 1.65) * device_sms(), fp64 ? 32 : 80);
   // the memory variables' copies reach one plane ahead; the prefetches add
   // to that only where the variables come from DRAM
   c.prefetch = streams ? kPrefetchDefault : 0;
@@ -1415,7 +1419,7 @@ class Engine final : public EngineBase {
     for (int q : active) tiles += tiles_of(shots_[q]->d);
     for (int q : active) {
       const ShotDesc<T> &d = shots_[q]->d;
-      const int c = choice_.chunk > 0 ? C : flow_chunk(d.nz, tiles, per_sm_flow_ * num_sms_, 48);
+      const int c = choice_.chunk > 0 ? C : flow_chunk(d.nz, tiles, 2.0 * per_sm_flow_ * num_sms_, 48);
       shapes.push_back({d.nx, d.ny, d.nz, q, c});
       per_step += 2 * tiles_of(d) * ((d.nz + c - 1) / c);
     }

@@ -101,9 +101,9 @@ TuneChoice plan_choice(const ela3d_params &p);
 // not known yet): one tile for all, chunk 0 = sized for each shot.
 TuneChoice batch_choice(const std::vector<ela3d_params> &ps, int fp64);
 // Planes per z-chunk (at most `most`) of a dataflow schedule for a column of
-// nz planes, when the shots running have `tiles` tiles in all and there are
-// `blocks` blocks.
-int flow_chunk(int nz, long long tiles, int blocks, int most);
+// nz planes, when the shots running have `tiles` tiles in all and should make
+// about `items` work items per half-step.
+int flow_chunk(int nz, long long tiles, double items, int most);
 
 // Autotuner (ela3d_tune.cu): process-wide cache of measured best choices
 // keyed by the workload shape.
