@@ -175,6 +175,23 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, i
       : "memory");
 }
 
+// L2 policy of an access whose lines are the first to be evicted.
+__device__ __forceinline__ uint64_t evict_first() {
+  uint64_t p;
+  asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+  return p;
+}
+
+// tma_load_3d of lines that L2 is to give up first.
+__device__ __forceinline__ void tma_load_3d_first(void *dst, const CUtensorMap *map, int x, int y, int z,
+                                                  uint64_t *bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cta.global.mbarrier::complete_tx::bytes.L2::cache_hint"
+      " [%0], [%1, {%2, %3, %4}], [%5], %6;" ::"r"(smem_u32(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar)), "l"(evict_first())
+      : "memory");
+}
+
 // 16-byte asynchronous copy global -> shared through L2 (cp.async.cg);
 // the first src_bytes (0..16) are read, the rest of the 16 are zero-filled.
 // Both addresses 16-byte aligned.
@@ -192,6 +209,16 @@ __device__ __forceinline__ void cp_async_vec(void *dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
   else
     asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(dst)), "l"(src), "n"(B) : "memory");
+}
+
+// A 16-byte cp.async and a store of four floats, likewise.
+__device__ __forceinline__ void cp_async_16_first(void *dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src),
+               "l"(evict_first())
+               : "memory");
+}
+__device__ __forceinline__ void st_first(float *p, const float (&o)[4]) {
+  __stcs(reinterpret_cast<float4 *>(p), make_float4(o[0], o[1], o[2], o[3]));
 }
 
 // Arrive on bar once every cp.async this thread issued before has landed

@@ -1072,6 +1072,8 @@ class Engine final : public EngineBase {
     CK(cudaFuncSetAttribute(var_->velocity, cudaFuncAttributeMaxDynamicSharedMemorySize, var_->vel_smem));
     if (var_->flow)
       CK(cudaFuncSetAttribute(var_->flow, cudaFuncAttributeMaxDynamicSharedMemorySize, var_->flow_smem));
+    if (var_->flow_once)
+      CK(cudaFuncSetAttribute(var_->flow_once, cudaFuncAttributeMaxDynamicSharedMemorySize, var_->flow_smem));
     if (var_->flow_coef)
       CK(cudaFuncSetAttribute(var_->flow_coef, cudaFuncAttributeMaxDynamicSharedMemorySize, var_->flow_coef_smem));
     ela3d_status ost = occupancy(c);
@@ -1162,6 +1164,11 @@ class Engine final : public EngineBase {
     if (var_->flow) {
       int occ_f = 0;
       CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_f, var_->flow, var_->threads, var_->flow_smem));
+      if (var_->flow_once) {
+        int occ_o = 0;
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_o, var_->flow_once, var_->threads, var_->flow_smem));
+        occ_f = std::min(occ_f, occ_o);
+      }
       if (var_->flow_coef) {
         int occ_c = 0;
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_c, var_->flow_coef, var_->threads, var_->flow_coef_smem));
@@ -1477,6 +1484,15 @@ class Engine final : public EngineBase {
     if (st != ELA3D_OK) return st;
     flow_items_ = (int)items.size();
     flow_steps_ = K;
+    // Arrays that about fit the L2 (126 MB): the fields stay there if the model and
+    // the memory variables make room.  Gcell-updates/s without / with, 10 and 20
+    // layer cells: 64^3 (13 MB) 20.5 / 20.9, 101^3 (63) 39.2 / 41.4 and 33.4 /
+    // 37.0, 112^3 43.0 / 47.6 and 36.9 / 43.6, 128^3 (101) 48.1 / 50.8 and 41.0 /
+    // 46.0, 64x180x180 (100) 44.3 / 50.2 and 38.1 / 44.5.  Above, the halos and
+    // densities read again from HBM cost more: 180x64x180 (106) 40.7 / 41.6 but
+    // 35.4 / 33.9, 96x160x160 (118) 44.8 / 43.5, 100x150x140 (129) 36.0 / 35.4,
+    // 160^3 (197) 45.7 / 42.2, 256^3 49.8 / 47.8.
+    flow_once_ = var_->flow_once && bytes < 105e6;
     flow_coef_ = var_->flow_coef != nullptr;
     for (int q : active) flow_coef_ = flow_coef_ && shots_[q]->coef;
     flags_used_ = flags;
@@ -1509,7 +1525,8 @@ class Engine final : public EngineBase {
     }
     const int grid = std::min(per_sm_flow_ * num_sms_, std::max(1, flow_items_));
     const bool coef = flow_coef_;
-    CK(cudaLaunchCooperativeKernel(coef ? var_->flow_coef : var_->flow, dim3(grid), dim3(var_->threads), args,
+    const void *kernel = coef ? var_->flow_coef : flow_once_ ? var_->flow_once : var_->flow;
+    CK(cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(var_->threads), args,
                                    coef ? var_->flow_coef_smem : var_->flow_smem, stream_));
     if (timing_) {
       CK(cudaEventRecord(e1, stream_));
@@ -1987,6 +2004,7 @@ class Engine final : public EngineBase {
   int flow_passes_ = kFlowPasses;
   static constexpr long long kFlowMaxItems = 1 << 20, kFlowBatchItems = 1 << 14;
   int flow_walks_ = kFlowPasses;   // walks of the list in one launch
+  bool flow_once_ = false;         // the list runs var_->flow_once
   bool flow_coef_ = false;         // every shot of the list has its coefficients
   static constexpr long long kCoefBytes = 8ll << 30;
   FlowItem *d_flow_ = nullptr;

@@ -22,6 +22,7 @@ struct Variant {
   const void *velocity;
   const void *flow;     // dataflow kernel (many steps per launch); null if not compiled
   int flow_smem;
+  const void *flow_once;  // the same with model and memory variables first to leave L2; null if not compiled
   const void *flow_coef;  // the same with coefficients from arrays; null if not compiled
   int flow_coef_smem;
 };

@@ -29,14 +29,18 @@ static Variant make_variant() {
   v.velocity = reinterpret_cast<const void *>(&velocity_kernel<T, TX, TY, NSV, CPT, MB, LOAD>);
   v.flow = nullptr;
   v.flow_smem = 0;
+  v.flow_once = nullptr;
   v.flow_coef = nullptr;
   v.flow_coef_smem = 0;
   if constexpr (LOAD == LOAD_TMA) {
-    v.flow = reinterpret_cast<const void *>(&flow_kernel<T, TX, TY, NS, CPT, MB, false>);
+    v.flow = reinterpret_cast<const void *>(&flow_kernel<T, TX, TY, NS, CPT, MB, false, false>);
     v.flow_smem = Flow<G, T, NS>::SMEM;
+    // FP32 tiles of seven or eight warps: also with the L2 hints
+    if constexpr (sizeof(T) == 4 && G::NCW >= 7)
+      v.flow_once = reinterpret_cast<const void *>(&flow_kernel<T, TX, TY, NS, CPT, MB, false, true>);
     // FP64 with one cell per thread: also with coefficients from arrays
     if constexpr (sizeof(T) == 8 && CPT == 1 && MB == 0) {
-      v.flow_coef = reinterpret_cast<const void *>(&flow_kernel<T, TX, TY, NS, CPT, MB, true>);
+      v.flow_coef = reinterpret_cast<const void *>(&flow_kernel<T, TX, TY, NS, CPT, MB, true, false>);
       v.flow_coef_smem = Flow<Geo<T, TX, TY, NS, CPT, MB, true>, T, NS>::SMEM;
     }
   }

@@ -34,9 +34,14 @@ namespace ela3d {
 
 // COEF: the update coefficients (dt lambda and so on) come from arrays
 // computed once per plan instead of from the model (FP64 dataflow kernels).
-template <typename T, int TX_, int TY_, int NS_, int CPT_ = Vec<T>::N, int MINB_ = 0, bool COEF_ = false>
+// ONCE: the model and the C-PML memory variables, which a step reads (and
+// writes) once or twice, are the first lines that L2 gives up, so that the
+// fields, which pass from half-step to half-step and to the neighbouring tiles,
+// stay there (FP32 dataflow kernels of shots whose arrays about fill the L2).
+template <typename T, int TX_, int TY_, int NS_, int CPT_ = Vec<T>::N, int MINB_ = 0, bool COEF_ = false,
+          bool ONCE_ = false>
 struct Geo {
-  static constexpr bool COEF = COEF_;
+  static constexpr bool COEF = COEF_, ONCE = ONCE_;
   static constexpr int VEC = CPT_;       // cells per thread (consecutive in x)
   static constexpr int H = Vec<T>::N;    // halo width in x (16 bytes, the TMA x alignment)
   static constexpr int TX = TX_, TY = TY_, NS = NS_;
@@ -528,6 +533,12 @@ struct ItemPrefetch {
 };
 
 // ------------------------------------------------------- stage loads ----
+template <bool ONCE>
+__device__ __forceinline__ void load_model(void *dst, const CUtensorMap *map, int x, int y, int z, uint64_t *bar) {
+  if constexpr (ONCE) tma_load_3d_first(dst, map, x, y, z, bar);
+  else tma_load_3d(dst, map, x, y, z, bar);
+}
+
 // The two parts of one stress plane (box shapes in ela3d_device.cuh, ShotMaps):
 // vx vy cs rho with their halos | vz with its halo, cp and the six stresses.
 template <typename G, int LOAD, typename T>
@@ -548,8 +559,8 @@ __device__ __forceinline__ void stress_issue_a(const ShotDesc<T> &sd, const Shot
     tma_load_3d(st + G::S_VX, &m[0], x0, y0, k, bar);
     tma_load_3d(st + G::S_VY, &m[1], x0 - H, y0 - 1, k, bar);
     if constexpr (!G::COEF) {
-      tma_load_3d(st + G::S_CS, &m[3], x0 - H, y0, k, bar);
-      tma_load_3d(st + G::S_RHO, &m[4], x0 - H, y0, k, bar);
+      load_model<G::ONCE>(st + G::S_CS, &m[3], x0 - H, y0, k, bar);
+      load_model<G::ONCE>(st + G::S_RHO, &m[4], x0 - H, y0, k, bar);
     }
   }
 }
@@ -574,7 +585,7 @@ __device__ __forceinline__ void stress_issue_b(const ShotDesc<T> &sd, const Shot
 #pragma unroll
       for (int c = 0; c < 5; ++c) tma_load_3d(st + G::S_CP + c * G::SC, &maps.coef[c], x0, y0, k, bar);
     } else {
-      tma_load_3d(st + G::S_CP, &m[5], x0, y0, k, bar);
+      load_model<G::ONCE>(st + G::S_CP, &m[5], x0, y0, k, bar);
     }
 #pragma unroll
     for (int c = 0; c < 6; ++c) tma_load_3d(st + G::S_SIG + c * G::SC, &m[6 + c], x0, y0, k, bar);
@@ -597,7 +608,7 @@ __device__ __forceinline__ void velocity_issue_a(const ShotDesc<T> &sd, const Sh
     const CUtensorMap *m = maps.vel;
     mbar_arrive_expect_tx(bar, G::V_TXA);
     tma_load_3d(st + G::V_SZZ, &m[2], x0, y0, k, bar);
-    if constexpr (!G::COEF) tma_load_3d(st + G::V_RHO, &m[6], x0 - H, y0, k, bar);
+    if constexpr (!G::COEF) load_model<G::ONCE>(st + G::V_RHO, &m[6], x0 - H, y0, k, bar);
   }
 }
 
@@ -688,15 +699,18 @@ __device__ __forceinline__ bool flow_ready(uint64_t *ready, uint32_t parity, uns
 // the plane's update.  Built-in choices, 10 layer cells, Gcell-updates/s:
 // 101^3 33.2 -> 36.5, 128^3 36.0 -> 40.7, 192^3 41.1 -> 42.2, 256^3 47.5 ->
 // 48.7; the two kernels at 128^3 29.8 -> 33.5.
-template <typename T, int NT, int V>
+template <typename T, int NT, int V, bool ONCE>
 struct PsiSlots {
   unsigned char *base;   // this thread's slot of variable 0
   static constexpr int B = V * (int)sizeof(T);
+  static_assert(!ONCE || B == 16, "accesses with an L2 policy are 16 bytes");
   __device__ __forceinline__ PsiSlots(unsigned char *psi, int tid) : base(psi + tid * B) {}
   // variables 0..2 of `axis` from p, p + stride, p + 2 stride
   __device__ __forceinline__ void fetch(int axis, const T *p, long long stride) const {
 #pragma unroll
-    for (int v = 0; v < 3; ++v) cp_async_vec<B>(base + (axis * 3 + v) * NT * B, p + v * stride);
+    for (int v = 0; v < 3; ++v)
+      if constexpr (ONCE) cp_async_16_first(base + (axis * 3 + v) * NT * B, p + v * stride);
+      else cp_async_vec<B>(base + (axis * 3 + v) * NT * B, p + v * stride);
   }
   // d <- d / K + psi with psi <- b psi + a d, written back to p.  RAW: d
   // holds plain differences, to be multiplied by 1/h first.  AFIRST: which
@@ -720,7 +734,8 @@ struct PsiSlots {
       fma_v(q, b, q, t);
     }
     fma_v(d, x, ik, q);
-    st_vec(p, q);
+    if constexpr (ONCE) st_first(p, q);
+    else st_vec(p, q);
   }
 };
 
@@ -820,7 +835,7 @@ __device__ __forceinline__ bool stress_item(const ShotDesc<T> &sd, const Item &i
   long long g = (long long)item.k0 * plane + rowoff;
   // the memory variables of the first plane; each plane then copies the next
   // one's as it has used its own
-  const PsiSlots<T, G::NT, V> slots(psi, tid);
+  const PsiSlots<T, G::NT, V, G::ONCE> slots(psi, tid);
   auto fetch_z = [&](int k) {
     if (live && (k < zl || k >= zr)) {
       const int zs = k < zl ? k : zl + (k - zr);
@@ -1200,7 +1215,7 @@ __device__ __forceinline__ bool velocity_item(const ShotDesc<T> &sd, const Item 
   long long g = (long long)item.k0 * plane + rowoff;
   // the memory variables of the first plane; each plane then copies the next
   // one's as it has used its own
-  const PsiSlots<T, G::NT, V> slots(psi, tid);
+  const PsiSlots<T, G::NT, V, G::ONCE> slots(psi, tid);
   auto fetch_z = [&](int k) {
     if (live && (k < zl || k >= zr)) {
       const int zs = k < zl ? k : zl + (k - zr);
@@ -1636,12 +1651,12 @@ __device__ __forceinline__ bool flow_wait_deps(const ShotDesc<T> &sd, const Flow
   return true;
 }
 
-template <typename T, int TX, int TY, int NS, int CPT, int MB, bool COEF>
+template <typename T, int TX, int TY, int NS, int CPT, int MB, bool COEF, bool ONCE>
 __global__ void __launch_bounds__(Geo<T, TX, TY, NS, CPT, MB>::THREADS, Geo<T, TX, TY, NS, CPT, MB>::MINB)
     flow_kernel(const ShotDesc<T> *__restrict__ shots, const ShotMaps *__restrict__ maps,
                 const FlowItem *__restrict__ items, int nitems, int list_steps, int nsteps, int tick,
                 const int *__restrict__ dtick, unsigned *__restrict__ err, int ctl, int *__restrict__ claim) {
-  using G = Geo<T, TX, TY, NS, CPT, MB, COEF>;
+  using G = Geo<T, TX, TY, NS, CPT, MB, COEF, ONCE>;
   using F = Flow<G, T, NS>;
   extern __shared__ __align__(1024) unsigned char smem[];
   using R = typename F::R;

@@ -163,3 +163,23 @@ def test_fp64_coefficients_follow_a_restored_model(built):
             alone = _run(*s, variant=first, schedule=1, chunk=8)
             assert np.array_equal(b.seismograms(q), alone[0])
             assert np.array_equal(b.field(q, 2), alone[4])
+
+
+@pytest.mark.parametrize("nz", [133, 134], ids=["hinted", "plain"])
+@pytest.mark.parametrize("tile", [(128, 7), (64, 14), (112, 8), (56, 16), (32, 28), (128, 8), (64, 16), (32, 32),
+                                  (112, 9), (56, 18)], ids=lambda t: "%dx%d" % t)
+def test_l2_hints_equal_two_kernels(tile, nz):
+    """128x128xnz: the arrays of 133 planes are just below the size up to which
+    the dataflow kernel runs with L2 hints, those of 134 just above."""
+    from ela3d_gb300 import ShotParams, media, variants
+
+    rec = np.stack([np.arange(40, 80), np.full(40, 60), np.full(40, 66)], axis=1).astype(np.int32)
+    p = ShotParams(nx=128, ny=128, nz=nz, nstep=9, dt=1e-3, npml=12, f0=25.0, t0=0.004, k_max=1.5, src=(63, 60, 66),
+                   rec=rec)
+    cp, cs, rho = media.anticline_layers(128, 128, nz, depths=(40, 80, 100, 2 * nz), amp=13, sigma=26, seed=4)
+    number = next(i for i, v in enumerate(variants()) if (v.tile_x, v.tile_y) == tile and not v.fp64 and v.loads == 0)
+    want = _run(p, cp, cs, rho, variant=0, schedule=1, chunk=8)
+    got = _run(p, cp, cs, rho, variant=number, schedule=4, chunk=12)
+    assert np.abs(want[0]).max() > 0
+    for a, b in zip(got, want):
+        assert np.array_equal(a, b)
