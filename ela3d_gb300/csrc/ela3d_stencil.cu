@@ -7,9 +7,9 @@
 
 namespace ela3d {
 
-// NSV: stages of the velocity kernel's ring (its stage is smaller than the
+// NSV: places of the velocity kernel's rings (its planes are smaller than the
 // stress kernel's, so it can hold more of them); the dataflow kernel runs
-// both half-steps in one ring of NS stages.
+// both half-steps in rings of NS places.
 template <typename T, int TX, int TY, int NS, int CPT = Vec<T>::N, int MB = 0, int LOAD = LOAD_TMA, int NSV = NS>
 static Variant make_variant() {
   using G = Geo<T, TX, TY, NS, CPT, MB>;
@@ -48,8 +48,8 @@ static Variant make_variant() {
 }
 
 static const Variant kVariants[] = {
-    // velocity ring of 5 stages (5 x 38 KB; the stress ring's 4 x 46 KB):
-    // more bytes in flight per SM, 1.2% less velocity time at 256^3
+    // velocity rings of 5 places: more bytes in flight per SM, 1.2% less
+    // velocity time at 256^3
     make_variant<float, 128, 7, 4, 4, 0, LOAD_TMA, 5>(),
     make_variant<float, 128, 6, 5>(),
     make_variant<float, 128, 5, 6>(),

@@ -1,17 +1,20 @@
-// ela3d_stencil.cuh -- the two time-loop kernels: stress half-step and
-// velocity half-step, templated on the real type and the x-y tile.
+// ela3d_stencil.cuh -- the time-loop kernels, templated on the real type and
+// the x-y tile: the stress and the velocity half-step (stress_item,
+// velocity_item), as a kernel each and as items of one persistent dataflow
+// kernel (flow_kernel).
 //
-// Scheme (2.5-D z-march, one launch per half-step):
+// Scheme (2.5-D z-march):
 //  - a block owns a list of work items (shot, x-y tile, z-run [k0, k1));
 //  - one producer warp walks the block's planes and, for each, issues TMA
 //    tiled loads of every input array's x-y tile (with the one-cell halos
-//    the stencil needs) into a ring of NS shared-memory stages; each stage
-//    has a "full" mbarrier (TMA bytes landed) and an "empty" mbarrier (all
-//    consumer warps done), so refills start as soon as a stage is released;
+//    the stencil needs) into two rings of shared-memory places (what the
+//    plane below reads too, and the rest); each place has a "full" mbarrier
+//    (TMA bytes landed) and an "empty" mbarrier (all consumer warps done), so
+//    refills start as soon as a place is released;
 //  - out-of-grid halo cells arrive as zeros (the TMA fill), which is also
 //    the zero plane above k = nz-1 that the reference's sigma_xz/sigma_yz
 //    loop reads (simpelmodel.cpp:450,477);
-//  - consumer warps compute plane k from stages k and k+1 (the z+1
+//  - consumer warps compute plane k from places k and k+1 (the z+1
 //    neighbours) and keep the z-1 neighbours in registers; each thread owns
 //    16 bytes of consecutive x cells of one row (float4 / double2);
 //  - C-PML memory variables are read and written only in the PML slabs, each
