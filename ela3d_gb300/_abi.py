@@ -69,6 +69,7 @@ SIGNATURES = [
     ("ela3d_batch_get_field", _c.c_int, [_P, _c.c_int32, _c.c_int32, _P]),
     ("ela3d_batch_get_source_trace", _c.c_int, [_P, _c.c_int32, _P]),
     ("ela3d_batch_info", _c.c_int, [_P, _c.c_int32, _P]),
+    ("ela3d_batch_inject_list_failure", _c.c_int, [_P, _c.c_int32]),
     ("ela3d_batch_destroy", _c.c_int, [_P]),
     ("ela3d_server_config_default", _c.c_int, [_P]),
     ("ela3d_server_create", _c.c_int, [_P, _c.POINTER(_P)]),
@@ -524,6 +525,11 @@ class Batch:
         i = PlanInfo()
         _check(self._lib.ela3d_batch_info(self._h, shot, ctypes.byref(i)), "ela3d_batch_info")
         return i
+
+    def inject_list_failure(self, builds: int) -> None:
+        """Test hook: the next `builds` work-list allocations fail
+        (ela3d_batch_inject_list_failure)."""
+        _check(self._lib.ela3d_batch_inject_list_failure(self._h, builds), "ela3d_batch_inject_list_failure")
 
     def close(self) -> None:
         if getattr(self, "_h", None) is not None and self._h.value:

@@ -563,6 +563,11 @@ ela3d_status ela3d_batch_info(ela3d_batch *b, int32_t shot, ela3d_plan_info *out
   return b->eng->info(shot, out);
 }
 
+ela3d_status ela3d_batch_inject_list_failure(ela3d_batch *b, int32_t builds) {
+  if (!b) return ELA3D_ERR_INVALID_ARG;
+  return b->eng->inject_list_failure(builds);
+}
+
 ela3d_status ela3d_batch_destroy(ela3d_batch *b) {
   delete b;
   return ELA3D_OK;

@@ -1192,6 +1192,7 @@ class Engine final : public EngineBase {
   void set_retire(bool on) override { retire_ = on; }
 
   ela3d_status launch_step(int tick, const int *dtick) {
+    if (!sched_valid_ || flow_on() || !d_items_ || !d_ranges_) BAD("internal: no work items to launch");
     int ctl = (inject_ > 0 ? CTL_WITHHOLD_LOADS : 0) | prefetch_;
     if (inject_ > 0) --inject_;
     void *args[] = {&d_desc_, &d_maps_, &d_items_, &d_ranges_, &tick, &dtick, &d_err_, &ctl};
@@ -1236,9 +1237,11 @@ class Engine final : public EngineBase {
     if (nsteps < 0) BAD("nsteps must be >= 0");
     while (nsteps > 0) {
       int seg = nsteps;
-      if (retire_) {
+      if (retire_ || !sched_valid_) {
         ela3d_status st = rebuild_schedule();
         if (st != ELA3D_OK) return st;
+      }
+      if (retire_) {
         // (the dataflow kernel passes over finished shots itself: a launch
         // ends at a shot's last step only for an explosive source's sake,
         // whose last injection comes after the launch)
@@ -1336,6 +1339,7 @@ class Engine final : public EngineBase {
 
   // Shot descriptors and tensor maps to the device (once per composition).
   ela3d_status upload_tables() {
+    tables_dirty_ = true;   // until both are on the device
     std::vector<ShotDesc<T>> descs;
     std::vector<ShotMaps> maps;
     for (auto &sp : shots_) { descs.push_back(sp->d); maps.push_back(sp->maps); }
@@ -1348,11 +1352,33 @@ class Engine final : public EngineBase {
     CK(cudaMemcpyAsync(d_desc_, descs.data(), descs.size() * sizeof(ShotDesc<T>), cudaMemcpyHostToDevice, stream_));
     CK(cudaMemcpyAsync(d_maps_, maps.data(), maps.size() * sizeof(ShotMaps), cudaMemcpyHostToDevice, stream_));
     CK(cudaStreamSynchronize(stream_));
+    tables_dirty_ = false;
+    return ELA3D_OK;
+  }
+
+  // Room for n elements; the old ones are given up if they are too few.  (The
+  // test hook's failures come here, as if memory had run out.)
+  template <typename U>
+  ela3d_status grow(U *&p, size_t &cap, size_t n) {
+    if (n <= cap && fail_lists_ == 0) return ELA3D_OK;
+    if (p) CK(cudaFree(p));
+    p = nullptr;
+    cap = 0;
+    if (fail_lists_ > 0) {
+      --fail_lists_;
+      set_last_error("injected failure of a work list's allocation");
+      return ELA3D_ERR_OOM;
+    }
+    CK(cudaMalloc(&p, n * sizeof(U)));
+    cap = n;
     return ELA3D_OK;
   }
 
   // Work items for the shots active at the next step (all shots unless
   // retirement is on).  Invalidates the cached graph when the split changes.
+  // The schedule counts as valid only once every list and table of it is on
+  // the device: after an error there is none, nothing is launched, and the
+  // next enqueue builds it again.
   ela3d_status rebuild_schedule() {
     std::vector<ShotShape> shapes;
     std::vector<int> key;
@@ -1367,23 +1393,23 @@ class Engine final : public EngineBase {
       CK(cudaStreamSynchronize(stream_));  // no launch reads the old tables any more
       ela3d_status st = upload_tables();
       if (st != ELA3D_OK) return st;
-      tables_dirty_ = false;
     }
     if (!sched_key_.empty() && key == sched_key_ && sched_valid_) return ELA3D_OK;
-    sched_key_ = key;
-    sched_valid_ = true;
+    sched_valid_ = false;
+    nblocks_ = nitems_ = flow_items_ = flow_steps_ = 0;
     steps_on_schedule_ = 0;
     invalidate_graph();
-    if (shapes.empty()) {
-      nblocks_ = 0;
-      return ELA3D_OK;
+    if (!shapes.empty()) {
+      ela3d_status st = flow_on() ? rebuild_flow(key) : rebuild_items(shapes);
+      if (st != ELA3D_OK) return st;
     }
-    flow_items_ = 0;
-    flow_steps_ = 0;
-    if (flow_on()) {
-      nblocks_ = 1;   // (something is active)
-      return rebuild_flow(key);
-    }
+    sched_key_ = key;
+    sched_valid_ = true;
+    return ELA3D_OK;
+  }
+
+  // The work items of the half-step kernels.
+  ela3d_status rebuild_items(const std::vector<ShotShape> &shapes) {
     std::vector<Item> items;
     std::vector<int2> ranges;
     const int kind = choice_.kind >= kScheduleFlow ? 1 : choice_.kind;
@@ -1393,18 +1419,9 @@ class Engine final : public EngineBase {
     for (const Item &it : items)
       if (it.k1 <= it.k0) BAD("internal: empty work item");
     CK(cudaStreamSynchronize(stream_));  // kernels in flight may still read the old tables
-    if (items.size() > items_cap_) {
-      if (d_items_) CK(cudaFree(d_items_));
-      d_items_ = nullptr;
-      CK(cudaMalloc(&d_items_, items.size() * sizeof(Item)));
-      items_cap_ = items.size();
-    }
-    if (ranges.size() > ranges_cap_) {
-      if (d_ranges_) CK(cudaFree(d_ranges_));
-      d_ranges_ = nullptr;
-      CK(cudaMalloc(&d_ranges_, ranges.size() * sizeof(int2)));
-      ranges_cap_ = ranges.size();
-    }
+    ela3d_status st = grow(d_items_, items_cap_, items.size());
+    if (st == ELA3D_OK) st = grow(d_ranges_, ranges_cap_, ranges.size());
+    if (st != ELA3D_OK) return st;
     CK(cudaMemcpy(d_items_, items.data(), items.size() * sizeof(Item), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(d_ranges_, ranges.data(), ranges.size() * sizeof(int2), cudaMemcpyHostToDevice));
     nblocks_ = (int)ranges.size();
@@ -1458,32 +1475,22 @@ class Engine final : public EngineBase {
                              &off, &nch, &nflags, &why))
       BAD(why);
     CK(cudaStreamSynchronize(stream_));
-    if (items.size() > flow_cap_) {
-      if (d_flow_) CK(cudaFree(d_flow_));
-      d_flow_ = nullptr;
-      flow_cap_ = 0;
-      CK(cudaMalloc(&d_flow_, items.size() * sizeof(FlowItem)));
-      flow_cap_ = items.size();
-    }
     // the claim counter sits behind the flags, on a line of its own
     const size_t flags = ((size_t)nflags + 31) / 32 * 32 + 32;
-    if (flags > flags_cap_) {
-      if (d_flags_) CK(cudaFree(d_flags_));
-      d_flags_ = nullptr;
-      flags_cap_ = 0;
-      CK(cudaMalloc(&d_flags_, flags * sizeof(int)));
-      flags_cap_ = flags;
-    }
+    ela3d_status st = grow(d_flow_, flow_cap_, items.size());
+    if (st == ELA3D_OK) st = grow(d_flags_, flags_cap_, flags);
+    if (st != ELA3D_OK) return st;
     CK(cudaMemcpy(d_flow_, items.data(), items.size() * sizeof(FlowItem), cudaMemcpyHostToDevice));
     for (size_t a = 0; a < active.size(); ++a) {
       ShotDesc<T> &d = shots_[active[a]]->d;
       d.flow_flags = d_flags_ + off[a];
       d.flow_chunks = nch[a];
     }
-    ela3d_status st = upload_tables();
+    st = upload_tables();
     if (st != ELA3D_OK) return st;
     flow_items_ = (int)items.size();
     flow_steps_ = K;
+    nblocks_ = 1;   // (something is active)
     // Arrays that about fit the L2 (126 MB): the fields stay there if the model and
     // the memory variables make room.  Gcell-updates/s without / with, 10 and 20
     // layer cells: 64^3 (13 MB) 20.5 / 20.9, 101^3 (63) 39.2 / 41.4 and 33.4 /
@@ -1501,6 +1508,7 @@ class Engine final : public EngineBase {
 
   // One launch of the dataflow kernel: steps tick .. tick + nsteps - 1.
   ela3d_status launch_flow(int tick, int nsteps) {
+    if (!sched_valid_ || !d_flow_ || !d_flags_) BAD("internal: no work list to launch");
     int ctl = (inject_ > 0 ? CTL_WITHHOLD_LOADS : 0) | prefetch_ | (retire_ ? CTL_RETIRE : 0);
     inject_ = std::max(0, inject_ - nsteps);
     const int *dtick = nullptr;
@@ -1828,6 +1836,12 @@ class Engine final : public EngineBase {
     return ELA3D_OK;
   }
 
+  ela3d_status inject_list_failure(int builds) override {
+    if (builds < 0) BAD("builds must be >= 0");
+    fail_lists_ = builds;
+    return ELA3D_OK;
+  }
+
   int64_t launches() const override { return launches_; }
 
   int64_t device_bytes() const override {
@@ -1972,6 +1986,7 @@ class Engine final : public EngineBase {
   cudaStream_t setup_ = nullptr;
   int tick_ = 0;
   int inject_ = 0;   // steps left whose launches withhold their loads (test hook)
+  int fail_lists_ = 0;   // work lists whose allocation is still to fail (test hook)
   int prefetch_ = kPrefetchDefault;  // memory-variable prefetch hints (x slab to L1, y/z slabs to L2)
   int prefetch_env_ = -1;
   size_t guard_ = 0;   // bytes of each debug guard zone (0 = off)

@@ -144,6 +144,7 @@ class EngineBase {
   virtual ela3d_status info(int shot, ela3d_plan_info *out) = 0;
   virtual ela3d_status set_timing(bool on) = 0;
   virtual ela3d_status inject_timeout(int launches) = 0;
+  virtual ela3d_status inject_list_failure(int builds) = 0;
   virtual ela3d_status poison_padding(double value) = 0;
   virtual ela3d_status check_guards() = 0;
   virtual void set_retire(bool on) = 0;

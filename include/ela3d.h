@@ -363,6 +363,12 @@ ela3d_status ela3d_batch_get_seismograms(ela3d_batch *b, int32_t shot, float *ou
 ela3d_status ela3d_batch_get_field(ela3d_batch *b, int32_t shot, int32_t comp, float *out);
 ela3d_status ela3d_batch_get_source_trace(ela3d_batch *b, int32_t shot, float *out);
 ela3d_status ela3d_batch_info(ela3d_batch *b, int32_t shot, ela3d_plan_info *out);
+/* Test hook: the next `builds` work lists that the batch allocates (again
+ * whenever shots retire) fail with ELA3D_ERR_OOM, as if device memory had
+ * run out.  The run that meets the failure launches nothing after it; a later
+ * run builds the list again and continues from the step reached
+ * (ela3d_batch_info). */
+ela3d_status ela3d_batch_inject_list_failure(ela3d_batch *b, int32_t builds);
 ela3d_status ela3d_batch_destroy(ela3d_batch *b);
 
 /* ---- serving: continuous batching ---------------------------------------- */
