@@ -2,6 +2,8 @@
 // maps, work schedule and the time-step loop.
 #include "ela3d_engine.h"
 
+#include "ela3d_hostrange.h"
+
 #include <cudaTypedefs.h>
 #include <sys/mman.h>
 #include <unistd.h>
@@ -581,17 +583,18 @@ TuneChoice batch_choice(const std::vector<ela3d_params> &ps, int fp64) {
 }
 
 // ------------------------------------------------------------ TMA maps --
+// A function of the driver's interface as of CUDA version `version`, or null.
+static void *driver_entry(const char *name, unsigned version) {
+  void *p = nullptr;
+  cudaDriverEntryPointQueryResult q;
+  if (cudaGetDriverEntryPointByVersion(name, &p, version, cudaEnableDefault, &q) != cudaSuccess ||
+      q != cudaDriverEntryPointSuccess)
+    return nullptr;
+  return p;
+}
+
 static PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void *p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) ==
-            cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-  });
+  static const auto fn = (PFN_cuTensorMapEncodeTiled_v12000)driver_entry("cuTensorMapEncodeTiled", 12000);
   return fn;
 }
 
@@ -618,6 +621,27 @@ static ela3d_status encode_map(CUtensorMap *m, const T *base, int nx, int ny, in
 }
 
 // -------------------------------------------------------------- engine --
+// Where a kernel may read a page-locked host array, or null: for arrays that
+// are not page-locked, that do not start on 16 bytes, or of which one
+// page-locked range (an allocation or a registration) does not hold all.  A copy
+// from an array that is locked in part is the driver's to refuse; a kernel
+// would read past the range.
+static const float *mapped_array(const float *p, size_t bytes) {
+  cudaPointerAttributes at{};
+  const bool locked = cudaPointerGetAttributes(&at, p) == cudaSuccess && at.type == cudaMemoryTypeHost && at.devicePointer;
+  cudaGetLastError();   // (a pointer CUDA does not know is no error)
+  if (!locked || (uintptr_t)at.devicePointer % 16 != 0) return nullptr;
+  static const auto attribute = (PFN_cuPointerGetAttribute_v4000)driver_entry("cuPointerGetAttribute", 4000);
+  CUdeviceptr start = 0;
+  size_t size = 0;
+  const CUdeviceptr at0 = (CUdeviceptr)(uintptr_t)at.devicePointer;
+  if (!attribute || attribute(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, at0) != CUDA_SUCCESS ||
+      attribute(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, at0) != CUDA_SUCCESS ||
+      !range_holds(start, size, at0, bytes))
+    return nullptr;
+  return static_cast<const float *>(at.devicePointer);
+}
+
 template <typename T>
 struct Shot {
   ela3d_params p{};
@@ -889,14 +913,10 @@ class Engine final : public EngineBase {
       for (int c = 0; c < 3; ++c) {
         // page-locked arrays: the kernel that pads (and widens) the rows reads
         // them over the link
-        cudaPointerAttributes at{};
-        const bool mapped = cudaPointerGetAttributes(&at, src[c]) == cudaSuccess && at.type == cudaMemoryTypeHost &&
-                            at.devicePointer && (uintptr_t)at.devicePointer % 16 == 0;
-        if (mapped) {
-          CK(Fp<T>::pad(static_cast<const float *>(at.devicePointer), dst[c], nx, ny, nz, px, setup_));
+        if (const float *mapped = mapped_array(src[c], compact)) {
+          CK(Fp<T>::pad(mapped, dst[c], nx, ny, nz, px, setup_));
           continue;
         }
-        cudaGetLastError();   // (a pointer CUDA does not know is no error)
         if (sizeof(T) == 4 && px == nx) {
           CK(cudaMemcpyAsync(dst[c], src[c], compact, cudaMemcpyHostToDevice, setup_));
           continue;
