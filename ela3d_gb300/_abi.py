@@ -58,6 +58,7 @@ SIGNATURES = [
     ("ela3d_select_device", _c.c_int, [_c.c_int32]),
     ("ela3d_host_alloc", _c.c_int, [_c.c_size_t, _c.POINTER(_P)]),
     ("ela3d_builtin_tuning", _c.c_int, [_c.POINTER(CParams), _P]),
+    ("ela3d_open_tuning", _c.c_int, [_c.c_int32, _P, _P]),
     ("ela3d_host_free", _c.c_int, [_P]),
     ("ela3d_run_timed", _c.c_int, [_P, _c.c_int32, _c.POINTER(_c.c_double)]),
     ("ela3d_slab_extent", _c.c_int, [_P, _P, _c.c_int32, _c.POINTER(_c.c_int32), _c.POINTER(_c.c_int32)]),
@@ -228,9 +229,23 @@ def load_library(path: str | None = None) -> ctypes.CDLL:
     return lib
 
 
+def open_tuning(*shots) -> "Tuning":
+    """The choice of a plan (one ShotParams) or batch (several) whose tuning
+    is left open (ela3d_open_tuning; host only)."""
+    structs = (CParams * len(shots))()
+    keep = []
+    for i, p in enumerate(shots):
+        structs[i], rec = p.to_c()
+        keep.append(rec)
+    t = Tuning()
+    _check(load_library().ela3d_open_tuning(len(shots), ctypes.addressof(structs), ctypes.addressof(t)),
+           "ela3d_open_tuning")
+    return t
+
+
 def builtin_tuning(p) -> "Tuning":
-    """The built-in kernel choice for a single shot with parameters p
-    (ela3d_builtin_tuning; host only)."""
+    """The fixed choice that fills in what a single shot's tuning leaves open
+    beside the fields set (ela3d_builtin_tuning; host only)."""
     c, _rec = p.to_c()
     t = Tuning()
     _check(load_library().ela3d_builtin_tuning(ctypes.byref(c), ctypes.addressof(t)), "ela3d_builtin_tuning")

@@ -128,6 +128,11 @@ ela3d_status ela3d_variant_get(int32_t index, ela3d_variant_info *out) {
   return ELA3D_OK;
 }
 
+// The library's own choice for a plan or batch whose tuning is left open.
+static TuneChoice open_choice(const std::vector<ela3d_params> &ps) {
+  return ps.size() == 1 ? plan_choice(ps[0]) : batch_choice(ps, ps[0].precision == ELA3D_FP64);
+}
+
 // The choice for a workload: fields the caller set win; the rest come from
 // the autotuner's cache (tuning on a miss when ELA3D_AUTOTUNE=1), else the
 // built-in default.
@@ -138,11 +143,10 @@ static TuneChoice resolve_tuning(const std::vector<ela3d_params> &ps, const floa
   // round-robin chunks enough to go around)
   const bool open = !t || (t->variant < 0 && t->schedule < 0 && t->chunk <= 0 && t->blocks_per_sm < 0 &&
                            t->prefetch < 0 && t->lag < 0);
-  TuneChoice c = ps.size() != 1 ? (open ? batch_choice(ps, p.precision == ELA3D_FP64)
-                                        : default_choice(p.precision == ELA3D_FP64, 0, 0, 0))
-                 : open         ? plan_choice(p)
-                                : default_choice(p.precision == ELA3D_FP64, p.nx, p.ny, p.nz,
-                                                 p.src_kind == ELA3D_SRC_EXPLOSIVE);
+  TuneChoice c = open             ? open_choice(ps)
+                 : ps.size() != 1 ? default_choice(p.precision == ELA3D_FP64, 0, 0, 0)
+                                  : default_choice(p.precision == ELA3D_FP64, p.nx, p.ny, p.nz,
+                                                   p.src_kind == ELA3D_SRC_EXPLOSIVE);
   const bool explicit_variant = t && t->variant >= 0;
   if (!explicit_variant) {
     TuneChoice cached{};
@@ -424,6 +428,23 @@ ela3d_status ela3d_builtin_tuning(const ela3d_params *p, ela3d_tuning *out) {
   if (!p || !out) return ELA3D_ERR_INVALID_ARG;
   const TuneChoice c = default_choice(p->precision == ELA3D_FP64, p->nx, p->ny, p->nz,
                                       p->src_kind == ELA3D_SRC_EXPLOSIVE);
+  out->variant = c.variant;
+  out->schedule = c.kind;
+  out->chunk = c.chunk;
+  out->blocks_per_sm = c.blocks_per_sm;
+  out->prefetch = c.prefetch;
+  out->lag = c.lag;
+  return ELA3D_OK;
+}
+
+ela3d_status ela3d_open_tuning(int32_t nshots, const ela3d_params *params, ela3d_tuning *out) {
+  if (nshots < 1 || !params || !out) return ELA3D_ERR_INVALID_ARG;
+  for (int i = 0; i < nshots; ++i) {
+    ela3d_status st = validate_params(params[i]);
+    if (st != ELA3D_OK) return st;
+    if (params[i].precision != params[0].precision) return ELA3D_ERR_INVALID_ARG;
+  }
+  const TuneChoice c = open_choice(std::vector<ela3d_params>(params, params + nshots));
   out->variant = c.variant;
   out->schedule = c.kind;
   out->chunk = c.chunk;

@@ -231,7 +231,8 @@ bool build_flow_schedule(const std::vector<FlowShape> &shots, int tx, int ty, in
   *nflags = 0;
   bool sized = true;
   for (const FlowShape &f : shots) sized = sized && (f.chunk == 0 ? chunk >= 2 : f.chunk >= 2);
-  if (!sized || (shots.empty() && chunk < 2) || gap < 1 || nsteps < 1 || nsteps > 255 || tx < 1 || ty < 1 || shots.size() >= (1u << 16)) {
+  if (!sized || (shots.empty() && chunk < 2) || gap < 1 || nsteps < 1 || nsteps > 255 || tx < 1 || ty < 1 ||
+      shots.size() > kFlowMaxShots) {
     *why = "dataflow schedule: chunk >= 2, gap >= 1, 1 <= nsteps <= 255, fewer than 65536 shots";
     return false;
   }
@@ -552,7 +553,7 @@ TuneChoice plan_choice(const ela3d_params &p) {
 
 // Shots that run together.  Known ones (a batch) take the dataflow kernel with
 // the tile that suits all of them best and chunks of up to 48 planes, no
-// prefetch; Gcell-updates/s against the two kernels with 128x7 tiles and
+// prefetch (more than a dataflow list holds keep the two kernels); Gcell-updates/s against the two kernels with 128x7 tiles and
 // 10-plane chunks: eight 192^3 shots of one model 45.2 against 36.6, ten uneven
 // grids (edges 64-320) 39.0 against 35.6.  (80 planes 43.8 and 38.3; with all
 // prefetches 43.7 and 38.0.)
@@ -566,7 +567,7 @@ TuneChoice batch_choice(const std::vector<ela3d_params> &ps, int fp64) {
   TuneChoice c = default_choice(fp64, 0, 0, 0);
   int n = 0;
   const Variant *v = variants(&n);
-  if (!v[c.variant].flow || (fp64 && ps.empty())) return c;
+  if (!v[c.variant].flow || (fp64 && ps.empty()) || ps.size() > kFlowMaxShots) return c;
   c.prefetch = 0;
   c.lag = 0;
   c.chunk = 0;

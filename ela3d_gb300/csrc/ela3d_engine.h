@@ -72,6 +72,7 @@ struct FlowShape {
   int id;   // shot index written into the items
   int chunk = 0;   // planes per z-chunk of this shot (0: the schedule's)
 };
+constexpr size_t kFlowMaxShots = 65535;   // of one dataflow list
 bool build_flow_schedule(const std::vector<FlowShape> &shots, int tx, int ty, int chunk, int gap, bool overlap,
                          int nsteps, std::vector<FlowItem> *items, std::vector<int> *flag_off,
                          std::vector<int> *nchunks, int *nflags, std::string *why);

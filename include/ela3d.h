@@ -286,14 +286,16 @@ typedef struct ela3d_tuning {
  * one is done.  Results are bit-identical to schedules 0-2.  The work list
  * is built on the host for the shots running, again whenever shots join or
  * retire, so these schedules suit a plan or a batch of shots that run
- * together; the autotuner tries them for single shots, and schedule 4 is
- * the built-in choice for a single FP32 shot without an explosive source,
- * its z-chunks sized for about 1.5 work items per block (ela3d_builtin_tuning
- * reports the choice).  A plan whose caller leaves every field open refines
- * that choice, and takes schedule 4 for an explosive source and in FP64 too:
- * the tile that wastes least of the grid, z-chunks for about two items per
- * block and of at most 80 planes (FP64 32).  A batch with open fields takes
- * schedule 4 as well, one tile for all its shots and chunks for each. */
+ * together; the autotuner tries them for single shots.  A plan whose caller
+ * leaves every field open takes schedule 4 with the tile that wastes least of
+ * the grid, z-chunks for about two items per block (1.65 near the L2 size) and
+ * of at most 80 planes (FP64 32).  A batch with open fields takes schedule 4
+ * as well, one tile for all its shots and chunks for each (65536 shots or more,
+ * which one work list cannot hold: the two kernels).  ela3d_open_tuning reports
+ * these choices.  A plan with some fields set takes the others from a fixed
+ * choice (ela3d_builtin_tuning): schedule 4 for a single FP32 shot without an
+ * explosive source, its z-chunks sized for about 1.5 work items per block,
+ * else the two kernels. */
 
 /* Times every compiled variant with the candidate schedules on these shots
  * (`steps` time steps each, after a warm-up) and returns the fastest choice;
@@ -451,11 +453,18 @@ ela3d_status ela3d_server_destroy(ela3d_server *s);
  * simpelmodel.cpp:89-106).  lo == hi == n when the layer covers the axis. */
 ela3d_status ela3d_slab_extent(const double *a_full, const double *a_half, int32_t n,
                                int32_t *lo, int32_t *hi);
-/* Host-only: the built-in kernel choice for a single shot with these
- * parameters (variant, schedule, chunk, prefetch; no tuning cache, no
- * device work; the current device's SM count, 152 without a device).  No
- * reference counterpart. */
+/* Host-only: the choice that fills in the fields left open in a single
+ * shot's tuning when the caller sets others (variant, schedule, chunk,
+ * prefetch; no tuning cache, no device work; the current device's SM count,
+ * 152 without a device).  A tuning with every field open takes
+ * ela3d_open_tuning's choice instead.  No reference counterpart. */
 ela3d_status ela3d_builtin_tuning(const ela3d_params *p, ela3d_tuning *out);
+/* Host-only: what a plan (nshots = 1) or batch of these shots runs when every
+ * field of its tuning is left open and no tuned choice is cached.  chunk 0:
+ * each shot's z-chunks are sized for the shots running.  Passed to
+ * ela3d_plan_create_tuned it makes the same plan.  The SM count as for
+ * ela3d_builtin_tuning. */
+ela3d_status ela3d_open_tuning(int32_t nshots, const ela3d_params *params, ela3d_tuning *out);
 /* Host-only test hook: the dataflow work list (schedules 3 and 4) of one
  * nx*ny*nz shot for `nsteps` steps, tiles tile_x*tile_y, z-chunks of
  * `chunk` planes, `gap` places after each item's last dependency, steps
