@@ -150,16 +150,18 @@ static TuneChoice resolve_tuning(const std::vector<ela3d_params> &ps, const floa
   const bool explicit_variant = t && t->variant >= 0;
   if (!explicit_variant) {
     TuneChoice cached{};
-    if (tune_lookup(ps, &cached)) {
-      c = cached;
-    } else {
+    bool hit = tune_lookup(ps, &cached);
+    if (!hit) {
       const char *env = std::getenv("ELA3D_AUTOTUNE");
       if (env && env[0] == '1' && cp && cs && rho) {
         std::vector<const float *> a(cp, cp + ps.size()), b(cs, cs + ps.size()), r(rho, rho + ps.size());
         TuneChoice tuned{};
-        if (autotune(ps, a, b, r, 10, &tuned, nullptr, nullptr) == ELA3D_OK) c = tuned;
+        hit = autotune(ps, a, b, r, 10, &tuned, nullptr, nullptr) == ELA3D_OK && tune_lookup(ps, &cached);
       }
     }
+    // (a batch's open choice, chunk 0, has nothing to fill in beside fields
+    // that the caller set)
+    if (hit && (open || cached.chunk > 0)) c = cached;
   }
   if (!t) return c;
   if (t->variant >= 0) c.variant = t->variant;

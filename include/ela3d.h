@@ -300,7 +300,9 @@ typedef struct ela3d_tuning {
 /* Times every compiled variant with the candidate schedules on these shots
  * (`steps` time steps each, after a warm-up) and returns the fastest choice;
  * it is also cached for the workload's shape, so later plans and batches of
- * that shape use it.  ELA3D_TUNE_CACHE=<file> keeps the cache across
+ * that shape use it.  For several shots the candidates are the two kernels'
+ * schedules, and where the open choice (ela3d_open_tuning) is faster than the
+ * best of them, that one is cached instead.  ELA3D_TUNE_CACHE=<file> keeps the cache across
  * processes; ELA3D_AUTOTUNE=1 makes plan and batch creation tune on a cache
  * miss.  candidates (may be NULL) receives the number of choices timed.
  * No reference counterpart. */
