@@ -1266,7 +1266,7 @@ class Engine final : public EngineBase {
         // (the dataflow kernel passes over finished shots itself: a launch
         // ends at a shot's last step only for an explosive source's sake,
         // whose last injection comes after the launch)
-        if (flow_on() && flow_steps_ > 0 && !any_explosive_)
+        if (nblocks_ > 0 && flow_on() && !any_explosive_)
           seg = std::min({seg, steps_to_last(), std::max(1, flow_steps_ * flow_walks_)});
         else
           seg = std::min(seg, steps_to_boundary());
@@ -1415,7 +1415,7 @@ class Engine final : public EngineBase {
       ela3d_status st = upload_tables();
       if (st != ELA3D_OK) return st;
     }
-    if (!sched_key_.empty() && key == sched_key_ && sched_valid_) return ELA3D_OK;
+    if (sched_valid_ && key == sched_key_) return ELA3D_OK;
     sched_valid_ = false;
     nblocks_ = nitems_ = flow_items_ = flow_steps_ = 0;
     steps_on_schedule_ = 0;

@@ -1,6 +1,9 @@
 """The work lists of a running batch, which are built again whenever a shot
 ends: a list whose allocation fails launches nothing, and the batch goes on from
-there once there is memory again."""
+there once there is memory again; time that passes with no shot left costs
+nothing."""
+import time
+
 import numpy as np
 import pytest
 
@@ -44,3 +47,19 @@ def test_failed_list_launches_nothing_and_the_batch_goes_on(built, schedule, pre
         assert np.abs(w[0]).max() > 0
         for x, y in zip(g, w):
             assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("schedule", [-1, 1], ids=["open", "two kernels"])
+def test_time_passes_at_once_after_the_last_shot(built, schedule):
+    from ela3d_gb300 import Batch
+
+    shots = _shots()
+    with Batch(shots, schedule=schedule) as b:
+        b.run(31)
+        done = [b.seismograms(q) for q in range(3)]
+        t = time.perf_counter()
+        b.run(1_000_000_000)
+        assert time.perf_counter() - t < 5.0
+        assert all(b.info(q).step == 1_000_000_031 for q in range(3))
+        assert all(np.array_equal(b.seismograms(q), done[q]) for q in range(3))
+        assert all(np.abs(d).max() > 0 for d in done)
