@@ -161,8 +161,9 @@ __global__ void explosive_kernel(const ShotDesc<T> *shots, int nshots, int tick,
 // spends as few FP64 operations as it can: the strain energy is one quotient
 // (ss D - lambda tr^2) / (4 mu D) with D = 3 lambda + 2 mu, the quotients of
 // four cells are brought to one denominator, and the twelve values of a cell
-// are widened with integer operations (widen_normal).  The denominators' product stays
-// in range for moduli between 1e-38 and 1e38.  FP64 plans, whose values may be
+// are widened with integer operations (widen_normal).  Where a product of two
+// denominators leaves 2^-332 .. 2^332 (moduli below about 1e-25 or above 1e25)
+// or the quotient is not finite, each cell is divided by itself.  FP64 plans, whose values may be
 // larger, keep one division per term.  FP32, ms a call before and now: 101^3
 // 0.23 and 0.12, 201^3 1.57 and 0.59, 256^3 2.54 and 1.10, 400^3 9.2 and 4.1.
 __device__ __forceinline__ double block_sum_f64(double v) {
@@ -187,6 +188,15 @@ __device__ __forceinline__ double widen_normal(float f) {
 __device__ __forceinline__ bool subnormal_or_special(float f) {   // also infinities and NaN
   const unsigned b = __float_as_uint(f) << 1;
   return b != 0 && (b < 0x01000000u || b >= 0xff000000u);
+}
+
+// |d| within 2^-332 .. 2^333, and a value that is neither infinite nor NaN, by
+// their exponents.
+__device__ __forceinline__ bool mid_range(double d) {
+  return (((unsigned)__double2hiint(d) >> 20) & 0x7ffu) - (1023u - 332u) <= 664u;
+}
+__device__ __forceinline__ bool finite_bits(double d) {
+  return ((unsigned)__double2hiint(d) & 0x7ff00000u) != 0x7ff00000u;
 }
 
 // Twice the kinetic energy density of one cell, and its strain energy density
@@ -245,7 +255,10 @@ __global__ void __launch_bounds__(kEnergyThreads)
     }
     const double n01 = n[0] * d[1] + n[1] * d[0], d01 = d[0] * d[1];
     const double n23 = n[2] * d[3] + n[3] * d[2], d23 = d[2] * d[3];
-    strain += (n01 * d23 + n23 * d01) / (d01 * d23);
+    double s = (n01 * d23 + n23 * d01) / (d01 * d23);
+    if (!mid_range(d01) || !mid_range(d23) || !finite_bits(s))
+      s = (n[0] / d[0] + n[1] / d[1]) + (n[2] / d[2] + n[3] / d[3]);
+    strain += s;
   }
   const double acc = block_sum_f64(0.5 * kin + 0.25 * strain);
   if (threadIdx.x == 0) part[(long long)blockIdx.y * gridDim.x + blockIdx.x] = acc;
