@@ -266,13 +266,14 @@ __device__ __forceinline__ float dt_over_rho(float dt, float R) { return __fdivi
 // each SM) bounds the FP64 kernels.  R is a sum of two float32 model values.
 // Its reciprocal is found in pairs of float32 numbers on the FP32 unit (R = rh
 // + rl; y = yf + yl from the hardware reciprocal yf of rh and one cubic Newton
-// step, e = 1 - R yf, yl = yf (e + e^2); relative error about 2^-44), and the
+// step, e = 1 - R yf, yl = yf (e + e^2); relative error below 2^-45), and the
 // quotient takes one Markstein correction (P. Markstein, "Computation of
 // elementary functions on the IBM RISC System/6000 processor", 1990): q + (2
-// dt - q R) y is off by 2^-88 before its rounding, while a quotient by a
-// 26-bit R stays 2^-80 away from the midpoints between doubles, so it rounds
-// to the IEEE quotient (2e8 random quotients agree).  Floats are widened by
-// integer operations.  Sums outside [2^-60, 2^60) divide as usual.
+// dt - q R) y, whose remainder is exact for an R of 33 bits, is off by 2^-90
+// before its rounding, while a quotient by such an R stays 2^-87 away from the
+// midpoints between doubles, so it rounds to the IEEE quotient.  Floats are
+// widened by integer operations.  Sums of more bits (densities about 512 times
+// apart or more) and sums outside [2^-60, 2^60) divide as usual.
 __device__ __forceinline__ double widen_signed(float f) {   // (0 becomes 2^-127)
   const unsigned b = __float_as_uint(f);
   return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(b << 29));
@@ -280,8 +281,8 @@ __device__ __forceinline__ double widen_signed(float f) {   // (0 becomes 2^-127
 __device__ __forceinline__ double dt_over_rho(double dt, double R) {
   const double a = 2.0 * dt;
   const int hi = __double2hiint(R);
-  if ((unsigned)(hi - 0x3c300000) >= 0x07800000u) return a / R;
   const unsigned lo = (unsigned)__double2loint(R);
+  if ((unsigned)(hi - 0x3c300000) >= 0x07800000u || (lo & 0xfffffu) != 0) return a / R;
   const unsigned hb = ((unsigned)(hi - 0x38000000) << 3) | (lo >> 29);   // rh: the first 24 bits
   const float rh = __uint_as_float(hb);
   const float rl = (float)(lo & 0x1fffffffu) * __uint_as_float((hb & 0x7f800000u) - (52u << 23));
