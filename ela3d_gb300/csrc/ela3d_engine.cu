@@ -469,6 +469,10 @@ static int device_sms() {
   return sms;
 }
 
+// Bytes of the twelve arrays of a grid (nx cells or, padding included, px
+// elements a row).
+static double array_bytes(int nx, int ny, int nz, size_t word) { return 12.0 * word * nx * ny * nz; }
+
 // The tile: the share of its threads that hold cells, times a weight for its
 // shape.  Narrow tiles read more halo, which costs little while the arrays are
 // near the L2 (126 MB) and more once they stream from HBM.  Single shots,
@@ -540,7 +544,7 @@ TuneChoice plan_choice(const ela3d_params &p) {
   if (!v[c.variant].flow) return c;
   c.kind = kScheduleFlowOverlap;
   c.lag = 0;
-  const double bytes = 12.0 * p.nx * p.ny * p.nz * 4.0;
+  const double bytes = array_bytes(p.nx, p.ny, p.nz, sizeof(float));
   const bool streams = !fp64 && bytes > 400e6;
   c.variant = pick_tile({p}, fp64, streams, c.variant);
   const int tx = v[c.variant].tx, ty = v[c.variant].ty;
@@ -1450,10 +1454,10 @@ class Engine final : public EngineBase {
     return ELA3D_OK;
   }
 
-  // The dataflow list of the active shots for up to kFlowSteps steps (fewer
-  // when the list would pass kFlowMaxItems items; a launch walks it up to
-  // flow_passes_ times), their completion counters, and the descriptors that
-  // point at them.
+  // The dataflow list of the active shots, their completion counters, and the
+  // descriptors that point at them.  The list holds up to kFlowSteps steps (ten
+  // for a shot near the L2 size or in FP64, fewer when it would pass kFlowMaxItems
+  // items, for several shots kFlowBatchItems); a launch walks it flow_walks_ times.
   ela3d_status rebuild_flow(const std::vector<int> &active) {
     std::vector<FlowShape> shapes;
     long long per_step = 0, tiles = 0;
@@ -1469,18 +1473,21 @@ class Engine final : public EngineBase {
       per_step += 2 * tiles_of(d) * ((d.nz + c - 1) / c);
     }
     // The list's steps: building it costs the host about 16 us per 1000 items.
-    // A plan that streams from HBM gets all of flow_max_steps_ (512^3: 50 steps
-    // 51.0 Gcell-updates/s, 16 50.0); near the L2 size, and in FP64, ten do as
-    // well (101^3 35.4 and 35.3, 128^3 43.1 and 43.1).  Shots that run together change more
+    // A plan whose arrays, padding included, are far beyond the L2 gets all of
+    // flow_max_steps_ (512^3: 50 steps 51.0 Gcell-updates/s, 16 50.0; 201^3, 434
+    // MB, 197.3 us a step, with ten 199.1); near the L2 size, and in FP64, ten do
+    // as well (101^3 35.4 and 35.3 Gcell-updates/s, 128^3 43.1 and 43.1).  (The
+    // line is not plan_choice's for streaming, which counts no padding and
+    // decides the tile and the prefetch: 201^3 lies between them.)  Shots that run together change more
     // often than a plan's, and their longer steps hide the seam between two
     // walks of a short list.
     double bytes = 0.0;
-    for (int q : active) bytes += 12.0 * sizeof(T) * shots_[q]->d.px * shots_[q]->d.ny * shots_[q]->d.nz;
-    const bool together = active.size() > 1, streams = sizeof(T) == 4 && bytes > 400e6;
+    for (int q : active) bytes += array_bytes(shots_[q]->d.px, shots_[q]->d.ny, shots_[q]->d.nz, sizeof(T));
+    const bool together = active.size() > 1, far = sizeof(T) == 4 && bytes > 400e6;
     const long long most = together ? kFlowBatchItems : kFlowMaxItems;
-    const int steps = together || streams ? flow_max_steps_ : std::min(flow_max_steps_, 10);
+    const int steps = together || far ? flow_max_steps_ : std::min(flow_max_steps_, 10);
     const int K = (int)std::max<long long>(1, std::min<long long>(steps, most / std::max(1ll, per_step)));
-    flow_walks_ = std::max(flow_passes_, (together || !streams) ? (kFlowSteps * kFlowPasses + K - 1) / K : 0);
+    flow_walks_ = std::max(flow_passes_, (together || !far) ? (kFlowSteps * kFlowPasses + K - 1) / K : 0);
     std::vector<FlowItem> items;
     std::vector<int> off, nch;
     int nflags = 0;
@@ -1512,7 +1519,7 @@ class Engine final : public EngineBase {
     flow_items_ = (int)items.size();
     flow_steps_ = K;
     nblocks_ = 1;   // (something is active)
-    // Arrays that about fit the L2 (126 MB): the fields stay there if the model and
+    // Arrays that, padding included, about fit the L2 (126 MB): the fields stay there if the model and
     // the memory variables make room.  Gcell-updates/s without / with, 10 and 20
     // layer cells: 64^3 (13 MB) 20.5 / 20.9, 101^3 (63) 39.2 / 41.4 and 33.4 /
     // 37.0, 112^3 43.0 / 47.6 and 36.9 / 43.6, 128^3 (101) 48.1 / 50.8 and 41.0 /
@@ -1998,7 +2005,7 @@ class Engine final : public EngineBase {
   int2 *d_ranges_ = nullptr;
   unsigned *d_err_ = nullptr;
   double *d_energy_ = nullptr;
-  int energy_cap_ = 0;   // doubles held by d_energy_
+  int energy_cap_ = 0;   // planes d_energy_ has room for, plus one
   int nblocks_ = 0, nitems_ = 0, per_sm_ = 1;
   size_t items_cap_ = 0, ranges_cap_ = 0;
   std::vector<int> sched_key_;
@@ -2008,7 +2015,7 @@ class Engine final : public EngineBase {
   int tick_ = 0;
   int inject_ = 0;   // steps left whose launches withhold their loads (test hook)
   int fail_lists_ = 0;   // work lists whose allocation is still to fail (test hook)
-  int prefetch_ = kPrefetchDefault;  // memory-variable prefetch hints (x slab to L1, y/z slabs to L2)
+  int prefetch_ = kPrefetchDefault;  // memory-variable prefetch hints (CTL_PF_*), into L2
   int prefetch_env_ = -1;
   size_t guard_ = 0;   // bytes of each debug guard zone (0 = off)
   int steps_on_schedule_ = 0;  // steps run with the current work items
@@ -2027,10 +2034,10 @@ class Engine final : public EngineBase {
   std::vector<cudaEvent_t> free_events_;
   double t_stress_ = 0.0, t_vel_ = 0.0;
   int64_t n_stress_ = 0, n_vel_ = 0;
-  // dataflow path (schedule kind 3)
+  // dataflow path (schedule kinds 3 and 4)
   static constexpr int kFlowSteps = 50;
-  // passes over the list per dataflow launch: a launch runs up to
-  // kFlowSteps * kFlowPasses steps, the list is built for kFlowSteps
+  // passes over a list of kFlowSteps steps per dataflow launch (shorter lists
+  // are walked more often): a launch runs up to kFlowSteps * kFlowPasses steps
   // (measured: 200-step launches 1% faster than 50-step ones at 101^3 and
   // 256^3; a 200-step list would take 25-40 ms to build on the host)
   static constexpr int kFlowPasses = 4;

@@ -56,6 +56,14 @@ def test_named_sizes(built):
     assert pick(configs.anticline_256(n=128, precision=E.FP64)[0]) == ((16, 16), 4, 26, 0)
 
 
+def test_prefetch_from_the_size_that_streams(built):
+    """The line is 400 MB of arrays without the rows' padding: 201x201x206 lies
+    below (399.5 MB; 445 with padding), one plane more above."""
+    import ela3d_gb300 as E
+
+    assert [E.open_tuning(_params((201, 201, nz))).prefetch for nz in (201, 206, 207)] == [0, 0, 6]
+
+
 def test_batch_choice_up_to_the_most_shots_a_list_holds(built):
     """65535 shots share one dataflow list; more run on the two kernels."""
     import ela3d_gb300 as E
