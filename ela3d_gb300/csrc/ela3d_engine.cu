@@ -727,6 +727,8 @@ class Engine final : public EngineBase {
     if (const char *e = std::getenv("ELA3D_FLOW_PASSES")) flow_passes_ = std::max(1, std::atoi(e));
     // ELA3D_PSI_PREFETCH=<bits> overrides the tuned prefetch mode (experiments)
     if (const char *e = std::getenv("ELA3D_PSI_PREFETCH")) prefetch_env_ = std::atoi(e) & (CTL_PF_X | CTL_PF_YZ);
+    // ELA3D_COEF_BYTES=<bytes> replaces kCoefBytes (0: FP64 without coefficient arrays)
+    if (const char *e = std::getenv("ELA3D_COEF_BYTES")) coef_budget_ = std::max(0ll, std::atoll(e));
     // ELA3D_GUARD_ZONES=<bytes> (debug): guard zones around every pool array
     if (const char *e = std::getenv("ELA3D_GUARD_ZONES")) {
       const long long b = std::atoll(e);
@@ -1159,7 +1161,7 @@ class Engine final : public EngineBase {
       size_t fr = 0, tot = 0;
       CK(cudaMemGetInfo(&fr, &tot));
       if (bytes > fr / 4) return ELA3D_OK;
-      if ((coef_bytes_held() += (long long)bytes) > kCoefBytes) {
+      if ((coef_bytes_held() += (long long)bytes) > coef_budget_) {
         coef_bytes_held() -= (long long)bytes;
         return ELA3D_OK;
       }
@@ -2050,6 +2052,7 @@ class Engine final : public EngineBase {
   bool flow_once_ = false;         // the list runs var_->flow_once
   bool flow_coef_ = false;         // every shot of the list has its coefficients
   static constexpr long long kCoefBytes = 8ll << 30;
+  long long coef_budget_ = kCoefBytes;
   FlowItem *d_flow_ = nullptr;
   int *d_flags_ = nullptr;
   size_t flow_cap_ = 0, flags_cap_ = 0, flags_used_ = 0;

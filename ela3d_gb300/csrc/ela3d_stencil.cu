@@ -38,7 +38,7 @@ static Variant make_variant() {
     // FP32 tiles of seven or eight warps: also with the L2 hints
     if constexpr (sizeof(T) == 4 && G::NCW >= 7)
       v.flow_once = reinterpret_cast<const void *>(&flow_kernel<T, TX, TY, NS, CPT, MB, false, true>);
-    // FP64 with one cell per thread: also with coefficients from arrays
+    // FP64 with one cell per thread and one block per SM: also with coefficients from arrays
     if constexpr (sizeof(T) == 8 && CPT == 1 && MB == 0) {
       v.flow_coef = reinterpret_cast<const void *>(&flow_kernel<T, TX, TY, NS, CPT, MB, true, false>);
       v.flow_coef_smem = Flow<Geo<T, TX, TY, NS, CPT, MB, true>, T, NS>::SMEM;
