@@ -75,7 +75,9 @@ static const Variant kVariants[] = {
     // FP32 tiles of eight consumer warps (their launch splits its registers
     // unevenly): grids are often multiples of 8 or 16 rows, and near the L2
     // size the warps are what limits the kernel (128^3 43.6 -> 46.2
-    // Gcell-updates/s, 192^3 46.6 -> 47.7)
+    // Gcell-updates/s, 192^3 46.6 -> 47.7).  At 168 registers a thread seven of
+    // their dataflow instances spill 24 bytes (112x9 and 56x18, and all five
+    // with the L2 hints)
     make_variant<float, 128, 8, 4>(),
     make_variant<float, 64, 16, 4>(),
     make_variant<float, 32, 32, 4>(),

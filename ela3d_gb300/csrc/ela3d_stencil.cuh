@@ -389,9 +389,13 @@ __device__ __forceinline__ void prefetch_l2(const void *p, int bytes) {
 // consumers of a tile will copy into their slots (PsiSlots, which reach one
 // plane ahead and read through L2): issued by the producer warp's lanes (one
 // (variable, row) pair per lane) when a plane's stage is requested, NS-2
-// planes ahead of the consumers.  A hint: no result depends on it.  The x
-// slab's row ends are short and unaligned (CTL_PF_X, line by line); the rows
-// of the y and z slabs are whole (CTL_PF_YZ, bulk prefetches).
+// planes ahead of the consumers.  A hint: no result depends on it.  A lane has
+// one pair, so of a tile with more than 32 of them (three variables of more
+// than ten rows) only the first 32 are prefetched: all of the 7- to 9-row
+// tiles' pairs, 32 of 64x16's 48, of 32x32's 96 one variable's (pick_tile's
+// weights for grids that stream were measured so).  The x slab's row ends are
+// short and unaligned (CTL_PF_X, line by line); the rows of the y and z slabs
+// are whole (CTL_PF_YZ, bulk prefetches).
 __device__ __forceinline__ void prefetch_l2_bulk(const void *p, int bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }

@@ -347,14 +347,15 @@ ela3d_status ela3d_model_generate(const ela3d_model_spec *model, int32_t nx, int
                                   float *cp, float *cs, float *rho);
 
 /* ---- batches of shots ---------------------------------------------------- */
-/* Many shots resident together and advanced by the same two launches per
- * time step (the persistent kernels deal (shot, tile, z-run) items to all
- * SMs).  Shots may differ in size, model, source, receivers, dt and nstep
+/* Many shots resident together and advanced by the same launches: with an open
+ * tuning the dataflow kernel, up to 200 steps a launch, else as the tuning says
+ * (two kernels per time step whose blocks take (shot, tile, z-run) items, or
+ * the dataflow kernel).  Shots may differ in size, model, source, receivers, dt and nstep
  * (same precision).  Shots whose cp, cs and rho pointers and grid equal an
  * earlier shot's share that shot's device model.  A shot stops being
  * computed once it has done its nstep steps; its results stay readable.
- * Runs of 50 or more steps replay a captured CUDA graph.  The reference runs
- * one shot per process (no counterpart). */
+ * On the two kernels runs of 50 or more steps replay a captured CUDA graph.  The
+ * reference runs one shot per process (no counterpart). */
 typedef struct ela3d_batch ela3d_batch;
 ela3d_status ela3d_batch_create(int32_t nshots, const ela3d_params *params, const float *const *cp,
                                 const float *const *cs, const float *const *rho, const ela3d_tuning *tune,
